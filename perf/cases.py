@@ -59,27 +59,27 @@ def _case(name, kind, requests, tokens, history=0, size="0.9b", dtype="bf16", **
 def listed():
     return [
         # a server with eight live chats, each some 4000 tokens long: one token for each of them
-        _case("decode step, 8 chats", "decode_step", 8, 8, CONTEXT - 8),
+        _case("decode step 8 chats", "decode_step", 8, 8, CONTEXT - 8),
         # a document of 2048 tokens arrives: a step at the engine's token budget
         _case("prompt of 2048", "prompt", 1, 2048),
         # the same for its layers: two prompts that share a step
-        _case("attention, 2 prompts", "gqa_attention", 2, 2048),
-        _case("feed-forward, 2048 rows", "swiglu", 1, 2048),
+        _case("attention 2 prompts", "gqa_attention", 2, 2048),
+        _case("feed-forward 2048 rows", "swiglu", 1, 2048),
         # a prompt through the windowed attention with a distance bias, in a step of its own
-        _case("windowed attention, prompt", "window_attention", 1, 2048),
+        _case("windowed attention prompt", "window_attention", 1, 2048),
         # the second half of a long document: compressed keys and values of the first half are in the cache
-        _case("latent attention, prompt", "latent_attention", 1, 1024, 1024),
+        _case("latent attention prompt", "latent_attention", 1, 1024, 1024),
         # eight chats through differential attention
-        _case("diff attention, 8 chats", "diff_attention", 8, 8, CONTEXT - 8),
+        _case("diff attention 8 chats", "diff_attention", 8, 8, CONTEXT - 8),
         # a prompt through the delta rule
-        _case("delta rule, prompt", "recurrence", 1, 2048, rule="channel_delta"),
+        _case("delta rule prompt", "recurrence", 1, 2048, rule="channel_delta"),
         # four prompts that share a step, in a larger model with gated linear attention
-        _case("gated recurrence, 4 prompts", "recurrence", 4, 2048, size="3b", rule="gated"),
+        _case("gated recurrence 4 prompts", "recurrence", 4, 2048, size="3b", rule="gated"),
         # an odd pair of short prompts in the 32-bit mode that checks and small experiments use
-        _case("decay recurrence, 32-bit", "recurrence", 2, 777, dtype="f32", rule="decay"),
+        _case("decay recurrence 32-bit", "recurrence", 2, 777, dtype="f32", rule="decay"),
         # routed experts behind a full prompt step and behind a decode step
-        _case("experts, 2048 rows", "experts", 1, 2048),
-        _case("experts, 8 rows", "experts", 8, 8),
+        _case("experts 2048 rows", "experts", 1, 2048),
+        _case("experts 8 rows", "experts", 8, 8),
     ]
 
 
