@@ -1,0 +1,194 @@
+"""The chunked form of the matrix-state recurrences (csrc/chunked_recurrence.cu) against the recurrence walked in float64,
+beside the kernels that walk it token by token: every kind of decay, both widths, portions around the edges of a chunk (64
+tokens) and of its sub-chunks (16), several requests of unequal length with a state of their own, strided rows, decays that
+underflow, and non-finite tokens, which no earlier token may see."""
+import math
+
+import pytest
+import torch
+
+F64 = torch.float64
+
+
+def _walk(q, k, v, g, S, beta=None, bonus=None):
+    """o_t = S_t^T q_t over the tokens in float64; ``beta``: the delta rule; ``bonus``: outputs read the state before."""
+    out = []
+    for t in range(len(q)):
+        if bonus is not None:
+            out.append(torch.einsum("hdv,hd->hv", S, q[t]) + (bonus * q[t] * k[t]).sum(-1, keepdim=True) * v[t])
+        S = g[t][..., None] * S
+        u = v[t] if beta is None else beta[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t]))
+        S = S + k[t][..., None] * u[:, None]
+        if bonus is None:
+            out.append(torch.einsum("hdv,hd->hv", S, q[t]))
+    return torch.stack(out), S
+
+
+def _norm(o, w, eps):
+    return o / torch.sqrt((o * o).mean(-1, keepdim=True) + eps) * w
+
+
+class Case:
+    """Inputs of a step in ``dtype`` and its oracle; ``call(ops, segments)`` runs one of the entry points."""
+
+    def __init__(self, rule, K, V, lengths, dtype, seed=0, H=4, strong=0.0):
+        self.rule, self.K, self.V, self.lengths, self.dtype, self.H = rule, K, V, list(lengths), dtype, H
+        gen = torch.Generator().manual_seed(seed)
+        n = sum(lengths)
+        r = lambda *s: torch.randn(*s, generator=gen)  # noqa: E731
+        self.G = G = 2 if rule in ("channel", "head", "step") else H
+        self.n, self.eps = n, 1e-6
+        cols = (G if rule == "forget" else 2 * G) * K + H * V + (H * V if rule == "bonus" else 0)
+        self.rows = r(n, cols + 16).to(dtype)[:, :cols]                          # a view with a longer row
+        self.a = (r(n, H if rule in ("head", "step") else H * K) + strong).to(dtype)
+        self.b, self.gate = r(n, H).to(dtype), r(n, H * V).to(dtype)
+        self.a_log = {"constant": 1 - 2.0 ** -(2 + torch.arange(H).float()), "gated": torch.full((H,), 0.125),
+                      "forget": torch.rand(H * K, generator=gen) * 0.9, "bonus": r(H * K)}.get(rule, r(H) * 0.3)
+        self.bias = torch.rand(H if rule in ("head", "step") else H * K, generator=gen) * 3 - 2
+        self.norm_w = 1 + 0.1 * r(H * V if rule in ("constant", "bonus") else V)
+        slots = len(lengths)
+        self.state = r(slots + 1, H * K * V + 8)[:, :H * K * V] * 0.1            # a free stride between the slots
+        order = list(range(slots))[::-1]                                         # requests in slots of another order
+        self.slot = torch.cat([torch.full((m,), order[i], dtype=torch.int32) for i, m in enumerate(lengths)])
+        ends = torch.tensor(lengths).cumsum(0)
+        self.last = torch.cat([torch.full((m,), int(e) - 1, dtype=torch.int32) for m, e in zip(lengths, ends)])
+        self.first = [int(e) - m for m, e in zip(lengths, ends)]
+        self.order = order
+
+    def oracle(self):
+        H, G, K, V, rule = self.H, self.G, self.K, self.V, self.rule
+        d = self.rows.to(F64)
+        a, bias, a_log, gate = self.a.to(F64), self.bias.to(F64), self.a_log.to(F64), self.gate.to(F64)
+        silu, plus = torch.nn.functional.silu, torch.nn.functional.softplus
+        out, states = torch.zeros(self.n, H * V, dtype=F64), self.state.to(F64).clone()
+        for r0, m, s in zip(self.first, self.lengths, self.order):
+            x, ar = d[r0:r0 + m], a[r0:r0 + m]
+            S, beta, bonus = states[s].view(H, K, V), None, None
+            vec = lambda at, w, heads: x[:, at:at + heads * w].reshape(m, heads, w)  # noqa: E731
+            q = vec(0, K, G)
+            if rule == "forget":
+                v = vec(G * K, V, H)
+                low = a_log.view(H, K)
+                g = low + (1 - low) * torch.sigmoid(ar.view(m, H, K) + bias.view(H, K))
+                q, k = silu(q), 1 - g
+            else:
+                k, v = vec(G * K, K, G), vec(2 * G * K, V, H)
+                if rule in ("channel", "head"):
+                    q, k = (t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6) for t in (q, k))
+                    q, beta = q * K ** -0.5, torch.sigmoid(self.b[r0:r0 + m].to(F64))
+                    z = (ar + bias).view(m, H, -1)
+                    g = torch.exp(-torch.exp(a_log)[:, None] * plus(z)).expand(m, H, K)
+                elif rule == "constant":
+                    q, k, v, g = silu(q), silu(k), silu(v), a_log[:, None].expand(m, H, K)
+                elif rule == "gated":
+                    q, g = q * K ** -0.5, torch.exp(-plus(-(ar + bias)).view(m, H, K) * a_log[:, None])
+                elif rule == "step":
+                    dt = plus(ar + bias)
+                    g, v = torch.exp(-torch.exp(a_log) * dt)[..., None].expand(m, H, K), v * dt[..., None]
+                else:
+                    g, bonus = torch.exp(-torch.exp((ar + bias).view(m, H, K))), a_log.view(H, K)
+            q, k = (t.repeat_interleave(H // t.shape[1], 1) for t in (q, k))
+            o, S = _walk(q, k, v, g, S, beta, bonus)
+            states[s] = S.reshape(-1)
+            gr = gate[r0:r0 + m]
+            if rule == "constant":
+                y = _norm(o.flatten(1), self.norm_w.to(F64), self.eps) * torch.sigmoid(gr)
+            elif rule == "step":
+                y = o.flatten(1)
+            elif rule == "bonus":
+                y = _norm(o, self.norm_w.to(F64).view(H, V), self.eps).flatten(1) * silu(x[:, -H * V:])
+            else:
+                y = _norm(o, self.norm_w.to(F64), self.eps).flatten(1)
+                y = y if rule == "forget" else y * (silu(gr) if rule == "gated" else torch.sigmoid(gr))
+            out[r0:r0 + m] = y
+        return out, states
+
+    def call(self, ops, segments):
+        c = lambda t: t.cuda()  # noqa: E731
+        wide = torch.empty(self.n, self.rows.shape[1] + 16, dtype=self.dtype, device="cuda")
+        rows = wide[:, :self.rows.shape[1]]
+        rows.copy_(self.rows)
+        held = torch.empty(self.state.shape[0], self.state.shape[1] + 8, device="cuda")
+        state = held[:, :self.state.shape[1]]
+        state.copy_(self.state)
+        out = torch.zeros(self.n, self.H * self.V, dtype=self.dtype, device="cuda")
+        tail = dict(requests=len(self.lengths), segments=segments)
+        at = (c(self.slot), c(self.last), self.H)
+        if self.rule in ("channel", "head"):
+            ops.delta_rule(rows, c(self.b), c(self.a), c(self.gate), c(self.a_log), c(self.bias), c(self.norm_w), self.eps, 1e-6,
+                           self.K ** -0.5, state, out, *at, self.G, self.K, self.V, decay_per_head=self.rule == "head", **tail)
+        elif self.rule == "constant":
+            ops.linear_attention(rows, c(self.gate), c(self.a_log), c(self.norm_w), self.eps, state, out, *at, self.K, self.V, **tail)
+        elif self.rule == "forget":
+            ops.forget_gate_recurrence(rows, c(self.a), c(self.a_log), c(self.bias), c(self.norm_w), self.eps, state, out, *at,
+                                       self.K, self.V, **tail)
+        elif self.rule == "gated":
+            ops.gated_linear_attention(rows, c(self.a), c(self.a_log), c(self.bias), c(self.gate), c(self.norm_w), self.eps,
+                                       self.K ** -0.5, state, out, *at, self.K, self.V, **tail)
+        elif self.rule == "step":
+            out = ops.state_space_scan(rows, c(self.a), c(self.a_log), c(self.bias), state, *at, self.G, self.K, self.V, **tail)
+        else:
+            ops.time_mix(rows, c(self.a), c(self.a_log), c(self.bias), c(self.norm_w), self.eps, state, out, *at, self.K, **tail)
+        return out.double().cpu(), state.double().cpu()
+
+    def segments(self, chunked):
+        return torch.tensor(self.first, dtype=torch.int32, device="cuda"), len(self.first), 10 ** 6 if chunked else 1
+
+
+def _off(got, want):
+    return float((got - want).norm() / want.norm())
+
+
+RULES = ["channel", "head", "constant", "forget", "gated", "step", "bonus"]
+
+
+def _compare(case):
+    from tiny_inference_server_b200.kernels import ops
+    want_o, want_s = case.oracle()
+    walked_o, walked_s = case.call(ops, case.segments(False))
+    before = ops.launches
+    got_o, got_s = case.call(ops, case.segments(True))
+    assert ops.launches - before >= 3                                       # the chunked form ran
+    # 32-bit sums of at most K + 64 products a chunk, errors of one chunk carried on by decays <= 1: a few times 2^-23
+    # relative to the whole; and never much worse than the walk, whose chain is as long as the portion
+    limit = 3e-6 if case.dtype == torch.float32 or case.rule == "step" else 4e-3
+    assert _off(got_o, want_o) < limit, (_off(got_o, want_o), _off(walked_o, want_o))
+    assert _off(got_s, want_s) < 3e-6, (_off(got_s, want_s), _off(walked_s, want_s))
+    assert _off(got_s, want_s) < 2 * _off(walked_s, want_s) + 3e-7
+    assert torch.equal(got_s[-1], case.state[-1].double())                  # nobody's slot
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", RULES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("K,V,lengths", [(128, 128, (130, 1, 63)), (64, 128, (65,)), (128, 64, (16, 64, 17)), (64, 64, (15, 129))])
+def test_chunks_against_the_walk(rule, dtype, K, V, lengths):
+    if rule == "bonus" and K != V:
+        V = K
+    _compare(Case(rule, K, V, lengths, dtype))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", ["channel", "head", "gated", "bonus", "step"])
+def test_decays_that_underflow(rule):
+    """Decays far below the smallest float beside ones near 1: products are zero, never a division by them."""
+    case = Case(rule, 64, 64, (100, 70), torch.float32, seed=3, strong=0.0)
+    case.a[::7] += -120.0 if rule == "gated" else 120.0
+    case.a[3::7] += 40.0 if rule == "gated" else -40.0
+    if rule == "gated":
+        case.a_log.fill_(1.0)
+    _compare(case)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", RULES)
+def test_a_token_that_is_not_finite_shows_in_no_earlier_one(rule):
+    from tiny_inference_server_b200.kernels import ops
+    case = Case(rule, 64, 64, (90, 40), torch.float32, seed=5)
+    clean, _ = case.call(ops, case.segments(True))
+    for bad, row in ((math.inf, 37), (math.nan, 70)):
+        broken = Case(rule, 64, 64, (90, 40), torch.float32, seed=5)
+        broken.rows[row] = bad
+        got, states = broken.call(ops, broken.segments(True))
+        assert torch.equal(got[:row], clean[:row]) and torch.equal(got[90:], clean[90:])
+        assert not torch.isfinite(states[broken.order[0]]).all()

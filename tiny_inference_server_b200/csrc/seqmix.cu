@@ -9,7 +9,7 @@
 //
 // Rows of a step: row r belongs to request slot row_slot[r] (negative: padding) at positions[r]; the rows of a
 // request are consecutive and in order, row_last[r] is the last row of r's request in this step.
-#include "common.cuh"
+#include "recurrence.cuh"
 
 // ------------------------------------------------------------------------------------------------------------
 // y[r, c] = (residual ? x[r, c] : 0) + bias[c] + sum_j w[j, c] * x(t - taps + 1 + j)[c], optionally through silu (the
@@ -784,29 +784,7 @@ TIS_API int tis_window_attention(int dtype, const void* q, int ldq, const void* 
 // ------------------------------------------------------------------------------------------------------------
 constexpr int DELTA_CHUNK = 16;
 
-__device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
-__device__ __forceinline__ float silu_f(float x) { return x / (1.f + expf(-x)); }
-// what a gate does to the projection it is made from: 0 sigmoid, 1 silu
-__device__ __forceinline__ float gate_f(float x, int act) { const float s = 1.f / (1.f + expf(-x)); return act == 1 ? x * s : s; }
-// where the decay of a token comes from: a projection per head and key channel, a projection per head, or a constant
-// per head (`A_log` then holds the constants themselves and the recurrence is plain linear attention: q, k and v pass
-// silu instead of the unit norms, and the state takes k v^T without the correction towards v)
-// or (DECAY_FORGET_GATE) a forget gate per head and key channel that also decides what is written: with `a_in` the
-// gate's projection, `dt_bias` its bias and `A_log` a lower bound per head and key channel, f = low + (1 - low) *
-// sigmoid(a + bias), S <- diag(f) S + (1 - f) v^T, o = S^T silu(q): the key is 1 - f, there is no key projection (a
-// row of `qkv` holds the queries and then the values), no unit norms and no correction towards v
-// or (DECAY_LOG_SIGMOID) a gate per head and key channel raised to a power: with `a_in` the gate's projection, `dt_bias`
-// its bias and `A_log` the power itself per head (1 / tau), g = sigmoid(a + bias)^power = exp(-power * softplus(-(a + bias))),
-// S <- diag(g) S + k v^T, o = S^T (q * q_scale): gated linear attention, no unit norms, no correction
-// or (DECAY_STEP) a step size per head and token: with `a_in` (n, H) its projection and `dt_bias` (H) its bias,
-// dt = softplus(a + bias), S <- exp(-exp(A_log[head]) * dt) S + k (dt v)^T, o = S^T q: a selective state space in its
-// recurrent form (k is the input matrix B, q the output matrix C, v the head's inputs); the outputs leave unnormalised
-// or (DECAY_BONUS) a decay per head and key channel with a bonus for the current token: with `a_in` the decay's projection,
-// `dt_bias` its bias and `A_log` the bonus u per head and key channel, g = exp(-exp(a + bias)), o = (S + diag(u) k v^T)^T q,
-// then S <- diag(g) S + k v^T: the outputs read the state before the token.  The bonus' share of o is (sum_i u_i q_i k_i) v,
-// one number a token (kept where the other forms keep beta).  The norm's weights are the head's own (H * v_dim of them)
-enum { DECAY_PER_CHANNEL = 0, DECAY_PER_HEAD = 1, DECAY_CONSTANT = 2, DECAY_FORGET_GATE = 3, DECAY_LOG_SIGMOID = 4,
-       DECAY_STEP = 5, DECAY_BONUS = 6 };
+// (softplus, the gates and the kinds of decay, with what each computes: recurrence.cuh)
 
 template <typename T, int DIM>
 __global__ void __launch_bounds__(DIM > 0 ? 256 : 1024)
@@ -1511,7 +1489,7 @@ static int matrix_state_recurrence(int dtype, const void* qkv, int ld, const voi
                                    float eps, float unit_eps, float q_scale, float* state, size_t state_stride, void* out,
                                    int ldo, float* o_raw, const int* row_slot, const int* row_last, int n, int H, int G,
                                    int k_dim, int v_dim, int narrow, const int* seg_row0, int segments, int decay_mode,
-                                   int gate_act, cudaStream_t stream) {
+                                   int gate_act, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
     if (n <= 0) return TIS_OK;
     if (decay_mode < DECAY_PER_CHANNEL || decay_mode > DECAY_BONUS || gate_act < 0 || gate_act > 1 ||
         ((decay_mode == DECAY_CONSTANT || decay_mode == DECAY_STEP) && o_raw == nullptr)) {
@@ -1522,6 +1500,21 @@ static int matrix_state_recurrence(int dtype, const void* qkv, int ld, const voi
     if (n > 65535) {
         tis_set_error("delta_rule: %d rows in one step (at most 65535)", n);
         return TIS_BAD_SIZE;
+    }
+    if (chunk_scratch != nullptr) {                     // long portions: in chunks of tokens (chunked_recurrence.cu)
+        ChunkArgs p = {};
+        p.qkv = qkv; p.ld = ld; p.b_in = b_in; p.ldb = ldb; p.a_in = a_in; p.lda = lda; p.gate = gate; p.ldg = ldg;
+        p.A_log = A_log; p.dt_bias = dt_bias; p.norm_w = norm_w; p.eps = eps; p.unit_eps = unit_eps; p.q_scale = q_scale;
+        p.state = state; p.state_stride = state_stride; p.out = out; p.ldo = ldo; p.o_raw = o_raw; p.row_slot = row_slot;
+        p.row_last = row_last; p.seg_row0 = seg_row0; p.segments = segments; p.n = n; p.H = H; p.G = G; p.mode = decay_mode;
+        p.gate_act = gate_act;
+        if (chunked_recurrence_takes(dtype, p, k_dim, v_dim)) {
+            const int st = chunked_recurrence(dtype, p, k_dim, v_dim, chunk_scratch, chunk_floats, stream);
+            if (st != TIS_OK || decay_mode != DECAY_CONSTANT) return st;
+            TIS_DISPATCH_DTYPE(dtype, T, tis_launch(row_out_norm_kernel<T>, dim3(n), dim3(256), 0, stream, (const float*)o_raw,
+                               (const T*)gate, ldg, norm_w, eps, (T*)out, ldo, row_slot, H * v_dim));
+            return tis_check_launch("row_out_norm");
+        }
     }
     // (the walk with a bonus reads its rows in 16-byte vectors)
     const bool rows_fit = decay_mode != DECAY_BONUS || (ld % 8 == 0 && lda % 8 == 0 && ((uintptr_t)qkv | (uintptr_t)a_in) % 16 == 0);
@@ -1583,6 +1576,9 @@ static int matrix_state_recurrence(int dtype, const void* qkv, int ld, const voi
     return TIS_OK;
 }
 
+// The entry points below: `chunk_scratch`, `chunk_floats` (tis_chunked_recurrence_floats of them; null: none): the step
+// holds long portions and may be walked in chunks of tokens.
+
 // The delta rule.  decay_per_head 0: `a_in` (n, H * k_dim) and `dt_bias` (H * k_dim), a decay per head and key channel;
 // 1: `a_in` (n, H) and `dt_bias` (H), one per head.  gate_act: 0 sigmoid, 1 silu.
 TIS_API int tis_delta_rule(int dtype, const void* qkv, int ld, const void* b_in, int ldb, const void* a_in, int lda,
@@ -1590,11 +1586,11 @@ TIS_API int tis_delta_rule(int dtype, const void* qkv, int ld, const void* b_in,
                            float eps, float unit_eps, float q_scale, float* state, size_t state_stride, void* out,
                            int ldo, float* o_raw, const int* row_slot, const int* row_last, int n, int H, int G,
                            int k_dim, int v_dim, int narrow, const int* seg_row0, int segments, int decay_per_head,
-                           int gate_act, cudaStream_t stream) {
+                           int gate_act, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
     return matrix_state_recurrence(dtype, qkv, ld, b_in, ldb, a_in, lda, gate, ldg, A_log, dt_bias, norm_w, eps, unit_eps,
                                    q_scale, state, state_stride, out, ldo, o_raw, row_slot, row_last, n, H, G, k_dim, v_dim,
                                    narrow, seg_row0, segments, decay_per_head ? DECAY_PER_HEAD : DECAY_PER_CHANNEL, gate_act,
-                                   stream);
+                                   chunk_scratch, chunk_floats, stream);
 }
 
 // Linear attention with a constant decay per head (`decay`, H numbers): S <- decay S + silu(k) silu(v)^T, o = S^T silu(q);
@@ -1603,10 +1599,10 @@ TIS_API int tis_delta_rule(int dtype, const void* qkv, int ld, const void* b_in,
 TIS_API int tis_linear_attention(int dtype, const void* qkv, int ld, const void* gate, int ldg, const float* decay,
                                  const float* norm_w, float eps, float* state, size_t state_stride, void* out, int ldo,
                                  float* o_raw, const int* row_slot, const int* row_last, int n, int H, int k_dim, int v_dim,
-                                 int narrow, const int* seg_row0, int segments, cudaStream_t stream) {
+                                 int narrow, const int* seg_row0, int segments, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
     return matrix_state_recurrence(dtype, qkv, ld, nullptr, 0, nullptr, 0, gate, ldg, decay, nullptr, norm_w, eps, 0.f, 1.f,
                                    state, state_stride, out, ldo, o_raw, row_slot, row_last, n, H, H, k_dim, v_dim, narrow,
-                                   seg_row0, segments, DECAY_CONSTANT, 0, stream);
+                                   seg_row0, segments, DECAY_CONSTANT, 0, chunk_scratch, chunk_floats, stream);
 }
 
 // The recurrence with a forget gate per head and key channel (DECAY_FORGET_GATE): a row of `qv` holds the queries of H
@@ -1617,10 +1613,10 @@ TIS_API int tis_forget_gate_recurrence(int dtype, const void* qv, int ld, const 
                                        const float* f_bias, const float* norm_w, float eps, float* state,
                                        size_t state_stride, void* out, int ldo, float* o_raw, const int* row_slot,
                                        const int* row_last, int n, int H, int k_dim, int v_dim, int narrow,
-                                       const int* seg_row0, int segments, cudaStream_t stream) {
+                                       const int* seg_row0, int segments, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
     return matrix_state_recurrence(dtype, qv, ld, nullptr, 0, f_in, ldf, nullptr, 0, lower, f_bias, norm_w, eps, 0.f, 1.f,
                                    state, state_stride, out, ldo, o_raw, row_slot, row_last, n, H, H, k_dim, v_dim, narrow,
-                                   seg_row0, segments, DECAY_FORGET_GATE, 0, stream);
+                                   seg_row0, segments, DECAY_FORGET_GATE, 0, chunk_scratch, chunk_floats, stream);
 }
 
 // Gated linear attention (DECAY_LOG_SIGMOID): a row of `qkv` holds the queries and keys of H heads (k_dim each) and the
@@ -1632,10 +1628,10 @@ TIS_API int tis_gated_linear_attention(int dtype, const void* qkv, int ld, const
                                        const float* a_bias, const void* gate, int ldg, const float* norm_w, float eps,
                                        float q_scale, float* state, size_t state_stride, void* out, int ldo, float* o_raw,
                                        const int* row_slot, const int* row_last, int n, int H, int k_dim, int v_dim,
-                                       int narrow, const int* seg_row0, int segments, int gate_act, cudaStream_t stream) {
+                                       int narrow, const int* seg_row0, int segments, int gate_act, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
     return matrix_state_recurrence(dtype, qkv, ld, nullptr, 0, a_in, lda, gate, ldg, power, a_bias, norm_w, eps, 0.f, q_scale,
                                    state, state_stride, out, ldo, o_raw, row_slot, row_last, n, H, H, k_dim, v_dim, narrow,
-                                   seg_row0, segments, DECAY_LOG_SIGMOID, gate_act, stream);
+                                   seg_row0, segments, DECAY_LOG_SIGMOID, gate_act, chunk_scratch, chunk_floats, stream);
 }
 
 // A selective state space in its recurrent form (DECAY_STEP): a row of `cbx` holds the output matrices C and then the input
@@ -1645,10 +1641,10 @@ TIS_API int tis_gated_linear_attention(int dtype, const void* qkv, int ld, const
 TIS_API int tis_state_space_scan(int dtype, const void* cbx, int ld, const void* dt_in, int ldd, const float* A_log,
                                  const float* dt_bias, float* state, size_t state_stride, float* o_raw, const int* row_slot,
                                  const int* row_last, int n, int H, int G, int state_dim, int v_dim, int narrow,
-                                 const int* seg_row0, int segments, cudaStream_t stream) {
+                                 const int* seg_row0, int segments, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
     return matrix_state_recurrence(dtype, cbx, ld, nullptr, 0, dt_in, ldd, nullptr, 0, A_log, dt_bias, nullptr, 0.f, 0.f, 1.f,
                                    state, state_stride, nullptr, 0, o_raw, row_slot, row_last, n, H, G, state_dim, v_dim,
-                                   narrow, seg_row0, segments, DECAY_STEP, 0, stream);
+                                   narrow, seg_row0, segments, DECAY_STEP, 0, chunk_scratch, chunk_floats, stream);
 }
 
 // The recurrence with a bonus for the current token (DECAY_BONUS): a row of `rkvg` holds r, k and v of H heads (dim each) and
@@ -1658,9 +1654,9 @@ TIS_API int tis_state_space_scan(int dtype, const void* cbx, int ld, const void*
 TIS_API int tis_time_mix(int dtype, const void* rkvg, int ld, const void* w_in, int ldw, const float* u, const float* w_bias,
                          const float* norm_w, float eps, float* state, size_t state_stride, void* out, int ldo, float* o_raw,
                          const int* row_slot, const int* row_last, int n, int H, int dim, int narrow, const int* seg_row0,
-                         int segments, cudaStream_t stream) {
+                         int segments, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
     const size_t gate_at = (size_t)3 * H * dim * (dtype == TIS_BF16 ? 2 : 4);
     return matrix_state_recurrence(dtype, rkvg, ld, nullptr, 0, w_in, ldw, (const char*)rkvg + gate_at, ld, u, w_bias, norm_w,
                                    eps, 0.f, 1.f, state, state_stride, out, ldo, o_raw, row_slot, row_last, n, H, H, dim, dim,
-                                   narrow, seg_row0, segments, DECAY_BONUS, 1, stream);
+                                   narrow, seg_row0, segments, DECAY_BONUS, 1, chunk_scratch, chunk_floats, stream);
 }

@@ -16,13 +16,14 @@ class SegmentPlanner(StepPlanner):
         return rows
 
     def plan(self, segments: Sequence[Tuple[int, int]]):
-        return {"row0": [first for first, _ in segments]}, len(segments)
+        return {"row0": [first for first, _ in segments]}, (len(segments), max((rows for _, rows in segments), default=0))
 
     def plan_decode(self, rows: int):
-        return {"row0": list(range(rows))}, rows
+        return {"row0": list(range(rows))}, (rows, 1)
 
     def bind(self, arrays: Dict[str, torch.Tensor], facts):
-        return arrays["row0"], int(facts)
+        """(first rows, number of requests, rows of the longest)"""
+        return arrays["row0"], int(facts[0]), int(facts[1])
 
 
 _planner = SegmentPlanner()
