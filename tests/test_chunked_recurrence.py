@@ -190,5 +190,6 @@ def test_a_token_that_is_not_finite_shows_in_no_earlier_one(rule):
         broken = Case(rule, 64, 64, (90, 40), torch.float32, seed=5)
         broken.rows[row] = bad
         got, states = broken.call(ops, broken.segments(True))
-        assert torch.equal(got[:row], clean[:row]) and torch.equal(got[90:], clean[90:])
+        # the block of 16 tokens around a broken one is summed another way: 32-bit sums of up to 128 products, not the same bits
+        assert _off(got[:row], clean[:row]) < 3e-6 and torch.equal(got[90:], clean[90:])
         assert not torch.isfinite(states[broken.order[0]]).all()

@@ -20,16 +20,19 @@
 // Every product of decays is a product of factors <= 1 in the direction the tokens run (within sub-chunks of 16 tokens,
 // over whole sub-chunks between them): nothing is divided by a decay, so a decay of zero and a long product that
 // underflows are what they are in the walk.  No token's output meets a later token's vectors, not even times zero.
-// Everything is 32-bit (CUDA cores: 3 x tf32 on mma.sync measured 266 / 3 TFLOP/s against 67 here, and would have to
-// split its operands first).
+// Operands, states and sums are 32-bit.  The dense products run on the tensor cores as three tf32 products of operands
+// split in two (x = hi + lo: lo hi + hi lo + hi hi; what is left out is 2^-22 of a product): the CUDA cores read a word
+// from shared memory for every one to four multiply-adds, and at a quarter of their rate that is what the first form of
+// these kernels spent its time on (delta rule, 2048 tokens, 12 heads of 128 x 128: 135 + 113 + 51 us; now 80 + 99 + 41).
+// Straight-line code is kept short: a kernel's code is read anew at every launch, and unrolled over a chunk's tokens the
+// exponentials of the preparation took longer to fetch than to run.  A product of a masked zero and a number that is not finite would not be zero: blocks on the diagonal look at their operands first.
 #include "recurrence.cuh"
 
 namespace {
 
 constexpr int C = REC_CHUNK, SUB = 16, NSUB = C / SUB;
-constexpr int DCOLS = 16;                       // columns of the state that a CTA of chunk_delta_kernel takes
 
-__device__ __forceinline__ void copy16(float* smem, const float* gmem) {
+__device__ __forceinline__ void copy16(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem));
 }
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::); }
@@ -70,6 +73,60 @@ template <int N> __device__ __forceinline__ void store_run(bf16* p, const float 
     if constexpr (N == 4) *reinterpret_cast<uint2*>(p) = *reinterpret_cast<uint2*>(h);
     else *reinterpret_cast<__nv_bfloat162*>(p) = h[0];
 }
+
+// ---- products of 16 x 8 (x 8) tiles in three tf32 products; lane = 4 r + c holds rows r, r + 8 and columns c, c + 4 of A
+// (16 x 8), rows c, c + 4 of column r of B (8 x 8), columns 2 c, 2 c + 1 of rows r, r + 8 of the sum.  The order of the
+// summed index is free as long as A and B agree: where it suits the layout, c and c + 4 stand for tokens 2 c and 2 c + 1.
+// EXACT (32-bit activations): lo is rounded as well, and the sums of every step are added up outside the tensor cores,
+// whose own additions truncate; against 64 bits the products are then no further off than the CUDA
+// cores' (measured at 777 rows, state: 7.1e-7 of its norm before, 1.1e-6 with three truncating products).
+template <bool EXACT> __device__ __forceinline__ void split_tf32(float x, unsigned& hi, unsigned& lo) {
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+    const float rest = x - __uint_as_float(hi);
+    if (EXACT) asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(rest));
+    else lo = __float_as_uint(rest);
+}
+template <bool EXACT> struct FragA {
+    unsigned hi[4], lo[4];
+    __device__ __forceinline__ void set(float a0, float a1, float a2, float a3) {
+        split_tf32<EXACT>(a0, hi[0], lo[0]); split_tf32<EXACT>(a1, hi[1], lo[1]);
+        split_tf32<EXACT>(a2, hi[2], lo[2]); split_tf32<EXACT>(a3, hi[3], lo[3]);
+    }
+};
+template <bool EXACT> struct FragB {
+    unsigned hi[2], lo[2];
+    __device__ __forceinline__ void set(float b0, float b1) { split_tf32<EXACT>(b0, hi[0], lo[0]); split_tf32<EXACT>(b1, hi[1], lo[1]); }
+};
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// c[i] += A B[i] for N tiles side by side (independent sums between dependent ones)
+template <int N, bool EXACT>
+__device__ __forceinline__ void mma_split(float (&c)[N][4], const FragA<EXACT>& a, const FragB<EXACT> (&b)[N]) {
+    if constexpr (EXACT) {
+        float d[N][4] = {};
+#pragma unroll
+        for (int i = 0; i < N; ++i) mma_tf32(d[i], a.lo, b[i].hi);
+#pragma unroll
+        for (int i = 0; i < N; ++i) mma_tf32(d[i], a.hi, b[i].lo);
+#pragma unroll
+        for (int i = 0; i < N; ++i) mma_tf32(d[i], a.hi, b[i].hi);
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) c[i][k] += d[i][k];
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) mma_tf32(c[i], a.lo, b[i].hi);
+#pragma unroll
+        for (int i = 0; i < N; ++i) mma_tf32(c[i], a.hi, b[i].lo);
+#pragma unroll
+        for (int i = 0; i < N; ++i) mma_tf32(c[i], a.hi, b[i].hi);
+    }
+}
+__device__ __forceinline__ bool finite_f(float x) { return fabsf(x) <= 3.402823466e38f; }
 
 // The rows of segment `seg`, 0 if it is padding or goes on where the one before it ended.
 __device__ __forceinline__ int segment_rows(const ChunkArgs& p, int seg, int& row0) {
@@ -116,31 +173,31 @@ __device__ __forceinline__ int first_chunk(const ChunkArgs& p, int seg, int& row
     return before;
 }
 
-template <int K> struct PrepareSmem {
-    static constexpr int ROW = K + 4;                       // padding: neighbouring tokens lie four banks apart
-    static constexpr size_t bytes(bool delta) {
-        return sizeof(float) * (3 * (size_t)C * ROW + NSUB * K + C + (delta ? SUB * SUB * NSUB * (NSUB + 1) / 2 : 0));
-    }
-};
+__host__ __device__ constexpr int m_row(int a) { return SUB * (a + 1) + 4; }    // a row of sub-chunk a's part of M
+__host__ __device__ constexpr int m_at(int a) { return 128 * a * (a + 1) + 64 * a; }                // where that part begins
+constexpr size_t prepare_smem(int K, bool delta) {
+    return sizeof(float) * (3 * (size_t)C * (K + 4) + NSUB * K + C + (delta ? m_at(NSUB) : 0));
+}
 
-// Bound by the issue of shared-memory loads and multiply-adds (1.5 M multiply-adds a chunk and head of 128 x 128, two CTAs
-// an SM).  Blocks of A and L on the diagonal (16 x 16 tokens) are walked with a running key, P(s, t] k_s, so that they
-// need neither divisions nor exponentials; the others factor at the sub-chunk edges.
+// Two CTAs an SM (shared memory).  Blocks of A and L on the diagonal (16 x 16 tokens) are walked with a running key,
+// P(s, t] k_s, four tokens s and a sixteenth of the channels a thread, so that they need neither divisions nor
+// exponentials; the others factor at the sub-chunk edges and are products.
 template <typename T, int K, int V, bool DELTA>
 __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p) {
-    constexpr int ROW = PrepareSmem<K>::ROW, CPL = K / 32;
+    constexpr bool EXACT = sizeof(T) == 4;
+    constexpr int ROW = K + 4, CPL = K / 32;                // padding: neighbouring tokens lie four banks apart
     extern __shared__ __align__(16) float smem[];
     float* qs = smem;                                       // [C][ROW]  q, then q P(start of its sub-chunk, t]
     float* ks = qs + C * ROW;                               // k, then the same product
     float* gs = ks + C * ROW;                               // decays, then k P(t, end of its sub-chunk]
     float* subp = gs + C * ROW;                             // [NSUB][K] decay of a whole sub-chunk
     float* betas = subp + NSUB * K;                         // [C]
-    float* M = betas + C;                                   // diag(beta) L, sub-chunk a's rows 16 (a + 1) long
+    float* M = betas + C;                                   // diag(beta) L below the diagonal, sub-chunk by sub-chunk
     pdl_launch_dependents();
     const int head = blockIdx.x, chunk = blockIdx.y;
     int row0, rows;
     if (!find_chunk(p, chunk, row0, rows)) return;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fc = lane & 3;
     const int kvh = head / (p.H / p.G), mode = p.mode;
     const bool forget = mode == DECAY_FORGET_GATE, plain = mode == DECAY_CONSTANT, bonus = mode == DECAY_BONUS;
     const bool per_head = mode == DECAY_PER_HEAD || mode == DECAY_STEP;
@@ -156,65 +213,87 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
         low[i] = (forget || bonus) ? p.A_log[head * K + ch0 + i] : 0.f;
     }
     pdl_wait();
-    // ---- the chunk's token vectors: a warp a token; tokens behind the end change nothing (k 0, decay 1)
-#pragma unroll 4
-    for (int t = warp; t < C; t += 8) {
-        float q[CPL], k[CPL], g[CPL], beta = 0.f;
+    // ---- the chunk's token vectors, a warp a token.  First as they are, every load of a thread on its way at once; then
+    // token by token in a loop that is short enough to stay in the instruction cache (a token takes some hundred
+    // instructions).  A thread reads back what it wrote itself.
 #pragma unroll
-        for (int i = 0; i < CPL; ++i) { q[i] = 0.f; k[i] = 0.f; g[i] = 1.f; }
-        if (t < rows) {
-            const size_t rr = (size_t)(row0 + t);
-            float a[CPL];
-            load_run<CPL>(qkv + rr * p.ld + q_off + ch0, q);
-            if (!forget) load_run<CPL>(qkv + rr * p.ld + k_off + ch0, k);
-            if (per_head) a[0] = to_f32(a_in[rr * p.lda + head]);
-            else if (!plain) load_run<CPL>(a_in + rr * p.lda + (size_t)head * K + ch0, a);
-            if (DELTA) {
-                beta = 1.f / (1.f + expf(-to_f32(((const T*)p.b_in)[rr * p.ldb + head])));
-                float sq = 0.f, sk = 0.f;
+    for (int u = 0; u < C / 8; ++u) {
+        const int t = warp + 8 * u;
+        const size_t rr = (size_t)(row0 + min(t, rows - 1));
+        float q[CPL], k[CPL], g[CPL];
+        load_run<CPL>(qkv + rr * p.ld + q_off + ch0, q);
+        load_run<CPL>(forget ? qkv + rr * p.ld + q_off + ch0 : qkv + rr * p.ld + k_off + ch0, k);
+        if (!per_head && !plain) load_run<CPL>(a_in + rr * p.lda + (size_t)head * K + ch0, g);
+        store_run<CPL>(qs + t * ROW + ch0, q);
+        store_run<CPL>(ks + t * ROW + ch0, k);
+        if (!per_head && !plain) store_run<CPL>(gs + t * ROW + ch0, g);
+    }
+    float head_in[2] = {0.f, 0.f};                          // a lane a token: its decay's and its beta's projections
+    if (lane < C / 8) {
+        const size_t rr = (size_t)(row0 + min(warp + 8 * lane, rows - 1));
+        if (per_head) head_in[0] = to_f32(a_in[rr * p.lda + head]);
+        if (DELTA) head_in[1] = to_f32(((const T*)p.b_in)[rr * p.ldb + head]);
+    }
+#pragma unroll 1
+    for (int u = 0; u < C / 8; ++u) {
+        const int t = warp + 8 * u;
+        float q[CPL], k[CPL], g[CPL], beta = 1.f;
+        load_run<CPL>(qs + t * ROW + ch0, q);
+        load_run<CPL>(ks + t * ROW + ch0, k);
+        const float step_in = __shfl_sync(0xffffffffu, head_in[0], u), beta_in = __shfl_sync(0xffffffffu, head_in[1], u);
+        if (!per_head && !plain) load_run<CPL>(gs + t * ROW + ch0, g);
+        if (DELTA) {
+            float sq = 0.f, sk = 0.f;
 #pragma unroll
-                for (int i = 0; i < CPL; ++i) { sq = fmaf(q[i], q[i], sq); sk = fmaf(k[i], k[i], sk); }
-                sq = warp_sum(sq);
-                sk = warp_sum(sk);
-                const float fq = p.q_scale / sqrtf(sq + p.unit_eps), fk = 1.f / sqrtf(sk + p.unit_eps);
-                const float whole = per_head ? expf(-rate * softplus_f(a[0] + bias[0])) : 0.f;
+            for (int i = 0; i < CPL; ++i) { sq = fmaf(q[i], q[i], sq); sk = fmaf(k[i], k[i], sk); }
 #pragma unroll
-                for (int i = 0; i < CPL; ++i) {
-                    q[i] *= fq;
-                    k[i] *= fk;
-                    g[i] = per_head ? whole : expf(-rate * softplus_f(a[i] + bias[i]));
-                }
-            } else if (plain) {
-                beta = 1.f;
-#pragma unroll
-                for (int i = 0; i < CPL; ++i) { q[i] = silu_f(q[i]); k[i] = silu_f(k[i]); g[i] = rate; }
-            } else if (forget) {
-                beta = 1.f;
-#pragma unroll
-                for (int i = 0; i < CPL; ++i) {
-                    const float open = 1.f / (1.f + expf(a[i] + bias[i]));      // 1 - sigmoid of the gate
-                    q[i] = silu_f(q[i]);
-                    k[i] = (1.f - low[i]) * open;
-                    g[i] = low[i] + (1.f - low[i]) * (1.f - open);
-                }
-            } else if (bonus) {
-#pragma unroll
-                for (int i = 0; i < CPL; ++i) {
-                    q[i] *= p.q_scale;
-                    g[i] = expf(-expf(a[i] + bias[i]));
-                    beta = fmaf(q[i] * low[i], k[i], beta);
-                }
-                beta = warp_sum(beta);
-            } else {
-                const bool stepped = mode == DECAY_STEP;
-                beta = stepped ? softplus_f(a[0] + bias[0]) : 1.f;
-                const float whole = stepped ? expf(-rate * beta) : 0.f;
-#pragma unroll
-                for (int i = 0; i < CPL; ++i) {
-                    q[i] *= p.q_scale;
-                    g[i] = stepped ? whole : expf(-rate * softplus_f(-(a[i] + bias[i])));
-                }
+            for (int o = 16; o > 0; o >>= 1) {
+                sq += __shfl_xor_sync(0xffffffffu, sq, o);
+                sk += __shfl_xor_sync(0xffffffffu, sk, o);
             }
+            const float fq = p.q_scale / sqrtf(sq + p.unit_eps), fk = 1.f / sqrtf(sk + p.unit_eps);
+            beta = 1.f / (1.f + expf(-beta_in));
+            const float whole = per_head ? expf(-rate * softplus_f(step_in + bias[0])) : 0.f;
+#pragma unroll
+            for (int i = 0; i < CPL; ++i) {
+                g[i] = per_head ? whole : expf(-rate * softplus_f(g[i] + bias[i]));
+                q[i] *= fq;
+                k[i] *= fk;
+            }
+        } else if (plain) {
+#pragma unroll
+            for (int i = 0; i < CPL; ++i) { q[i] = silu_f(q[i]); k[i] = silu_f(k[i]); g[i] = rate; }
+        } else if (forget) {
+#pragma unroll
+            for (int i = 0; i < CPL; ++i) {
+                const float open = 1.f / (1.f + expf(g[i] + bias[i]));              // 1 - sigmoid of the gate
+                q[i] = silu_f(q[i]);
+                k[i] = (1.f - low[i]) * open;
+                g[i] = low[i] + (1.f - low[i]) * (1.f - open);
+            }
+        } else if (bonus) {
+            float now = 0.f;
+#pragma unroll
+            for (int i = 0; i < CPL; ++i) {
+                q[i] *= p.q_scale;
+                g[i] = expf(-expf(g[i] + bias[i]));
+                now = fmaf(q[i] * low[i], k[i], now);
+            }
+            beta = warp_sum(now);
+        } else {
+            const bool stepped = mode == DECAY_STEP;
+            if (stepped) beta = softplus_f(step_in + bias[0]);
+            const float whole = stepped ? expf(-rate * beta) : 0.f;
+#pragma unroll
+            for (int i = 0; i < CPL; ++i) {
+                q[i] *= p.q_scale;
+                g[i] = stepped ? whole : expf(-rate * softplus_f(-(g[i] + bias[i])));
+            }
+        }
+        if (t >= rows) {                                    // behind the end: changes nothing
+#pragma unroll
+            for (int i = 0; i < CPL; ++i) { q[i] = 0.f; k[i] = 0.f; g[i] = 1.f; }
+            beta = 0.f;
         }
         store_run<CPL>(qs + t * ROW + ch0, q);
         store_run<CPL>(ks + t * ROW + ch0, k);
@@ -224,53 +303,74 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
     __syncthreads();
     const size_t unit = (size_t)chunk * p.H + head;
     float* A = p.a + unit * C * C;
-    // ---- blocks on the diagonal: a thread per (token s, quarter of the channels), down the tokens t of its sub-chunk
+    // ---- blocks on the diagonal: a thread four tokens s.. and every sixteenth float4 of the channels, down the tokens t
+    // of its sub-chunk; the sixteen threads of four tokens add their sums up at once
     {
-        const int slice = tid & 3, s = tid >> 2, a0 = s & ~(SUB - 1);
-        float4 w[K / 16];
+        constexpr int J = K / 64, SUMS = DELTA ? 8 : 4;
+        const int slice = tid & 15, grp = tid >> 4, a = grp >> 2, a0 = a * SUB, s0 = a0 + (grp & 3) * 4;
+        float4 w[4][J];
 #pragma unroll
-        for (int j = 0; j < K / 16; ++j) w[j] = *reinterpret_cast<const float4*>(ks + s * ROW + (j * 4 + slice) * 4);
-#pragma unroll 1
-        for (int t = a0; t < a0 + SUB; ++t) {
-            const float* qt = qs + t * ROW + slice * 4;
-            const float* kt = ks + t * ROW + slice * 4;
-            const float* gt = gs + t * ROW + slice * 4;
-            float da = 0.f, db = 0.f, la = 0.f, lb = 0.f;
-            if (!bonus && t > s) {
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < K / 16; ++j) {
-                    const float4 g = *reinterpret_cast<const float4*>(gt + j * 16);
-                    w[j].x *= g.x; w[j].y *= g.y; w[j].z *= g.z; w[j].w *= g.w;
+            for (int j = 0; j < J; ++j) w[i][j] = *reinterpret_cast<const float4*>(ks + (s0 + i) * ROW + j * 64 + slice * 4);
+#pragma unroll 2
+        for (int t = a0 + (s0 & 8); t < a0 + SUB; ++t) {
+            float4 q[J], k[J], g[J];
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const int at = t * ROW + j * 64 + slice * 4;
+                q[j] = *reinterpret_cast<const float4*>(qs + at);
+                g[j] = *reinterpret_cast<const float4*>(gs + at);
+                if (DELTA) k[j] = *reinterpret_cast<const float4*>(ks + at);
+            }
+            float sum[SUMS];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const bool later = t > s0 + i;
+                if (!bonus && later) {
+#pragma unroll
+                    for (int j = 0; j < J; ++j) { w[i][j].x *= g[j].x; w[i][j].y *= g[j].y; w[i][j].z *= g[j].z; w[i][j].w *= g[j].w; }
+                }
+                float da = 0.f, db = 0.f, la = 0.f, lb = 0.f;
+#pragma unroll
+                for (int j = 0; j < J; ++j) {
+                    da = fmaf(q[j].x, w[i][j].x, fmaf(q[j].y, w[i][j].y, da));
+                    db = fmaf(q[j].z, w[i][j].z, fmaf(q[j].w, w[i][j].w, db));
+                    if (DELTA) {
+                        la = fmaf(k[j].x, w[i][j].x, fmaf(k[j].y, w[i][j].y, la));
+                        lb = fmaf(k[j].z, w[i][j].z, fmaf(k[j].w, w[i][j].w, lb));
+                    }
+                }
+                sum[i] = da + db;
+                if (DELTA) sum[SUMS - 4 + i] = la + lb;
+                if (bonus && later) {
+#pragma unroll
+                    for (int j = 0; j < J; ++j) { w[i][j].x *= g[j].x; w[i][j].y *= g[j].y; w[i][j].z *= g[j].z; w[i][j].w *= g[j].w; }
                 }
             }
+            int which = 0;
 #pragma unroll
-            for (int j = 0; j < K / 16; ++j) {
-                const float4 q = *reinterpret_cast<const float4*>(qt + j * 16);
-                da = fmaf(q.x, w[j].x, fmaf(q.y, w[j].y, da));
-                db = fmaf(q.z, w[j].z, fmaf(q.w, w[j].w, db));
-                if (DELTA) {
-                    const float4 k = *reinterpret_cast<const float4*>(kt + j * 16);
-                    la = fmaf(k.x, w[j].x, fmaf(k.y, w[j].y, la));
-                    lb = fmaf(k.z, w[j].z, fmaf(k.w, w[j].w, lb));
+            for (int half = SUMS / 2, o = 8; o > 0; half >>= 1, o >>= 1) {
+                if (half > 0) {
+                    const bool upper = (slice & o) != 0;
+#pragma unroll
+                    for (int i = 0; i < SUMS / 2; ++i)
+                        if (i < half) {
+                            const float give = upper ? sum[i] : sum[i + half], keep = upper ? sum[i + half] : sum[i];
+                            sum[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                        }
+                    which += upper ? half : 0;
+                } else {
+                    sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
                 }
             }
-            if (bonus && t > s) {
-#pragma unroll
-                for (int j = 0; j < K / 16; ++j) {
-                    const float4 g = *reinterpret_cast<const float4*>(gt + j * 16);
-                    w[j].x *= g.x; w[j].y *= g.y; w[j].z *= g.z; w[j].w *= g.w;
+            const int s = s0 + (which & 3);
+            if ((slice & (DELTA ? 1 : 3)) == 0) {
+                if (which < 4) {
+                    if (t >= s) A[t * C + s] = (bonus && t == s) ? betas[t] : sum[0];
+                } else if (t > s) {
+                    M[m_at(a) + (t - a0) * m_row(a) + s] = betas[t] * sum[0];
                 }
-            }
-            float d = da + db;
-            d += __shfl_xor_sync(0xffffffffu, d, 1);
-            d += __shfl_xor_sync(0xffffffffu, d, 2);
-            if (slice == 0 && t >= s) A[t * C + s] = (bonus && t == s) ? betas[t] : d;
-            if (DELTA) {
-                float l = la + lb;
-                l += __shfl_xor_sync(0xffffffffu, l, 1);
-                l += __shfl_xor_sync(0xffffffffu, l, 2);
-                const int sub = a0 / SUB;
-                if (slice == 0 && t > s) M[SUB * SUB * sub * (sub + 1) / 2 + (t - a0) * SUB * (sub + 1) + s] = betas[t] * l;
             }
         }
     }
@@ -298,45 +398,51 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
         }
     }
     __syncthreads();
-    // ---- blocks below the diagonal: a warp each, rows (lane / 4) + 8 i, columns (lane % 4) + 4 j
+    // ---- blocks below the diagonal: a warp each
     if (warp < 6) {
         const int a = warp < 3 ? 3 : (warp < 5 ? 2 : 1), b = warp < 3 ? warp : (warp < 5 ? warp - 3 : 0);
-        const int t0 = a * SUB + (lane >> 2), s0 = b * SUB + (lane & 3);
+        const int t0 = a * SUB + fr, s0 = b * SUB + fr;
         float acc[2][4] = {}, accl[2][4] = {};
-        for (int c = 0; c < K; c += 4) {
-            float4 between = make_float4(1.f, 1.f, 1.f, 1.f);
-            for (int m = b + 1; m < a; ++m) {
-                const float4 d = *reinterpret_cast<const float4*>(subp + m * K + c);
-                between.x *= d.x; between.y *= d.y; between.z *= d.z; between.w *= d.w;
-            }
-            float4 kv[4];
+#pragma unroll 2
+        for (int c = fc; c < K; c += 8) {
+            float f0 = 1.f, f1 = 1.f;                       // whole sub-chunks between the two
+            for (int m = b + 1; m < a; ++m) { f0 *= subp[m * K + c]; f1 *= subp[m * K + c + 4]; }
+            FragB<EXACT> kb[2];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                kv[j] = *reinterpret_cast<const float4*>(gs + (s0 + 4 * j) * ROW + c);
-                kv[j].x *= between.x; kv[j].y *= between.y; kv[j].z *= between.z; kv[j].w *= between.w;
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const float4 q = *reinterpret_cast<const float4*>(qs + (t0 + 8 * i) * ROW + c);
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    acc[i][j] = fmaf(q.x, kv[j].x, fmaf(q.y, kv[j].y, fmaf(q.z, kv[j].z, fmaf(q.w, kv[j].w, acc[i][j]))));
-                if (DELTA) {
-                    const float4 k = *reinterpret_cast<const float4*>(ks + (t0 + 8 * i) * ROW + c);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        accl[i][j] = fmaf(k.x, kv[j].x, fmaf(k.y, kv[j].y, fmaf(k.z, kv[j].z, fmaf(k.w, kv[j].w, accl[i][j]))));
-                }
+            for (int j = 0; j < 2; ++j) kb[j].set(gs[(s0 + 8 * j) * ROW + c] * f0, gs[(s0 + 8 * j) * ROW + c + 4] * f1);
+            FragA<EXACT> f;
+            f.set(qs[t0 * ROW + c], qs[(t0 + 8) * ROW + c], qs[t0 * ROW + c + 4], qs[(t0 + 8) * ROW + c + 4]);
+            mma_split<2, EXACT>(acc, f, kb);
+            if (DELTA) {
+                f.set(ks[t0 * ROW + c], ks[(t0 + 8) * ROW + c], ks[t0 * ROW + c + 4], ks[(t0 + 8) * ROW + c + 4]);
+                mma_split<2, EXACT>(accl, f, kb);
             }
         }
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int t = t0 + 8 * i, s = s0 + 4 * j;
-                A[t * C + s] = acc[i][j];
-                if (DELTA) M[SUB * SUB * a * (a + 1) / 2 + (t - a * SUB) * SUB * (a + 1) + s] = betas[t] * accl[i][j];
+            for (int i = 0; i < 2; ++i) {
+                const int t = t0 + 8 * i, s = b * SUB + 8 * j + 2 * fc;
+                *reinterpret_cast<float2*>(A + t * C + s) = make_float2(acc[j][2 * i], acc[j][2 * i + 1]);
+                if (DELTA)
+                    *reinterpret_cast<float2*>(M + m_at(a) + (t - a * SUB) * m_row(a) + s) =
+                        make_float2(betas[t] * accl[j][2 * i], betas[t] * accl[j][2 * i + 1]);
             }
+    } else if (DELTA) {
+        // meanwhile: (I + M)^-1 - I of the blocks on the diagonal, in their place, a thread a column
+        const int i = tid - 192, a = i >> 4, j = i & 15;
+        float* m = M + m_at(a) + a * SUB;
+        float x[SUB];
+#pragma unroll
+        for (int t = 0; t < SUB; ++t) {
+            float y = t == j ? 1.f : 0.f;
+#pragma unroll
+            for (int s = 0; s < t; ++s) y = fmaf(-m[t * m_row(a) + s], x[s], y);
+            x[t] = t < j ? 0.f : y;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < SUB; ++t) m[t * m_row(a) + j] = t > j ? x[t] : 0.f;
     }
     // ---- what the other kernels read: q P(0, t], the chunk's decay, k P(t, C]
     float* qb = p.qb + unit * C * K;
@@ -356,59 +462,8 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
         p.decay[unit * K + ch] = d;
     }
     float* ub = p.u + unit * C * V;
-    __syncthreads();                                        // gs, qs and M are complete, nobody reads gs as it was
-    if (DELTA) {
-        float* kd = p.kd + unit * C * K;
-        for (int idx = tid; idx < K / 4 * C; idx += 256) {
-            const int ch = idx % (K / 4) * 4, t = idx / (K / 4), sub = t / SUB;
-            float4 k = *reinterpret_cast<const float4*>(gs + t * ROW + ch);
-            for (int m = sub + 1; m < NSUB; ++m) {
-                const float4 d = *reinterpret_cast<const float4*>(subp + m * K + ch);
-                k.x *= d.x; k.y *= d.y; k.z *= d.z; k.w *= d.w;
-            }
-            *reinterpret_cast<float4*>(kd + t * K + ch) = k;
-        }
-        // the triangular system, a thread a column of [beta K P(0, .] | beta V]
-        for (int col = tid; col < K + V; col += 256) {
-            float x[C];
-            const bool key = col < K;
-            if (key) {
-                float pre = 1.f;
-#pragma unroll
-                for (int t = 0; t < C; ++t) {
-                    if (t > 0 && t % SUB == 0) pre *= subp[(t / SUB - 1) * K + col];
-                    x[t] = betas[t] * ks[t * ROW + col] * pre;
-                }
-            } else {
-#pragma unroll
-                for (int t = 0; t < C; ++t)
-                    x[t] = t < rows ? betas[t] * to_f32(qkv[(size_t)(row0 + t) * p.ld + v_off + col - K]) : 0.f;
-            }
-            float* dst = key ? p.w + unit * C * K + col : ub + (col - K);
-            const int ldd = key ? K : V;
-#pragma unroll
-            for (int t = 0; t < C; ++t) {
-                const int sub = t / SUB;
-                const float* m = M + SUB * SUB * sub * (sub + 1) / 2 + (t - sub * SUB) * SUB * (sub + 1);
-                float y0 = x[t], y1 = 0.f;
-#pragma unroll
-                for (int s = 0; s + 3 < t; s += 4) {
-                    const float4 v = *reinterpret_cast<const float4*>(m + s);
-                    y0 = fmaf(-v.x, x[s], y0);
-                    y1 = fmaf(-v.y, x[s + 1], y1);
-                    y0 = fmaf(-v.z, x[s + 2], y0);
-                    y1 = fmaf(-v.w, x[s + 3], y1);
-                }
-#pragma unroll
-                for (int s = t & ~3; s < t; ++s) y0 = fmaf(-m[s], x[s], y0);
-                x[t] = y0 + y1;
-                dst[(size_t)t * ldd] = x[t];
-            }
-        }
-        return;
-    }
-    // ---- the chunk's share of the state, sum_s (k_s P(s, C]) u_s^T: a thread 8 x 8 of it
-    float* us = smem;                                       // [C][V], over the queries and keys
+    __syncthreads();                                        // qs is written out, gs and M are complete
+    float* kd = DELTA ? p.kd + unit * C * K : gs;
     for (int idx = tid; idx < K / 4 * C; idx += 256) {
         const int ch = idx % (K / 4) * 4, t = idx / (K / 4), sub = t / SUB;
         float4 k = *reinterpret_cast<const float4*>(gs + t * ROW + ch);
@@ -416,8 +471,104 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
             const float4 d = *reinterpret_cast<const float4*>(subp + m * K + ch);
             k.x *= d.x; k.y *= d.y; k.z *= d.z; k.w *= d.w;
         }
-        *reinterpret_cast<float4*>(gs + t * ROW + ch) = k;
+        *reinterpret_cast<float4*>(kd + t * (DELTA ? K : ROW) + ch) = k;
     }
+    if (DELTA) {
+        // the triangular system, 16 columns of [beta K P(0, .] | beta V] a warp, transposed: the sums of one block of
+        // tokens are, lane by lane, the operands of the next
+        for (int tile = warp; tile < (K + V) / 16; tile += 8) {
+            const bool key = tile < K / 16;
+            const int col = (key ? tile : tile - K / 16) * 16 + fr;
+            float x[C / 8][4];
+            float pre[2] = {1.f, 1.f};
+#pragma unroll
+            for (int j = 0; j < C / 8; ++j) {
+                if (key && j > 0 && j % 2 == 0) { pre[0] *= subp[(j / 2 - 1) * K + col]; pre[1] *= subp[(j / 2 - 1) * K + col + 8]; }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int t = 8 * j + 2 * fc + (e & 1), c = col + (e >> 1) * 8;
+                    x[j][e] = key ? ks[t * ROW + c] * pre[e >> 1]
+                                  : to_f32(qkv[(size_t)(row0 + min(t, rows - 1)) * p.ld + v_off + c]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < C / 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int t = 8 * j + 2 * fc + (e & 1);
+                    x[j][e] = t < rows ? x[j][e] * betas[t] : 0.f;
+                }
+#pragma unroll
+            for (int a = 0; a < NSUB; ++a) {
+                const float* m = M + m_at(a) + fr * m_row(a) + 2 * fc;
+                float y[2][4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { y[0][e] = x[2 * a][e]; y[1][e] = x[2 * a + 1][e]; }
+#pragma unroll
+                for (int j = 0; j < 2 * a; ++j) {
+                    FragA<EXACT> f;
+                    f.set(x[j][0], x[j][2], x[j][1], x[j][3]);
+                    FragB<EXACT> mb[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const float2 v = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + 8 * j);
+                        mb[i].set(-v.x, -v.y);
+                    }
+                    mma_split<2, EXACT>(y, f, mb);
+                }
+                bool fine = true;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) fine = fine && finite_f(y[0][e]) && finite_f(y[1][e]);
+                float r[2][4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { r[0][e] = y[0][e]; r[1][e] = y[1][e]; }
+                if (__all_sync(0xffffffffu, fine)) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        FragA<EXACT> f;
+                        f.set(r[j][0], r[j][2], r[j][1], r[j][3]);
+                        FragB<EXACT> mb[2];
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const float2 v = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + a * SUB + 8 * j);
+                            mb[i].set(v.x, v.y);
+                        }
+                        mma_split<2, EXACT>(y, f, mb);
+                    }
+                } else {                                    // token by token: none meets a later one
+                    const float* own = M + m_at(a) + a * SUB;
+                    for (int s = 0; s < SUB; ++s) {
+                        const int from = (lane & ~3) | ((s & 7) >> 1);
+                        float rs[2];
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const float even = s < 8 ? r[0][2 * i] : r[1][2 * i], odd = s < 8 ? r[0][2 * i + 1] : r[1][2 * i + 1];
+                            rs[i] = __shfl_sync(0xffffffffu, (s & 1) ? odd : even, from);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 2; ++j)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const int t = 8 * j + 2 * fc + (e & 1);
+                                if (t > s) y[j][e] = fmaf(own[t * m_row(a) + s], rs[e >> 1], y[j][e]);
+                            }
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { x[2 * a][e] = y[0][e]; x[2 * a + 1][e] = y[1][e]; }
+            }
+            float* dst = key ? p.w + unit * C * K : ub;
+            const int ldd = key ? K : V;
+#pragma unroll
+            for (int j = 0; j < C / 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dst[(8 * j + 2 * fc + (e & 1)) * ldd + col + (e >> 1) * 8] = x[j][e];
+        }
+        return;
+    }
+    // ---- the chunk's share of the state, sum_s (k_s P(s, C]) u_s^T
+    constexpr int UROW = V + 4;
+    float* us = smem;                                       // [C][UROW], over the queries and keys
     for (int idx = tid; idx < V / 4 * C; idx += 256) {
         const int col = idx % (V / 4) * 4, t = idx / (V / 4);
         float v[4] = {0.f, 0.f, 0.f, 0.f};
@@ -425,42 +576,36 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
         const float f = mode == DECAY_STEP ? betas[t] : 1.f;
 #pragma unroll
         for (int e = 0; e < 4; ++e) v[e] = plain ? silu_f(v[e]) : v[e] * f;
-        store_run<4>(us + t * V + col, v);
+        store_run<4>(us + t * UROW + col, v);
         store_run<4>(ub + t * V + col, v);
     }
     __syncthreads();
-    constexpr int RK = K / 64, RV = V / 64;                 // groups of four rows and columns a thread takes
-    const int ty = tid >> 4, tx = tid & 15;
-    float acc[RK * 4][RV * 4];
+    constexpr int MW = K / 32, NT = V / 8 / (8 / MW);       // warps along the channels (32 each), column tiles of a warp
+    const int mb = (warp % MW) * 32, nb = (warp / MW) * NT * 8;
+    float acc[2][NT][4] = {};
+#pragma unroll 1
+    for (int t0 = 0; t0 < C; t0 += 8) {
+        const int t = t0 + 2 * fc;
+        FragB<EXACT> u[NT];
 #pragma unroll
-    for (int i = 0; i < RK * 4; ++i)
+        for (int j = 0; j < NT; ++j) u[j].set(us[t * UROW + nb + 8 * j + fr], us[(t + 1) * UROW + nb + 8 * j + fr]);
 #pragma unroll
-        for (int j = 0; j < RV * 4; ++j) acc[i][j] = 0.f;
-#pragma unroll 2
-    for (int t = 0; t < C; ++t) {
-        float x[RK * 4], y[RV * 4];
-#pragma unroll
-        for (int i = 0; i < RK; ++i) {
-            const float4 v = *reinterpret_cast<const float4*>(gs + t * ROW + i * 64 + ty * 4);
-            x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+        for (int i = 0; i < 2; ++i) {
+            const float* at = gs + t * ROW + mb + 16 * i + fr;
+            FragA<EXACT> f;
+            f.set(at[0], at[8], at[ROW], at[ROW + 8]);
+            mma_split<NT, EXACT>(acc[i], f, u);
         }
-#pragma unroll
-        for (int i = 0; i < RV; ++i) {
-            const float4 v = *reinterpret_cast<const float4*>(us + t * V + i * 64 + tx * 4);
-            y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
-        }
-#pragma unroll
-        for (int i = 0; i < RK * 4; ++i)
-#pragma unroll
-            for (int j = 0; j < RV * 4; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
     }
     float* dS = p.s + unit * K * V;
 #pragma unroll
-    for (int i = 0; i < RK * 4; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < RV; ++j)
-            *reinterpret_cast<float4*>(dS + (size_t)((i / 4) * 64 + ty * 4 + i % 4) * V + j * 64 + tx * 4) =
-                make_float4(acc[i][4 * j], acc[i][4 * j + 1], acc[i][4 * j + 2], acc[i][4 * j + 3]);
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float2*>(dS + (size_t)(mb + 16 * i + 8 * h + fr) * V + nb + 8 * j + 2 * fc) =
+                    make_float2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
 }
 
 // s[chunk] holds what the chunk adds to the state and gets the state in front of the chunk.  A thread four elements,
@@ -502,183 +647,170 @@ __global__ void __launch_bounds__(256) chunk_state_kernel(const ChunkArgs p) {
     *reinterpret_cast<float4*>(dst) = S;
 }
 
-template <int K> struct DeltaSmem {
-    static constexpr int ROW = K + 16;                      // a token's row: neighbouring rows lie 16 banks apart
-    static constexpr int SROW = DCOLS + 4;
-    static constexpr size_t bytes = sizeof(float) * (2 * (size_t)C * ROW + 2 * C * DCOLS + K * SROW + K);
+template <int K, int NT> struct DeltaSmem {
+    static constexpr int ROW = K + 4, COLS = 8 * NT;
+    static constexpr int SROW = COLS + 8, UROW = COLS + 4;  // rows of the state and of U: fragments meet every bank once
+    static constexpr int STAGE = 2 * C * ROW + C * COLS + K;                    // W, Kd, U0, decay of a chunk
+    static constexpr size_t bytes = sizeof(float) * (2 * (size_t)STAGE + C * UROW + K * SROW);
 };
 
-// The chain of the delta rule: per chunk U = U0 - W S and S <- diag(decay) S + Kd^T U, 16 columns of one head's state a CTA,
-// the state and U in shared memory.  Bound by its own two products (512 multiply-adds a thread each, four and two ways
-// split along the sum) and four barriers; the operands of the next product are copied while the current one runs.
-template <int K, int V>
-__global__ void __launch_bounds__(256) chunk_delta_kernel(const ChunkArgs p) {
-    constexpr int ROW = DeltaSmem<K>::ROW, SROW = DeltaSmem<K>::SROW;
+// The chain of the delta rule: per chunk U = U0 - W S and S <- diag(decay) S + Kd^T U, 8 NT columns of one head's state a
+// CTA.  The state lives in the registers of the warps that sum it and, for the next chunk's first product, in shared
+// memory; the next chunk's operands are copied while this one's run.  Bound by the two products' tensor instructions
+// (768 cycles each at 16 columns) and what stands between them: two barriers, the operands' split.
+template <int K, int V, int NT, bool EXACT>
+__global__ void __launch_bounds__(256, 1) chunk_delta_kernel(const ChunkArgs p) {
+    typedef DeltaSmem<K, NT> L;
+    constexpr int ROW = L::ROW, COLS = L::COLS, SROW = L::SROW, UROW = L::UROW;
     extern __shared__ __align__(16) float smem[];
-    float* ws = smem;                                       // [C][ROW]
-    float* kds = ws + C * ROW;                              // [C][ROW]
-    float* u0s = kds + C * ROW;                             // [C][DCOLS]
-    float* us = u0s + C * DCOLS;                            // [C][DCOLS]
-    float* S = us + C * DCOLS;                              // [K][SROW]
-    float* ds = S + K * SROW;                               // [K]
+    float* us = smem + 2 * L::STAGE;                        // [C][UROW]
+    float* S = us + C * UROW;                               // [K][SROW]
     pdl_launch_dependents();
-    const int col0 = blockIdx.x * DCOLS, head = blockIdx.y;
+    const int col0 = blockIdx.x * COLS, head = blockIdx.y;
     int row0, rows;
     const int first = first_chunk(p, blockIdx.z, row0, rows);
     if (rows <= 0) return;
     const int chunks = (rows + C - 1) / C;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fc = lane & 3;
     float* state = p.state + (size_t)p.row_slot[row0] * p.state_stride + (size_t)head * K * V + col0;
     pdl_wait();
-    auto fetch_w = [&](int c) {
+    auto fetch = [&](int c) {
         const size_t unit = (size_t)(first + c) * p.H + head;
-        for (int i = tid; i < C * K / 4; i += 256)
-            copy16(ws + i / (K / 4) * ROW + i % (K / 4) * 4, p.w + unit * C * K + (size_t)i * 4);
-        for (int i = tid; i < C * DCOLS / 4; i += 256)
-            copy16(u0s + i * 4, p.u + unit * C * V + (size_t)(i / (DCOLS / 4)) * V + col0 + i % (DCOLS / 4) * 4);
-        copy_commit();
-    };
-    auto fetch_kd = [&](int c) {
-        const size_t unit = (size_t)(first + c) * p.H + head;
-        for (int i = tid; i < C * K / 4; i += 256)
-            copy16(kds + i / (K / 4) * ROW + i % (K / 4) * 4, p.kd + unit * C * K + (size_t)i * 4);
+        float* ws = smem + (c & 1) * L::STAGE;
+        float* kds = ws + C * ROW;
+        float* u0s = kds + C * ROW;
+        float* ds = u0s + C * COLS;
+        for (int i = tid; i < C * K / 4; i += 256) copy16(ws + i / (K / 4) * ROW + i % (K / 4) * 4, p.w + unit * C * K + (size_t)i * 4);
+        for (int i = tid; i < C * COLS / 4; i += 256)
+            copy16(u0s + i * 4, p.u + unit * C * V + (size_t)(i / (COLS / 4)) * V + col0 + i % (COLS / 4) * 4);
+        for (int i = tid; i < C * K / 4; i += 256) copy16(kds + i / (K / 4) * ROW + i % (K / 4) * 4, p.kd + unit * C * K + (size_t)i * 4);
         for (int i = tid; i < K / 4; i += 256) copy16(ds + i * 4, p.decay + unit * K + (size_t)i * 4);
         copy_commit();
     };
-    fetch_w(0);
-    fetch_kd(0);
-    for (int i = tid; i < K * DCOLS / 4; i += 256)
-        *reinterpret_cast<float4*>(S + i / 4 * SROW + i % 4 * 4) =
-            *reinterpret_cast<const float4*>(state + (size_t)(i / 4) * V + i % 4 * 4);
+    fetch(0);
+    // the part of the state that this warp sums: rows sm.., SN column tiles from sn on
+    constexpr int SM = K / 16, SW = 8 / SM, SN = NT / SW;   // row tiles, warps that share one, column tiles of each
+    const int sm = warp / SW * 16, sn = warp % SW * SN * 8;
+    float s[SN][4];
+#pragma unroll
+    for (int j = 0; j < SN; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float2 v = *reinterpret_cast<const float2*>(state + (size_t)(sm + fr + 8 * h) * V + sn + 8 * j + 2 * fc);
+            s[j][2 * h] = v.x; s[j][2 * h + 1] = v.y;
+        }
+    // the part of U that this warp sums: tokens um.., half of the column tiles
+    constexpr int UN = NT / 2;
+    const int um = (warp & 3) * 16, un = (warp >> 2) * UN * 8;
     for (int c = 0; c < chunks; ++c) {
         const size_t unit = (size_t)(first + c) * p.H + head;
-        copy_wait<1>();
-        __syncthreads();                                    // W, U0 and the state of this chunk are there
-        for (int i = tid; i < K * DCOLS / 4; i += 256)
-            *reinterpret_cast<float4*>(p.s + unit * K * V + (size_t)(i / 4) * V + col0 + i % 4 * 4) =
-                *reinterpret_cast<const float4*>(S + i / 4 * SROW + i % 4 * 4);
-        {   // U = U0 - W S: rows rg + 16 i, columns 4 cg.., a quarter of the sum each
-            const int cg = tid & 3, kq = (tid >> 2) & 3, rg = tid >> 4;
-            float acc[4][4] = {};
-#pragma unroll 2
-            for (int k0 = 0; k0 < K; k0 += 16) {
-                const int k = k0 + kq * 4;
-                float4 w[4], s[4];
+        const float* ws = smem + (c & 1) * L::STAGE;
+        const float* kds = ws + C * ROW;
+        const float* u0s = kds + C * ROW;
+        const float* ds = u0s + C * COLS;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(ws + (rg + 16 * i) * ROW + k);
+        for (int j = 0; j < SN; ++j)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s[j] = *reinterpret_cast<const float4*>(S + (k + j) * SROW + cg * 4);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float wi[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        acc[i][0] = fmaf(wi[j], s[j].x, acc[i][0]);
-                        acc[i][1] = fmaf(wi[j], s[j].y, acc[i][1]);
-                        acc[i][2] = fmaf(wi[j], s[j].z, acc[i][2]);
-                        acc[i][3] = fmaf(wi[j], s[j].w, acc[i][3]);
-                    }
-                }
+            for (int h = 0; h < 2; ++h) {
+                const float2 v = make_float2(s[j][2 * h], s[j][2 * h + 1]);
+                const int k = sm + fr + 8 * h, col = sn + 8 * j + 2 * fc;
+                *reinterpret_cast<float2*>(S + k * SROW + col) = v;
+                *reinterpret_cast<float2*>(p.s + unit * K * V + (size_t)k * V + col0 + col) = v;
             }
-            // the four quarters: every lane ends with one row of its four
-            float half[2][4], mine[4];
-            const bool up1 = (kq & 1) != 0, up2 = (kq & 2) != 0;
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float give = up1 ? acc[i][e] : acc[i + 2][e], keep = up1 ? acc[i + 2][e] : acc[i][e];
-                    half[i][e] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
-                }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float give = up2 ? half[0][e] : half[1][e], keep = up2 ? half[1][e] : half[0][e];
-                mine[e] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
-            }
-            const int row = rg + 16 * ((up1 ? 2 : 0) + (up2 ? 1 : 0));
-            const float4 u0 = *reinterpret_cast<const float4*>(u0s + row * DCOLS + cg * 4);
-            const float4 u = make_float4(u0.x - mine[0], u0.y - mine[1], u0.z - mine[2], u0.w - mine[3]);
-            *reinterpret_cast<float4*>(us + row * DCOLS + cg * 4) = u;
-            *reinterpret_cast<float4*>(p.u + unit * C * V + (size_t)row * V + col0 + cg * 4) = u;
-        }
-        __syncthreads();                                    // U is complete, W and U0 are free
-        if (c + 1 < chunks) fetch_w(c + 1); else copy_commit();
-        copy_wait<1>();
-        __syncthreads();                                    // Kd and the decay are there
-        {   // S <- diag(decay) S + Kd^T U: rows 4 kg.., columns 4 cg.., every SPLIT-th token
-            constexpr int SPLIT = 256 / K;                  // 2 (K 128), 4 (K 64)
-            const int cg = tid & 3, sq = (tid >> 2) & (SPLIT - 1), kg = tid / (4 * SPLIT);
-            float acc[4][4] = {};
+        copy_wait<0>();
+        __syncthreads();                                    // the chunk's operands and the state; the other stage is free
+        if (c + 1 < chunks) fetch(c + 1);
+        {   // U = U0 - W S
+            float acc[2][UN][4] = {};                       // even and odd steps: independent sums
 #pragma unroll 4
-            for (int t = sq; t < C; t += SPLIT) {
-                const float4 kv = *reinterpret_cast<const float4*>(kds + t * ROW + kg * 4);
-                const float4 uv = *reinterpret_cast<const float4*>(us + t * DCOLS + cg * 4);
-                const float ki[4] = {kv.x, kv.y, kv.z, kv.w};
+            for (int k0 = 0; k0 < K; k0 += 16)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    acc[i][0] = fmaf(ki[i], uv.x, acc[i][0]);
-                    acc[i][1] = fmaf(ki[i], uv.y, acc[i][1]);
-                    acc[i][2] = fmaf(ki[i], uv.z, acc[i][2]);
-                    acc[i][3] = fmaf(ki[i], uv.w, acc[i][3]);
+                for (int half = 0; half < 2; ++half) {
+                    const int k = k0 + 8 * half + fc;
+                    const float* w = ws + (um + fr) * ROW + k;
+                    FragA<EXACT> f;
+                    f.set(w[0], w[8 * ROW], w[4], w[8 * ROW + 4]);
+                    FragB<EXACT> b[UN];
+#pragma unroll
+                    for (int j = 0; j < UN; ++j) b[j].set(S[k * SROW + un + 8 * j + fr], S[(k + 4) * SROW + un + 8 * j + fr]);
+                    mma_split<UN, EXACT>(acc[half], f, b);
                 }
-            }
-            const bool up1 = (sq & 1) != 0, up2 = (sq & 2) != 0;
-            float half[2][4];
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
+            for (int j = 0; j < UN; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float give = up1 ? acc[i][e] : acc[i + 2][e], keep = up1 ? acc[i + 2][e] : acc[i][e];
-                    half[i][e] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+                for (int h = 0; h < 2; ++h) {
+                    const int t = um + fr + 8 * h, col = un + 8 * j + 2 * fc;
+                    const float2 u0 = *reinterpret_cast<const float2*>(u0s + t * COLS + col);
+                    const float2 u = make_float2(u0.x - (acc[0][j][2 * h] + acc[1][j][2 * h]),
+                                                 u0.y - (acc[0][j][2 * h + 1] + acc[1][j][2 * h + 1]));
+                    *reinterpret_cast<float2*>(us + t * UROW + col) = u;
+                    *reinterpret_cast<float2*>(p.u + unit * C * V + (size_t)t * V + col0 + col) = u;
                 }
-            auto add = [&](int k, const float (&v)[4]) {
-                float4* at = reinterpret_cast<float4*>(S + k * SROW + cg * 4);
-                const float g = ds[k];
-                const float4 s = *at;
-                *at = make_float4(fmaf(s.x, g, v[0]), fmaf(s.y, g, v[1]), fmaf(s.z, g, v[2]), fmaf(s.w, g, v[3]));
-            };
-            if (SPLIT == 2) {
-                add(kg * 4 + (up1 ? 2 : 0), half[0]);
-                add(kg * 4 + (up1 ? 3 : 1), half[1]);
-            } else {
-                float mine[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float give = up2 ? half[0][e] : half[1][e], keep = up2 ? half[1][e] : half[0][e];
-                    mine[e] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
-                }
-                add(kg * 4 + (up1 ? 2 : 0) + (up2 ? 1 : 0), mine);
-            }
         }
-        __syncthreads();                                    // the new state is complete, Kd is free
-        if (c + 1 < chunks) fetch_kd(c + 1); else copy_commit();
+        __syncthreads();                                    // U is complete, nobody reads the state any more
+        {   // S <- diag(decay) S + Kd^T U
+            float acc[2][SN][4] = {};
+#pragma unroll 4
+            for (int t0 = 0; t0 < C; t0 += 16)
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int t = t0 + 8 * half + 2 * fc;
+                    const float* kd = kds + t * ROW + sm + fr;
+                    FragA<EXACT> f;
+                    f.set(kd[0], kd[8], kd[ROW], kd[ROW + 8]);
+                    FragB<EXACT> b[SN];
+#pragma unroll
+                    for (int j = 0; j < SN; ++j) b[j].set(us[t * UROW + sn + 8 * j + fr], us[(t + 1) * UROW + sn + 8 * j + fr]);
+                    mma_split<SN, EXACT>(acc[half], f, b);
+                }
+            const float g0 = ds[sm + fr], g1 = ds[sm + fr + 8];
+#pragma unroll
+            for (int j = 0; j < SN; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[j][e] = fmaf(s[j][e], e < 2 ? g0 : g1, acc[0][j][e] + acc[1][j][e]);
+        }
     }
-    copy_wait<0>();
-    for (int i = tid; i < K * DCOLS / 4; i += 256)
-        *reinterpret_cast<float4*>(state + (size_t)(i / 4) * V + i % 4 * 4) =
-            *reinterpret_cast<const float4*>(S + i / 4 * SROW + i % 4 * 4);
+#pragma unroll
+    for (int j = 0; j < SN; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            *reinterpret_cast<float2*>(state + (size_t)(sm + fr + 8 * h) * V + sn + 8 * j + 2 * fc) =
+                make_float2(s[j][2 * h], s[j][2 * h + 1]);
 }
 
 constexpr int OUT_TILE = 32;                    // of the sum, a stage of chunk_output_kernel
-constexpr size_t output_smem(int V) { return sizeof(float) * 2 * (size_t)(C * (OUT_TILE + 4) + OUT_TILE * V); }
+constexpr size_t output_smem(int V, size_t type) {
+    return sizeof(float) * 2 * (size_t)(C * (OUT_TILE + 4) + OUT_TILE * (V + 8)) + type * C * V;
+}
 
-// o = [q P | A] [S_0; U] of a chunk and head: a warp eight tokens with all value columns, so that a token's norm is a sum
-// over its warp; tiles of 32 along the sum, two in flight.  A's part ends at the warp's own tokens.  Modes whose norm is
-// not per head leave 32-bit outputs in o_raw.
+// o = [q P | A] [S_0; U] of a chunk and head: a warp a sub-chunk's 16 tokens and half of the value columns; tiles of 32 along
+// the sum, two in flight.  A's part ends with the warp's own tokens.  Modes whose norm is not per head leave 32-bit
+// outputs in o_raw.
 template <typename T, int K, int V>
-__global__ void __launch_bounds__(256) chunk_output_kernel(const ChunkArgs p) {
-    constexpr int KT = OUT_TILE, XROW = KT + 4, VC = V / 32;
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 3) chunk_output_kernel(const ChunkArgs p) {
+    constexpr bool EXACT = sizeof(T) == 4;
+    constexpr int KT = OUT_TILE, XROW = KT + 4, YROW = V + 8, NT = V / 16;
     extern __shared__ __align__(16) float smem[];
     float* xs = smem;                                       // [2][C][XROW]
-    float* ys = smem + 2 * C * XROW;                        // [2][KT][V]
+    float* ys = smem + 2 * C * XROW;                        // [2][KT][YROW]
+    T* gs = reinterpret_cast<T*>(ys + 2 * KT * YROW);       // [C][V]
     pdl_launch_dependents();
     const int head = blockIdx.x, chunk = blockIdx.y;
     int row0, rows;
     if (!find_chunk(p, chunk, row0, rows)) return;
-    const int tid = threadIdx.x, lane = tid & 31, r0 = (tid >> 5) * 8;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fc = lane & 3;
+    const int a = warp & 3, r0 = a * SUB + fr, n0 = (warp >> 2) * (V / 2);
     const size_t unit = (size_t)chunk * p.H + head;
     constexpr int TILES = (K + C) / KT;
+    const bool raw = p.mode == DECAY_CONSTANT || p.mode == DECAY_STEP, gated = !raw && p.gate != nullptr;
     pdl_wait();
+    if (gated) {                                            // what the last step reads, on its way from the beginning
+        constexpr int PER = 16 / (int)sizeof(T);
+        for (int i = tid; i < C * V / PER; i += 256) {
+            const int t = i / (V / PER), at = i % (V / PER) * PER;
+            copy16(gs + t * V + at, (const T*)p.gate + (size_t)(row0 + min(t, rows - 1)) * p.ldg + (size_t)head * V + at);
+        }
+    }
     auto fetch = [&](int tile) {
         const int buf = tile & 1, at = tile * KT;
         const float* x = at < K ? p.qb + unit * C * K + at : p.a + unit * C * C + at - K;
@@ -686,79 +818,99 @@ __global__ void __launch_bounds__(256) chunk_output_kernel(const ChunkArgs p) {
         const int ldx = at < K ? K : C;
         for (int i = tid; i < C * KT / 4; i += 256)
             copy16(xs + buf * C * XROW + i / (KT / 4) * XROW + i % (KT / 4) * 4, x + (size_t)(i / (KT / 4)) * ldx + i % (KT / 4) * 4);
-        for (int i = tid; i < KT * V / 4; i += 256) copy16(ys + buf * KT * V + i * 4, y + (size_t)i * 4);
+        for (int i = tid; i < KT * V / 4; i += 256)
+            copy16(ys + buf * KT * YROW + i / (V / 4) * YROW + i % (V / 4) * 4, y + (size_t)i * 4);
         copy_commit();
     };
-    float acc[8][VC];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int e = 0; e < VC; ++e) acc[i][e] = 0.f;
+    float acc[NT][4] = {};
     fetch(0);
     for (int tile = 0; tile < TILES; ++tile) {
         if (tile + 1 < TILES) fetch(tile + 1); else copy_commit();
         copy_wait<1>();
         __syncthreads();
-        const float* x = xs + (tile & 1) * C * XROW;
-        const float* y = ys + (tile & 1) * KT * V;
+        const float* x = xs + (tile & 1) * C * XROW + r0 * XROW;
+        const float* y = ys + (tile & 1) * KT * YROW + n0 + fr;
         const int s0 = tile * KT - K;                       // first token of A's columns in this tile (negative: q P)
-        const int whole = s0 < 0 ? KT : min(KT, max(0, r0 - s0));           // columns that every token of the warp sees
-#pragma unroll 2
-        for (int j = 0; j < whole; j += 4) {
-            float4 xv[8];
+        const int whole = s0 < 0 ? KT : min(KT, max(0, a * SUB - s0));      // columns that every token of the warp sees
+#pragma unroll 1
+        for (int j = 0; j < whole; j += 8) {
+            const int k = j + fc;
+            FragA<EXACT> f;
+            f.set(x[k], x[8 * XROW + k], x[k + 4], x[8 * XROW + k + 4]);
+            FragB<EXACT> b[NT];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) xv[i] = *reinterpret_cast<const float4*>(x + (r0 + i) * XROW + j);
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                float yv[VC];
-                load_run<VC>(y + (j + m) * V + lane * VC, yv);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float xi = m == 0 ? xv[i].x : m == 1 ? xv[i].y : m == 2 ? xv[i].z : xv[i].w;
-#pragma unroll
-                    for (int e = 0; e < VC; ++e) acc[i][e] = fmaf(xi, yv[e], acc[i][e]);
-                }
-            }
+            for (int i = 0; i < NT; ++i) b[i].set(y[k * YROW + 8 * i], y[(k + 4) * YROW + 8 * i]);
+            mma_split<NT, EXACT>(acc, f, b);
         }
-        if (s0 >= 0 && r0 >= s0 && r0 < s0 + KT) {          // the warp's own tokens: each sees those up to itself
+        const int d0 = a * SUB - s0;                        // where the warp's own tokens lie in this tile
+        if (s0 >= 0 && d0 >= 0 && d0 < KT) {
+            bool fine = true;
 #pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                float yv[VC];
-                load_run<VC>(y + (r0 - s0 + m) * V + lane * VC, yv);
+            for (int j = 0; j < SUB; j += 4)
 #pragma unroll
-                for (int i = m; i < 8; ++i) {
-                    const float xi = x[(r0 + i) * XROW + r0 - s0 + m];
+                for (int i = 0; i < NT; ++i) fine = fine && finite_f(y[(d0 + j + fc) * YROW + 8 * i]);
+            if (__all_sync(0xffffffffu, fine)) {
 #pragma unroll
-                    for (int e = 0; e < VC; ++e) acc[i][e] = fmaf(xi, yv[e], acc[i][e]);
+                for (int j = 0; j < SUB; j += 8) {
+                    const int k = d0 + j + fc, s = j + fc;
+                    FragA<EXACT> f;                                // a token sees those up to itself
+                    f.set(fr >= s ? x[k] : 0.f, fr + 8 >= s ? x[8 * XROW + k] : 0.f, fr >= s + 4 ? x[k + 4] : 0.f,
+                          fr + 8 >= s + 4 ? x[8 * XROW + k + 4] : 0.f);
+                    FragB<EXACT> b[NT];
+#pragma unroll
+                    for (int i = 0; i < NT; ++i) b[i].set(y[k * YROW + 8 * i], y[(k + 4) * YROW + 8 * i]);
+                    mma_split<NT, EXACT>(acc, f, b);
                 }
+            } else {
+                const float* yt = ys + (tile & 1) * KT * YROW + n0 + 2 * fc;
+                for (int s = 0; s < SUB; ++s)
+#pragma unroll
+                    for (int i = 0; i < NT; ++i)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (fr + 8 * (e >> 1) >= s)
+                                acc[i][e] = fmaf(x[8 * (e >> 1) * XROW + d0 + s], yt[(d0 + s) * YROW + 8 * i + (e & 1)], acc[i][e]);
             }
         }
         __syncthreads();
     }
     copy_wait<0>();
-    const bool raw = p.mode == DECAY_CONSTANT || p.mode == DECAY_STEP;
-    const float* nw = p.norm_w + (p.mode == DECAY_BONUS ? (size_t)head * V : 0) + lane * VC;
+    // through shared memory, so that a warp has eight whole tokens: their norms, gates and stores
+    constexpr int OROW = V + 4, VC = V / 32;
+    float* os = smem;                                       // [C][OROW], over the tiles
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        if (r0 + i >= rows) break;
-        const size_t rr = (size_t)(row0 + r0 + i);
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            *reinterpret_cast<float2*>(os + (r0 + 8 * h) * OROW + n0 + 8 * i + 2 * fc) = make_float2(acc[i][2 * h], acc[i][2 * h + 1]);
+    const int t0 = warp * 8, col = lane * VC;
+    float nw[VC];
+#pragma unroll
+    for (int e = 0; e < VC; ++e) nw[e] = raw ? 1.f : p.norm_w[(p.mode == DECAY_BONUS ? head * V : 0) + col + e];
+    __syncthreads();
+    const int count = min(8, rows - t0);
+#pragma unroll 1
+    for (int i = 0; i < count; ++i) {                       // (a loop that stays in the instruction cache)
+        const size_t rr = (size_t)(row0 + t0 + i);
+        float o[VC];
+        load_run<VC>(os + (t0 + i) * OROW + col, o);
         if (raw) {
-            store_run<VC>(p.o_raw + rr * p.H * V + (size_t)head * V + lane * VC, acc[i]);
+            store_run<VC>(p.o_raw + rr * p.H * V + (size_t)head * V + col, o);
             continue;
         }
         float ss = 0.f;
 #pragma unroll
-        for (int e = 0; e < VC; ++e) ss = fmaf(acc[i][e], acc[i][e], ss);
+        for (int e = 0; e < VC; ++e) ss = fmaf(o[e], o[e], ss);
         ss = warp_sum(ss);
         const float f = rsqrtf(ss / (float)V + p.eps);
-        float o[VC], g[VC];
-        if (p.gate != nullptr) load_run<VC>((const T*)p.gate + rr * p.ldg + (size_t)head * V + lane * VC, g);
+        float g[VC];
+        if (gated) load_run<VC>(gs + (t0 + i) * V + col, g);
 #pragma unroll
         for (int e = 0; e < VC; ++e) {
-            o[e] = acc[i][e] * f * nw[e];
-            if (p.gate != nullptr) o[e] *= gate_f(g[e], p.gate_act);
+            o[e] = o[e] * f * nw[e];
+            if (gated) o[e] *= gate_f(g[e], p.gate_act);
         }
-        store_run<VC>((T*)p.out + rr * p.ldo + (size_t)head * V + lane * VC, o);
+        store_run<VC>((T*)p.out + rr * p.ldo + (size_t)head * V + col, o);
     }
 }
 
@@ -766,7 +918,7 @@ template <typename T, int K, int V>
 int launch_chunked(const ChunkArgs& p, cudaStream_t stream) {
     const bool delta = p.mode == DECAY_PER_CHANNEL || p.mode == DECAY_PER_HEAD;
     const dim3 per_chunk(p.H, p.chunks);
-    const size_t smem = PrepareSmem<K>::bytes(delta);
+    const size_t smem = prepare_smem(K, delta);
     if (delta) {
         cudaFuncSetAttribute(chunk_prepare_kernel<T, K, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         tis_launch(chunk_prepare_kernel<T, K, V, true>, per_chunk, dim3(256), smem, stream, p);
@@ -777,15 +929,21 @@ int launch_chunked(const ChunkArgs& p, cudaStream_t stream) {
     int st = tis_check_launch("chunk_prepare");
     if (st != TIS_OK) return st;
     if (delta) {
-        cudaFuncSetAttribute(chunk_delta_kernel<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaSmem<K>::bytes);
-        tis_launch(chunk_delta_kernel<K, V>, dim3(V / DCOLS, p.H, p.segments), dim3(256), DeltaSmem<K>::bytes, stream, p);
+        // 16 columns a CTA while all CTAs are resident (one an SM), else 32
+        if (p.H * (V / 16) * p.segments <= 148) {
+            cudaFuncSetAttribute(chunk_delta_kernel<K, V, 2, sizeof(T) == 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaSmem<K, 2>::bytes);
+            tis_launch(chunk_delta_kernel<K, V, 2, sizeof(T) == 4>, dim3(V / 16, p.H, p.segments), dim3(256), DeltaSmem<K, 2>::bytes, stream, p);
+        } else {
+            cudaFuncSetAttribute(chunk_delta_kernel<K, V, 4, sizeof(T) == 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaSmem<K, 4>::bytes);
+            tis_launch(chunk_delta_kernel<K, V, 4, sizeof(T) == 4>, dim3(V / 32, p.H, p.segments), dim3(256), DeltaSmem<K, 4>::bytes, stream, p);
+        }
     } else {
         tis_launch(chunk_state_kernel<K, V>, dim3(K * V / 1024, p.H, p.segments), dim3(256), 0, stream, p);
     }
     st = tis_check_launch("chunk_state");
     if (st != TIS_OK) return st;
-    cudaFuncSetAttribute(chunk_output_kernel<T, K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)output_smem(V));
-    tis_launch(chunk_output_kernel<T, K, V>, per_chunk, dim3(256), output_smem(V), stream, p);
+    cudaFuncSetAttribute(chunk_output_kernel<T, K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)output_smem(V, sizeof(T)));
+    tis_launch(chunk_output_kernel<T, K, V>, per_chunk, dim3(256), output_smem(V, sizeof(T)), stream, p);
     return tis_check_launch("chunk_output");
 }
 

@@ -1090,9 +1090,9 @@ def _recurrence_spread(requests: Optional[int], num_heads: int, v_dim: int) -> i
 
 #: rows of a step's longest request from which the matrix-state recurrences run in chunks of 64 tokens
 #: (csrc/chunked_recurrence.cu) instead of token by token.  Measured on a B200 at 12 heads of 128 x 128 in bfloat16, us token by
-#: token / in chunks: delta rule, one request of 128 rows 82 / 90, of 192 rows 120 / 92, of 2048 rows 1080 / 300, 16 requests of 128
-#: rows 268 / 259; gated linear attention, one request of 128 rows 59 / 65, of 192 rows 85 / 71
-CHUNKED_MIN_ROWS = int(os.environ.get("TIS_CHUNKED_MIN_ROWS", "160"))
+#: token / in chunks: delta rule, one request of 96 rows 62 / 57, of 128 rows 82 / 58, 4 requests of 96 rows 140 / 88; gated
+#: linear attention, one request of 96 rows 45 / 64, of 128 rows 59 / 57, 4 requests of 96 rows 113 / 67
+CHUNKED_MIN_ROWS = int(os.environ.get("TIS_CHUNKED_MIN_ROWS", "112"))
 #: scratch of the chunked form above which a step is walked token by token all the same (it grows with the rows: 220 KB a
 #: chunk and head of 128 x 128)
 CHUNKED_MAX_BYTES = 1 << 30
