@@ -4,7 +4,9 @@
 #pragma once
 #include "common.cuh"
 #include <cuda.h>
+#include <map>
 #include <mutex>
+#include <tuple>
 #include <unordered_map>
 
 namespace tc {
@@ -41,6 +43,11 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
                  ::"r"(smem_u32(dst)), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, unsigned long long* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
+                 ::"r"(smem_u32(dst)), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
                  : "memory");
 }
 __device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
@@ -200,6 +207,34 @@ inline bool tensor_map(const void* ptr, long long inner, long long outer, long l
     const CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { tis_set_error("cuTensorMapEncodeTiled failed with %d", (int)r); return false; }
+    if (cache.size() > 4096) cache.clear();
+    cache.emplace(key, m);
+    *out = m;
+    return true;
+}
+
+// A map of the rows of a pool of pages: `width` elements a row, `rows` rows a page (all its kv heads), read in boxes of 64
+// elements x `box_rows` rows with the 128-byte swizzle.  Kept by address and shape.
+inline bool page_map(const void* ptr, int width, int rows, int num_pages, size_t row_stride, size_t page_stride, int box_rows,
+                     CUtensorMap* out) {
+    typedef std::tuple<const void*, int, int, int, size_t, size_t, int> Key;
+    static std::mutex mu;
+    static std::map<Key, CUtensorMap> cache;
+    const Key key(ptr, width, rows, num_pages, row_stride, page_stride, box_rows);
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = cache.find(key);
+    if (it != cache.end()) { *out = it->second; return true; }
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) { tis_set_error("the driver has no cuTensorMapEncodeTiled"); return false; }
+    const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)rows, (cuuint64_t)num_pages};
+    const cuuint64_t strides[2] = {(cuuint64_t)row_stride * 2, (cuuint64_t)page_stride * 2};
+    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    CUtensorMap m;
+    const CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { tis_set_error("cuTensorMapEncodeTiled failed with %d", (int)r); return false; }
     if (cache.size() > 4096) cache.clear();
     cache.emplace(key, m);

@@ -989,6 +989,7 @@ def window_attention_library(k_dim: int, v_dim: int):
         lib.tis_window_attention_mma_dims(ctypes.byref(kd), ctypes.byref(vd))
         if (kd.value, vd.value) != (k_dim, v_dim):
             raise KernelError(f"windowed attention library built for widths {kd.value}/{vd.value}, wanted {k_dim}/{v_dim}")
+        lib.tc_forms = int(lib.tis_window_attention_tc_forms())
         _wattn_libs[(k_dim, v_dim)] = lib
     return lib
 
@@ -1011,6 +1012,22 @@ def window_attention_mma_usable(q: torch.Tensor, gate, out: torch.Tensor, k_page
             and k_pages.data_ptr() % 16 == 0 and v_pages.data_ptr() % 16 == 0)
 
 
+#: long portions of prompts run on the tcgen05 kernel where it takes their widths and pages;
+#: TIS_WINDOW_ATTENTION_TC=0 keeps them on the mma.sync kernel
+WINDOW_ATTENTION_TC = os.environ.get("TIS_WINDOW_ATTENTION_TC", "1") != "0"
+
+
+def _window_boxes(k_pages: torch.Tensor, v_pages: torch.Tensor, page_size: int) -> int:
+    """Whether key and value rows can be read in boxes of whole pages: 0 no; 1 yes; 2 yes, and the values are the first elements
+    of the key rows."""
+    heads, k_dim, v_dim = k_pages.shape[1], k_pages.shape[3], v_pages.shape[3]
+    if page_size not in (16, 32, 64, 128) or not (heads == 1 or k_pages.stride(1) == page_size * k_dim):
+        return 0
+    if v_pages.data_ptr() == k_pages.data_ptr() and v_pages.stride() == k_pages.stride():
+        return 2
+    return int(v_pages.stride(2) == v_dim and (heads == 1 or v_pages.stride(1) == page_size * v_dim))
+
+
 def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor, k_pages: torch.Tensor,
                      v_pages: torch.Tensor, block_table: torch.Tensor, positions: torch.Tensor, row_slot: torch.Tensor,
                      num_heads: int, page_size: int, window: Optional[int], scale: float,
@@ -1027,8 +1044,8 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
     wider rows (``v_pages`` with a row stride above its width, for instance the first elements of the key rows).
 
     float32, and widths that are not multiples of 16: a CUDA-core kernel, a CTA per row and head.  bfloat16 inside
-    a step (``step`` given, with the tiles of ``kernels.window_plan``): the tensor-core kernel, a CTA per tile of rows
-    and kv head; the warps of a decode row's CTA split its keys."""
+    a step (``step`` given, with the tiles of ``kernels.window_plan``): long portions on the tcgen05 kernel where it takes them,
+    else the mma.sync kernel, a CTA per tile of rows and kv head; the warps of a decode row's CTA split its keys."""
     lib = library()
     n = q.shape[0]
     kv_heads, k_dim, v_dim = k_pages.shape[1], k_pages.shape[3], v_pages.shape[3]
@@ -1038,8 +1055,25 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
     if step is not None and num_heads // kv_heads <= 64 and window_attention_mma_usable(q, gate, out, k_pages, v_pages,
                                                                                           gate_per_head):
         from . import window_plan
-        row0, rows, count = step.plan(window_plan.planner(num_heads // kv_heads))
+        tiles = step.plan(window_plan.planner(num_heads // kv_heads))
+        row0, rows, count = tiles.rows
         wlib = window_attention_library(k_dim, v_dim)
+        gate_row = gate.stride(0) if gate is not None else 0
+        boxes = _window_boxes(k_pages, v_pages, page_size)
+        wide0, wide, wide_count = tiles.wide
+        tc = (WINDOW_ATTENTION_TC and wide_count and boxes & wlib.tc_forms and scale > 0 and out.stride(0) % 8 == 0
+              and out.data_ptr() % 16 == 0
+              and (gate is None or gate_per_head or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0)))
+        if tc and (wide_count >= TC_ATTENTION_MIN_TILES or getattr(step, "max_position", 0) < TC_ATTENTION_SHORT_CONTEXT):
+            calls["window_attention_tc"] += 1
+            _check(wlib.tis_window_attention_tc(_p(q), q.stride(0), n, _p(gate), gate_row, int(gate_per_head), _p(out), out.stride(0),
+                                                _p(k_pages), kps, _p(v_pages), vps, int(boxes == 2), _p(block_table),
+                                                block_table.stride(0), k_pages.shape[0], _p(positions), _p(row_slot), _p(wide0),
+                                                _p(wide), wide_count, num_heads, kv_heads, page_size, code, _f(scale), _f(cap),
+                                                _p(bias_slope), _p(bias_rate), _p(sink), _p(fault), _stream()), wlib)
+            row0, rows, count = row0[tiles.rows_in_wide:], rows[tiles.rows_in_wide:], count - tiles.rows_in_wide
+            if not count:
+                return out
         calls["window_attention_mma"] += 1
         # a decode step has few tiles, each with many keys to walk: share the keys of a tile out over several CTAs
         # (about two CTAs per SM in all), whose partial results a second launch merges
@@ -1054,7 +1088,7 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
                                       device=q.device)
                 global launches
                 launches += 1
-        _check(wlib.tis_window_attention_mma(_p(q), q.stride(0), _p(gate), gate.stride(0) if gate is not None else 0,
+        _check(wlib.tis_window_attention_mma(_p(q), q.stride(0), _p(gate), gate_row,
                                              _p(out), out.stride(0), _p(k_pages), kps, khs, _p(v_pages), vps, vhs,
                                              _p(block_table), block_table.stride(0), k_pages.shape[0], _p(positions),
                                              _p(row_slot), _p(row0), _p(rows), count, num_heads, kv_heads, page_size,
