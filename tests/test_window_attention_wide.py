@@ -2,7 +2,7 @@
 kernel: long portions on the tcgen05 kernel (csrc/window_attention_tc.cu): widths, shared value rows, windows and chunks, biases
 (also ones that vary by more than the first pass's slack within a tile), sinks, bounds, both gates, portions around the edges of
 a tile of 128 rows behind cached keys, page sizes, requests side by side with single rows, and pages whose unseen rows are not
-finite."""
+finite; the rows of decode steps on the kernel whose key shares are a cluster (csrc/window_attention_decode.cu), likewise."""
 import math
 
 import pytest
@@ -145,6 +145,27 @@ def test_biases(bias, window):
 @pytest.mark.parametrize("K,shared", [(128, False), (192, True)])
 def test_sinks_bounds_and_gates(options, K, shared):
     _check(_run("tc", K, 128, 4, 1, [(130, 200), (0, 70)], 16, shared=shared, **options))
+
+
+# single rows: one key, the edges of a tile of 64 keys, few and many shares of the keys
+ROWS = [[(0, 1), (63, 1), (64, 1), (65, 1), (700, 1)], [(2500, 1)], [(h * 37 % 400, 1) for h in range(40)]]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K,V,H,G,shared", [(128, 128, 12, 3, False), (192, 128, 12, 1, True), (128, 128, 16, 1, True), (64, 128, 4, 2, False),
+                                            (128, 64, 6, 2, False), (256, 128, 4, 4, False), (64, 64, 2, 2, False)])
+@pytest.mark.parametrize("portions", ROWS)
+def test_single_rows(K, V, H, G, shared, portions):
+    _check(_run("decode", K, V, H, G, portions, 16, shared=shared))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("options", [{"sink": True}, {"cap": 3.0}, {"gate": "head", "sink": True}, {"gate": "element", "bias": 0.5},
+                                     {"bias": 30.0}, {"cap": 3.0, "window": -128, "sink": True}, {"window": 1}, {"window": 100},
+                                     {"window": 64, "bias": 0.5}])
+@pytest.mark.parametrize("page", [16, 64, 128])
+def test_single_rows_with_all_they_may_ask_for(options, page):
+    _check(_run("decode", 128, 128, 8, 2, ROWS[0] + [(1500, 1)], page, **options))
 
 
 def test_tiles_cover_the_rows_once():

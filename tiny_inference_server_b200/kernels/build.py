@@ -43,7 +43,7 @@ def _nvcc() -> str:
 #: sources compiled once per head size (-DTIS_HD=<hd>) into libraries of their own
 PER_HEAD_SIZE = ("attention_mma.cu", "attention_tc.cu")
 #: sources compiled once per (key width, value width) (-DTIS_KD=<kd> -DTIS_VD=<vd>)
-PER_WIDTHS = ("window_attention_mma.cu", "window_attention_tc.cu")
+PER_WIDTHS = ("window_attention_mma.cu", "window_attention_tc.cu", "window_attention_decode.cu")
 
 
 def sources():

@@ -990,6 +990,7 @@ def window_attention_library(k_dim: int, v_dim: int):
         if (kd.value, vd.value) != (k_dim, v_dim):
             raise KernelError(f"windowed attention library built for widths {kd.value}/{vd.value}, wanted {k_dim}/{v_dim}")
         lib.tc_forms = int(lib.tis_window_attention_tc_forms())
+        lib.decode_forms = int(lib.tis_window_attention_decode_forms())
         _wattn_libs[(k_dim, v_dim)] = lib
     return lib
 
@@ -1015,6 +1016,11 @@ def window_attention_mma_usable(q: torch.Tensor, gate, out: torch.Tensor, k_page
 #: long portions of prompts run on the tcgen05 kernel where it takes their widths and pages;
 #: TIS_WINDOW_ATTENTION_TC=0 keeps them on the mma.sync kernel
 WINDOW_ATTENTION_TC = os.environ.get("TIS_WINDOW_ATTENTION_TC", "1") != "0"
+
+
+#: decode steps of at most 16 query heads a kv head run on the kernel whose key shares are a cluster, where it takes their
+#: widths and pages; TIS_WINDOW_ATTENTION_DECODE=0 keeps them on the mma.sync kernel
+WINDOW_ATTENTION_DECODE = os.environ.get("TIS_WINDOW_ATTENTION_DECODE", "1") != "0"
 
 
 def _window_boxes(k_pages: torch.Tensor, v_pages: torch.Tensor, page_size: int) -> int:
@@ -1060,6 +1066,21 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
         wlib = window_attention_library(k_dim, v_dim)
         gate_row = gate.stride(0) if gate is not None else 0
         boxes = _window_boxes(k_pages, v_pages, page_size)
+        decode = getattr(step, "decode_only", False) and count > 0
+        keys = 0
+        if decode:
+            keys = step.max_position + 1 if not window else min(int(window), step.max_position + 1)
+        if decode and count == n and boxes & wlib.decode_forms and num_heads // kv_heads <= 16 and WINDOW_ATTENTION_DECODE:
+            # shares of the keys: as many as keep all CTAs resident (two an SM), one cluster at most, a tile of keys each
+            want = min(16, keys // 64 + 1, WINDOW_ATTENTION_CTAS // (count * kv_heads))
+            splits = 1 << max(0, want.bit_length() - 1)
+            calls["window_attention_decode"] += 1
+            _check(wlib.tis_window_attention_decode(_p(q), q.stride(0), _p(gate), gate_row, int(gate_per_head), _p(out), out.stride(0),
+                                                    _p(k_pages), kps, _p(v_pages), vps, int(boxes == 2), _p(block_table),
+                                                    block_table.stride(0), k_pages.shape[0], _p(positions), _p(row_slot), n,
+                                                    num_heads, kv_heads, page_size, code, _f(scale), _f(cap), _p(bias_slope),
+                                                    _p(bias_rate), _p(sink), splits, _p(fault), _stream()), wlib)
+            return out
         wide0, wide, wide_count = tiles.wide
         tc = (WINDOW_ATTENTION_TC and wide_count and boxes & wlib.tc_forms and scale > 0 and out.stride(0) % 8 == 0
               and out.data_ptr() % 16 == 0
@@ -1078,8 +1099,7 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
         # a decode step has few tiles, each with many keys to walk: share the keys of a tile out over several CTAs
         # (about two CTAs per SM in all), whose partial results a second launch merges
         splits, partial = 1, None
-        if getattr(step, "decode_only", False) and count > 0:
-            keys = step.max_position + 1 if not window else min(int(window), step.max_position + 1)
+        if decode:
             key_tiles = keys // 64 + 1
             splits = max(1, min(key_tiles, WINDOW_ATTENTION_CTAS // max(1, count * kv_heads), 64))
             if splits > 1:
