@@ -74,6 +74,63 @@ __device__ __forceinline__ void fill_f32(float* dst, const T* __restrict__ src, 
     }
 }
 
+// What the router makes of a row's logits, by one warp, for at most 32 experts (lane e holds z_e): the choice as described
+// below, step by step as one thread would take it, so that ties and sums come out alike.
+struct RouteForm { int E, groups, keep, top; float weight_eps; int score_kind, group_best, renorm; };
+__device__ __forceinline__ void route_select(float z, const RouteForm& f, const float* __restrict__ corr, int* __restrict__ chosen,
+                                             float* __restrict__ weights) {
+    const int lane = threadIdx.x & 31;
+    const bool expert = lane < f.E;
+    float s = f.score_kind != 0 ? z : 1.f / (1.f + expf(-z));
+    const float c = corr != nullptr && expert ? corr[lane] : 0.f;
+    float pick = corr != nullptr ? s + c : ((f.groups == 0 || f.group_best) ? z : s);
+    if (f.score_kind == 2) {                               // the softmax over all experts
+        const float big = warp_max(expert ? s : -INFINITY);
+        const float part = expert ? expf(s - big) : 0.f;
+        s = part * (1.f / warp_sum(part));
+        if (corr != nullptr) pick = s + c;                 // (else the picks are the logits)
+    }
+    if (f.groups > 0) {
+        const int per = f.E / f.groups, g = min(lane, f.E - 1) / per;
+        float a = -INFINITY, b = -INFINITY;                // the two largest picks of the lane's group
+        for (int i = 0; i < per; ++i) {
+            const float v = __shfl_sync(0xffffffffu, pick, g * per + i);
+            if (v > a) { b = a; a = v; } else if (v > b) b = v;
+        }
+        const float strength = per > 1 && !f.group_best ? a + b : a;
+        int stronger = 0;                                  // groups in front of the lane's
+        for (int h = 0; h < f.groups; ++h) {
+            const float v = __shfl_sync(0xffffffffu, strength, h * per);
+            if (v > strength || (v == strength && h < g)) ++stronger;
+        }
+        if (stronger >= f.keep) pick = -INFINITY;
+    }
+    if (!expert || !(pick > -INFINITY)) pick = -INFINITY;
+    float mine = 0.f, total = 0.f;                         // lane k: the k-th choice's weight
+    int best_mine = 0;
+    for (int k = 0; k < f.top; ++k) {
+        const float big = warp_max(pick);
+        const int best = big > -INFINITY ? __ffs(__ballot_sync(0xffffffffu, pick == big)) - 1 : 0;
+        const float w = __shfl_sync(0xffffffffu, s, best);
+        if (lane == best) pick = -INFINITY;
+        if (lane == k) { mine = w; best_mine = best; }
+        total += w;
+    }
+    if (f.score_kind == 1) {                               // softmax over the chosen logits
+        const float big = warp_max(lane < f.top ? mine : -INFINITY);
+        mine = lane < f.top ? expf(mine - big) : 0.f;
+        total = 0.f;
+        for (int k = 0; k < f.top; ++k) total += __shfl_sync(0xffffffffu, mine, k);
+        mine /= total;
+    } else if (f.renorm) {
+        mine *= 1.f / (total + f.weight_eps);
+    }
+    if (lane < f.top) {
+        chosen[lane] = best_mine;
+        weights[lane] = mine;
+    }
+}
+
 // ------------------------------------------------------------------------------------------------------------
 // The router, a CTA a row:  s = sigmoid(W x) over E experts (W float32 (E, d));  pick = s + correction;  with
 // groups > 0 the experts form that many groups of E / groups neighbours, a group's strength is the sum of its two
@@ -111,6 +168,7 @@ moe_route_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ wr,
         if (lane == 0) {
             for (int j = 0; j < (e1 != e0 ? 2 : 1); ++j) {
                 const int e = j == 0 ? e0 : e1;
+                if (E <= 32 && e < E) { sc[e] = z[j]; continue; }           // the logits, for route_select
                 const float s = (score_kind != 0 && e < E) ? z[j] : 1.f / (1.f + expf(-z[j]));
                 // (without a correction the logits choose: the order is the same, and scores that round to one another keep it)
                 if (e < E) { sc[e] = s; pick[e] = corr != nullptr ? s + corr[e] : ((groups == 0 || group_best) ? z[j] : s); }
@@ -120,6 +178,11 @@ moe_route_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ wr,
     }
     __syncthreads();
     if (warp != 0) return;
+    if (E <= 32) {
+        const RouteForm f = {E, groups, keep, top, weight_eps, score_kind, group_best, renorm};
+        route_select(lane < E ? sc[lane] : 0.f, f, corr, chosen + (size_t)r * top, weights + (size_t)r * top);
+        return;
+    }
     if (score_kind == 2) {                                 // the softmax over all experts, by one warp
         float big = -INFINITY;
         for (int e = lane; e < E; e += 32) big = fmaxf(big, sc[e]);
@@ -184,6 +247,68 @@ moe_route_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ wr,
     if (!renorm) return;
     const float inv = 1.f / (total + weight_eps);
     for (int k = 0; k < top; ++k) weights[(size_t)r * top + k] *= inv;
+}
+
+// The router for few experts (at most ROUTE_DOTS sums a row) and widths of 128 NV: a warp keeps one expert's row of the router's
+// matrix in registers, loaded before the kernel waits for the rows, and takes its sum for every row of the CTA; then every warp
+// chooses for a row.  (A CTA a row with the matrix read anew: 2048 rows of 1536, 16 experts 31 us, 8 rows 16 us; now
+// 15.5 and 6.2 us, cold, under the profiler.)
+// The sums run in the order of the other kernel.
+constexpr int ROUTE_DOTS = 18, ROUTE_ROWS = 16;
+template <typename T, int NV>
+__global__ void __launch_bounds__(32 * ROUTE_DOTS)
+moe_route_rows_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ wr, const float* __restrict__ corr,
+                      const float* __restrict__ w_sg, int n, int rows, const RouteForm f, int* __restrict__ chosen,
+                      float* __restrict__ weights, float* __restrict__ shared_gate) {
+    extern __shared__ __align__(16) unsigned char route_rows[];            // [count][128 NV] the CTA's rows, as they are
+    __shared__ float zs[ROUTE_ROWS][ROUTE_DOTS];
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, dots = blockDim.x >> 5;
+    const int r0 = blockIdx.x * rows, count = min(rows, n - r0);
+    float4 w[NV];
+    const float* mine = (warp < f.E ? wr + (size_t)warp * NV * 128 : w_sg) + lane * 4;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) w[j] = __ldg(reinterpret_cast<const float4*>(mine + j * 128));
+    pdl_wait();
+    constexpr int VECS = NV * 128 * (int)sizeof(T) / 16;   // of a row
+    for (int i = threadIdx.x; i < count * VECS; i += blockDim.x)
+        reinterpret_cast<uint4*>(route_rows)[i] = *reinterpret_cast<const uint4*>(x + (size_t)(r0 + i / VECS) * ldx + i % VECS * (16 / sizeof(T)));
+    __syncthreads();
+    for (int i = 0; i < count; ++i) {
+        const T* at = reinterpret_cast<const T*>(route_rows) + (size_t)i * NV * 128 + lane * 4;
+        float z = 0.f;
+        constexpr int PART = NV <= 12 ? NV : 4;             // of the row, held at a time
+#pragma unroll
+        for (int j0 = 0; j0 < NV; j0 += PART) {
+            if constexpr (sizeof(T) == 4) {
+                float4 v[PART];
+#pragma unroll
+                for (int j = 0; j < PART; ++j) v[j] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(at) + (j0 + j) * 128);
+#pragma unroll
+                for (int j = 0; j < PART; ++j)
+                    z = fmaf(w[j0 + j].w, v[j].w, fmaf(w[j0 + j].z, v[j].z, fmaf(w[j0 + j].y, v[j].y, fmaf(w[j0 + j].x, v[j].x, z))));
+            } else {
+                uint2 v[PART];
+#pragma unroll
+                for (int j = 0; j < PART; ++j) v[j] = *reinterpret_cast<const uint2*>(at + (j0 + j) * 128);
+#pragma unroll
+                for (int j = 0; j < PART; ++j) {
+                    z = fmaf(w[j0 + j].x, __uint_as_float(v[j].x << 16), z);
+                    z = fmaf(w[j0 + j].y, __uint_as_float(v[j].x & 0xffff0000u), z);
+                    z = fmaf(w[j0 + j].z, __uint_as_float(v[j].y << 16), z);
+                    z = fmaf(w[j0 + j].w, __uint_as_float(v[j].y & 0xffff0000u), z);
+                }
+            }
+        }
+        z = warp_sum(z);
+        if (lane == 0) zs[i][warp] = z;
+    }
+    __syncthreads();
+    for (int i = warp; i < count; i += dots) {
+        const int r = r0 + i;
+        if (w_sg != nullptr && lane == 0) shared_gate[r] = 1.f / (1.f + expf(-zs[i][f.E]));
+        route_select(lane < f.E ? zs[i][lane] : 0.f, f, corr, chosen + (size_t)r * f.top, weights + (size_t)r * f.top);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -319,6 +444,30 @@ TIS_API int tis_moe_route(int dtype, const void* x, int ldx, const float* wr, co
         tis_set_error("moe_route: %d experts, top %d, %d groups of which %d kept", E, top, groups, keep);
         return TIS_BAD_SIZE;
     }
+    const int dots = E + (w_sg != nullptr ? 1 : 0);
+    if (dots <= ROUTE_DOTS && ldx % 8 == 0 && ((uintptr_t)x | (uintptr_t)wr | (uintptr_t)w_sg) % 16 == 0) {
+        // as many rows a CTA as spread the step over all SMs once, and fit its shared memory
+        const size_t row_bytes = (size_t)d * (dtype == TIS_BF16 ? 2 : 4);
+        const int fit = (int)(98304 / row_bytes), most = fit < ROUTE_ROWS ? fit : ROUTE_ROWS;
+        const int rows = n < 148 * most ? (n + 147) / 148 : most;
+        const RouteForm f = {E, groups, keep, top, weight_eps, score_kind, group_best, renorm};
+#define TIS_ROUTE(NV)                                                                                                  \
+    if (d == 128 * NV) {                                                                                               \
+        TIS_DISPATCH_DTYPE(dtype, T, {                                                                                 \
+            const int st = set_smem(moe_route_rows_kernel<T, NV>, rows * row_bytes + 4096, "moe_route");  /* zs beside it */ \
+            if (st != TIS_OK) return st;                                                                               \
+            tis_launch(moe_route_rows_kernel<T, NV>, dim3((n + rows - 1) / rows), dim3(32 * dots), rows * row_bytes, stream,  \
+                       (const T*)x, ldx, wr, corr, w_sg, n, rows, f, chosen, weights, shared_gate);                    \
+        });                                                                                                            \
+        return tis_check_launch("moe_route");                                                                          \
+    }
+        TIS_ROUTE(4)
+        TIS_ROUTE(8)
+        TIS_ROUTE(12)
+        TIS_ROUTE(16)
+        TIS_ROUTE(24)
+#undef TIS_ROUTE
+    }
     const size_t smem = sizeof(float) * ((size_t)d + 2 * (size_t)E + (size_t)(groups > 0 ? groups : 1));
     TIS_DISPATCH_DTYPE(dtype, T, {
         const int st = set_smem(moe_route_kernel<T>, smem, "moe_route");
@@ -394,29 +543,52 @@ moe_sort_kernel(const int* __restrict__ chosen, int pairs, int E, int tile_rows,
     pdl_wait();
     for (int i = tid; i < max_rows; i += nthr) sorted_pair[i] = -1;
     __syncthreads();
-    for (int p = tid; p < pairs; p += nthr) {
-        const int e = chosen[p];
-        if (e >= 0 && e < E) atomicAdd(&counts[e], 1);
-    }
+    // pairs of one expert in a warp count together: one atomic addition each, not one a pair on the same few words.  The
+    // first HELD pairs of a thread stay in registers.
+    constexpr int HELD = 8;
+    const int lane = tid & 31, rounds = (pairs + nthr - 1) / nthr;
+    int held[HELD];
+#pragma unroll
+    for (int i = 0; i < HELD; ++i) held[i] = i * nthr + tid < pairs ? chosen[i * nthr + tid] : -1;
+    auto count_in = [&](int e) {
+        const unsigned same = __match_any_sync(0xffffffffu, e);
+        if (e >= 0 && e < E && lane == __ffs(same) - 1) atomicAdd(&counts[e], __popc(same));
+    };
+#pragma unroll
+    for (int i = 0; i < HELD; ++i)
+        if (i < rounds) count_in(held[i]);
+    for (int i = HELD; i < rounds; ++i) count_in(i * nthr + tid < pairs ? chosen[i * nthr + tid] : -1);
     __syncthreads();
     if (tid == 0) {
         int tile = 0;
         for (int e = 0; e < E; ++e) {
             starts[e] = tile * tile_rows;
-            const int tiles = (counts[e] + tile_rows - 1) / tile_rows;
-            for (int t = 0; t < tiles && tile < max_tiles; ++t) tile_expert[tile++] = e;
+            tile += (counts[e] + tile_rows - 1) / tile_rows;
         }
-        for (; tile < max_tiles; ++tile) tile_expert[tile] = -1;
+    }
+    __syncthreads();
+    for (int e = tid; e < E; e += nthr) {
+        const int first = starts[e] / tile_rows, end = min(first + (counts[e] + tile_rows - 1) / tile_rows, max_tiles);
+        for (int t = first; t < end; ++t) tile_expert[t] = e;
+        if (e == E - 1)
+            for (int t = end; t < max_tiles; ++t) tile_expert[t] = -1;
     }
     __syncthreads();
     for (int e = tid; e < E; e += nthr) counts[e] = 0;      // now the next free place of every expert
     __syncthreads();
-    for (int p = tid; p < pairs; p += nthr) {
-        const int e = chosen[p];
-        if (e < 0 || e >= E) { pair_place[p] = -1; continue; }
-        const int place = starts[e] + atomicAdd(&counts[e], 1);
-        if (place < max_rows) { sorted_pair[place] = p; pair_place[p] = place; } else pair_place[p] = -1;
-    }
+    auto place_in = [&](int p, int e) {
+        const unsigned same = __match_any_sync(0xffffffffu, e);
+        const bool ok = e >= 0 && e < E;
+        int place = 0;
+        if (ok && lane == __ffs(same) - 1) place = starts[e] + atomicAdd(&counts[e], __popc(same));
+        place = __shfl_sync(0xffffffffu, place, __ffs(same) - 1) + __popc(same & ((1u << lane) - 1u));
+        if (p >= pairs) return;
+        if (ok && place < max_rows) { sorted_pair[place] = p; pair_place[p] = place; } else pair_place[p] = -1;
+    };
+#pragma unroll
+    for (int i = 0; i < HELD; ++i)
+        if (i < rounds) place_in(i * nthr + tid, held[i]);
+    for (int i = HELD; i < rounds; ++i) place_in(i * nthr + tid, i * nthr + tid < pairs ? chosen[i * nthr + tid] : -1);
 }
 
 __device__ __forceinline__ void g_ldmatrix_x4(unsigned (&r)[4], const void* smem) {
@@ -577,6 +749,47 @@ moe_combine_kernel(const bf16* __restrict__ y, int ldy, const int* __restrict__ 
     }
 }
 
+// The same with 16-byte vectors (widths and row strides that are multiples of eight), the choices' rows loaded four at a time
+// before any is added.  2048 rows of 1536, three choices and a shared unit: 18 -> 13 us (cold).
+__global__ void __launch_bounds__(256)
+moe_combine_vec_kernel(const bf16* __restrict__ y, int ldy, const int* __restrict__ pair_place, const float* __restrict__ weights,
+                       const bf16* __restrict__ shared, int lds, const float* __restrict__ shared_gate, bf16* __restrict__ out,
+                       int n, int d, int top) {
+    pdl_launch_dependents();
+    const int per_row = d / 8;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)n * per_row) return;
+    const int r = (int)(i / per_row), c = (int)(i % per_row) * 8;
+    pdl_wait();
+    float sum[8] = {};
+    float sv[8] = {};
+    const float sg = shared != nullptr ? (shared_gate != nullptr ? shared_gate[r] : 1.f) : 0.f;
+    if (shared != nullptr) Vec16<bf16>::load(shared + (size_t)r * lds + c, sv);
+    for (int k0 = 0; k0 < top; k0 += 4) {
+        float v[4][8], w[4];
+        int place[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            place[j] = k0 + j < top ? pair_place[(size_t)r * top + k0 + j] : -1;
+            w[j] = k0 + j < top && weights != nullptr ? weights[(size_t)r * top + k0 + j] : 1.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (place[j] >= 0) Vec16<bf16>::load(y + (size_t)place[j] * ldy + c, v[j]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (place[j] >= 0) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) sum[e] = fmaf(w[j], v[j][e], sum[e]);
+            }
+    }
+    if (shared != nullptr) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sum[e] = fmaf(sg, sv[e], sum[e]);
+    }
+    Vec16<bf16>::store(out + (size_t)r * d + c, sum);
+}
+
 }  // namespace
 
 // The sort and the weighted sum, for the tile kernels of this file and of moe_tc.cu.
@@ -589,6 +802,11 @@ int tis_moe_sort_launch(const int* chosen, int pairs, int E, int tile_rows, int*
 
 int tis_moe_combine_launch(const void* y, int ldy, const int* pair_place, const float* weights, const void* shared, int lds,
                            const float* shared_gate, void* out, int n, int d, int top, cudaStream_t stream) {
+    if (d % 8 == 0 && ldy % 8 == 0 && (shared == nullptr || lds % 8 == 0) && ((uintptr_t)y | (uintptr_t)shared | (uintptr_t)out) % 16 == 0) {
+        tis_launch(moe_combine_vec_kernel, dim3((unsigned)(((long long)n * (d / 8) + 255) / 256)), dim3(256), 0, stream, (const bf16*)y, ldy,
+                   pair_place, weights, (const bf16*)shared, lds, shared_gate, (bf16*)out, n, d, top);
+        return tis_check_launch("moe_combine");
+    }
     tis_launch(moe_combine_kernel, dim3(n), dim3(256), 0, stream, (const bf16*)y, ldy, pair_place, weights, (const bf16*)shared,
                lds, shared_gate, (bf16*)out, d, top);
     return tis_check_launch("moe_combine");

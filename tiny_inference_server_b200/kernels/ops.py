@@ -1706,6 +1706,10 @@ def bitmap_set(bitmap_row: torch.Tensor, tokens: torch.Tensor) -> None:
     _check(lib.tis_bitmap_set(_p(bitmap_row), _p(tokens), tokens.numel(), _stream()), lib)
 
 
+#: (row, choice) pairs up to which bfloat16 experts run with every chosen expert's matrices streamed once (csrc/moe_few.cu), and
+#: the experts up to which they do (its launches have CTAs for every expert); TIS_MOE_FEW_MAX_PAIRS overrides (0: never)
+MOE_FEW_MAX_PAIRS = int(os.environ.get("TIS_MOE_FEW_MAX_PAIRS", "96"))
+MOE_FEW_MAX_EXPERTS = 128
 #: (token, choice) pairs from which bfloat16 expert products go to the tiles on the tensor cores (rows sorted by expert on
 #: the device) instead of one dot product per output element; TIS_MOE_GROUPED_MIN_PAIRS overrides (0: never)
 MOE_GROUPED_MIN_PAIRS = int(os.environ.get("TIS_MOE_GROUPED_MIN_PAIRS", "96"))
@@ -1724,10 +1728,23 @@ def moe_experts(x: torch.Tensor, chosen: torch.Tensor, weights: torch.Tensor, w_
     float32: ``moe_gate_up`` and ``moe_down`` (a dot product per output element, the weights read where they lie).  Many
     bfloat16 rows: the rows are sorted by expert on the device and every expert's rows run as tiles on the tensor
     cores; nothing is read back, so either way the step can be captured in a graph."""
+    global launches
     n, d = x.shape
     top = chosen.shape[1]
     experts, hidden = w_gate_up.shape[0], w_gate_up.shape[-2]
     act_code = ACTIVATIONS[act] if act is not None else -1
+    if (n * top <= MOE_FEW_MAX_PAIRS and x.dtype == torch.bfloat16 and experts <= MOE_FEW_MAX_EXPERTS and d % 32 == 0 and hidden % 32 == 0
+            and x.stride(1) == 1 and x.stride(0) % 8 == 0 and (x.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0
+            and (shared is None or shared.stride(1) == 1)):
+        lib = library()
+        hid = torch.empty((n * top, hidden), dtype=x.dtype, device=x.device)
+        out = torch.empty((n, d), dtype=x.dtype, device=x.device)
+        calls["moe_few"] += 1
+        launches += 1
+        _check(lib.tis_moe_few(_p(x), x.stride(0), _p(chosen), _p(weights), _p(w_gate_up), _p(w_down), _p(shared),
+                               shared.stride(0) if shared is not None else 0, _p(shared_gate), _p(out), _p(hid), n, d, top, experts,
+                               hidden, act_code, form, int(weigh_input), _stream()), lib)
+        return out
     grouped = (x.dtype == torch.bfloat16 and MOE_GROUPED_MIN_PAIRS > 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
                and x.data_ptr() % 16 == 0 and (shared is None or (shared.stride(1) == 1 and shared.stride(0) % 2 == 0)))
     if grouped and MOE_TC_MIN_PAIRS > 0 and n * top >= MOE_TC_MIN_PAIRS and d % 64 == 0 and hidden % 64 == 0:
@@ -1742,7 +1759,6 @@ def moe_experts(x: torch.Tensor, chosen: torch.Tensor, weights: torch.Tensor, w_
         y = torch.empty((tiles * 128, d), dtype=x.dtype, device=dev)
         out = torch.empty((n, d), dtype=x.dtype, device=dev)
         calls["moe_grouped_tc"] += 1
-        global launches
         launches += 4
         _check(lib.tis_moe_grouped_tc(_p(x), x.stride(0), _p(chosen), _p(weights), _p(w_gate_up), _p(w_down), _p(shared),
                                       shared.stride(0) if shared is not None else 0, _p(shared_gate), _p(out), _p(sorted_pair),
