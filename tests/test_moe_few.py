@@ -40,11 +40,12 @@ def _experts(n, d, F, E, top, act=None, weigh=False, shared=False, chosen=None, 
     xc.copy_(x)
     keep, ops.MOE_FEW_MAX_PAIRS = ops.MOE_FEW_MAX_PAIRS, 384 if few else 0
     grouped, ops.MOE_GROUPED_MIN_PAIRS = ops.MOE_GROUPED_MIN_PAIRS, 0
+    many, ops.MOE_FEW_MAX_EXPERTS = ops.MOE_FEW_MAX_EXPERTS, 128
     before = ops.calls["moe_few"]
     try:
         got = ops.moe_experts(xc, c(chosen).int(), c(w), c(gu), c(down), c(sh), c(sg) if shared else None, act=act, weigh_input=weigh)
     finally:
-        ops.MOE_FEW_MAX_PAIRS, ops.MOE_GROUPED_MIN_PAIRS = keep, grouped
+        ops.MOE_FEW_MAX_PAIRS, ops.MOE_GROUPED_MIN_PAIRS, ops.MOE_FEW_MAX_EXPERTS = keep, grouped, many
     assert ops.calls["moe_few"] - before == int(few)
     return float((got.double().cpu() - want).norm() / want.norm())
 
@@ -55,7 +56,7 @@ def _check(*args, **options):
     assert few < 4e-3 and few < 1.1 * dots + 1e-4, (few, dots)
 
 
-@pytest.mark.parametrize("n,d,F,E,top", [(1, 64, 32, 4, 2), (8, 1536, 1024, 16, 3), (31, 96, 160, 5, 3), (33, 160, 64, 40, 1), (96, 128, 96, 7, 4)])
+@pytest.mark.parametrize("n,d,F,E,top", [(1, 64, 32, 4, 2), (8, 1536, 1024, 16, 3), (3, 768, 64, 70, 5), (5, 2400, 96, 9, 2), (31, 96, 160, 5, 3), (33, 160, 64, 40, 1), (96, 128, 96, 7, 4)])
 @pytest.mark.parametrize("options", [{}, {"act": "relu2"}, {"weigh": True, "shared": True}])
 def test_few_rows(n, d, F, E, top, options):
     _check(n, d, F, E, top, **options)
@@ -89,9 +90,9 @@ def test_router_with_its_matrix_in_registers(dtype, d, E, top, groups, keep, sco
         assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("n,d,F,E,top", [(400, 192, 64, 6, 3), (350, 200, 64, 6, 5)])
+@pytest.mark.parametrize("n,d,F,E,top", [(400, 192, 64, 6, 3), (350, 200, 64, 6, 5), (33, 512, 64, 6, 3), (40, 576, 128, 32, 4)])
 def test_many_rows_sorted_and_summed(n, d, F, E, top):
-    """Widths of whole vectors and not, choices of four and more a row, through the sorted path."""
+    """Widths of whole vectors and not, choices of four and more a row, through the sorted path; from width 512 with few pairs too."""
     from tiny_inference_server_b200.kernels import ops
     import kernel_refs as ref
     gen = torch.Generator().manual_seed(d)
@@ -100,5 +101,7 @@ def test_many_rows_sorted_and_summed(n, d, F, E, top):
     chosen = torch.stack([torch.randperm(E, generator=gen)[:top] for _ in range(n)]).int()
     w, sg = torch.rand(n, top, generator=gen), torch.rand(n, generator=gen)
     want = ref.moe_experts(x, chosen, w, gu, down, sh, sg).double()
+    before = ops.calls["moe_grouped_tc"]
     got = ops.moe_experts(x.cuda(), chosen.cuda(), w.cuda(), gu.cuda(), down.cuda(), sh.cuda(), sg.cuda()).double().cpu()
+    assert ops.calls["moe_grouped_tc"] - before == int(d % 64 == 0)
     assert float((got - want).norm() / want.norm()) < 8e-3

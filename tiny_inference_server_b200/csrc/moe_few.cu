@@ -5,15 +5,14 @@
 // rows of an mma.sync tile and up to 32 (row, choice) pairs of the expert its columns.  The summed index may run in any order
 // that both operands agree on: a lane's 16 bytes of a matrix row (eight neighbouring elements) are its share of two products,
 // and the same eight elements of its column's input row, so both come from global memory in 16-byte loads, as they lie.
-// 8 rows of 1536, 16 experts of 1024 hidden elements, 3 a row: 25 + 21 us before, 21 + 23 us now (cold, under the profiler); inside
-// the layer, with the router below, 72 -> 67 us.  More rows share an expert's bytes, where before each read them again.
+// 8 rows of 1536, 16 experts of 1024 hidden elements, 3 a row: 25 + 21 us before, 21 + 23 us now (cold, under the profiler).  More rows share an expert's bytes, where before each read them again.
 #include "common.cuh"
 
 namespace {
 
 constexpr int FEATURES = 16;             // matrix rows of a tile
 constexpr int GROUPS = 4;                // column groups of eight pairs that one pass over a matrix serves
-constexpr int FIRST_WARPS = 4, SECOND_WARPS = 16, SHARES = 4;
+constexpr int FIRST_WARPS = 4, SHARES = 4;
 
 __device__ __forceinline__ void mma_few(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -22,6 +21,15 @@ __device__ __forceinline__ void mma_few(float (&c)[4], unsigned a0, unsigned a1,
 __device__ __forceinline__ uint4 load_once(const bf16* p) {
     uint4 v;
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ float cluster_read(const float* mine, int rank) {
+    unsigned at;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(mine)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(at) : "memory");
     return v;
 }
 __device__ __forceinline__ float few_act(float x, int kind) {
@@ -137,60 +145,79 @@ moe_few_first_kernel(const bf16* __restrict__ x, int ldx, const int* __restrict_
     }
 }
 
-// out[r][c] = sum_k weights[r][k] * (Wd[e_k][c] . hidden[r * top + k]) (+ shared_gate[r] * shared[r][c]).  A CTA per 16 output
-// columns and all experts: its warps take (expert, quarter of the sum) in turn and leave the pairs' results in shared memory.
-__global__ void __launch_bounds__(SECOND_WARPS * 32)
+// out[r][c] = sum_k weights[r][k] * (Wd[e_k][c] . hidden[r * top + k]) (+ shared_gate[r] * shared[r][c]).  A cluster of 1, 2 or 4 CTAs
+// per 16 output columns takes the chosen experts in turn, four warps an expert, a quarter of the sum each, and leaves the pairs'
+// results in its CTAs' shared memory, where they are added up in the order of the choices whatever the size of the cluster.
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
 moe_few_second_kernel(const bf16* __restrict__ hidden, const int* __restrict__ chosen, const float* __restrict__ weights, int pairs, int top,
                       const bf16* __restrict__ w, const bf16* __restrict__ shared, int lds, const float* __restrict__ shared_gate,
-                      bf16* __restrict__ out, int d, int E, int F) {
+                      bf16* __restrict__ out, int d, int E, int F, int ctas) {
     extern __shared__ __align__(16) float smem[];
     float* part = smem;                                     // [SHARES][pairs][FEATURES]
     int* all = reinterpret_cast<int*>(part + (size_t)SHARES * pairs * FEATURES);        // [pairs] the choices
     int* list = all + pairs + (threadIdx.x >> 5) * pairs;   // [pairs] a warp's own
+    unsigned* met = reinterpret_cast<unsigned*>(all + (WARPS + 1) * pairs);      // [E / 32] a bit for each chosen expert
     pdl_launch_dependents();
-    const int c0 = blockIdx.x * FEATURES;
+    const int rank = blockIdx.x % ctas, c0 = blockIdx.x / ctas * FEATURES;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fc = lane & 3;
-    const int blocks = F / 32;
-    pdl_wait();
-    for (int i = tid; i < pairs; i += SECOND_WARPS * 32) all[i] = chosen[i];
+    const int blocks = F / 32, words = (E + 31) / 32, share = warp % SHARES;
+    for (int i = tid; i < words; i += WARPS * 32) met[i] = 0;
     __syncthreads();
-    for (int task = warp; task < E * SHARES; task += SECOND_WARPS) {
-        const int e = task / SHARES, share = task % SHARES;
-        const int count = pairs_of(all, pairs, e, list);
-        for (int p0 = 0; p0 < count; p0 += 8 * GROUPS) {
-            const int groups = min(GROUPS, (count - p0 + 7) / 8);
-            const bf16* const wm[1] = {w + ((size_t)e * d + c0 + fr) * F + fc * 8};
-            const bf16* xg[GROUPS];
-#pragma unroll
-            for (int g = 0; g < GROUPS; ++g) xg[g] = hidden + (size_t)list[min(p0 + 8 * g + fr, count - 1)] * F + fc * 8;
-            float acc[1][GROUPS][4] = {};
-            stream<1>(wm, (size_t)8 * F, xg, groups, blocks * share / SHARES, blocks * (share + 1) / SHARES, acc);
-#pragma unroll
-            for (int g = 0; g < GROUPS; ++g)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int k = p0 + 8 * g + 2 * fc + (i & 1);
-                    if (g < groups && k < count) part[((size_t)share * pairs + list[k]) * FEATURES + fr + (i >> 1) * 8] = acc[0][g][i];
-                }
-        }
-        __syncwarp();                                       // the list is written anew
+    pdl_wait();
+    for (int i = tid; i < pairs; i += WARPS * 32) {
+        const int e = chosen[i];
+        all[i] = e;
+        if (e >= 0 && e < E) atomicOr(&met[e >> 5], 1u << (e & 31));
     }
     __syncthreads();
-    for (int i = tid; i < pairs / top * FEATURES; i += SECOND_WARPS * 32) {
+    int turn = 0;                                           // chosen experts passed so far
+    for (int word = 0; word < words; ++word)
+        for (unsigned left = met[word]; left != 0; left &= left - 1, ++turn) {
+            if (turn % ctas != rank || turn / ctas % (WARPS / SHARES) != warp / SHARES) continue;
+            const int e = word * 32 + __ffs(left) - 1;
+            const int count = pairs_of(all, pairs, e, list);
+            for (int p0 = 0; p0 < count; p0 += 8 * GROUPS) {
+                const int groups = min(GROUPS, (count - p0 + 7) / 8);
+                const bf16* const wm[1] = {w + ((size_t)e * d + c0 + fr) * F + fc * 8};
+                const bf16* xg[GROUPS];
+#pragma unroll
+                for (int g = 0; g < GROUPS; ++g) xg[g] = hidden + (size_t)list[min(p0 + 8 * g + fr, count - 1)] * F + fc * 8;
+                float acc[1][GROUPS][4] = {};
+                stream<1>(wm, (size_t)8 * F, xg, groups, blocks * share / SHARES, blocks * (share + 1) / SHARES, acc);
+#pragma unroll
+                for (int g = 0; g < GROUPS; ++g)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int k = p0 + 8 * g + 2 * fc + (i & 1);
+                        if (g < groups && k < count) part[((size_t)share * pairs + list[k]) * FEATURES + fr + (i >> 1) * 8] = acc[0][g][i];
+                    }
+            }
+            __syncwarp();                                   // the list is written anew
+        }
+    if (ctas > 1) { cluster_arrive(); cluster_wait(); } else __syncthreads();
+    for (int i = rank * WARPS * 32 + tid; i < pairs / top * FEATURES; i += ctas * WARPS * 32) {
         const int r = i / FEATURES, c = i % FEATURES;
         float acc = 0.f;
         for (int k = 0; k < top; ++k) {
             const int pair = r * top + k, e = all[pair];
             if (e < 0 || e >= E) continue;
+            int home = __popc(met[e >> 5] & ((1u << (e & 31)) - 1u));        // the expert's turn, and with it its CTA
+            for (int word = 0; word < e >> 5; ++word) home += __popc(met[word]);
+            home %= ctas;
             float v = 0.f;
 #pragma unroll
-            for (int s = 0; s < SHARES; ++s) v += part[((size_t)s * pairs + pair) * FEATURES + c];
+            for (int s = 0; s < SHARES; ++s) {
+                const float* at = part + ((size_t)s * pairs + pair) * FEATURES + c;
+                v += ctas > 1 ? cluster_read(at, home) : *at;
+            }
             acc = fmaf(weights != nullptr ? weights[pair] : 1.f, v, acc);
         }
         if (shared != nullptr)
             acc = fmaf(shared_gate != nullptr ? shared_gate[r] : 1.f, __bfloat162float(shared[(size_t)r * lds + c0 + c]), acc);
         out[(size_t)r * d + c0 + c] = __float2bfloat16_rn(acc);
     }
+    if (ctas > 1) { cluster_arrive(); cluster_wait(); }     // no CTA leaves while a neighbour reads its shared memory
 }
 
 }  // namespace
@@ -215,10 +242,33 @@ TIS_API int tis_moe_few(const void* x, int ldx, const int* chosen, const float* 
                (int)pairs, top, (const bf16*)w_gu, (bf16*)hidden, d, F, act, gate, in_weights);
     const int st = tis_check_launch("moe_few_first");
     if (st != TIS_OK) return st;
-    const size_t smem = (sizeof(float) * SHARES * FEATURES + sizeof(int) * (SECOND_WARPS + 1)) * (size_t)pairs;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(moe_few_second_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    tis_launch(moe_few_second_kernel, dim3(d / FEATURES), dim3(SECOND_WARPS * 32), smem, stream, (const bf16*)hidden, chosen,
-               weigh_input ? (const float*)nullptr : weights, (int)pairs, top, (const bf16*)w_down, (const bf16*)shared, lds, shared_gate,
-               (bf16*)out, d, E, F);
+    // Columns for fewer groups than SMs: 16 warps a CTA, one CTA an SM, and clusters of as many as the SMs hold.  For more: 8 warps, two
+    // CTAs an SM (a second wave of a few CTAs would cost as much as the first).  us a layer, 64 experts of 512, width 1024, 4 rows of 6:
+    // 37 alone, 29 as pairs, 40 as fours; 16 of 256, width 512, 32 rows of 3: 17.4, 14.6, 12.9; 16 of 1408, width 2048, 8 rows: 59, 64, 74;
+    // 16 of 2048, width 3072, 4 rows: 99 with 16 warps a CTA, 87 with 8.
+    const int columns = d / FEATURES, sms = 148;
+    const int warps = columns <= sms ? 16 : 8, ctas = columns * 4 <= sms ? 4 : columns * 2 <= sms ? 2 : 1;
+    auto second = warps == 16 ? moe_few_second_kernel<16> : moe_few_second_kernel<8>;
+    const size_t smem = (sizeof(float) * SHARES * FEATURES + sizeof(int) * (warps + 1)) * (size_t)pairs + (size_t)(E + 31) / 32 * 4;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(second, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(columns * ctas);
+    cfg.blockDim = dim3(warps * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int attrs = 0;
+    if (ctas > 1) {
+        attr[attrs].id = cudaLaunchAttributeClusterDimension;
+        attr[attrs].val.clusterDim.x = ctas; attr[attrs].val.clusterDim.y = 1; attr[attrs++].val.clusterDim.z = 1;
+    }
+    if (tis_pdl_enabled()) {
+        attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = attrs;
+    cudaLaunchKernelEx(&cfg, second, (const bf16*)hidden, chosen, weigh_input ? (const float*)nullptr : weights, (int)pairs, top,
+                       (const bf16*)w_down, (const bf16*)shared, lds, shared_gate, (bf16*)out, d, E, F, ctas);
     return tis_check_launch("moe_few_second");
 }

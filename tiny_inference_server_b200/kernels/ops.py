@@ -1706,16 +1706,27 @@ def bitmap_set(bitmap_row: torch.Tensor, tokens: torch.Tensor) -> None:
     _check(lib.tis_bitmap_set(_p(bitmap_row), _p(tokens), tokens.numel(), _stream()), lib)
 
 
-#: (row, choice) pairs up to which bfloat16 experts run with every chosen expert's matrices streamed once (csrc/moe_few.cu), and
-#: the experts up to which they do (its launches have CTAs for every expert); TIS_MOE_FEW_MAX_PAIRS overrides (0: never)
+#: (row, choice) pairs up to which bfloat16 experts run with every chosen expert's matrices streamed once (csrc/moe_few.cu);
+#: TIS_MOE_FEW_MAX_PAIRS overrides (0: never).  us, 16 experts of 1024, width 1536, 3 a row, against a dot product per element: 1 row
+#: 22 -> 15, 8 rows 43 -> 42, 16 rows 66 -> 46, 31 rows 103 -> 47; experts of 2048, width 3072: 4 rows 87 -> 87, 16 rows 191 -> 146
 MOE_FEW_MAX_PAIRS = int(os.environ.get("TIS_MOE_FEW_MAX_PAIRS", "96"))
-MOE_FEW_MAX_EXPERTS = 128
+#: the experts, and the width, up to which they always do; beyond either, one row of 128 experts at most, and three
+#: pairs an expert or more: between these
+#: rows seldom share an expert, and a dot product per pair spreads better (32 experts of 768, width 2048, 4 a row: 1 row 25 -> 18 us,
+#: but 8 rows 50 -> 56; 24 rows 121 -> 78; 8 of 2048, width 4096, 2 a row: 4 rows 70 -> 75, 16 rows 206 -> 91)
+MOE_FEW_MAX_EXPERTS, MOE_FEW_MAX_WIDTH = 16, 3072
 #: (token, choice) pairs from which bfloat16 expert products go to the tiles on the tensor cores (rows sorted by expert on
 #: the device) instead of one dot product per output element; TIS_MOE_GROUPED_MIN_PAIRS overrides (0: never)
 MOE_GROUPED_MIN_PAIRS = int(os.environ.get("TIS_MOE_GROUPED_MIN_PAIRS", "96"))
 #: pairs from which they go to the tcgen05 kernel (tiles of 128 rows, TMA-fed, accumulator in tensor memory) where width and
 #: hidden size are multiples of 64; TIS_MOE_TC_MIN_PAIRS overrides (0: never)
 MOE_TC_MIN_PAIRS = int(os.environ.get("TIS_MOE_TC_MIN_PAIRS", "1024"))
+#: the same for the width MOE_TC_WIDE and more, up to MOE_TC_WIDE_MAX_EXPERTS experts: the mma.sync tiles walk the width with few CTAs in
+#: flight, TMA keeps more of it on its way.  us, 16 experts: 1024 of width 1536, 128 rows 110 -> 57; 2048 of 3072, 64 rows 208 -> 127;
+#: 256 of 512, 40 rows 33 -> 22.5; 128 of 256, 40 rows 19.7 -> 20.1
+#: (hence the width); 128 experts of 512, width 1024, 12 rows of 8: 90 -> 101 (hence the experts)
+MOE_TC_WIDE_MIN_PAIRS = int(os.environ.get("TIS_MOE_TC_WIDE_MIN_PAIRS", "96"))
+MOE_TC_WIDE, MOE_TC_WIDE_MAX_EXPERTS = 512, 32
 
 
 def moe_experts(x: torch.Tensor, chosen: torch.Tensor, weights: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor,
@@ -1724,16 +1735,18 @@ def moe_experts(x: torch.Tensor, chosen: torch.Tensor, weights: torch.Tensor, w_
     """``out[r] = sum_k weights[r, k] * unit(chosen[r, k])(x[r]) (+ shared_gate[r] * shared[r], or + shared[r])`` with the gated
     units ``unit(e)(x) = Wd[e] gated(Wg[e] x, Wu[e] x)`` in the form ``form``: ``w_gate_up`` (E, 2, F, d), ``w_down`` (E, d, F); or, with ``act``
     (``ACTIVATIONS``), units without a gate, ``Wd[e] act(Wu[e] x)`` and ``w_gate_up`` (E, F, d).  ``weigh_input``: ``sum_k unit(chosen[r, k])(weights[r, k] *
-    x[r])`` instead (the weight multiplies both projections of the unit in 32-bit).  Few rows, and
-    float32: ``moe_gate_up`` and ``moe_down`` (a dot product per output element, the weights read where they lie).  Many
-    bfloat16 rows: the rows are sorted by expert on the device and every expert's rows run as tiles on the tensor
-    cores; nothing is read back, so either way the step can be captured in a graph."""
+    x[r])`` instead (the weight multiplies both projections of the unit in 32-bit).  Few
+    bfloat16 rows: every chosen expert's matrices are streamed once, its rows the columns of tensor-core tiles.  Few rows of
+    many experts, and float32: ``moe_gate_up`` and ``moe_down`` (a dot product per output element, the weights read where they lie).
+    Many bfloat16 rows: the rows are sorted by expert on the device and every expert's rows run as tiles on the tensor
+    cores.  Nothing is read back, so either way the step can be captured in a graph."""
     global launches
     n, d = x.shape
     top = chosen.shape[1]
     experts, hidden = w_gate_up.shape[0], w_gate_up.shape[-2]
     act_code = ACTIVATIONS[act] if act is not None else -1
-    if (n * top <= MOE_FEW_MAX_PAIRS and x.dtype == torch.bfloat16 and experts <= MOE_FEW_MAX_EXPERTS and d % 32 == 0 and hidden % 32 == 0
+    streamed = (experts <= MOE_FEW_MAX_EXPERTS and d <= MOE_FEW_MAX_WIDTH) or (n == 1 and experts <= 128) or n * top >= 3 * experts
+    if (n * top <= MOE_FEW_MAX_PAIRS and x.dtype == torch.bfloat16 and streamed and d % 32 == 0 and hidden % 32 == 0
             and x.stride(1) == 1 and x.stride(0) % 8 == 0 and (x.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0
             and (shared is None or shared.stride(1) == 1)):
         lib = library()
@@ -1747,7 +1760,9 @@ def moe_experts(x: torch.Tensor, chosen: torch.Tensor, weights: torch.Tensor, w_
         return out
     grouped = (x.dtype == torch.bfloat16 and MOE_GROUPED_MIN_PAIRS > 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
                and x.data_ptr() % 16 == 0 and (shared is None or (shared.stride(1) == 1 and shared.stride(0) % 2 == 0)))
-    if grouped and MOE_TC_MIN_PAIRS > 0 and n * top >= MOE_TC_MIN_PAIRS and d % 64 == 0 and hidden % 64 == 0:
+    wide = d >= MOE_TC_WIDE and experts <= MOE_TC_WIDE_MAX_EXPERTS
+    tc_from = min(MOE_TC_MIN_PAIRS, MOE_TC_WIDE_MIN_PAIRS) if wide else MOE_TC_MIN_PAIRS
+    if grouped and MOE_TC_MIN_PAIRS > 0 and n * top >= tc_from and d % 64 == 0 and hidden % 64 == 0:
         # many rows: 128-row tiles on the tcgen05 tensor cores, the stacked weights as TMA boxes where they lie
         lib = library()
         tiles = lib.tis_moe_tc_tiles(n * top, experts)
