@@ -11,6 +11,13 @@ import torch
 F64 = torch.float64
 
 
+@pytest.fixture(autouse=True)
+def steps_of_any_size(monkeypatch):
+    """The tcgen05 kernel also where a step's work is too small for it to pay."""
+    from tiny_inference_server_b200.kernels import ops
+    monkeypatch.setattr(ops, "WINDOW_ATTENTION_TC_MIN_WORK", 0)
+
+
 class _Step:
     def __init__(self, pos, slot, decode_only):
         self.positions, self.row_slot, self.max_position, self.decode_only = pos, slot, int(pos.max()), decode_only

@@ -1016,6 +1016,11 @@ def window_attention_mma_usable(q: torch.Tensor, gate, out: torch.Tensor, k_page
 #: long portions of prompts run on the tcgen05 kernel where it takes their widths and pages;
 #: TIS_WINDOW_ATTENTION_TC=0 keeps them on the mma.sync kernel
 WINDOW_ATTENTION_TC = os.environ.get("TIS_WINDOW_ATTENTION_TC", "1") != "0"
+#: (rows * keys a row can see * query heads) of a step from which they do.  Below, a layer takes the host longer than the device,
+#: and the kernel's tensor maps, and a second launch for the short portions, cost more there than the device gains: 1200 rows in three
+#: prompts, 12 heads, 96 us a layer with the mma.sync kernel, 103 with this one, 154 rows in two 97 and 113; 2048 rows at a window
+#: of 1024 177 and 105 us
+WINDOW_ATTENTION_TC_MIN_WORK = 1 << 24
 
 
 #: decode steps of at most 16 query heads a kv head run on the kernel whose key shares are a cluster, where it takes their
@@ -1023,15 +1028,14 @@ WINDOW_ATTENTION_TC = os.environ.get("TIS_WINDOW_ATTENTION_TC", "1") != "0"
 WINDOW_ATTENTION_DECODE = os.environ.get("TIS_WINDOW_ATTENTION_DECODE", "1") != "0"
 
 
-def _window_boxes(k_pages: torch.Tensor, v_pages: torch.Tensor, page_size: int) -> int:
+def _window_boxes(page_size: int, heads: int, k_dim: int, v_dim: int, k_strides, v_strides, same_start: bool) -> int:
     """Whether key and value rows can be read in boxes of whole pages: 0 no; 1 yes; 2 yes, and the values are the first elements
-    of the key rows."""
-    heads, k_dim, v_dim = k_pages.shape[1], k_pages.shape[3], v_pages.shape[3]
-    if page_size not in (16, 32, 64, 128) or not (heads == 1 or k_pages.stride(1) == page_size * k_dim):
+    of the key rows.  ``*_strides``: page, head and row strides as ``_page_strides`` gave them."""
+    if page_size not in (16, 32, 64, 128) or not (heads == 1 or k_strides[1] == page_size * k_dim):
         return 0
-    if v_pages.data_ptr() == k_pages.data_ptr() and v_pages.stride() == k_pages.stride():
+    if same_start and k_strides == v_strides:
         return 2
-    return int(v_pages.stride(2) == v_dim and (heads == 1 or v_pages.stride(1) == page_size * v_dim))
+    return int(v_strides[2] == v_dim and (heads == 1 or v_strides[1] == page_size * v_dim))
 
 
 def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor, k_pages: torch.Tensor,
@@ -1065,7 +1069,8 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
         row0, rows, count = tiles.rows
         wlib = window_attention_library(k_dim, v_dim)
         gate_row = gate.stride(0) if gate is not None else 0
-        boxes = _window_boxes(k_pages, v_pages, page_size)
+        boxes = _window_boxes(page_size, kv_heads, k_dim, v_dim, (kps.value, khs.value, k_dim), (vps.value, vhs.value, v_row),
+                              k_pages.data_ptr() == v_pages.data_ptr())
         decode = getattr(step, "decode_only", False) and count > 0
         keys = 0
         if decode:
@@ -1085,6 +1090,8 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
         tc = (WINDOW_ATTENTION_TC and wide_count and boxes & wlib.tc_forms and scale > 0 and out.stride(0) % 8 == 0
               and out.data_ptr() % 16 == 0
               and (gate is None or gate_per_head or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0)))
+        reach = getattr(step, "max_position", 0) + 1
+        tc = tc and n * (min(int(window), reach) if window else reach) * num_heads >= WINDOW_ATTENTION_TC_MIN_WORK
         if tc and (wide_count >= TC_ATTENTION_MIN_TILES or getattr(step, "max_position", 0) < TC_ATTENTION_SHORT_CONTEXT):
             calls["window_attention_tc"] += 1
             _check(wlib.tis_window_attention_tc(_p(q), q.stride(0), n, _p(gate), gate_row, int(gate_per_head), _p(out), out.stride(0),
