@@ -271,6 +271,9 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                         *reinterpret_cast<uint4*>(pg_smem + r * 128 + (c >> 3) * HALF_BYTES + ((c & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
                     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 }
+                // it follows every phase of o_done all the same: a wait for the last one alone could return a phase early (the
+                // parity of the phase before the one before), and the merge below writes where P lies
+                if (i > 0 && !__all_sync(0xffffffffu, mbar_wait(&o_done[g], (i - 1) & 1, abort, p.fault, 6))) { ok = false; break; }
                 fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&p_full[g]);
