@@ -20,10 +20,15 @@
 // Every product of decays is a product of factors <= 1 in the direction the tokens run (within sub-chunks of 16 tokens,
 // over whole sub-chunks between them): nothing is divided by a decay, so a decay of zero and a long product that
 // underflows are what they are in the walk.  No token's output meets a later token's vectors, not even times zero.
-// Operands, states and sums are 32-bit.  The dense products run on the tensor cores as three tf32 products of operands
-// split in two (x = hi + lo: lo hi + hi lo + hi hi; what is left out is 2^-22 of a product): the CUDA cores read a word
-// from shared memory for every one to four multiply-adds, and at a quarter of their rate that is what the first form of
-// these kernels spent its time on (delta rule, 2048 tokens, 12 heads of 128 x 128: 135 + 113 + 51 us; now 80 + 99 + 41).
+// Operands, states and sums are 32-bit, with 32-bit and with bfloat16 activations alike: the state goes on from step to step
+// whatever the activations are.  The dense products run on the tensor cores as bfloat16 products of operands split in
+// three, whose parts hold all 24 bits (mma_split); products of decays are kept as sums of two numbers until they are used.
+// Against the walk in 64 bits (2-norms of the difference over the result, five shapes of 128 to 2048 tokens, both
+// activations): states 0.5 to 1.05 times as far off as token by token in 32 bits, 32-bit outputs 0.87 to 1.0 times.
+// Three tf32 products of operands split in two (2^-22 left out) cost the same tensor time and were 1.1 to 1.7 times as far
+// off, with sums left to the tensor cores, which truncate, up to 6.5 times.  On the CUDA cores, which read a word from
+// shared memory for every one to four multiply-adds, the kernels took longer (delta rule, 2048 tokens, 12 heads of 128 x 128,
+// a layer: 422 us; 271 in tf32, 311 now).
 // Straight-line code is kept short: a kernel's code is read anew at every launch, and unrolled over a chunk's tokens the
 // exponentials of the preparation took longer to fetch than to run.  A product of a masked zero and a number that is not finite would not be zero: blocks on the diagonal look at their operands first.
 #include "recurrence.cuh"
@@ -74,56 +79,71 @@ template <int N> __device__ __forceinline__ void store_run(bf16* p, const float 
     else *reinterpret_cast<__nv_bfloat162*>(p) = h[0];
 }
 
-// ---- products of 16 x 8 (x 8) tiles in three tf32 products; lane = 4 r + c holds rows r, r + 8 and columns c, c + 4 of A
-// (16 x 8), rows c, c + 4 of column r of B (8 x 8), columns 2 c, 2 c + 1 of rows r, r + 8 of the sum.  The order of the
-// summed index is free as long as A and B agree: where it suits the layout, c and c + 4 stand for tokens 2 c and 2 c + 1.
-// EXACT (32-bit activations): lo is rounded as well, and the sums of every step are added up outside the tensor cores,
-// whose own additions truncate; against 64 bits the products are then no further off than the CUDA
-// cores' (measured at 777 rows, state: 7.1e-7 of its norm before, 1.1e-6 with three truncating products).
-template <bool EXACT> __device__ __forceinline__ void split_tf32(float x, unsigned& hi, unsigned& lo) {
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
-    const float rest = x - __uint_as_float(hi);
-    if (EXACT) asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(rest));
-    else lo = __float_as_uint(rest);
+// ---- products of 16 x 16 (x 8) tiles of 32-bit operands in six bfloat16 products.  An operand is the sum of three bfloat16
+// numbers (8 + 8 + 8 bits: all of its 24), x = h + m + l; what is left out of a product (m l, l m, l l) is below 2^-26 of it.
+// Lane = 4 r + c holds rows r, r + 8 of A (16 x 16) in four columns, column r of B (16 x 8) in the same four, and columns 2 c,
+// 2 c + 1 of rows r, r + 8 of the sum.  Which four of the sixteen summed indices is free as long as A and B agree.
+// The tensor cores truncate what they add up.  So the sums of every step are added outside, and the large product runs a
+// second time with its own rounded sum to be taken off: what the rounding lost, to which the small products are added.
+// (A step's sum against 64 bits: 4.8e-8 of its norm with a bias of -3.9e-8 in one chain, 0.7e-8 without a bias so.)
+__device__ __forceinline__ void split_pair(float x, float y, unsigned& h, unsigned& m, unsigned& l) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(y), "f"(x));
+    x -= __uint_as_float(h << 16); y -= __uint_as_float(h & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(m) : "f"(y), "f"(x));
+    x -= __uint_as_float(m << 16); y -= __uint_as_float(m & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(l) : "f"(y), "f"(x));
 }
-template <bool EXACT> struct FragA {
-    unsigned hi[4], lo[4];
-    __device__ __forceinline__ void set(float a0, float a1, float a2, float a3) {
-        split_tf32<EXACT>(a0, hi[0], lo[0]); split_tf32<EXACT>(a1, hi[1], lo[1]);
-        split_tf32<EXACT>(a2, hi[2], lo[2]); split_tf32<EXACT>(a3, hi[3], lo[3]);
+struct FragA {
+    unsigned h[4], m[4], l[4];
+    // (row r, row r + 8) of the lane's first index, then of its second, third and fourth
+    __device__ __forceinline__ void set(float a0, float b0, float a1, float b1, float a2, float b2, float a3, float b3) {
+        split_pair(a0, a1, h[0], m[0], l[0]); split_pair(b0, b1, h[1], m[1], l[1]);
+        split_pair(a2, a3, h[2], m[2], l[2]); split_pair(b2, b3, h[3], m[3], l[3]);
     }
 };
-template <bool EXACT> struct FragB {
-    unsigned hi[2], lo[2];
-    __device__ __forceinline__ void set(float b0, float b1) { split_tf32<EXACT>(b0, hi[0], lo[0]); split_tf32<EXACT>(b1, hi[1], lo[1]); }
+struct FragB {
+    unsigned h[2], m[2], l[2];
+    __device__ __forceinline__ void set(float b0, float b1, float b2, float b3) {
+        split_pair(b0, b1, h[0], m[0], l[0]); split_pair(b2, b3, h[1], m[1], l[1]);
+    }
 };
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// c[i] += A B[i] for N tiles side by side (independent sums between dependent ones)
-template <int N, bool EXACT>
-__device__ __forceinline__ void mma_split(float (&c)[N][4], const FragA<EXACT>& a, const FragB<EXACT> (&b)[N]) {
-    if constexpr (EXACT) {
-        float d[N][4] = {};
+// c[i] += A B_i for N tiles side by side, up to four at a time; operands(i, b) makes B_i.
+template <int N, typename Operands>
+__device__ __forceinline__ void mma_split(float (&c)[N][4], const FragA& a, Operands operands) {
+    constexpr int G = N < 4 ? N : 4;
 #pragma unroll
-        for (int i = 0; i < N; ++i) mma_tf32(d[i], a.lo, b[i].hi);
+    for (int i0 = 0; i0 < N; i0 += G) {
+        FragB b[G];
+        float h[G][4] = {}, d[G][4];
 #pragma unroll
-        for (int i = 0; i < N; ++i) mma_tf32(d[i], a.hi, b[i].lo);
+        for (int i = 0; i < G; ++i) operands(i0 + i, b[i]);
 #pragma unroll
-        for (int i = 0; i < N; ++i) mma_tf32(d[i], a.hi, b[i].hi);
+        for (int i = 0; i < G; ++i) mma_bf16(h[i], a.h, b[i].h);
 #pragma unroll
-        for (int i = 0; i < N; ++i)
+        for (int i = 0; i < G; ++i) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) c[i][k] += d[i][k];
-    } else {
+            for (int k = 0; k < 4; ++k) d[i][k] = -h[i][k];
+            mma_bf16(d[i], a.h, b[i].h);
+        }
 #pragma unroll
-        for (int i = 0; i < N; ++i) mma_tf32(c[i], a.lo, b[i].hi);
+        for (int i = 0; i < G; ++i) mma_bf16(d[i], a.l, b[i].h);
 #pragma unroll
-        for (int i = 0; i < N; ++i) mma_tf32(c[i], a.hi, b[i].lo);
+        for (int i = 0; i < G; ++i) mma_bf16(d[i], a.h, b[i].l);
 #pragma unroll
-        for (int i = 0; i < N; ++i) mma_tf32(c[i], a.hi, b[i].hi);
+        for (int i = 0; i < G; ++i) mma_bf16(d[i], a.m, b[i].m);
+#pragma unroll
+        for (int i = 0; i < G; ++i) mma_bf16(d[i], a.m, b[i].h);
+#pragma unroll
+        for (int i = 0; i < G; ++i) mma_bf16(d[i], a.h, b[i].m);
+#pragma unroll
+        for (int i = 0; i < G; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) c[i0 + i][k] = (c[i0 + i][k] + d[i][k]) + h[i][k];
     }
 }
 __device__ __forceinline__ bool finite_f(float x) { return fabsf(x) <= 3.402823466e38f; }
@@ -176,7 +196,7 @@ __device__ __forceinline__ int first_chunk(const ChunkArgs& p, int seg, int& row
 __host__ __device__ constexpr int m_row(int a) { return SUB * (a + 1) + 4; }    // a row of sub-chunk a's part of M
 __host__ __device__ constexpr int m_at(int a) { return 128 * a * (a + 1) + 64 * a; }                // where that part begins
 constexpr size_t prepare_smem(int K, bool delta) {
-    return sizeof(float) * (3 * (size_t)C * (K + 4) + NSUB * K + C + (delta ? m_at(NSUB) : 0));
+    return sizeof(float) * (3 * (size_t)C * (K + 4) + NSUB * K + 2 * C + 4 + (delta ? m_at(NSUB) : 0));
 }
 
 // Two CTAs an SM (shared memory).  Blocks of A and L on the diagonal (16 x 16 tokens) are walked with a running key,
@@ -184,7 +204,6 @@ constexpr size_t prepare_smem(int K, bool delta) {
 // exponentials; the others factor at the sub-chunk edges and are products.
 template <typename T, int K, int V, bool DELTA>
 __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p) {
-    constexpr bool EXACT = sizeof(T) == 4;
     constexpr int ROW = K + 4, CPL = K / 32;                // padding: neighbouring tokens lie four banks apart
     extern __shared__ __align__(16) float smem[];
     float* qs = smem;                                       // [C][ROW]  q, then q P(start of its sub-chunk, t]
@@ -192,7 +211,8 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
     float* gs = ks + C * ROW;                               // decays, then k P(t, end of its sub-chunk]
     float* subp = gs + C * ROW;                             // [NSUB][K] decay of a whole sub-chunk
     float* betas = subp + NSUB * K;                         // [C]
-    float* M = betas + C;                                   // diag(beta) L below the diagonal, sub-chunk by sub-chunk
+    float* powers = betas + C;                              // [C + 4] of a constant decay
+    float* M = powers + C + 4;                              // diag(beta) L below the diagonal, sub-chunk by sub-chunk
     pdl_launch_dependents();
     const int head = blockIdx.x, chunk = blockIdx.y;
     int row0, rows;
@@ -206,6 +226,12 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
     const int q_off = kvh * K, k_off = p.G * K + kvh * K, v_off = (forget ? 1 : 2) * p.G * K + head * V;
     const float rate = (plain || mode == DECAY_LOG_SIGMOID) ? p.A_log[head] : ((forget || bonus) ? 0.f : expf(p.A_log[head]));
     const int ch0 = lane * CPL;
+    if (plain && tid <= C) {                                // each rounded once: an error here is every channel's and every token's
+        double power = 1., base = rate;
+        for (int e = tid; e > 0; e >>= 1, base *= base)
+            if (e & 1) power *= base;
+        powers[tid] = (float)power;
+    }
     float bias[CPL], low[CPL];
 #pragma unroll
     for (int i = 0; i < CPL; ++i) {
@@ -262,7 +288,7 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
             }
         } else if (plain) {
 #pragma unroll
-            for (int i = 0; i < CPL; ++i) { q[i] = silu_f(q[i]); k[i] = silu_f(k[i]); g[i] = rate; }
+            for (int i = 0; i < CPL; ++i) { q[i] = silu_f(q[i]); k[i] = silu_f(k[i]); g[i] = 1.f; }      // (the decays: `powers`)
         } else if (forget) {
 #pragma unroll
             for (int i = 0; i < CPL; ++i) {
@@ -367,7 +393,7 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
             const int s = s0 + (which & 3);
             if ((slice & (DELTA ? 1 : 3)) == 0) {
                 if (which < 4) {
-                    if (t >= s) A[t * C + s] = (bonus && t == s) ? betas[t] : sum[0];
+                    if (t >= s) A[t * C + s] = (bonus && t == s) ? betas[t] : (plain ? sum[0] * powers[t - s] : sum[0]);
                 } else if (t > s) {
                     M[m_at(a) + (t - a0) * m_row(a) + s] = betas[t] * sum[0];
                 }
@@ -375,26 +401,33 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
         }
     }
     __syncthreads();
-    // ---- products of decays inside the sub-chunks
+    // ---- products of decays inside the sub-chunks, as sums of two numbers: each has one rounding in the end, not one a token
     for (int idx = tid; idx < K * NSUB; idx += 256) {
-        const int ch = idx % K, sub = idx / K;
-        float g[SUB], k[SUB], pre = 1.f;
+        const int ch = idx % K, sub = idx / K, live = min(SUB, max(0, rows - sub * SUB));
+        float g[SUB], k[SUB], hi = 1.f, lo = 0.f;
+        auto times = [&](float x) {
+            const float p = hi * x;
+            lo = fmaf(lo, x, fmaf(hi, x, -p));
+            hi = p;
+        };
 #pragma unroll
         for (int r = 0; r < SUB; ++r) {
             const int at = (sub * SUB + r) * ROW + ch;
             g[r] = gs[at];
             k[r] = ks[at];
-            if (!bonus) pre *= g[r];
-            qs[at] *= pre;
-            if (DELTA) ks[at] = k[r] * pre;
-            if (bonus) pre *= g[r];
+            if (plain) hi = powers[min(r + 1, live)];
+            else if (!bonus) times(g[r]);
+            qs[at] = fmaf(qs[at], hi, qs[at] * lo);
+            if (DELTA) ks[at] = fmaf(k[r], hi, k[r] * lo);
+            if (bonus) times(g[r]);
         }
-        subp[sub * K + ch] = pre;
-        float suf = 1.f;
+        subp[sub * K + ch] = hi + lo;
+        hi = 1.f; lo = 0.f;
 #pragma unroll
         for (int r = SUB - 1; r >= 0; --r) {
-            gs[(sub * SUB + r) * ROW + ch] = k[r] * suf;
-            suf *= g[r];
+            if (plain) hi = powers[max(0, live - 1 - r)];
+            gs[(sub * SUB + r) * ROW + ch] = fmaf(k[r], hi, k[r] * lo);
+            if (!plain) times(g[r]);
         }
     }
     __syncthreads();
@@ -403,19 +436,30 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
         const int a = warp < 3 ? 3 : (warp < 5 ? 2 : 1), b = warp < 3 ? warp : (warp < 5 ? warp - 3 : 0);
         const int t0 = a * SUB + fr, s0 = b * SUB + fr;
         float acc[2][4] = {}, accl[2][4] = {};
+        auto rows_of = [&](const float* x, int c, FragA& f) {
+            const float *x0 = x + t0 * ROW + c, *x8 = x0 + 8 * ROW;
+            f.set(x0[0], x8[0], x0[4], x8[4], x0[8], x8[8], x0[12], x8[12]);
+        };
 #pragma unroll 2
-        for (int c = fc; c < K; c += 8) {
-            float f0 = 1.f, f1 = 1.f;                       // whole sub-chunks between the two
-            for (int m = b + 1; m < a; ++m) { f0 *= subp[m * K + c]; f1 *= subp[m * K + c + 4]; }
-            FragB<EXACT> kb[2];
+        for (int c = fc; c < K; c += 16) {
+            float f[4];                                     // whole sub-chunks between the two
 #pragma unroll
-            for (int j = 0; j < 2; ++j) kb[j].set(gs[(s0 + 8 * j) * ROW + c] * f0, gs[(s0 + 8 * j) * ROW + c + 4] * f1);
-            FragA<EXACT> f;
-            f.set(qs[t0 * ROW + c], qs[(t0 + 8) * ROW + c], qs[t0 * ROW + c + 4], qs[(t0 + 8) * ROW + c + 4]);
-            mma_split<2, EXACT>(acc, f, kb);
+            for (int e = 0; e < 4; ++e) {
+                f[e] = 1.f;
+                for (int m = b + 1; m < a; ++m) f[e] *= subp[m * K + c + 4 * e];
+            }
+            FragB kb[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float* k = gs + (s0 + 8 * j) * ROW + c;
+                kb[j].set(k[0] * f[0], k[4] * f[1], k[8] * f[2], k[12] * f[3]);
+            }
+            FragA x;
+            rows_of(qs, c, x);
+            mma_split<2>(acc, x, [&](int j, FragB& o) { o = kb[j]; });
             if (DELTA) {
-                f.set(ks[t0 * ROW + c], ks[(t0 + 8) * ROW + c], ks[t0 * ROW + c + 4], ks[(t0 + 8) * ROW + c + 4]);
-                mma_split<2, EXACT>(accl, f, kb);
+                rows_of(ks, c, x);
+                mma_split<2>(accl, x, [&](int j, FragB& o) { o = kb[j]; });
             }
         }
 #pragma unroll
@@ -459,7 +503,7 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
         float d = 1.f;
 #pragma unroll
         for (int m = 0; m < NSUB; ++m) d *= subp[m * K + ch];
-        p.decay[unit * K + ch] = d;
+        p.decay[unit * K + ch] = plain ? powers[min(C, rows)] : d;
     }
     float* ub = p.u + unit * C * V;
     __syncthreads();                                        // qs is written out, gs and M are complete
@@ -501,21 +545,22 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
 #pragma unroll
             for (int a = 0; a < NSUB; ++a) {
                 const float* m = M + m_at(a) + fr * m_row(a) + 2 * fc;
-                float y[2][4];
+                // (what earlier blocks take away is summed apart: a sum of smaller numbers, rounded finer)
+                float y[2][4], less[2][4] = {};
 #pragma unroll
-                for (int e = 0; e < 4; ++e) { y[0][e] = x[2 * a][e]; y[1][e] = x[2 * a + 1][e]; }
-#pragma unroll
-                for (int j = 0; j < 2 * a; ++j) {
-                    FragA<EXACT> f;
-                    f.set(x[j][0], x[j][2], x[j][1], x[j][3]);
-                    FragB<EXACT> mb[2];
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
+                for (int j = 0; j < 2 * a; j += 2) {
+                    FragA f;
+                    f.set(x[j][0], x[j][2], x[j][1], x[j][3], x[j + 1][0], x[j + 1][2], x[j + 1][1], x[j + 1][3]);
+                    mma_split<2>(less, f, [&](int i, FragB& o) {
                         const float2 v = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + 8 * j);
-                        mb[i].set(-v.x, -v.y);
-                    }
-                    mma_split<2, EXACT>(y, f, mb);
+                        const float2 w = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + 8 * j + 8);
+                        o.set(v.x, v.y, w.x, w.y);
+                    });
                 }
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) y[i][e] = x[2 * a + i][e] - less[i][e];
                 bool fine = true;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) fine = fine && finite_f(y[0][e]) && finite_f(y[1][e]);
@@ -523,18 +568,18 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
 #pragma unroll
                 for (int e = 0; e < 4; ++e) { r[0][e] = y[0][e]; r[1][e] = y[1][e]; }
                 if (__all_sync(0xffffffffu, fine)) {
+                    FragA f;
+                    f.set(r[0][0], r[0][2], r[0][1], r[0][3], r[1][0], r[1][2], r[1][1], r[1][3]);
+                    float more[2][4] = {};
+                    mma_split<2>(more, f, [&](int i, FragB& o) {
+                        const float2 v = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + a * SUB);
+                        const float2 w = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + a * SUB + 8);
+                        o.set(v.x, v.y, w.x, w.y);
+                    });
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        FragA<EXACT> f;
-                        f.set(r[j][0], r[j][2], r[j][1], r[j][3]);
-                        FragB<EXACT> mb[2];
+                    for (int i = 0; i < 2; ++i)
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            const float2 v = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + a * SUB + 8 * j);
-                            mb[i].set(v.x, v.y);
-                        }
-                        mma_split<2, EXACT>(y, f, mb);
-                    }
+                        for (int e = 0; e < 4; ++e) y[i][e] += more[i][e];
                 } else {                                    // token by token: none meets a later one
                     const float* own = M + m_at(a) + a * SUB;
                     for (int s = 0; s < SUB; ++s) {
@@ -584,17 +629,25 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
     const int mb = (warp % MW) * 32, nb = (warp / MW) * NT * 8;
     float acc[2][NT][4] = {};
 #pragma unroll 1
-    for (int t0 = 0; t0 < C; t0 += 8) {
-        const int t = t0 + 2 * fc;
-        FragB<EXACT> u[NT];
-#pragma unroll
-        for (int j = 0; j < NT; ++j) u[j].set(us[t * UROW + nb + 8 * j + fr], us[(t + 1) * UROW + nb + 8 * j + fr]);
+    for (int t0 = 0; t0 < C; t0 += 16) {
+        const int t = t0 + 2 * fc;                          // a lane's tokens: t, t + 1, t + 8, t + 9
+        FragA f[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const float* at = gs + t * ROW + mb + 16 * i + fr;
-            FragA<EXACT> f;
-            f.set(at[0], at[8], at[ROW], at[ROW + 8]);
-            mma_split<NT, EXACT>(acc[i], f, u);
+            const float *at = gs + t * ROW + mb + 16 * i + fr, *at8 = at + 8 * ROW;
+            f[i].set(at[0], at[8], at[ROW], at[ROW + 8], at8[0], at8[8], at8[ROW], at8[ROW + 8]);
+        }
+#pragma unroll
+        for (int j = 0; j < NT; j += 2) {
+            FragB u[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float* at = us + t * UROW + nb + 8 * (j + e) + fr;
+                u[e].set(at[0], at[UROW], at[8 * UROW], at[9 * UROW]);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                mma_split<2>(reinterpret_cast<float(&)[2][4]>(acc[i][j]), f[i], [&](int e, FragB& o) { o = u[e]; });
         }
     }
     float* dS = p.s + unit * K * V;
@@ -658,7 +711,7 @@ template <int K, int NT> struct DeltaSmem {
 // CTA.  The state lives in the registers of the warps that sum it and, for the next chunk's first product, in shared
 // memory; the next chunk's operands are copied while this one's run.  Bound by the two products' tensor instructions
 // (768 cycles each at 16 columns) and what stands between them: two barriers, the operands' split.
-template <int K, int V, int NT, bool EXACT>
+template <int K, int V, int NT>
 __global__ void __launch_bounds__(256, 1) chunk_delta_kernel(const ChunkArgs p) {
     typedef DeltaSmem<K, NT> L;
     constexpr int ROW = L::ROW, COLS = L::COLS, SROW = L::SROW, UROW = L::UROW;
@@ -721,53 +774,48 @@ __global__ void __launch_bounds__(256, 1) chunk_delta_kernel(const ChunkArgs p) 
         __syncthreads();                                    // the chunk's operands and the state; the other stage is free
         if (c + 1 < chunks) fetch(c + 1);
         {   // U = U0 - W S
-            float acc[2][UN][4] = {};                       // even and odd steps: independent sums
-#pragma unroll 4
-            for (int k0 = 0; k0 < K; k0 += 16)
+            float acc[UN][4] = {};
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const int k = k0 + 8 * half + fc;
-                    const float* w = ws + (um + fr) * ROW + k;
-                    FragA<EXACT> f;
-                    f.set(w[0], w[8 * ROW], w[4], w[8 * ROW + 4]);
-                    FragB<EXACT> b[UN];
-#pragma unroll
-                    for (int j = 0; j < UN; ++j) b[j].set(S[k * SROW + un + 8 * j + fr], S[(k + 4) * SROW + un + 8 * j + fr]);
-                    mma_split<UN, EXACT>(acc[half], f, b);
-                }
+            for (int k0 = 0; k0 < K; k0 += 16) {
+                const int k = k0 + fc;
+                const float *w = ws + (um + fr) * ROW + k, *w8 = w + 8 * ROW;
+                FragA f;
+                f.set(w[0], w8[0], w[4], w8[4], w[8], w8[8], w[12], w8[12]);
+                mma_split<UN>(acc, f, [&](int j, FragB& o) {
+                    const float* at = S + k * SROW + un + 8 * j + fr;
+                    o.set(at[0], at[4 * SROW], at[8 * SROW], at[12 * SROW]);
+                });
+            }
 #pragma unroll
             for (int j = 0; j < UN; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int t = um + fr + 8 * h, col = un + 8 * j + 2 * fc;
                     const float2 u0 = *reinterpret_cast<const float2*>(u0s + t * COLS + col);
-                    const float2 u = make_float2(u0.x - (acc[0][j][2 * h] + acc[1][j][2 * h]),
-                                                 u0.y - (acc[0][j][2 * h + 1] + acc[1][j][2 * h + 1]));
+                    const float2 u = make_float2(u0.x - acc[j][2 * h], u0.y - acc[j][2 * h + 1]);
                     *reinterpret_cast<float2*>(us + t * UROW + col) = u;
                     *reinterpret_cast<float2*>(p.u + unit * C * V + (size_t)t * V + col0 + col) = u;
                 }
         }
         __syncthreads();                                    // U is complete, nobody reads the state any more
         {   // S <- diag(decay) S + Kd^T U
-            float acc[2][SN][4] = {};
-#pragma unroll 4
-            for (int t0 = 0; t0 < C; t0 += 16)
+            float acc[SN][4] = {};
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const int t = t0 + 8 * half + 2 * fc;
-                    const float* kd = kds + t * ROW + sm + fr;
-                    FragA<EXACT> f;
-                    f.set(kd[0], kd[8], kd[ROW], kd[ROW + 8]);
-                    FragB<EXACT> b[SN];
-#pragma unroll
-                    for (int j = 0; j < SN; ++j) b[j].set(us[t * UROW + sn + 8 * j + fr], us[(t + 1) * UROW + sn + 8 * j + fr]);
-                    mma_split<SN, EXACT>(acc[half], f, b);
-                }
+            for (int t0 = 0; t0 < C; t0 += 16) {
+                const int t = t0 + 2 * fc;
+                const float *kd = kds + t * ROW + sm + fr, *kd8 = kd + 8 * ROW;
+                FragA f;
+                f.set(kd[0], kd[8], kd[ROW], kd[ROW + 8], kd8[0], kd8[8], kd8[ROW], kd8[ROW + 8]);
+                mma_split<SN>(acc, f, [&](int j, FragB& o) {
+                    const float* at = us + t * UROW + sn + 8 * j + fr;
+                    o.set(at[0], at[UROW], at[8 * UROW], at[9 * UROW]);
+                });
+            }
             const float g0 = ds[sm + fr], g1 = ds[sm + fr + 8];
 #pragma unroll
             for (int j = 0; j < SN; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) s[j][e] = fmaf(s[j][e], e < 2 ? g0 : g1, acc[0][j][e] + acc[1][j][e]);
+                for (int e = 0; e < 4; ++e) s[j][e] = fmaf(s[j][e], e < 2 ? g0 : g1, acc[j][e]);
         }
     }
 #pragma unroll
@@ -788,7 +836,6 @@ constexpr size_t output_smem(int V, size_t type) {
 // outputs in o_raw.
 template <typename T, int K, int V>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 3) chunk_output_kernel(const ChunkArgs p) {
-    constexpr bool EXACT = sizeof(T) == 4;
     constexpr int KT = OUT_TILE, XROW = KT + 4, YROW = V + 8, NT = V / 16;
     extern __shared__ __align__(16) float smem[];
     float* xs = smem;                                       // [2][C][XROW]
@@ -832,15 +879,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 3) chunk_output_kern
         const float* y = ys + (tile & 1) * KT * YROW + n0 + fr;
         const int s0 = tile * KT - K;                       // first token of A's columns in this tile (negative: q P)
         const int whole = s0 < 0 ? KT : min(KT, max(0, a * SUB - s0));      // columns that every token of the warp sees
+        auto column = [&](int k, int i, FragB& o) {
+            const float* at = y + k * YROW + 8 * i;
+            o.set(at[0], at[4 * YROW], at[8 * YROW], at[12 * YROW]);
+        };
 #pragma unroll 1
-        for (int j = 0; j < whole; j += 8) {
+        for (int j = 0; j < whole; j += 16) {
             const int k = j + fc;
-            FragA<EXACT> f;
-            f.set(x[k], x[8 * XROW + k], x[k + 4], x[8 * XROW + k + 4]);
-            FragB<EXACT> b[NT];
-#pragma unroll
-            for (int i = 0; i < NT; ++i) b[i].set(y[k * YROW + 8 * i], y[(k + 4) * YROW + 8 * i]);
-            mma_split<NT, EXACT>(acc, f, b);
+            const float* x8 = x + 8 * XROW;
+            FragA f;
+            f.set(x[k], x8[k], x[k + 4], x8[k + 4], x[k + 8], x8[k + 8], x[k + 12], x8[k + 12]);
+            mma_split<NT>(acc, f, [&](int i, FragB& o) { column(k, i, o); });
         }
         const int d0 = a * SUB - s0;                        // where the warp's own tokens lie in this tile
         if (s0 >= 0 && d0 >= 0 && d0 < KT) {
@@ -850,17 +899,16 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 3) chunk_output_kern
 #pragma unroll
                 for (int i = 0; i < NT; ++i) fine = fine && finite_f(y[(d0 + j + fc) * YROW + 8 * i]);
             if (__all_sync(0xffffffffu, fine)) {
+                const int k = d0 + fc;
+                float v[8];                                 // a token sees those up to itself
 #pragma unroll
-                for (int j = 0; j < SUB; j += 8) {
-                    const int k = d0 + j + fc, s = j + fc;
-                    FragA<EXACT> f;                                // a token sees those up to itself
-                    f.set(fr >= s ? x[k] : 0.f, fr + 8 >= s ? x[8 * XROW + k] : 0.f, fr >= s + 4 ? x[k + 4] : 0.f,
-                          fr + 8 >= s + 4 ? x[8 * XROW + k + 4] : 0.f);
-                    FragB<EXACT> b[NT];
-#pragma unroll
-                    for (int i = 0; i < NT; ++i) b[i].set(y[k * YROW + 8 * i], y[(k + 4) * YROW + 8 * i]);
-                    mma_split<NT, EXACT>(acc, f, b);
+                for (int e = 0; e < 4; ++e) {
+                    v[2 * e] = fr >= fc + 4 * e ? x[k + 4 * e] : 0.f;
+                    v[2 * e + 1] = fr + 8 >= fc + 4 * e ? x[8 * XROW + k + 4 * e] : 0.f;
                 }
+                FragA f;
+                f.set(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+                mma_split<NT>(acc, f, [&](int i, FragB& o) { column(k, i, o); });
             } else {
                 const float* yt = ys + (tile & 1) * KT * YROW + n0 + 2 * fc;
                 for (int s = 0; s < SUB; ++s)
@@ -931,11 +979,11 @@ int launch_chunked(const ChunkArgs& p, cudaStream_t stream) {
     if (delta) {
         // 16 columns a CTA while all CTAs are resident (one an SM), else 32
         if (p.H * (V / 16) * p.segments <= 148) {
-            cudaFuncSetAttribute(chunk_delta_kernel<K, V, 2, sizeof(T) == 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaSmem<K, 2>::bytes);
-            tis_launch(chunk_delta_kernel<K, V, 2, sizeof(T) == 4>, dim3(V / 16, p.H, p.segments), dim3(256), DeltaSmem<K, 2>::bytes, stream, p);
+            cudaFuncSetAttribute(chunk_delta_kernel<K, V, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaSmem<K, 2>::bytes);
+            tis_launch(chunk_delta_kernel<K, V, 2>, dim3(V / 16, p.H, p.segments), dim3(256), DeltaSmem<K, 2>::bytes, stream, p);
         } else {
-            cudaFuncSetAttribute(chunk_delta_kernel<K, V, 4, sizeof(T) == 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaSmem<K, 4>::bytes);
-            tis_launch(chunk_delta_kernel<K, V, 4, sizeof(T) == 4>, dim3(V / 32, p.H, p.segments), dim3(256), DeltaSmem<K, 4>::bytes, stream, p);
+            cudaFuncSetAttribute(chunk_delta_kernel<K, V, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DeltaSmem<K, 4>::bytes);
+            tis_launch(chunk_delta_kernel<K, V, 4>, dim3(V / 32, p.H, p.segments), dim3(256), DeltaSmem<K, 4>::bytes, stream, p);
         }
     } else {
         tis_launch(chunk_state_kernel<K, V>, dim3(K * V / 1024, p.H, p.segments), dim3(256), 0, stream, p);
