@@ -103,13 +103,14 @@ class Case:
             out[r0:r0 + m] = y
         return out, states
 
-    def call(self, ops, segments):
+    def call(self, ops, segments, rows_at=0, state_at=0):
+        """``rows_at``, ``state_at``: elements that the rows and the states begin beside a boundary."""
         c = lambda t: t.cuda()  # noqa: E731
         wide = torch.empty(self.n, self.rows.shape[1] + 16, dtype=self.dtype, device="cuda")
-        rows = wide[:, :self.rows.shape[1]]
+        rows = wide[:, rows_at:rows_at + self.rows.shape[1]]
         rows.copy_(self.rows)
         held = torch.empty(self.state.shape[0], self.state.shape[1] + 8, device="cuda")
-        state = held[:, :self.state.shape[1]]
+        state = held[:, state_at:state_at + self.state.shape[1]]
         state.copy_(self.state)
         out = torch.zeros(self.n, self.H * self.V, dtype=self.dtype, device="cuda")
         tail = dict(requests=len(self.lengths), segments=segments)
@@ -146,9 +147,9 @@ def _compare(case):
     from tiny_inference_server_b200.kernels import ops
     want_o, want_s = case.oracle()
     walked_o, walked_s = case.call(ops, case.segments(False))
-    before = ops.launches
+    before = ops.calls["recurrence_chunked"]
     got_o, got_s = case.call(ops, case.segments(True))
-    assert ops.launches - before >= 3                                       # the chunked form ran
+    assert ops.calls["recurrence_chunked"] == before + 1
     # 32-bit sums of at most K + 64 products a chunk, errors of one chunk carried on by decays <= 1: a few times 2^-23
     # relative to the whole; and never much worse than the walk, whose chain is as long as the portion
     limit = 3e-6 if case.dtype == torch.float32 or case.rule == "step" else 4e-3
@@ -212,3 +213,20 @@ def test_no_further_off_than_the_walk(rule, dtype):
         state.append(_off(got_s, want_s) / _off(walked_s, want_s))
     assert sum(state) / 5 < 1.15, state
     assert sum(out) / 5 < 1.05, out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", RULES)
+def test_operands_that_the_chunks_do_not_take_are_walked(rule):
+    """A state or rows that start beside a 16-byte boundary, and widths without the kernels: token by token, counted as that."""
+    from tiny_inference_server_b200.kernels import ops
+    for K, V, rows_at, state_at in ((64, 64, 1, 0), (64, 64, 0, 1), (32, 32, 0, 0)):
+        if rule == "bonus" and rows_at:
+            continue                                                        # (its walk reads rows in 16-byte vectors as well)
+        case = Case(rule, K, V, (70, 9), torch.float32, seed=9)
+        want_o, want_s = case.oracle()
+        before, launched = ops.calls["recurrence_chunked"], ops.launches
+        got_o, got_s = case.call(ops, case.segments(True), rows_at, state_at)
+        assert ops.calls["recurrence_chunked"] == before
+        assert ops.launches - launched == (1 if rule == "step" else 2)
+        assert _off(got_o, want_o) < 3e-6 and _off(got_s, want_s) < 3e-6

@@ -997,13 +997,6 @@ int launch_chunked(const ChunkArgs& p, cudaStream_t stream) {
 
 }  // namespace
 
-// Floats of scratch for a step of n rows in `segments` requests; 0: the chunked kernels do not take these widths.
-TIS_API size_t tis_chunked_recurrence_floats(int n, int segments, int H, int k_dim, int v_dim, int delta) {
-    if (!((k_dim == 64 || k_dim == 128) && (v_dim == 64 || v_dim == 128)) || n <= 0 || segments <= 0 || H <= 0) return 0;
-    const size_t units = ((size_t)n / C + segments) * H;
-    return units * ((size_t)C * k_dim * (delta ? 3 : 1) + (size_t)C * v_dim + (size_t)C * C + (size_t)k_dim * v_dim + k_dim);
-}
-
 bool chunked_recurrence_takes(int dtype, const ChunkArgs& p, int k_dim, int v_dim) {
     const bool head_step = p.mode == DECAY_PER_HEAD || p.mode == DECAY_STEP || p.mode == DECAY_CONSTANT;
     const bool raw = p.mode == DECAY_CONSTANT || p.mode == DECAY_STEP;
@@ -1011,18 +1004,34 @@ bool chunked_recurrence_takes(int dtype, const ChunkArgs& p, int k_dim, int v_di
     if (!head_step) bases |= (uintptr_t)p.a_in;
     if (!raw) bases |= (uintptr_t)p.gate | (uintptr_t)p.out;
     else bases |= (uintptr_t)p.o_raw;
-    const bool chunks_fit = p.seg_row0 != nullptr && p.segments > 0 && p.segments <= 65535 && p.H > 0 && p.H <= 65535 && p.G > 0 &&
+    const bool chunks_fit = p.segments > 0 && p.segments <= 65535 && p.H > 0 && p.H <= 65535 && p.G > 0 &&
                             p.H % p.G == 0 && p.n / C + p.segments <= 65535;
     return chunks_fit && (k_dim == 64 || k_dim == 128) && (v_dim == 64 || v_dim == 128) && (dtype == TIS_F32 || dtype == TIS_BF16) &&
            bases % 16 == 0 && p.ld % 8 == 0 && (head_step || p.lda % 8 == 0) && p.state_stride % 4 == 0 &&
            (raw || (p.ldo % 8 == 0 && (p.gate == nullptr || p.ldg % 8 == 0)));
 }
 
+static size_t chunk_floats(const ChunkArgs& p, int k_dim, int v_dim) {
+    const bool delta = p.mode == DECAY_PER_CHANNEL || p.mode == DECAY_PER_HEAD;
+    const size_t units = ((size_t)p.n / C + p.segments) * p.H;
+    return units * ((size_t)C * k_dim * (delta ? 3 : 1) + (size_t)C * v_dim + (size_t)C * C + (size_t)k_dim * v_dim + k_dim);
+}
+// Floats of scratch for a step of n rows in `segments` requests; 0: the chunked kernels do not take these operands (o_raw lies on
+// a 16-byte boundary).
+TIS_API size_t tis_chunked_recurrence_floats(int dtype, int mode, const void* qkv, int ld, const void* a_in, int lda, const void* gate,
+                                             int ldg, const void* out, int ldo, const float* state, size_t state_stride, int n,
+                                             int segments, int H, int G, int k_dim, int v_dim) {
+    ChunkArgs p = {};
+    p.qkv = qkv; p.ld = ld; p.a_in = a_in; p.lda = lda; p.gate = gate; p.ldg = ldg; p.out = const_cast<void*>(out); p.ldo = ldo;
+    p.state = const_cast<float*>(state); p.state_stride = state_stride; p.n = n; p.segments = segments; p.H = H; p.G = G; p.mode = mode;
+    return chunked_recurrence_takes(dtype, p, k_dim, v_dim) ? chunk_floats(p, k_dim, v_dim) : 0;
+}
+
 int chunked_recurrence(int dtype, ChunkArgs p, int k_dim, int v_dim, float* scratch, size_t scratch_floats, cudaStream_t stream) {
     const bool delta = p.mode == DECAY_PER_CHANNEL || p.mode == DECAY_PER_HEAD;
     p.chunks = p.n / C + p.segments;
     if (scratch == nullptr || (uintptr_t)scratch % 16 != 0 ||
-        scratch_floats < tis_chunked_recurrence_floats(p.n, p.segments, p.H, k_dim, v_dim, delta)) {
+        scratch_floats < chunk_floats(p, k_dim, v_dim)) {
         tis_set_error("chunked recurrence: %zu floats of scratch for %d rows of %d requests, %d heads", scratch_floats, p.n,
                       p.segments, p.H);
         return TIS_BAD_SIZE;

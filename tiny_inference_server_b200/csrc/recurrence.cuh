@@ -44,5 +44,5 @@ struct ChunkArgs {
 };
 // Whether the chunked kernels take these widths, and, if so, whether these operands: 16-byte rows and states.
 bool chunked_recurrence_takes(int dtype, const ChunkArgs& args, int k_dim, int v_dim);
-// Launches them; `scratch` holds chunked_recurrence_floats(...) floats.
+// Launches them; `scratch` holds tis_chunked_recurrence_floats(...) floats.
 int chunked_recurrence(int dtype, ChunkArgs args, int k_dim, int v_dim, float* scratch, size_t scratch_floats, cudaStream_t stream);

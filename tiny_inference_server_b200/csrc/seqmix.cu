@@ -1508,13 +1508,16 @@ static int matrix_state_recurrence(int dtype, const void* qkv, int ld, const voi
         p.state = state; p.state_stride = state_stride; p.out = out; p.ldo = ldo; p.o_raw = o_raw; p.row_slot = row_slot;
         p.row_last = row_last; p.seg_row0 = seg_row0; p.segments = segments; p.n = n; p.H = H; p.G = G; p.mode = decay_mode;
         p.gate_act = gate_act;
-        if (chunked_recurrence_takes(dtype, p, k_dim, v_dim)) {
-            const int st = chunked_recurrence(dtype, p, k_dim, v_dim, chunk_scratch, chunk_floats, stream);
-            if (st != TIS_OK || decay_mode != DECAY_CONSTANT) return st;
-            TIS_DISPATCH_DTYPE(dtype, T, tis_launch(row_out_norm_kernel<T>, dim3(n), dim3(256), 0, stream, (const float*)o_raw,
-                               (const T*)gate, ldg, norm_w, eps, (T*)out, ldo, row_slot, H * v_dim));
-            return tis_check_launch("row_out_norm");
+        if (seg_row0 == nullptr || !chunked_recurrence_takes(dtype, p, k_dim, v_dim)) {
+            tis_set_error("chunked recurrence: %d rows of %d heads in %d requests, widths %d and %d, or operands that are not aligned",
+                          n, H, segments, k_dim, v_dim);
+            return TIS_BAD_SIZE;
         }
+        const int st = chunked_recurrence(dtype, p, k_dim, v_dim, chunk_scratch, chunk_floats, stream);
+        if (st != TIS_OK || decay_mode != DECAY_CONSTANT) return st;
+        TIS_DISPATCH_DTYPE(dtype, T, tis_launch(row_out_norm_kernel<T>, dim3(n), dim3(256), 0, stream, (const float*)o_raw,
+                           (const T*)gate, ldg, norm_w, eps, (T*)out, ldo, row_slot, H * v_dim));
+        return tis_check_launch("row_out_norm");
     }
     // (the walk with a bonus reads its rows in 16-byte vectors)
     const bool rows_fit = decay_mode != DECAY_BONUS || (ld % 8 == 0 && lda % 8 == 0 && ((uintptr_t)qkv | (uintptr_t)a_in) % 16 == 0);
@@ -1577,7 +1580,7 @@ static int matrix_state_recurrence(int dtype, const void* qkv, int ld, const voi
 }
 
 // The entry points below: `chunk_scratch`, `chunk_floats` (tis_chunked_recurrence_floats of them; null: none): the step
-// holds long portions and may be walked in chunks of tokens.
+// is taken in chunks of tokens.
 
 // The delta rule.  decay_per_head 0: `a_in` (n, H * k_dim) and `dt_bias` (H * k_dim), a decay per head and key channel;
 // 1: `a_in` (n, H) and `dt_bias` (H), one per head.  gate_act: 0 sigmoid, 1 silu.

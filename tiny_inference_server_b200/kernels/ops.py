@@ -19,7 +19,7 @@ import torch
 from . import build as _build
 
 _lib = None
-ABI_VERSION = 14
+ABI_VERSION = 15
 #: launches of this library's kernels so far (library matrix products are not counted)
 launches = 0
 #: calls by kind, for tests that must know which kernel a product or an attention went to
@@ -1159,19 +1159,33 @@ CHUNKED_MIN_ROWS = int(os.environ.get("TIS_CHUNKED_MIN_ROWS", "112"))
 CHUNKED_MAX_BYTES = 1 << 30
 
 
-def _chunk_scratch(lib, n: int, segments, num_heads: int, k_dim: int, v_dim: int, delta: bool, device):
-    """Scratch for the chunked form of a recurrence, or None: token by token."""
+#: the kinds of decay by the launchers' numbers (csrc/recurrence.cuh)
+_DECAYS = {"channel": 0, "head": 1, "constant": 2, "forget": 3, "gated": 4, "step": 5, "bonus": 6}
+
+
+def _chunk_scratch(lib, decay: str, qkv: torch.Tensor, a_in, gate, out, state: torch.Tensor, segments, num_heads: int,
+                   qk_heads: int, k_dim: int, v_dim: int):
+    """Scratch for the chunked form of a recurrence, or None: token by token.  ``gate``: a tensor, or its (address, row stride)."""
+    n = qkv.shape[0]
     if segments is None:
         return None
     longest = segments[2] if len(segments) > 2 else n // max(1, int(segments[1]))
     if longest < CHUNKED_MIN_ROWS:
         return None
-    floats = lib.tis_chunked_recurrence_floats(n, int(segments[1]), num_heads, k_dim, v_dim, int(delta))
+    rows = lambda t: (None, 0) if t is None else (t if isinstance(t, tuple) else (_p(t), t.stride(0)))  # noqa: E731
+    floats = lib.tis_chunked_recurrence_floats(_dt(qkv), _DECAYS[decay], *rows(qkv), *rows(a_in), *rows(gate), *rows(out), _p(state),
+                                               ctypes.c_size_t(state.stride(0)), n, int(segments[1]), num_heads, qk_heads, k_dim, v_dim)
     if not floats or 4 * floats > CHUNKED_MAX_BYTES:
         return None
+    calls["recurrence_chunked"] += 1
+    return torch.empty(floats, dtype=torch.float32, device=qkv.device)
+
+
+def _count_recurrence(lib, decay: str, chunked: bool, k_dim: int, v_dim: int) -> None:
+    """Counts what a recurrence launches beyond the one kernel that every call counts."""
     global launches
-    launches += 1                                # three kernels instead of two
-    return torch.empty(floats, dtype=torch.float32, device=device)
+    norm = decay == "constant" or (decay != "step" and not chunked and bool(lib.tis_delta_rule_splits(k_dim, v_dim)))
+    launches += (2 if chunked else 0) + int(norm)
 
 
 def _floats(scratch: Optional[torch.Tensor]):
@@ -1202,9 +1216,9 @@ def delta_rule(qkv: torch.Tensor, beta: torch.Tensor, decay_in: torch.Tensor, ga
     raw = None
     if lib.tis_delta_rule_splits(k_dim, v_dim):
         raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=qkv.device)
-        global launches
-        launches += 1
-    scratch = _chunk_scratch(lib, n, segments, num_heads, k_dim, v_dim, True, qkv.device)
+    decay = "head" if decay_per_head else "channel"
+    scratch = _chunk_scratch(lib, decay, qkv, decay_in, gate, out, state, segments, num_heads, qk_heads, k_dim, v_dim)
+    _count_recurrence(lib, decay, scratch is not None, k_dim, v_dim)
     _check(lib.tis_delta_rule(_dt(qkv), _p(qkv), qkv.stride(0), _p(beta), beta.stride(0), _p(decay_in), decay_in.stride(0),
                               _p(gate), gate.stride(0) if gate is not None else 0, _p(a_log), _p(dt_bias), _p(norm_weight),
                               _f(eps), _f(unit_eps), _f(q_scale), _p(state), ctypes.c_size_t(state.stride(0)), _p(out),
@@ -1228,9 +1242,8 @@ def linear_attention(qkv: torch.Tensor, gate: Optional[torch.Tensor], decay: tor
     n = qkv.shape[0]
     narrow = _recurrence_spread(requests, num_heads, v_dim)
     raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=qkv.device)
-    global launches
-    launches += 1
-    scratch = _chunk_scratch(lib, n, segments, num_heads, k_dim, v_dim, False, qkv.device)
+    scratch = _chunk_scratch(lib, "constant", qkv, None, gate, out, state, segments, num_heads, num_heads, k_dim, v_dim)
+    _count_recurrence(lib, "constant", scratch is not None, k_dim, v_dim)
     _check(lib.tis_linear_attention(_dt(qkv), _p(qkv), qkv.stride(0), _p(gate), gate.stride(0) if gate is not None else 0,
                                     _p(decay), _p(norm_weight), _f(eps), _p(state), ctypes.c_size_t(state.stride(0)),
                                     _p(out), out.stride(0), _p(raw), _p(row_slot), _p(row_last), n, num_heads, k_dim, v_dim,
@@ -1255,9 +1268,8 @@ def forget_gate_recurrence(qv: torch.Tensor, f_in: torch.Tensor, lower: torch.Te
     raw = None
     if lib.tis_delta_rule_splits(k_dim, v_dim):
         raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=qv.device)
-        global launches
-        launches += 1
-    scratch = _chunk_scratch(lib, n, segments, num_heads, k_dim, v_dim, False, qv.device)
+    scratch = _chunk_scratch(lib, "forget", qv, f_in, None, out, state, segments, num_heads, num_heads, k_dim, v_dim)
+    _count_recurrence(lib, "forget", scratch is not None, k_dim, v_dim)
     _check(lib.tis_forget_gate_recurrence(_dt(qv), _p(qv), qv.stride(0), _p(f_in), f_in.stride(0), _p(lower), _p(f_bias),
                                           _p(norm_weight), _f(eps), _p(state), ctypes.c_size_t(state.stride(0)), _p(out),
                                           out.stride(0), _p(raw), _p(row_slot), _p(row_last), n, num_heads, k_dim, v_dim,
@@ -1364,9 +1376,8 @@ def gated_linear_attention(qkv: torch.Tensor, a_in: torch.Tensor, power: torch.T
     raw = None
     if lib.tis_delta_rule_splits(k_dim, v_dim):
         raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=qkv.device)
-        global launches
-        launches += 1
-    scratch = _chunk_scratch(lib, n, segments, num_heads, k_dim, v_dim, False, qkv.device)
+    scratch = _chunk_scratch(lib, "gated", qkv, a_in, gate, out, state, segments, num_heads, num_heads, k_dim, v_dim)
+    _count_recurrence(lib, "gated", scratch is not None, k_dim, v_dim)
     _check(lib.tis_gated_linear_attention(_dt(qkv), _p(qkv), qkv.stride(0), _p(a_in), a_in.stride(0), _p(power), _p(a_bias),
                                           _p(gate), gate.stride(0) if gate is not None else 0, _p(norm_weight), _f(eps),
                                           _f(q_scale), _p(state), ctypes.c_size_t(state.stride(0)), _p(out), out.stride(0),
@@ -1388,10 +1399,8 @@ def state_space_scan(cbx: torch.Tensor, dt_in: torch.Tensor, a_log: torch.Tensor
     n = cbx.shape[0]
     narrow = _recurrence_spread(requests, num_heads, v_dim)
     raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=cbx.device)
-    scratch = _chunk_scratch(lib, n, segments, num_heads, state_dim, v_dim, False, cbx.device)
-    if scratch is not None:
-        global launches
-        launches += 1
+    scratch = _chunk_scratch(lib, "step", cbx, dt_in, None, None, state, segments, num_heads, groups, state_dim, v_dim)
+    _count_recurrence(lib, "step", scratch is not None, state_dim, v_dim)
     _check(lib.tis_state_space_scan(_dt(cbx), _p(cbx), cbx.stride(0), _p(dt_in), dt_in.stride(0), _p(a_log), _p(dt_bias),
                                     _p(state), ctypes.c_size_t(state.stride(0)), _p(raw), _p(row_slot), _p(row_last), n,
                                     num_heads, groups, state_dim, v_dim, int(narrow),
@@ -1465,9 +1474,9 @@ def time_mix(rkvg: torch.Tensor, w_in: torch.Tensor, u: torch.Tensor, w_bias: to
     raw = None
     if lib.tis_delta_rule_splits(dim, dim):
         raw = torch.empty((n, num_heads * dim), dtype=torch.float32, device=rkvg.device)
-        global launches
-        launches += 1
-    scratch = _chunk_scratch(lib, n, segments, num_heads, dim, dim, False, rkvg.device)
+    scratch = _chunk_scratch(lib, "bonus", rkvg, w_in, (_p(rkvg[:, 3 * num_heads * dim:]), rkvg.stride(0)), out, state, segments,
+                             num_heads, num_heads, dim, dim)
+    _count_recurrence(lib, "bonus", scratch is not None, dim, dim)
     _check(lib.tis_time_mix(_dt(rkvg), _p(rkvg), rkvg.stride(0), _p(w_in), w_in.stride(0), _p(u), _p(w_bias), _p(norm_weight),
                             _f(eps), _p(state), ctypes.c_size_t(state.stride(0)), _p(out), out.stride(0), _p(raw), _p(row_slot),
                             _p(row_last), n, num_heads, dim, int(narrow), _p(segments[0] if segments is not None else None),
