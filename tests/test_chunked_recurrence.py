@@ -230,3 +230,40 @@ def test_operands_that_the_chunks_do_not_take_are_walked(rule):
         assert ops.calls["recurrence_chunked"] == before
         assert ops.launches - launched == (1 if rule == "step" else 2)
         assert _off(got_o, want_o) < 3e-6 and _off(got_s, want_s) < 3e-6
+
+
+def _same_where_not_finite(got, walked):
+    """Infinities and NaN where the walk has them, and the same ones; elsewhere 32-bit sums of up to 128 products."""
+    assert torch.equal(torch.isnan(got), torch.isnan(walked))
+    inf = torch.isinf(walked)
+    assert torch.equal(got[inf], walked[inf]) and torch.equal(torch.isinf(got), inf)
+    fine = torch.isfinite(walked)
+    assert _off(got[fine], walked[fine]) < 3e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", RULES)
+@pytest.mark.parametrize("where", ["value", "key", "query", "decay", "state", "overflow"])
+def test_numbers_that_are_not_finite_are_what_the_walk_makes_of_them(rule, where):
+    from tiny_inference_server_b200.kernels import ops
+    if (where, rule) == ("overflow", "forget"):
+        pytest.skip("keys below 1: sums that end near the largest number, and how a sum is grouped decides whether it passes it")
+    case = Case(rule, 64, 64, (200, 40, 129), torch.float32, seed=11)
+    G, K, H, V = case.G, 64, case.H, 64
+    at = {"query": 3, "key": G * K + 3, "value": (G if rule == "forget" else 2 * G) * K + 2 * V + 5}
+    if where == "state":
+        case.state[case.order[0], 2 * K * V + 7 * V + 9] = math.inf
+    elif where == "decay":
+        case.a[77, case.a.shape[1] - 1] = math.nan
+    elif where == "overflow":                                               # each finite, their sums not
+        case.rows[60:90, at["value"]] = 3e38
+        case.rows[60:90, at["key"]:at["key"] + 40] = 30.0
+    else:
+        case.rows[100, at[where]] = math.inf
+        case.rows[240 + 100, at[where] + 1] = -math.inf
+    walked = case.call(ops, case.segments(False))
+    before = ops.calls["recurrence_chunked"]
+    got = case.call(ops, case.segments(True))
+    assert ops.calls["recurrence_chunked"] == before + 1
+    for g, w in zip(got, walked):
+        _same_where_not_finite(g, w)

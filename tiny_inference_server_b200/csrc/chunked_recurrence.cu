@@ -19,7 +19,13 @@
 //
 // Every product of decays is a product of factors <= 1 in the direction the tokens run (within sub-chunks of 16 tokens,
 // over whole sub-chunks between them): nothing is divided by a decay, so a decay of zero and a long product that
-// underflows are what they are in the walk.  No token's output meets a later token's vectors, not even times zero.
+// underflows are what they are in the walk.
+//
+// Numbers that are not finite take other ways through these products than through the walk (a masked zero times an infinity;
+// an infinity split in three).  Every one of them, and every sum that overflows on the way, leaves something that is not
+// finite in the outputs of its chunk or in the state behind the portion: those two places are looked at, and the walk
+// (delta_rule_kernel in seqmix.cu) takes the marked heads of a portion again from the state they began with, which is
+// still in the scratch as the state in front of the first chunk.
 // Operands, states and sums are 32-bit, with 32-bit and with bfloat16 activations alike: the state goes on from step to step
 // whatever the activations are.  The dense products run on the tensor cores as bfloat16 products of operands split in
 // three, whose parts hold all 24 bits (mma_split); products of decays are kept as sums of two numbers until they are used.
@@ -30,7 +36,7 @@
 // shared memory for every one to four multiply-adds, the kernels took longer (delta rule, 2048 tokens, 12 heads of 128 x 128,
 // a layer: 422 us; 271 in tf32, 311 now).
 // Straight-line code is kept short: a kernel's code is read anew at every launch, and unrolled over a chunk's tokens the
-// exponentials of the preparation took longer to fetch than to run.  A product of a masked zero and a number that is not finite would not be zero: blocks on the diagonal look at their operands first.
+// exponentials of the preparation took longer to fetch than to run.
 #include "recurrence.cuh"
 
 namespace {
@@ -155,9 +161,10 @@ __device__ __forceinline__ int segment_rows(const ChunkArgs& p, int seg, int& ro
     if (slot < 0 || (row0 > 0 && p.row_slot[row0 - 1] == slot)) return 0;
     return p.row_last[row0] - row0 + 1;
 }
-// Where chunk `chunk` of the step lies (all lanes of a warp together): its first row and number of rows; false: there is
-// no such chunk (the grid is sized by an upper bound).
-__device__ __forceinline__ bool find_chunk(const ChunkArgs& p, int chunk, int& row0, int& rows) {
+// Where chunk `chunk` of the step lies (all lanes of a warp together): its first row and number of rows, its segment and that
+// segment's first chunk; false: there is no such chunk (the grid is sized by an upper bound).
+struct Chunk { int row0, rows, segment, first; };
+__device__ __forceinline__ bool find_chunk(const ChunkArgs& p, int chunk, Chunk& at_chunk) {
     const int lane = threadIdx.x & 31;
     int before = 0;
     for (int s0 = 0; s0 < p.segments; s0 += 32) {
@@ -174,8 +181,10 @@ __device__ __forceinline__ bool find_chunk(const ChunkArgs& p, int chunk, int& r
         if (past) {
             const int at = __ffs(past) - 1;
             const int in_segment = chunk - before - __shfl_sync(0xffffffffu, upto - mine, at);
-            row0 = __shfl_sync(0xffffffffu, first, at) + in_segment * C;
-            rows = min(C, __shfl_sync(0xffffffffu, count, at) - in_segment * C);
+            at_chunk.row0 = __shfl_sync(0xffffffffu, first, at) + in_segment * C;
+            at_chunk.rows = min(C, __shfl_sync(0xffffffffu, count, at) - in_segment * C);
+            at_chunk.segment = s0 + at;
+            at_chunk.first = chunk - in_segment;
             return true;
         }
         before += __shfl_sync(0xffffffffu, upto, 31);
@@ -215,9 +224,19 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
     float* M = powers + C + 4;                              // diag(beta) L below the diagonal, sub-chunk by sub-chunk
     pdl_launch_dependents();
     const int head = blockIdx.x, chunk = blockIdx.y;
-    int row0, rows;
-    if (!find_chunk(p, chunk, row0, rows)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fc = lane & 3;
+    Chunk here;
+    const bool there = find_chunk(p, chunk, here);
+    if (chunk == 0) {                                       // nothing is to be taken again so far; who takes which rows
+        pdl_wait();
+        for (int seg = tid; seg < p.all_segments; seg += 256) {
+            const int r = p.seg_row0[seg];
+            if (seg < p.segments) p.again[seg * p.H + head] = 0;
+            if (p.row_slot[r] >= 0) p.chunked[(size_t)p.row_last[r] * p.H + head] = seg < p.segments;
+        }
+    }
+    if (!there) return;
+    const int row0 = here.row0, rows = here.rows;
     const int kvh = head / (p.H / p.G), mode = p.mode;
     const bool forget = mode == DECAY_FORGET_GATE, plain = mode == DECAY_CONSTANT, bonus = mode == DECAY_BONUS;
     const bool per_head = mode == DECAY_PER_HEAD || mode == DECAY_STEP;
@@ -561,46 +580,16 @@ __global__ void __launch_bounds__(256, 2) chunk_prepare_kernel(const ChunkArgs p
                 for (int i = 0; i < 2; ++i)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) y[i][e] = x[2 * a + i][e] - less[i][e];
-                bool fine = true;
+                FragA f;
+                f.set(y[0][0], y[0][2], y[0][1], y[0][3], y[1][0], y[1][2], y[1][1], y[1][3]);
+                float more[2][4] = {};
+                mma_split<2>(more, f, [&](int i, FragB& o) {
+                    const float2 v = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + a * SUB);
+                    const float2 w = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + a * SUB + 8);
+                    o.set(v.x, v.y, w.x, w.y);
+                });
 #pragma unroll
-                for (int e = 0; e < 4; ++e) fine = fine && finite_f(y[0][e]) && finite_f(y[1][e]);
-                float r[2][4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) { r[0][e] = y[0][e]; r[1][e] = y[1][e]; }
-                if (__all_sync(0xffffffffu, fine)) {
-                    FragA f;
-                    f.set(r[0][0], r[0][2], r[0][1], r[0][3], r[1][0], r[1][2], r[1][1], r[1][3]);
-                    float more[2][4] = {};
-                    mma_split<2>(more, f, [&](int i, FragB& o) {
-                        const float2 v = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + a * SUB);
-                        const float2 w = *reinterpret_cast<const float2*>(m + 8 * i * m_row(a) + a * SUB + 8);
-                        o.set(v.x, v.y, w.x, w.y);
-                    });
-#pragma unroll
-                    for (int i = 0; i < 2; ++i)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) y[i][e] += more[i][e];
-                } else {                                    // token by token: none meets a later one
-                    const float* own = M + m_at(a) + a * SUB;
-                    for (int s = 0; s < SUB; ++s) {
-                        const int from = (lane & ~3) | ((s & 7) >> 1);
-                        float rs[2];
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            const float even = s < 8 ? r[0][2 * i] : r[1][2 * i], odd = s < 8 ? r[0][2 * i + 1] : r[1][2 * i + 1];
-                            rs[i] = __shfl_sync(0xffffffffu, (s & 1) ? odd : even, from);
-                        }
-#pragma unroll
-                        for (int j = 0; j < 2; ++j)
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int t = 8 * j + 2 * fc + (e & 1);
-                                if (t > s) y[j][e] = fmaf(own[t * m_row(a) + s], rs[e >> 1], y[j][e]);
-                            }
-                    }
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) { x[2 * a][e] = y[0][e]; x[2 * a + 1][e] = y[1][e]; }
+                for (int e = 0; e < 4; ++e) { x[2 * a][e] = y[0][e] + more[0][e]; x[2 * a + 1][e] = y[1][e] + more[1][e]; }
             }
             float* dst = key ? p.w + unit * C * K : ub;
             const int ldd = key ? K : V;
@@ -698,6 +687,7 @@ __global__ void __launch_bounds__(256) chunk_state_kernel(const ChunkArgs p) {
         }
     }
     *reinterpret_cast<float4*>(dst) = S;
+    if (!(finite_f(S.x) && finite_f(S.y) && finite_f(S.z) && finite_f(S.w))) p.again[blockIdx.z * p.H + head] = first + 1;
 }
 
 template <int K, int NT> struct DeltaSmem {
@@ -818,12 +808,16 @@ __global__ void __launch_bounds__(256, 1) chunk_delta_kernel(const ChunkArgs p) 
                 for (int e = 0; e < 4; ++e) s[j][e] = fmaf(s[j][e], e < 2 ? g0 : g1, acc[j][e]);
         }
     }
+    bool fine = true;
 #pragma unroll
     for (int j = 0; j < SN; ++j)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < 2; ++h) {
             *reinterpret_cast<float2*>(state + (size_t)(sm + fr + 8 * h) * V + sn + 8 * j + 2 * fc) =
                 make_float2(s[j][2 * h], s[j][2 * h + 1]);
+            fine = fine && finite_f(s[j][2 * h]) && finite_f(s[j][2 * h + 1]);
+        }
+    if (!fine) p.again[blockIdx.z * p.H + head] = first + 1;
 }
 
 constexpr int OUT_TILE = 32;                    // of the sum, a stage of chunk_output_kernel
@@ -843,8 +837,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 3) chunk_output_kern
     T* gs = reinterpret_cast<T*>(ys + 2 * KT * YROW);       // [C][V]
     pdl_launch_dependents();
     const int head = blockIdx.x, chunk = blockIdx.y;
-    int row0, rows;
-    if (!find_chunk(p, chunk, row0, rows)) return;
+    Chunk here;
+    if (!find_chunk(p, chunk, here)) return;
+    const int row0 = here.row0, rows = here.rows;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, fr = lane >> 2, fc = lane & 3;
     const int a = warp & 3, r0 = a * SUB + fr, n0 = (warp >> 2) * (V / 2);
     const size_t unit = (size_t)chunk * p.H + head;
@@ -893,32 +888,16 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 3) chunk_output_kern
         }
         const int d0 = a * SUB - s0;                        // where the warp's own tokens lie in this tile
         if (s0 >= 0 && d0 >= 0 && d0 < KT) {
-            bool fine = true;
+            const int k = d0 + fc;
+            float v[8];                                 // a token sees those up to itself
 #pragma unroll
-            for (int j = 0; j < SUB; j += 4)
-#pragma unroll
-                for (int i = 0; i < NT; ++i) fine = fine && finite_f(y[(d0 + j + fc) * YROW + 8 * i]);
-            if (__all_sync(0xffffffffu, fine)) {
-                const int k = d0 + fc;
-                float v[8];                                 // a token sees those up to itself
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    v[2 * e] = fr >= fc + 4 * e ? x[k + 4 * e] : 0.f;
-                    v[2 * e + 1] = fr + 8 >= fc + 4 * e ? x[8 * XROW + k + 4 * e] : 0.f;
-                }
-                FragA f;
-                f.set(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
-                mma_split<NT>(acc, f, [&](int i, FragB& o) { column(k, i, o); });
-            } else {
-                const float* yt = ys + (tile & 1) * KT * YROW + n0 + 2 * fc;
-                for (int s = 0; s < SUB; ++s)
-#pragma unroll
-                    for (int i = 0; i < NT; ++i)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            if (fr + 8 * (e >> 1) >= s)
-                                acc[i][e] = fmaf(x[8 * (e >> 1) * XROW + d0 + s], yt[(d0 + s) * YROW + 8 * i + (e & 1)], acc[i][e]);
+            for (int e = 0; e < 4; ++e) {
+                v[2 * e] = fr >= fc + 4 * e ? x[k + 4 * e] : 0.f;
+                v[2 * e + 1] = fr + 8 >= fc + 4 * e ? x[8 * XROW + k + 4 * e] : 0.f;
             }
+            FragA f;
+            f.set(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+            mma_split<NT>(acc, f, [&](int i, FragB& o) { column(k, i, o); });
         }
         __syncthreads();
     }
@@ -926,6 +905,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 3) chunk_output_kern
     // through shared memory, so that a warp has eight whole tokens: their norms, gates and stores
     constexpr int OROW = V + 4, VC = V / 32;
     float* os = smem;                                       // [C][OROW], over the tiles
+    bool fine = true;
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) fine = fine && finite_f(acc[i][e]);
+    if (!fine) p.again[here.segment * p.H + head] = here.first + 1;
 #pragma unroll
     for (int i = 0; i < NT; ++i)
 #pragma unroll
@@ -1005,47 +990,48 @@ bool chunked_recurrence_takes(int dtype, const ChunkArgs& p, int k_dim, int v_di
     if (!raw) bases |= (uintptr_t)p.gate | (uintptr_t)p.out;
     else bases |= (uintptr_t)p.o_raw;
     const bool chunks_fit = p.segments > 0 && p.segments <= 65535 && p.H > 0 && p.H <= 65535 && p.G > 0 &&
-                            p.H % p.G == 0 && p.n / C + p.segments <= 65535;
+                            p.H % p.G == 0 && p.n > 0 && p.n / C + p.segments <= 65535;
     return chunks_fit && (k_dim == 64 || k_dim == 128) && (v_dim == 64 || v_dim == 128) && (dtype == TIS_F32 || dtype == TIS_BF16) &&
            bases % 16 == 0 && p.ld % 8 == 0 && (head_step || p.lda % 8 == 0) && p.state_stride % 4 == 0 &&
            (raw || (p.ldo % 8 == 0 && (p.gate == nullptr || p.ldg % 8 == 0)));
 }
 
-static size_t chunk_floats(const ChunkArgs& p, int k_dim, int v_dim) {
-    const bool delta = p.mode == DECAY_PER_CHANNEL || p.mode == DECAY_PER_HEAD;
-    const size_t units = ((size_t)p.n / C + p.segments) * p.H;
-    return units * ((size_t)C * k_dim * (delta ? 3 : 1) + (size_t)C * v_dim + (size_t)C * C + (size_t)k_dim * v_dim + k_dim);
-}
-// Floats of scratch for a step of n rows in `segments` requests; 0: the chunked kernels do not take these operands (o_raw lies on
-// a 16-byte boundary).
-TIS_API size_t tis_chunked_recurrence_floats(int dtype, int mode, const void* qkv, int ld, const void* a_in, int lda, const void* gate,
-                                             int ldg, const void* out, int ldo, const float* state, size_t state_stride, int n,
-                                             int segments, int H, int G, int k_dim, int v_dim) {
-    ChunkArgs p = {};
-    p.qkv = qkv; p.ld = ld; p.a_in = a_in; p.lda = lda; p.gate = gate; p.ldg = ldg; p.out = const_cast<void*>(out); p.ldo = ldo;
-    p.state = const_cast<float*>(state); p.state_stride = state_stride; p.n = n; p.segments = segments; p.H = H; p.G = G; p.mode = mode;
-    return chunked_recurrence_takes(dtype, p, k_dim, v_dim) ? chunk_floats(p, k_dim, v_dim) : 0;
-}
-
-int chunked_recurrence(int dtype, ChunkArgs p, int k_dim, int v_dim, float* scratch, size_t scratch_floats, cudaStream_t stream) {
+// Floats of scratch for p.n rows in p.segments portions of a step of p.all_rows rows, and the arrays in it.
+static size_t chunk_arrays(ChunkArgs& p, int k_dim, int v_dim, float* scratch) {
     const bool delta = p.mode == DECAY_PER_CHANNEL || p.mode == DECAY_PER_HEAD;
     p.chunks = p.n / C + p.segments;
-    if (scratch == nullptr || (uintptr_t)scratch % 16 != 0 ||
-        scratch_floats < chunk_floats(p, k_dim, v_dim)) {
+    const size_t units = (size_t)p.chunks * p.H;
+    size_t at = 0;
+    auto take = [&](size_t floats) { float* r = scratch + at; at += (floats + 3) / 4 * 4; return r; };
+    p.s = take(units * k_dim * v_dim);
+    p.qb = take(units * C * k_dim);
+    p.u = take(units * C * v_dim);
+    p.a = take(units * C * C);
+    p.decay = take(units * k_dim);
+    p.w = delta ? take(units * C * k_dim) : nullptr;
+    p.kd = delta ? take(units * C * k_dim) : nullptr;
+    p.again = reinterpret_cast<int*>(take((size_t)p.segments * p.H));
+    p.chunked = reinterpret_cast<int*>(take((size_t)p.all_rows * p.H));
+    return at;
+}
+// Floats of scratch for `rows` rows in `segments` portions of a step of `all_rows` rows; 0: the chunked kernels do not take these
+// operands (o_raw lies on a 16-byte boundary).
+TIS_API size_t tis_chunked_recurrence_floats(int dtype, int mode, const void* qkv, int ld, const void* a_in, int lda, const void* gate,
+                                             int ldg, const void* out, int ldo, const float* state, size_t state_stride, int rows,
+                                             int segments, int all_rows, int H, int G, int k_dim, int v_dim) {
+    ChunkArgs p = {};
+    p.qkv = qkv; p.ld = ld; p.a_in = a_in; p.lda = lda; p.gate = gate; p.ldg = ldg; p.out = const_cast<void*>(out); p.ldo = ldo;
+    p.state = const_cast<float*>(state); p.state_stride = state_stride; p.n = rows; p.segments = segments; p.all_rows = all_rows;
+    p.H = H; p.G = G; p.mode = mode;
+    return chunked_recurrence_takes(dtype, p, k_dim, v_dim) ? chunk_arrays(p, k_dim, v_dim, nullptr) : 0;
+}
+
+int chunked_recurrence(int dtype, ChunkArgs& p, int k_dim, int v_dim, float* scratch, size_t scratch_floats, cudaStream_t stream) {
+    if (scratch == nullptr || (uintptr_t)scratch % 16 != 0 || scratch_floats < chunk_arrays(p, k_dim, v_dim, scratch)) {
         tis_set_error("chunked recurrence: %zu floats of scratch for %d rows of %d requests, %d heads", scratch_floats, p.n,
                       p.segments, p.H);
         return TIS_BAD_SIZE;
     }
-    const size_t units = (size_t)p.chunks * p.H;
-    float* at = scratch;
-    auto take = [&](size_t floats) { float* r = at; at += units * floats; return r; };
-    p.s = take((size_t)k_dim * v_dim);
-    p.qb = take((size_t)C * k_dim);
-    p.u = take((size_t)C * v_dim);
-    p.a = take((size_t)C * C);
-    p.decay = take((size_t)k_dim);
-    p.w = delta ? take((size_t)C * k_dim) : nullptr;
-    p.kd = delta ? take((size_t)C * k_dim) : nullptr;
 #define TIS_CHUNKED(K, V) \
     if (k_dim == K && v_dim == V) TIS_DISPATCH_DTYPE(dtype, T, return (launch_chunked<T, K, V>(p, stream)));
     TIS_CHUNKED(64, 64)

@@ -26,7 +26,11 @@ __device__ __forceinline__ float gate_f(float x, int act) { const float s = 1.f 
 enum { DECAY_PER_CHANNEL = 0, DECAY_PER_HEAD = 1, DECAY_CONSTANT = 2, DECAY_FORGET_GATE = 3, DECAY_LOG_SIGMOID = 4,
        DECAY_STEP = 5, DECAY_BONUS = 6 };
 
-// What the three kernels of the chunked form get (chunked_recurrence.cu).  Scratch arrays are indexed by (chunk, head).
+// What the kernels of the chunked form get (chunked_recurrence.cu): the first `segments` of the `all_segments` requests of a
+// step of `all_rows` rows, n rows at most.  Scratch arrays are indexed by (chunk, head), but for
+//   again    (segment, head): 0, or 1 + the first chunk of a portion that the walk has to take again, because numbers
+//            that are not finite came up in it, from the state that `s` holds for that chunk
+//   chunked  (last row of a request, head): whether its rows are the chunked form's
 constexpr int REC_CHUNK = 64;
 struct ChunkArgs {
     const void* qkv; int ld;
@@ -39,10 +43,11 @@ struct ChunkArgs {
     void* out; int ldo;
     float* o_raw;
     const int *row_slot, *row_last, *seg_row0;
-    int segments, n, H, G, mode, gate_act, chunks;
+    int segments, all_segments, n, all_rows, H, G, mode, gate_act, chunks;
     float *qb, *kd, *w, *u, *a, *s, *decay;
+    int *again, *chunked;
 };
 // Whether the chunked kernels take these widths, and, if so, whether these operands: 16-byte rows and states.
 bool chunked_recurrence_takes(int dtype, const ChunkArgs& args, int k_dim, int v_dim);
-// Launches them; `scratch` holds tis_chunked_recurrence_floats(...) floats.
-int chunked_recurrence(int dtype, ChunkArgs args, int k_dim, int v_dim, float* scratch, size_t scratch_floats, cudaStream_t stream);
+// Launches them (scratch: tis_chunked_recurrence_floats), and leaves the arrays in the scratch in `args`.
+int chunked_recurrence(int dtype, ChunkArgs& args, int k_dim, int v_dim, float* scratch, size_t scratch_floats, cudaStream_t stream);

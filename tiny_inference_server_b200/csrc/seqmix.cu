@@ -793,10 +793,19 @@ delta_rule_kernel(const T* __restrict__ qkv, int ld, const T* __restrict__ b_in,
                   const float* __restrict__ dt_bias, const float* __restrict__ norm_w, float eps, float unit_eps,
                   float q_scale, float* __restrict__ state, size_t state_stride, T* __restrict__ out, int ldo,
                   const int* __restrict__ row_slot, const int* __restrict__ row_last, int H, int G, int k_dim_rt,
-                  int v_dim, int decay_mode, int gate_act, float* __restrict__ o_raw, int state_in_place) {
+                  int v_dim, int decay_mode, int gate_act, float* __restrict__ o_raw, int state_in_place,
+                  const int* __restrict__ seg_row0, const int* __restrict__ again, const float* __restrict__ again_state) {
     extern __shared__ float smem[];
     pdl_launch_dependents();
-    const int head = blockIdx.x, r0 = blockIdx.y;
+    // grid.y: every row (the CTAs of rows that are not the first of their request leave at once), or the requests of
+    // `seg_row0`, of which only those heads are walked that `again` marks (ChunkArgs), from the state in `again_state`
+    const int head = blockIdx.x, r0 = seg_row0 != nullptr ? seg_row0[blockIdx.y] : (int)blockIdx.y;
+    int from = 0;
+    if (again != nullptr) {
+        pdl_wait();
+        from = again[blockIdx.y * H + head];
+        if (from == 0) return;
+    }
     const int slot = row_slot[r0];
     if (slot < 0) return;
     if (r0 > 0 && row_slot[r0 - 1] == slot) return;
@@ -826,12 +835,13 @@ delta_rule_kernel(const T* __restrict__ qkv, int ld, const T* __restrict__ b_in,
     constexpr int REG = DIM > 0 ? DIM : 1;
     float S[REG];
     pdl_wait();
+    const float* S_from = again != nullptr ? again_state + ((size_t)(from - 1) * H + head) * k_dim * v_dim : S_glob;
     if (tid < v_dim) {
         if (DIM > 0) {
 #pragma unroll
-            for (int i = 0; i < REG; ++i) S[i] = S_glob[(size_t)i * v_dim + tid];
+            for (int i = 0; i < REG; ++i) S[i] = S_from[(size_t)i * v_dim + tid];
         } else if (!in_place) {
-            for (int i = 0; i < k_dim; ++i) S_sh[i * v_dim + tid] = S_glob[(size_t)i * v_dim + tid];
+            for (int i = 0; i < k_dim; ++i) S_sh[i * v_dim + tid] = S_from[(size_t)i * v_dim + tid];
         }
     }
     const int q_off = kvh * k_dim, k_off = G * k_dim + kvh * k_dim, v_off = (forget ? 1 : 2) * G * k_dim + head * v_dim;
@@ -1334,18 +1344,19 @@ delta_rule_split_kernel(const T* __restrict__ qkv, int ld, const T* __restrict__
 }
 
 // out[r, head, :] = o / sqrt(mean(o^2) + eps) * norm_w * act(gate) for every (row, head): a warp each.  own_weights: norm_w
-// holds v_dim weights for every head, else v_dim for all of them.
+// holds v_dim weights for every head, else v_dim for all of them.  `chunked` (null: none; ChunkArgs): rows that are done.
 template <typename T>
 __global__ void __launch_bounds__(128)
 delta_out_norm_kernel(const float* __restrict__ o_raw, const T* __restrict__ gate, int ldg, const float* __restrict__ norm_w,
                       float eps, T* __restrict__ out, int ldo, const int* __restrict__ row_slot, int n, int H, int v_dim,
-                      int gate_act, int own_weights) {
+                      int gate_act, int own_weights, const int* __restrict__ row_last, const int* __restrict__ chunked) {
     pdl_launch_dependents();
     const int idx = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (idx >= n * H) return;
     const int r = idx / H, head = idx - r * H;
     if (row_slot[r] < 0) return;
     pdl_wait();
+    if (chunked != nullptr && chunked[(size_t)row_last[r] * H + head] != 0) return;
     const float* o = o_raw + (size_t)r * H * v_dim + (size_t)head * v_dim;
     const float* w = norm_w + (own_weights ? (size_t)head * v_dim : 0);
     float ss = 0.f;
@@ -1408,7 +1419,8 @@ static int launch_delta_rule_split(const T* qkv, int ld, const T* b_in, int ldb,
                                    const float* A_log, const float* dt_bias, const float* norm_w, float eps, float unit_eps,
                                    float q_scale, float* state, size_t state_stride, T* out, int ldo, float* o_raw,
                                    const int* row_slot, const int* row_last, const int* seg_row0, int segments, int n,
-                                   int H, int G, int v_dim, int decay_mode, int gate_act, cudaStream_t stream) {
+                                   int H, int G, int v_dim, int decay_mode, int gate_act, const int* chunked,
+                                   cudaStream_t stream) {
     const dim3 grid(H, v_dim / COLS, seg_row0 != nullptr ? segments : n);
     if (decay_mode == DECAY_CONSTANT)
         tis_launch(delta_rule_split_kernel<T, DL, LANES, COLS, 1>, grid, dim3(COLS * LANES), 0, stream, qkv, ld, b_in, ldb, a_in,
@@ -1442,7 +1454,7 @@ static int launch_delta_rule_split(const T* qkv, int ld, const T* b_in, int ldb,
         return tis_check_launch("row_out_norm");
     }
     tis_launch(delta_out_norm_kernel<T>, dim3((n * H + 3) / 4), dim3(128), 0, stream, (const float*)o_raw, gate, ldg, norm_w, eps,
-               out, ldo, row_slot, n, H, v_dim, gate_act, (int)(decay_mode == DECAY_BONUS));
+               out, ldo, row_slot, n, H, v_dim, gate_act, (int)(decay_mode == DECAY_BONUS), row_last, chunked);
     return tis_check_launch("delta_out_norm");
 }
 
@@ -1451,7 +1463,8 @@ static int launch_delta_rule(const T* qkv, int ld, const T* b_in, int ldb, const
                              const float* A_log, const float* dt_bias, const float* norm_w, float eps, float unit_eps,
                              float q_scale, float* state, size_t state_stride, T* out, int ldo, const int* row_slot,
                              const int* row_last, int n, int H, int G, int k_dim, int v_dim, int decay_mode, int gate_act,
-                             float* o_raw, cudaStream_t stream) {
+                             float* o_raw, cudaStream_t stream, const int* seg_row0 = nullptr, int segments = 0,
+                             const int* again = nullptr, const float* again_state = nullptr) {
     int threads = (v_dim + 31) / 32 * 32;
     if (threads < 128) threads = 128;                  // warps to prepare and normalise a chunk with
     size_t smem = sizeof(float) * ((size_t)DELTA_CHUNK * (3 * k_dim + 2 * v_dim + 1) + (DIM > 0 ? 0 : (size_t)k_dim * v_dim));
@@ -1466,12 +1479,13 @@ static int launch_delta_rule(const T* qkv, int ld, const T* b_in, int ldb, const
     }
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(delta_rule_kernel<T, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    tis_launch(delta_rule_kernel<T, DIM>, dim3(H, n), dim3(threads), smem, stream, qkv, ld, b_in, ldb, a_in, lda, gate, ldg,
+    tis_launch(delta_rule_kernel<T, DIM>, dim3(H, seg_row0 != nullptr ? segments : n), dim3(threads), smem, stream, qkv, ld, b_in, ldb, a_in, lda, gate, ldg,
                A_log, dt_bias, norm_w, eps, unit_eps, q_scale, state, state_stride, out, ldo, row_slot, row_last, H, G,
                k_dim, v_dim, decay_mode, gate_act,
-               (decay_mode == DECAY_CONSTANT || decay_mode == DECAY_STEP) ? o_raw : (float*)nullptr, in_place);
+               (decay_mode == DECAY_CONSTANT || decay_mode == DECAY_STEP) ? o_raw : (float*)nullptr, in_place, seg_row0, again,
+               again_state);
     int st = tis_check_launch("delta_rule");
-    if (st != TIS_OK || decay_mode != DECAY_CONSTANT) return st;
+    if (st != TIS_OK || decay_mode != DECAY_CONSTANT || again != nullptr) return st;
     tis_launch(row_out_norm_kernel<T>, dim3(n), dim3(256), 0, stream, (const float*)o_raw, gate, ldg, norm_w, eps, out, ldo,
                row_slot, H * v_dim);
     return tis_check_launch("row_out_norm");
@@ -1489,7 +1503,8 @@ static int matrix_state_recurrence(int dtype, const void* qkv, int ld, const voi
                                    float eps, float unit_eps, float q_scale, float* state, size_t state_stride, void* out,
                                    int ldo, float* o_raw, const int* row_slot, const int* row_last, int n, int H, int G,
                                    int k_dim, int v_dim, int narrow, const int* seg_row0, int segments, int decay_mode,
-                                   int gate_act, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
+                                   int gate_act, float* chunk_scratch, size_t chunk_floats, int chunk_segments,
+                                   int chunk_rows, cudaStream_t stream) {
     if (n <= 0) return TIS_OK;
     if (decay_mode < DECAY_PER_CHANNEL || decay_mode > DECAY_BONUS || gate_act < 0 || gate_act > 1 ||
         ((decay_mode == DECAY_CONSTANT || decay_mode == DECAY_STEP) && o_raw == nullptr)) {
@@ -1501,23 +1516,39 @@ static int matrix_state_recurrence(int dtype, const void* qkv, int ld, const voi
         tis_set_error("delta_rule: %d rows in one step (at most 65535)", n);
         return TIS_BAD_SIZE;
     }
-    if (chunk_scratch != nullptr) {                     // long portions: in chunks of tokens (chunked_recurrence.cu)
+    const int* chunked = nullptr;
+    if (chunk_scratch != nullptr) {                     // the first requests of the list in chunks of tokens (chunked_recurrence.cu)
         ChunkArgs p = {};
         p.qkv = qkv; p.ld = ld; p.b_in = b_in; p.ldb = ldb; p.a_in = a_in; p.lda = lda; p.gate = gate; p.ldg = ldg;
         p.A_log = A_log; p.dt_bias = dt_bias; p.norm_w = norm_w; p.eps = eps; p.unit_eps = unit_eps; p.q_scale = q_scale;
         p.state = state; p.state_stride = state_stride; p.out = out; p.ldo = ldo; p.o_raw = o_raw; p.row_slot = row_slot;
-        p.row_last = row_last; p.seg_row0 = seg_row0; p.segments = segments; p.n = n; p.H = H; p.G = G; p.mode = decay_mode;
-        p.gate_act = gate_act;
-        if (seg_row0 == nullptr || !chunked_recurrence_takes(dtype, p, k_dim, v_dim)) {
-            tis_set_error("chunked recurrence: %d rows of %d heads in %d requests, widths %d and %d, or operands that are not aligned",
-                          n, H, segments, k_dim, v_dim);
+        p.row_last = row_last; p.seg_row0 = seg_row0; p.segments = chunk_segments; p.all_segments = segments; p.n = chunk_rows;
+        p.all_rows = n; p.H = H; p.G = G; p.mode = decay_mode; p.gate_act = gate_act;
+        if (seg_row0 == nullptr || chunk_segments > segments || chunk_rows > n || !chunked_recurrence_takes(dtype, p, k_dim, v_dim) ||
+            (chunk_segments < segments && o_raw == nullptr)) {
+            tis_set_error("chunked recurrence: %d rows of %d heads in %d of %d requests, widths %d and %d, or operands that are "
+                          "not aligned", chunk_rows, H, chunk_segments, segments, k_dim, v_dim);
             return TIS_BAD_SIZE;
         }
-        const int st = chunked_recurrence(dtype, p, k_dim, v_dim, chunk_scratch, chunk_floats, stream);
-        if (st != TIS_OK || decay_mode != DECAY_CONSTANT) return st;
-        TIS_DISPATCH_DTYPE(dtype, T, tis_launch(row_out_norm_kernel<T>, dim3(n), dim3(256), 0, stream, (const float*)o_raw,
-                           (const T*)gate, ldg, norm_w, eps, (T*)out, ldo, row_slot, H * v_dim));
-        return tis_check_launch("row_out_norm");
+        int st = chunked_recurrence(dtype, p, k_dim, v_dim, chunk_scratch, chunk_floats, stream);
+        if (st != TIS_OK) return st;
+        // the heads in which something was not finite, token by token
+#define TIS_WALK_AGAIN(D)                                                                                              \
+        TIS_DISPATCH_DTYPE(dtype, T, st = (launch_delta_rule<T, D>((const T*)qkv, ld, (const T*)b_in, ldb, (const T*)a_in, lda,       \
+            (const T*)gate, ldg, A_log, dt_bias, norm_w, eps, unit_eps, q_scale, state, state_stride, (T*)out, ldo, row_slot,         \
+            row_last, n, H, G, k_dim, v_dim, decay_mode, gate_act, o_raw, stream, seg_row0, chunk_segments, p.again, p.s)))
+        if (k_dim == 64) { TIS_WALK_AGAIN(64); } else { TIS_WALK_AGAIN(128); }
+#undef TIS_WALK_AGAIN
+        if (st != TIS_OK) return st;
+        if (chunk_segments == segments) {
+            if (decay_mode != DECAY_CONSTANT) return TIS_OK;
+            TIS_DISPATCH_DTYPE(dtype, T, tis_launch(row_out_norm_kernel<T>, dim3(n), dim3(256), 0, stream, (const float*)o_raw,
+                               (const T*)gate, ldg, norm_w, eps, (T*)out, ldo, row_slot, H * v_dim));
+            return tis_check_launch("row_out_norm");
+        }
+        seg_row0 += chunk_segments;                     // the others below
+        segments -= chunk_segments;
+        chunked = p.chunked;
     }
     // (the walk with a bonus reads its rows in 16-byte vectors)
     const bool rows_fit = decay_mode != DECAY_BONUS || (ld % 8 == 0 && lda % 8 == 0 && ((uintptr_t)qkv | (uintptr_t)a_in) % 16 == 0);
@@ -1527,7 +1558,7 @@ static int matrix_state_recurrence(int dtype, const void* qkv, int ld, const voi
         TIS_DISPATCH_DTYPE(dtype, T, return (launch_delta_rule_split<T, DL, LANES, COLS>((const T*)qkv, ld,            \
             (const T*)b_in, ldb, (const T*)a_in, lda, (const T*)gate, ldg, A_log, dt_bias, norm_w, eps, unit_eps,      \
             q_scale, state, state_stride, (T*)out, ldo, o_raw, row_slot, row_last, seg_row0, segments, n, H, G, v_dim,       \
-            decay_mode, gate_act, stream)));
+            decay_mode, gate_act, chunked, stream)));
         if (v_dim % 8 == 0 && narrow >= 2) {            // sixteen lanes a column, 8 columns a CTA: one or two requests
             TIS_DELTA_SPLIT(32, 2, 16, 8)
             TIS_DELTA_SPLIT(64, 4, 16, 8)
@@ -1579,8 +1610,8 @@ static int matrix_state_recurrence(int dtype, const void* qkv, int ld, const voi
     return TIS_OK;
 }
 
-// The entry points below: `chunk_scratch`, `chunk_floats` (tis_chunked_recurrence_floats of them; null: none): the step
-// is taken in chunks of tokens.
+// The entry points below: `chunk_scratch`, `chunk_floats` (tis_chunked_recurrence_floats of them; null: none): the first
+// `chunk_segments` requests of `seg_row0`, at most `chunk_rows` rows together, are taken in chunks of tokens, the others token by token.
 
 // The delta rule.  decay_per_head 0: `a_in` (n, H * k_dim) and `dt_bias` (H * k_dim), a decay per head and key channel;
 // 1: `a_in` (n, H) and `dt_bias` (H), one per head.  gate_act: 0 sigmoid, 1 silu.
@@ -1589,11 +1620,12 @@ TIS_API int tis_delta_rule(int dtype, const void* qkv, int ld, const void* b_in,
                            float eps, float unit_eps, float q_scale, float* state, size_t state_stride, void* out,
                            int ldo, float* o_raw, const int* row_slot, const int* row_last, int n, int H, int G,
                            int k_dim, int v_dim, int narrow, const int* seg_row0, int segments, int decay_per_head,
-                           int gate_act, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
+                           int gate_act, float* chunk_scratch, size_t chunk_floats, int chunk_segments,
+                                       int chunk_rows, cudaStream_t stream) {
     return matrix_state_recurrence(dtype, qkv, ld, b_in, ldb, a_in, lda, gate, ldg, A_log, dt_bias, norm_w, eps, unit_eps,
                                    q_scale, state, state_stride, out, ldo, o_raw, row_slot, row_last, n, H, G, k_dim, v_dim,
                                    narrow, seg_row0, segments, decay_per_head ? DECAY_PER_HEAD : DECAY_PER_CHANNEL, gate_act,
-                                   chunk_scratch, chunk_floats, stream);
+                                   chunk_scratch, chunk_floats, chunk_segments, chunk_rows, stream);
 }
 
 // Linear attention with a constant decay per head (`decay`, H numbers): S <- decay S + silu(k) silu(v)^T, o = S^T silu(q);
@@ -1602,10 +1634,11 @@ TIS_API int tis_delta_rule(int dtype, const void* qkv, int ld, const void* b_in,
 TIS_API int tis_linear_attention(int dtype, const void* qkv, int ld, const void* gate, int ldg, const float* decay,
                                  const float* norm_w, float eps, float* state, size_t state_stride, void* out, int ldo,
                                  float* o_raw, const int* row_slot, const int* row_last, int n, int H, int k_dim, int v_dim,
-                                 int narrow, const int* seg_row0, int segments, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
+                                 int narrow, const int* seg_row0, int segments, float* chunk_scratch, size_t chunk_floats, int chunk_segments,
+                                       int chunk_rows, cudaStream_t stream) {
     return matrix_state_recurrence(dtype, qkv, ld, nullptr, 0, nullptr, 0, gate, ldg, decay, nullptr, norm_w, eps, 0.f, 1.f,
                                    state, state_stride, out, ldo, o_raw, row_slot, row_last, n, H, H, k_dim, v_dim, narrow,
-                                   seg_row0, segments, DECAY_CONSTANT, 0, chunk_scratch, chunk_floats, stream);
+                                   seg_row0, segments, DECAY_CONSTANT, 0, chunk_scratch, chunk_floats, chunk_segments, chunk_rows, stream);
 }
 
 // The recurrence with a forget gate per head and key channel (DECAY_FORGET_GATE): a row of `qv` holds the queries of H
@@ -1616,10 +1649,11 @@ TIS_API int tis_forget_gate_recurrence(int dtype, const void* qv, int ld, const 
                                        const float* f_bias, const float* norm_w, float eps, float* state,
                                        size_t state_stride, void* out, int ldo, float* o_raw, const int* row_slot,
                                        const int* row_last, int n, int H, int k_dim, int v_dim, int narrow,
-                                       const int* seg_row0, int segments, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
+                                       const int* seg_row0, int segments, float* chunk_scratch, size_t chunk_floats, int chunk_segments,
+                                       int chunk_rows, cudaStream_t stream) {
     return matrix_state_recurrence(dtype, qv, ld, nullptr, 0, f_in, ldf, nullptr, 0, lower, f_bias, norm_w, eps, 0.f, 1.f,
                                    state, state_stride, out, ldo, o_raw, row_slot, row_last, n, H, H, k_dim, v_dim, narrow,
-                                   seg_row0, segments, DECAY_FORGET_GATE, 0, chunk_scratch, chunk_floats, stream);
+                                   seg_row0, segments, DECAY_FORGET_GATE, 0, chunk_scratch, chunk_floats, chunk_segments, chunk_rows, stream);
 }
 
 // Gated linear attention (DECAY_LOG_SIGMOID): a row of `qkv` holds the queries and keys of H heads (k_dim each) and the
@@ -1631,10 +1665,11 @@ TIS_API int tis_gated_linear_attention(int dtype, const void* qkv, int ld, const
                                        const float* a_bias, const void* gate, int ldg, const float* norm_w, float eps,
                                        float q_scale, float* state, size_t state_stride, void* out, int ldo, float* o_raw,
                                        const int* row_slot, const int* row_last, int n, int H, int k_dim, int v_dim,
-                                       int narrow, const int* seg_row0, int segments, int gate_act, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
+                                       int narrow, const int* seg_row0, int segments, int gate_act, float* chunk_scratch, size_t chunk_floats, int chunk_segments,
+                                       int chunk_rows, cudaStream_t stream) {
     return matrix_state_recurrence(dtype, qkv, ld, nullptr, 0, a_in, lda, gate, ldg, power, a_bias, norm_w, eps, 0.f, q_scale,
                                    state, state_stride, out, ldo, o_raw, row_slot, row_last, n, H, H, k_dim, v_dim, narrow,
-                                   seg_row0, segments, DECAY_LOG_SIGMOID, gate_act, chunk_scratch, chunk_floats, stream);
+                                   seg_row0, segments, DECAY_LOG_SIGMOID, gate_act, chunk_scratch, chunk_floats, chunk_segments, chunk_rows, stream);
 }
 
 // A selective state space in its recurrent form (DECAY_STEP): a row of `cbx` holds the output matrices C and then the input
@@ -1644,10 +1679,11 @@ TIS_API int tis_gated_linear_attention(int dtype, const void* qkv, int ld, const
 TIS_API int tis_state_space_scan(int dtype, const void* cbx, int ld, const void* dt_in, int ldd, const float* A_log,
                                  const float* dt_bias, float* state, size_t state_stride, float* o_raw, const int* row_slot,
                                  const int* row_last, int n, int H, int G, int state_dim, int v_dim, int narrow,
-                                 const int* seg_row0, int segments, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
+                                 const int* seg_row0, int segments, float* chunk_scratch, size_t chunk_floats, int chunk_segments,
+                                       int chunk_rows, cudaStream_t stream) {
     return matrix_state_recurrence(dtype, cbx, ld, nullptr, 0, dt_in, ldd, nullptr, 0, A_log, dt_bias, nullptr, 0.f, 0.f, 1.f,
                                    state, state_stride, nullptr, 0, o_raw, row_slot, row_last, n, H, G, state_dim, v_dim,
-                                   narrow, seg_row0, segments, DECAY_STEP, 0, chunk_scratch, chunk_floats, stream);
+                                   narrow, seg_row0, segments, DECAY_STEP, 0, chunk_scratch, chunk_floats, chunk_segments, chunk_rows, stream);
 }
 
 // The recurrence with a bonus for the current token (DECAY_BONUS): a row of `rkvg` holds r, k and v of H heads (dim each) and
@@ -1657,9 +1693,10 @@ TIS_API int tis_state_space_scan(int dtype, const void* cbx, int ld, const void*
 TIS_API int tis_time_mix(int dtype, const void* rkvg, int ld, const void* w_in, int ldw, const float* u, const float* w_bias,
                          const float* norm_w, float eps, float* state, size_t state_stride, void* out, int ldo, float* o_raw,
                          const int* row_slot, const int* row_last, int n, int H, int dim, int narrow, const int* seg_row0,
-                         int segments, float* chunk_scratch, size_t chunk_floats, cudaStream_t stream) {
+                         int segments, float* chunk_scratch, size_t chunk_floats, int chunk_segments,
+                                       int chunk_rows, cudaStream_t stream) {
     const size_t gate_at = (size_t)3 * H * dim * (dtype == TIS_BF16 ? 2 : 4);
     return matrix_state_recurrence(dtype, rkvg, ld, nullptr, 0, w_in, ldw, (const char*)rkvg + gate_at, ld, u, w_bias, norm_w,
                                    eps, 0.f, 1.f, state, state_stride, out, ldo, o_raw, row_slot, row_last, n, H, H, dim, dim,
-                                   narrow, seg_row0, segments, DECAY_BONUS, 1, chunk_scratch, chunk_floats, stream);
+                                   narrow, seg_row0, segments, DECAY_BONUS, 1, chunk_scratch, chunk_floats, chunk_segments, chunk_rows, stream);
 }

@@ -19,7 +19,7 @@ import torch
 from . import build as _build
 
 _lib = None
-ABI_VERSION = 15
+ABI_VERSION = 16
 #: launches of this library's kernels so far (library matrix products are not counted)
 launches = 0
 #: calls by kind, for tests that must know which kernel a product or an attention went to
@@ -1174,7 +1174,7 @@ def _chunk_scratch(lib, decay: str, qkv: torch.Tensor, a_in, gate, out, state: t
         return None
     rows = lambda t: (None, 0) if t is None else (t if isinstance(t, tuple) else (_p(t), t.stride(0)))  # noqa: E731
     floats = lib.tis_chunked_recurrence_floats(_dt(qkv), _DECAYS[decay], *rows(qkv), *rows(a_in), *rows(gate), *rows(out), _p(state),
-                                               ctypes.c_size_t(state.stride(0)), n, int(segments[1]), num_heads, qk_heads, k_dim, v_dim)
+                                               ctypes.c_size_t(state.stride(0)), n, int(segments[1]), n, num_heads, qk_heads, k_dim, v_dim)
     if not floats or 4 * floats > CHUNKED_MAX_BYTES:
         return None
     calls["recurrence_chunked"] += 1
@@ -1185,12 +1185,14 @@ def _count_recurrence(lib, decay: str, chunked: bool, k_dim: int, v_dim: int) ->
     """Counts what a recurrence launches beyond the one kernel that every call counts."""
     global launches
     norm = decay == "constant" or (decay != "step" and not chunked and bool(lib.tis_delta_rule_splits(k_dim, v_dim)))
-    launches += (2 if chunked else 0) + int(norm)
+    launches += (3 if chunked else 0) + int(norm)
 
 
-def _floats(scratch: Optional[torch.Tensor]):
-    """A scratch tensor as the launchers take it: its address and its length."""
-    return _p(scratch), ctypes.c_size_t(0 if scratch is None else scratch.numel())
+def _chunk_args(scratch: Optional[torch.Tensor], segments, n: int):
+    """What the launchers take for the chunked form: the scratch, its length, the requests and rows in chunks."""
+    if scratch is None:
+        return _p(None), ctypes.c_size_t(0), 0, 0
+    return _p(scratch), ctypes.c_size_t(scratch.numel()), int(segments[1]), n
 
 
 def delta_rule(qkv: torch.Tensor, beta: torch.Tensor, decay_in: torch.Tensor, gate: Optional[torch.Tensor],
@@ -1225,7 +1227,7 @@ def delta_rule(qkv: torch.Tensor, beta: torch.Tensor, decay_in: torch.Tensor, ga
                               out.stride(0), _p(raw), _p(row_slot), _p(row_last), n, num_heads, qk_heads, k_dim, v_dim,
                               int(narrow), _p(segments[0] if segments is not None else None),
                               int(segments[1]) if segments is not None else 0, int(bool(decay_per_head)),
-                              GATE_ACTS[gate_act], *_floats(scratch), _stream()), lib)
+                              GATE_ACTS[gate_act], *_chunk_args(scratch, segments, n), _stream()), lib)
     return out
 
 
@@ -1248,7 +1250,7 @@ def linear_attention(qkv: torch.Tensor, gate: Optional[torch.Tensor], decay: tor
                                     _p(decay), _p(norm_weight), _f(eps), _p(state), ctypes.c_size_t(state.stride(0)),
                                     _p(out), out.stride(0), _p(raw), _p(row_slot), _p(row_last), n, num_heads, k_dim, v_dim,
                                     int(narrow), _p(segments[0] if segments is not None else None),
-                                    int(segments[1]) if segments is not None else 0, *_floats(scratch), _stream()), lib)
+                                    int(segments[1]) if segments is not None else 0, *_chunk_args(scratch, segments, n), _stream()), lib)
     return out
 
 
@@ -1274,7 +1276,7 @@ def forget_gate_recurrence(qv: torch.Tensor, f_in: torch.Tensor, lower: torch.Te
                                           _p(norm_weight), _f(eps), _p(state), ctypes.c_size_t(state.stride(0)), _p(out),
                                           out.stride(0), _p(raw), _p(row_slot), _p(row_last), n, num_heads, k_dim, v_dim,
                                           int(narrow), _p(segments[0] if segments is not None else None),
-                                          int(segments[1]) if segments is not None else 0, *_floats(scratch), _stream()), lib)
+                                          int(segments[1]) if segments is not None else 0, *_chunk_args(scratch, segments, n), _stream()), lib)
     return out
 
 
@@ -1383,7 +1385,7 @@ def gated_linear_attention(qkv: torch.Tensor, a_in: torch.Tensor, power: torch.T
                                           _f(q_scale), _p(state), ctypes.c_size_t(state.stride(0)), _p(out), out.stride(0),
                                           _p(raw), _p(row_slot), _p(row_last), n, num_heads, k_dim, v_dim, int(narrow),
                                           _p(segments[0] if segments is not None else None),
-                                          int(segments[1]) if segments is not None else 0, GATE_ACTS[gate_act], *_floats(scratch), _stream()), lib)
+                                          int(segments[1]) if segments is not None else 0, GATE_ACTS[gate_act], *_chunk_args(scratch, segments, n), _stream()), lib)
     return out
 
 
@@ -1405,7 +1407,7 @@ def state_space_scan(cbx: torch.Tensor, dt_in: torch.Tensor, a_log: torch.Tensor
                                     _p(state), ctypes.c_size_t(state.stride(0)), _p(raw), _p(row_slot), _p(row_last), n,
                                     num_heads, groups, state_dim, v_dim, int(narrow),
                                     _p(segments[0] if segments is not None else None),
-                                    int(segments[1]) if segments is not None else 0, *_floats(scratch), _stream()), lib)
+                                    int(segments[1]) if segments is not None else 0, *_chunk_args(scratch, segments, n), _stream()), lib)
     return raw
 
 
@@ -1480,7 +1482,7 @@ def time_mix(rkvg: torch.Tensor, w_in: torch.Tensor, u: torch.Tensor, w_bias: to
     _check(lib.tis_time_mix(_dt(rkvg), _p(rkvg), rkvg.stride(0), _p(w_in), w_in.stride(0), _p(u), _p(w_bias), _p(norm_weight),
                             _f(eps), _p(state), ctypes.c_size_t(state.stride(0)), _p(out), out.stride(0), _p(raw), _p(row_slot),
                             _p(row_last), n, num_heads, dim, int(narrow), _p(segments[0] if segments is not None else None),
-                            int(segments[1]) if segments is not None else 0, *_floats(scratch), _stream()), lib)
+                            int(segments[1]) if segments is not None else 0, *_chunk_args(scratch, segments, n), _stream()), lib)
     return out
 
 
