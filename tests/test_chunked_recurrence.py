@@ -267,3 +267,52 @@ def test_numbers_that_are_not_finite_are_what_the_walk_makes_of_them(rule, where
     assert ops.calls["recurrence_chunked"] == before + 1
     for g, w in zip(got, walked):
         _same_where_not_finite(g, w)
+
+
+def test_who_is_taken_in_chunks():
+    """The requests of a step, the longest first; only portions that may be long enter the chunks, from a length that depends
+    on the rule, or from a shorter one where there are several."""
+    from tiny_inference_server_b200.kernels import ops, segment_plan
+    planner = segment_plan.planner()
+
+    def portions(decay, lengths):
+        first = [sum(lengths[:i]) for i in range(len(lengths))]
+        arrays, facts = planner.plan(list(zip(first, lengths)))
+        seg = planner.bind({k: torch.tensor(v) for k, v in arrays.items()}, facts)
+        assert seg.count == len(lengths) == len(seg.row0) and seg.longest == max(lengths)
+        ordered = [lengths[first.index(int(r))] for r in seg.row0]
+        assert sorted(ordered) == sorted(lengths) and ordered == sorted(lengths, reverse=True)
+        assert list(seg.rows) == [m for m in ordered if m >= segment_plan.LISTED_ROWS]
+        return ops._chunk_portions(decay, seg, sum(lengths))
+
+    assert portions("channel", [1] * 31 + [159]) == (0, 0)
+    assert portions("channel", [1] * 31 + [160]) == (1, 160)
+    assert portions("bonus", [1] * 31 + [511]) == (0, 0)
+    assert portions("gated", [1, 300, 1, 47, 48, 700]) == (3, 1048)
+    assert portions("channel", [112] * 4) == (4, 448)
+    assert portions("channel", [64] * 16) == (0, 0)                          # none of them long
+    assert portions("bonus", [112] * 4) == (0, 0)
+    assert portions("step", [1] * 8) == (0, 0)
+    arrays, facts = planner.plan_decode(5)
+    assert ops._chunk_portions("step", planner.bind({k: torch.tensor(v) for k, v in arrays.items()}, facts), 5) == (0, 0)
+    assert ops._chunk_portions("step", None, 5) == (0, 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", RULES)
+@pytest.mark.parametrize("lengths", [(1, 1, 200, 5, 530, 1), (530,) + (1,) * 40, (47, 600, 48)])
+def test_a_step_with_single_rows_beside_long_portions(rule, lengths):
+    """Long portions in chunks, the other requests token by token, both against the recurrence in float64."""
+    from tiny_inference_server_b200.kernels import ops, segment_plan
+    case = Case(rule, 64, 64, lengths, torch.float32, seed=13)
+    want_o, want_s = case.oracle()
+    planner = segment_plan.planner()
+    arrays, facts = planner.plan(list(zip(case.first, case.lengths)))
+    seg = planner.bind({k: torch.tensor(v, dtype=torch.int32, device="cuda") for k, v in arrays.items()}, facts)
+    before, launched = ops.calls["recurrence_chunked"], ops.launches
+    got_o, got_s = case.call(ops, seg)
+    assert ops.calls["recurrence_chunked"] == before + 1
+    assert ops.launches - launched == (5 if rule == "step" else 6)
+    assert _off(got_o, want_o) < 3e-6 and _off(got_s, want_s) < 3e-6
+    for r0, m in zip(case.first, case.lengths):                              # every request for itself
+        assert _off(got_o[r0:r0 + m], want_o[r0:r0 + m]) < 6e-6

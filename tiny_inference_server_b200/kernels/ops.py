@@ -12,7 +12,7 @@ import collections
 import ctypes
 import math
 import os
-from typing import Optional
+from typing import NamedTuple, Optional
 
 import torch
 
@@ -1150,12 +1150,18 @@ def _recurrence_spread(requests: Optional[int], num_heads: int, v_dim: int) -> i
 
 
 #: rows of a step's longest request from which the matrix-state recurrences run in chunks of 64 tokens
-#: (csrc/chunked_recurrence.cu) instead of token by token.  Measured on a B200 at 12 heads of 128 x 128 in bfloat16, us token by
-#: token / in chunks: delta rule, one request of 96 rows 62 / 57, of 128 rows 82 / 58, 4 requests of 96 rows 140 / 88; gated
-#: linear attention, one request of 96 rows 45 / 64, of 128 rows 59 / 57, 4 requests of 96 rows 113 / 67
-CHUNKED_MIN_ROWS = int(os.environ.get("TIS_CHUNKED_MIN_ROWS", "112"))
-#: scratch of the chunked form above which a step is walked token by token all the same (it grows with the rows: 220 KB a
-#: chunk and head of 128 x 128)
+#: (csrc/chunked_recurrence.cu) instead of token by token, by the kind of decay: the chunks have a time of their own, and the
+#: walks take unlike times a token.  Measured on a B200 at 12 heads of 128 x 128 in bfloat16, us token by token / in chunks,
+#: one request of 128, 200, 512 rows: delta rule 82 / 86, 126 / 106, 309 / 115; gated linear attention 59 / 68, 90 / 86,
+#: 218 / 80; state space 65 / 61, 100 / 76, 248 / 71; with a bonus 27 / 64, 40 / 81, 92 / 87
+CHUNKED_MIN_ROWS = {"channel": 160, "head": 160, "constant": 224, "forget": 208, "gated": 208, "step": 160, "bonus": 512}
+if "TIS_CHUNKED_MIN_ROWS" in os.environ:
+    CHUNKED_MIN_ROWS = dict.fromkeys(CHUNKED_MIN_ROWS, int(os.environ["TIS_CHUNKED_MIN_ROWS"]))
+#: several requests: from that many rows of the longest, and that many times the rows above in all that may be long.  Four
+#: requests of 112 rows: delta rule 163 / 119, gated 131 / 81, with a bonus 51 / 77; of 500: 713 / 236, 581 / 138, 212 / 133
+CHUNKED_PORTION_ROWS, CHUNKED_TOTAL = 96, 2
+#: scratch of the chunked form above which a step is walked token by token all the same (it grows with the rows: 147 KB a
+#: chunk and head of 128 x 128, 213 KB with the delta rule)
 CHUNKED_MAX_BYTES = 1 << 30
 
 
@@ -1163,36 +1169,60 @@ CHUNKED_MAX_BYTES = 1 << 30
 _DECAYS = {"channel": 0, "head": 1, "constant": 2, "forget": 3, "gated": 4, "step": 5, "bonus": 6}
 
 
-def _chunk_scratch(lib, decay: str, qkv: torch.Tensor, a_in, gate, out, state: torch.Tensor, segments, num_heads: int,
-                   qk_heads: int, k_dim: int, v_dim: int):
-    """Scratch for the chunked form of a recurrence, or None: token by token.  ``gate``: a tensor, or its (address, row stride)."""
-    n = qkv.shape[0]
+def _chunk_portions(decay: str, segments, n: int):
+    """(number, rows) of a step's requests, the longest first, that are taken in chunks; (0, 0): none."""
     if segments is None:
+        return 0, 0
+    count, longest = int(segments[1]), segments[2] if len(segments) > 2 else n // max(1, int(segments[1]))
+    least = CHUNKED_MIN_ROWS[decay]
+    if len(segments) < 4:                                                   # rows not known one by one: all or none
+        return (count, n) if longest >= least else (0, 0)
+    total = sum(segments[3])
+    if longest < least and not (longest >= CHUNKED_PORTION_ROWS and total >= CHUNKED_TOTAL * least):
+        return 0, 0
+    return len(segments[3]), total
+
+
+class _Chunks(NamedTuple):
+    """What of a step is taken in chunks: the scratch, the number of requests and their rows; whether others are left."""
+    scratch: torch.Tensor
+    requests: int
+    rows: int
+    others: bool
+
+
+def _chunks(lib, decay: str, qkv: torch.Tensor, a_in, gate, out, state: torch.Tensor, segments, num_heads: int, qk_heads: int,
+            k_dim: int, v_dim: int) -> Optional[_Chunks]:
+    """The chunked part of a recurrence, or None: token by token.  ``gate``: a tensor, or its (address, row stride)."""
+    n = qkv.shape[0]
+    requests, rows = _chunk_portions(decay, segments, n)
+    if not requests:
         return None
-    longest = segments[2] if len(segments) > 2 else n // max(1, int(segments[1]))
-    if longest < CHUNKED_MIN_ROWS:
-        return None
-    rows = lambda t: (None, 0) if t is None else (t if isinstance(t, tuple) else (_p(t), t.stride(0)))  # noqa: E731
-    floats = lib.tis_chunked_recurrence_floats(_dt(qkv), _DECAYS[decay], *rows(qkv), *rows(a_in), *rows(gate), *rows(out), _p(state),
-                                               ctypes.c_size_t(state.stride(0)), n, int(segments[1]), n, num_heads, qk_heads, k_dim, v_dim)
+    at = lambda t: (None, 0) if t is None else (t if isinstance(t, tuple) else (_p(t), t.stride(0)))  # noqa: E731
+    floats = lib.tis_chunked_recurrence_floats(_dt(qkv), _DECAYS[decay], *at(qkv), *at(a_in), *at(gate), *at(out), _p(state),
+                                               ctypes.c_size_t(state.stride(0)), rows, requests, n, num_heads, qk_heads, k_dim, v_dim)
     if not floats or 4 * floats > CHUNKED_MAX_BYTES:
         return None
     calls["recurrence_chunked"] += 1
-    return torch.empty(floats, dtype=torch.float32, device=qkv.device)
+    return _Chunks(torch.empty(floats, dtype=torch.float32, device=qkv.device), requests, rows, requests < int(segments[1]))
 
 
-def _count_recurrence(lib, decay: str, chunked: bool, k_dim: int, v_dim: int) -> None:
-    """Counts what a recurrence launches beyond the one kernel that every call counts."""
+def _recurrence(lib, decay: str, chunks: Optional[_Chunks], n: int, requests: Optional[int], num_heads: int, k_dim: int, v_dim: int,
+                device):
+    """(how the walk shares out a head's columns, 32-bit scratch for outputs that a launch of its own normalises, the launchers'
+    arguments for the chunked part); counts what is launched beyond the one kernel that every call counts."""
     global launches
-    norm = decay == "constant" or (decay != "step" and not chunked and bool(lib.tis_delta_rule_splits(k_dim, v_dim)))
-    launches += (3 if chunked else 0) + int(norm)
-
-
-def _chunk_args(scratch: Optional[torch.Tensor], segments, n: int):
-    """What the launchers take for the chunked form: the scratch, its length, the requests and rows in chunks."""
-    if scratch is None:
-        return _p(None), ctypes.c_size_t(0), 0, 0
-    return _p(scratch), ctypes.c_size_t(scratch.numel()), int(segments[1]), n
+    walked = chunks is None or chunks.others
+    apart = walked and bool(lib.tis_delta_rule_splits(k_dim, v_dim))       # the walk leaves its outputs to the norm
+    raw = None
+    if apart or decay in ("constant", "step"):
+        raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=device)
+    launches += (3 if chunks is not None else -1) + int(walked) + int(decay == "constant" or (apart and decay != "step"))
+    if chunks is None:
+        return _recurrence_spread(requests, num_heads, v_dim), raw, (_p(None), ctypes.c_size_t(0), 0, 0)
+    requests = None if requests is None else max(1, requests - chunks.requests)
+    return (_recurrence_spread(requests, num_heads, v_dim), raw,
+            (_p(chunks.scratch), ctypes.c_size_t(chunks.scratch.numel()), chunks.requests, chunks.rows))
 
 
 def delta_rule(qkv: torch.Tensor, beta: torch.Tensor, decay_in: torch.Tensor, gate: Optional[torch.Tensor],
@@ -1212,22 +1242,16 @@ def delta_rule(qkv: torch.Tensor, beta: torch.Tensor, decay_in: torch.Tensor, ga
     launches CTAs for the requests only, not for every row."""
     lib = library()
     n = qkv.shape[0]
-    narrow = _recurrence_spread(requests, num_heads, v_dim)
-    # widths that the kernel with a head's columns split over CTAs takes: the outputs pass through 32-bit scratch
-    # and a second launch normalises them
-    raw = None
-    if lib.tis_delta_rule_splits(k_dim, v_dim):
-        raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=qkv.device)
     decay = "head" if decay_per_head else "channel"
-    scratch = _chunk_scratch(lib, decay, qkv, decay_in, gate, out, state, segments, num_heads, qk_heads, k_dim, v_dim)
-    _count_recurrence(lib, decay, scratch is not None, k_dim, v_dim)
+    chunks = _chunks(lib, decay, qkv, decay_in, gate, out, state, segments, num_heads, qk_heads, k_dim, v_dim)
+    narrow, raw, chunk_args = _recurrence(lib, decay, chunks, n, requests, num_heads, k_dim, v_dim, qkv.device)
     _check(lib.tis_delta_rule(_dt(qkv), _p(qkv), qkv.stride(0), _p(beta), beta.stride(0), _p(decay_in), decay_in.stride(0),
                               _p(gate), gate.stride(0) if gate is not None else 0, _p(a_log), _p(dt_bias), _p(norm_weight),
                               _f(eps), _f(unit_eps), _f(q_scale), _p(state), ctypes.c_size_t(state.stride(0)), _p(out),
                               out.stride(0), _p(raw), _p(row_slot), _p(row_last), n, num_heads, qk_heads, k_dim, v_dim,
                               int(narrow), _p(segments[0] if segments is not None else None),
                               int(segments[1]) if segments is not None else 0, int(bool(decay_per_head)),
-                              GATE_ACTS[gate_act], *_chunk_args(scratch, segments, n), _stream()), lib)
+                              GATE_ACTS[gate_act], *chunk_args, _stream()), lib)
     return out
 
 
@@ -1242,15 +1266,13 @@ def linear_attention(qkv: torch.Tensor, gate: Optional[torch.Tensor], decay: tor
     ``requests`` and ``segments`` as for ``delta_rule``: the same kernels walk the recurrence."""
     lib = library()
     n = qkv.shape[0]
-    narrow = _recurrence_spread(requests, num_heads, v_dim)
-    raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=qkv.device)
-    scratch = _chunk_scratch(lib, "constant", qkv, None, gate, out, state, segments, num_heads, num_heads, k_dim, v_dim)
-    _count_recurrence(lib, "constant", scratch is not None, k_dim, v_dim)
+    chunks = _chunks(lib, "constant", qkv, None, gate, out, state, segments, num_heads, num_heads, k_dim, v_dim)
+    narrow, raw, chunk_args = _recurrence(lib, "constant", chunks, n, requests, num_heads, k_dim, v_dim, qkv.device)
     _check(lib.tis_linear_attention(_dt(qkv), _p(qkv), qkv.stride(0), _p(gate), gate.stride(0) if gate is not None else 0,
                                     _p(decay), _p(norm_weight), _f(eps), _p(state), ctypes.c_size_t(state.stride(0)),
                                     _p(out), out.stride(0), _p(raw), _p(row_slot), _p(row_last), n, num_heads, k_dim, v_dim,
                                     int(narrow), _p(segments[0] if segments is not None else None),
-                                    int(segments[1]) if segments is not None else 0, *_chunk_args(scratch, segments, n), _stream()), lib)
+                                    int(segments[1]) if segments is not None else 0, *chunk_args, _stream()), lib)
     return out
 
 
@@ -1266,17 +1288,13 @@ def forget_gate_recurrence(qv: torch.Tensor, f_in: torch.Tensor, lower: torch.Te
     and norm are 32-bit.  ``requests`` and ``segments`` as for ``delta_rule``: the same kernels walk the recurrence."""
     lib = library()
     n = qv.shape[0]
-    narrow = _recurrence_spread(requests, num_heads, v_dim)
-    raw = None
-    if lib.tis_delta_rule_splits(k_dim, v_dim):
-        raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=qv.device)
-    scratch = _chunk_scratch(lib, "forget", qv, f_in, None, out, state, segments, num_heads, num_heads, k_dim, v_dim)
-    _count_recurrence(lib, "forget", scratch is not None, k_dim, v_dim)
+    chunks = _chunks(lib, "forget", qv, f_in, None, out, state, segments, num_heads, num_heads, k_dim, v_dim)
+    narrow, raw, chunk_args = _recurrence(lib, "forget", chunks, n, requests, num_heads, k_dim, v_dim, qv.device)
     _check(lib.tis_forget_gate_recurrence(_dt(qv), _p(qv), qv.stride(0), _p(f_in), f_in.stride(0), _p(lower), _p(f_bias),
                                           _p(norm_weight), _f(eps), _p(state), ctypes.c_size_t(state.stride(0)), _p(out),
                                           out.stride(0), _p(raw), _p(row_slot), _p(row_last), n, num_heads, k_dim, v_dim,
                                           int(narrow), _p(segments[0] if segments is not None else None),
-                                          int(segments[1]) if segments is not None else 0, *_chunk_args(scratch, segments, n), _stream()), lib)
+                                          int(segments[1]) if segments is not None else 0, *chunk_args, _stream()), lib)
     return out
 
 
@@ -1374,18 +1392,14 @@ def gated_linear_attention(qkv: torch.Tensor, a_in: torch.Tensor, power: torch.T
     heads).  Gate, state and norm are 32-bit.  ``requests`` and ``segments`` as for ``delta_rule``."""
     lib = library()
     n = qkv.shape[0]
-    narrow = _recurrence_spread(requests, num_heads, v_dim)
-    raw = None
-    if lib.tis_delta_rule_splits(k_dim, v_dim):
-        raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=qkv.device)
-    scratch = _chunk_scratch(lib, "gated", qkv, a_in, gate, out, state, segments, num_heads, num_heads, k_dim, v_dim)
-    _count_recurrence(lib, "gated", scratch is not None, k_dim, v_dim)
+    chunks = _chunks(lib, "gated", qkv, a_in, gate, out, state, segments, num_heads, num_heads, k_dim, v_dim)
+    narrow, raw, chunk_args = _recurrence(lib, "gated", chunks, n, requests, num_heads, k_dim, v_dim, qkv.device)
     _check(lib.tis_gated_linear_attention(_dt(qkv), _p(qkv), qkv.stride(0), _p(a_in), a_in.stride(0), _p(power), _p(a_bias),
                                           _p(gate), gate.stride(0) if gate is not None else 0, _p(norm_weight), _f(eps),
                                           _f(q_scale), _p(state), ctypes.c_size_t(state.stride(0)), _p(out), out.stride(0),
                                           _p(raw), _p(row_slot), _p(row_last), n, num_heads, k_dim, v_dim, int(narrow),
                                           _p(segments[0] if segments is not None else None),
-                                          int(segments[1]) if segments is not None else 0, GATE_ACTS[gate_act], *_chunk_args(scratch, segments, n), _stream()), lib)
+                                          int(segments[1]) if segments is not None else 0, GATE_ACTS[gate_act], *chunk_args, _stream()), lib)
     return out
 
 
@@ -1399,15 +1413,13 @@ def state_space_scan(cbx: torch.Tensor, dt_in: torch.Tensor, a_log: torch.Tensor
     float32.  ``requests`` and ``segments`` as for ``delta_rule``: the same kernels walk the recurrence."""
     lib = library()
     n = cbx.shape[0]
-    narrow = _recurrence_spread(requests, num_heads, v_dim)
-    raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=cbx.device)
-    scratch = _chunk_scratch(lib, "step", cbx, dt_in, None, None, state, segments, num_heads, groups, state_dim, v_dim)
-    _count_recurrence(lib, "step", scratch is not None, state_dim, v_dim)
+    chunks = _chunks(lib, "step", cbx, dt_in, None, None, state, segments, num_heads, groups, state_dim, v_dim)
+    narrow, raw, chunk_args = _recurrence(lib, "step", chunks, n, requests, num_heads, state_dim, v_dim, cbx.device)
     _check(lib.tis_state_space_scan(_dt(cbx), _p(cbx), cbx.stride(0), _p(dt_in), dt_in.stride(0), _p(a_log), _p(dt_bias),
                                     _p(state), ctypes.c_size_t(state.stride(0)), _p(raw), _p(row_slot), _p(row_last), n,
                                     num_heads, groups, state_dim, v_dim, int(narrow),
                                     _p(segments[0] if segments is not None else None),
-                                    int(segments[1]) if segments is not None else 0, *_chunk_args(scratch, segments, n), _stream()), lib)
+                                    int(segments[1]) if segments is not None else 0, *chunk_args, _stream()), lib)
     return raw
 
 
@@ -1472,17 +1484,13 @@ def time_mix(rkvg: torch.Tensor, w_in: torch.Tensor, u: torch.Tensor, w_bias: to
     n = rkvg.shape[0]
     if rkvg.dtype != w_in.dtype or rkvg.stride(1) != 1 or w_in.stride(1) != 1:
         raise KernelError("time_mix: the rows and the decays' projection are dense and of one type")
-    narrow = _recurrence_spread(requests, num_heads, dim)
-    raw = None
-    if lib.tis_delta_rule_splits(dim, dim):
-        raw = torch.empty((n, num_heads * dim), dtype=torch.float32, device=rkvg.device)
-    scratch = _chunk_scratch(lib, "bonus", rkvg, w_in, (_p(rkvg[:, 3 * num_heads * dim:]), rkvg.stride(0)), out, state, segments,
-                             num_heads, num_heads, dim, dim)
-    _count_recurrence(lib, "bonus", scratch is not None, dim, dim)
+    chunks = _chunks(lib, "bonus", rkvg, w_in, (_p(rkvg[:, 3 * num_heads * dim:]), rkvg.stride(0)), out, state, segments,
+                     num_heads, num_heads, dim, dim)
+    narrow, raw, chunk_args = _recurrence(lib, "bonus", chunks, n, requests, num_heads, dim, dim, rkvg.device)
     _check(lib.tis_time_mix(_dt(rkvg), _p(rkvg), rkvg.stride(0), _p(w_in), w_in.stride(0), _p(u), _p(w_bias), _p(norm_weight),
                             _f(eps), _p(state), ctypes.c_size_t(state.stride(0)), _p(out), out.stride(0), _p(raw), _p(row_slot),
                             _p(row_last), n, num_heads, dim, int(narrow), _p(segments[0] if segments is not None else None),
-                            int(segments[1]) if segments is not None else 0, *_chunk_args(scratch, segments, n), _stream()), lib)
+                            int(segments[1]) if segments is not None else 0, *chunk_args, _stream()), lib)
     return out
 
 

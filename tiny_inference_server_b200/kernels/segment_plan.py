@@ -2,11 +2,24 @@
 time) and want one CTA per request instead of one per row (``parts.base.StepPlanner``)."""
 from __future__ import annotations
 
-from typing import Dict, Sequence, Tuple
+from typing import Dict, NamedTuple, Sequence, Tuple
 
 import torch
 
 from ..parts.base import StepPlanner
+
+
+#: rows from which a request may be taken otherwise than token by token
+LISTED_ROWS = 48
+
+
+class Segments(NamedTuple):
+    """The requests of a step, the longest first: their first rows (device), their number, the rows of the longest, and the rows
+    of each that has at least LISTED_ROWS."""
+    row0: torch.Tensor
+    count: int
+    longest: int
+    rows: Tuple[int, ...]
 
 
 class SegmentPlanner(StepPlanner):
@@ -16,14 +29,16 @@ class SegmentPlanner(StepPlanner):
         return rows
 
     def plan(self, segments: Sequence[Tuple[int, int]]):
-        return {"row0": [first for first, _ in segments]}, (len(segments), max((rows for _, rows in segments), default=0))
+        # the longest first: a request's rows are a chain, and the longest chain should not start last
+        ordered = sorted(segments, key=lambda s: -s[1])
+        return {"row0": [first for first, _ in ordered]}, (len(ordered), max((rows for _, rows in segments), default=0),
+                                                           *(rows for _, rows in ordered if rows >= LISTED_ROWS))
 
     def plan_decode(self, rows: int):
         return {"row0": list(range(rows))}, (rows, 1)
 
-    def bind(self, arrays: Dict[str, torch.Tensor], facts):
-        """(first rows, number of requests, rows of the longest)"""
-        return arrays["row0"], int(facts[0]), int(facts[1])
+    def bind(self, arrays: Dict[str, torch.Tensor], facts) -> Segments:
+        return Segments(arrays["row0"], int(facts[0]), int(facts[1]), tuple(int(r) for r in facts[2:]))
 
 
 _planner = SegmentPlanner()
