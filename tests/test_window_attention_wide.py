@@ -189,3 +189,15 @@ def test_tiles_cover_the_rows_once():
         covered = tiles.rows_in_wide
         assert rows((tiles.rows[0][:covered], tiles.rows[1][:covered])) == wide
         assert sum(len(v) for v in arrays.values()) <= planner.max_words(457)
+
+
+def test_shares_of_a_row_keep_all_clusters_resident():
+    from types import SimpleNamespace
+    from tiny_inference_server_b200.kernels import ops
+    # as a device answers whose clusters of 16 do not fill it: two CTAs an SM, and one
+    two = SimpleNamespace(decode_clusters={(0, 1): 296, (0, 2): 148, (0, 4): 72, (0, 8): 34, (0, 16): 14})
+    one = SimpleNamespace(decode_clusters={(0, 1): 148, (0, 2): 74, (0, 4): 36, (0, 8): 16, (0, 16): 7})
+    assert ops._decode_shares(two, 0, 14, 4096) == 16 and ops._decode_shares(two, 0, 15, 4096) == 8
+    assert ops._decode_shares(two, 0, 16, 1000) == 8 and ops._decode_shares(two, 0, 400, 4096) == 1
+    assert ops._decode_shares(one, 0, 8, 4096) == 8 and ops._decode_shares(one, 0, 32, 4096) == 4
+    assert ops._decode_shares(two, 0, 1, 63) == 1 and ops._decode_shares(two, 0, 1, 64) == 2       # a tile of keys each

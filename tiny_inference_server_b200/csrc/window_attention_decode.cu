@@ -7,6 +7,7 @@
 // swizzled) STAGES ahead; each of four warps takes 16 keys of every tile, with a running maximum and sum of its own, and no
 // barrier in the loop.  The warps' results are merged in shared memory, those of the cluster by reading the neighbours'
 // shared memory, every CTA a part of the outputs: no second launch, no scratch in global memory.
+// The shares are as many as keep all clusters resident at once (the device is asked how many it holds).
 // Keys that the row does not see come from pages that may hold anything: their scores are masked and their value elements
 // taken for zero.
 // What bounds it: the chain from the page table through the first boxes to the merge.  8 rows at 4096 keys, 8 query heads of 128
@@ -315,6 +316,26 @@ window_attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const 
 }
 
 template <bool SHARED>
+int resident_clusters(int splits) {
+    auto kernel = window_attention_decode_kernel<SHARED>;
+    constexpr int smem = smem_bytes<SHARED>();
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits, 1, 1);
+    cfg.blockDim = dim3((WARPS + 1) * 32);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return n;
+}
+
+template <bool SHARED>
 int launch_decode(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeParams& p, int rows, int splits, cudaStream_t stream) {
     auto kernel = window_attention_decode_kernel<SHARED>;
     constexpr int smem = smem_bytes<SHARED>();
@@ -341,6 +362,16 @@ int launch_decode(const CUtensorMap& mk, const CUtensorMap& mv, const DecodePara
 
 // Whether this pair of widths has the kernel (1), also with values that are the first elements of the key rows (3).
 TIS_API int tis_window_attention_decode_forms() { return TIS_KD >= TIS_VD ? 3 : 1; }
+
+// How many clusters of `splits` CTAs the device holds at once.
+TIS_API int tis_window_attention_decode_clusters(int shared, int splits) {
+    if (!shared) return resident_clusters<false>(splits);
+#if TIS_KD >= TIS_VD
+    return resident_clusters<true>(splits);
+#else
+    return 0;
+#endif
+}
 
 // Attention of `rows` single rows.  At most 16 query heads a kv head; `splits` 1, 2, 4, 8 or 16 shares of the keys; operands as
 // for tis_window_attention_tc, any sign of the scale.
@@ -386,6 +417,7 @@ TIS_API int tis_window_attention_decode(const void* q, int ldq, const void* gate
 #else
 
 TIS_API int tis_window_attention_decode_forms() { return 0; }
+TIS_API int tis_window_attention_decode_clusters(int, int) { return 0; }
 
 TIS_API int tis_window_attention_decode(const void*, int, const void*, int, int, void*, int, const void*, size_t, const void*,
                                         size_t, int, const int*, int, int, const int*, const int*, int, int, int, int, int, float,

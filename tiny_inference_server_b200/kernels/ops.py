@@ -991,6 +991,9 @@ def window_attention_library(k_dim: int, v_dim: int):
             raise KernelError(f"windowed attention library built for widths {kd.value}/{vd.value}, wanted {k_dim}/{v_dim}")
         lib.tc_forms = int(lib.tis_window_attention_tc_forms())
         lib.decode_forms = int(lib.tis_window_attention_decode_forms())
+        # (form - 1, shares of the keys) -> clusters that the device holds at once
+        lib.decode_clusters = {(f, 1 << i): int(lib.tis_window_attention_decode_clusters(f, 1 << i))
+                               for f in range(2) if lib.decode_forms >> f & 1 for i in range(5)}
         _wattn_libs[(k_dim, v_dim)] = lib
     return lib
 
@@ -1026,6 +1029,15 @@ WINDOW_ATTENTION_TC_MIN_WORK = 1 << 24
 #: decode steps of at most 16 query heads a kv head run on the kernel whose key shares are a cluster, where it takes their
 #: widths and pages; TIS_WINDOW_ATTENTION_DECODE=0 keeps them on the mma.sync kernel
 WINDOW_ATTENTION_DECODE = os.environ.get("TIS_WINDOW_ATTENTION_DECODE", "1") != "0"
+
+
+def _decode_shares(wlib, form: int, clusters: int, keys: int) -> int:
+    """Shares of the keys of a row, a cluster of CTAs: as many as keep all clusters resident at once, a tile of 64 keys each at least.
+    A second wave of a few clusters would cost as much as the first, and clusters do not fill the device as single CTAs do."""
+    splits = 16
+    while splits > 1 and (splits > keys // 64 + 1 or wlib.decode_clusters[form, splits] < clusters):
+        splits //= 2
+    return splits
 
 
 def _window_boxes(page_size: int, heads: int, k_dim: int, v_dim: int, k_strides, v_strides, same_start: bool) -> int:
@@ -1076,9 +1088,7 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
         if decode:
             keys = step.max_position + 1 if not window else min(int(window), step.max_position + 1)
         if decode and count == n and boxes & wlib.decode_forms and num_heads // kv_heads <= 16 and WINDOW_ATTENTION_DECODE:
-            # shares of the keys: as many as keep all CTAs resident (two an SM), one cluster at most, a tile of keys each
-            want = min(16, keys // 64 + 1, WINDOW_ATTENTION_CTAS // (count * kv_heads))
-            splits = 1 << max(0, want.bit_length() - 1)
+            splits = _decode_shares(wlib, boxes - 1, count * kv_heads, keys)
             calls["window_attention_decode"] += 1
             _check(wlib.tis_window_attention_decode(_p(q), q.stride(0), _p(gate), gate_row, int(gate_per_head), _p(out), out.stride(0),
                                                     _p(k_pages), kps, _p(v_pages), vps, int(boxes == 2), _p(block_table),
