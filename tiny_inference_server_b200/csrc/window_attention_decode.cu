@@ -243,6 +243,11 @@ window_attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const 
         }
     }
     __syncthreads();                                        // every tile has been read: the stages carry the warps' results
+    if (*abort) {
+        // a wait ran out: give boxes that may still be on their way time to land before the stages carry anything else, and
+        // before the shared memory is given up
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    }
     float* part = reinterpret_cast<float*>(tiles);          // [WARPS][ROWS][PROW]
     if (warp < WARPS) {
 #pragma unroll
