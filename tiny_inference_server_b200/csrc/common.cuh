@@ -145,7 +145,7 @@ __device__ __forceinline__ float gated_unit(float g, float u, const GateForm& f)
 __device__ __forceinline__ float gated_unit_fast(float g, float u, const GateForm& f) {
     g = fminf(g, f.limit);
     u = fminf(fmaxf(u, -f.limit), f.limit);
-    return __fdividef(g, 1.f + __expf(-g * fmaf(f.c3 * g, g, f.c1))) * (u + f.shift);
+    return g / (1.f + __expf(-g * fmaf(f.c3 * g, g, f.c1))) * (u + f.shift);
 }
 
 // Block-wide sum / max for blockDim.x a multiple of 32 (<= 1024); `red` holds 33 floats.

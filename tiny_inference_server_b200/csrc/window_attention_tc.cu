@@ -423,7 +423,7 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                             float gv[8];
                             Vec16<bf16>::load(gr + q * 8, gv);
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) o0[q * 8 + e] = __fdividef(o0[q * 8 + e], 1.f + __expf(-gv[e]));
+                            for (int e = 0; e < 8; ++e) o0[q * 8 + e] /= 1.f + __expf(-gv[e]);
                         }
                     }
                     bf16* dst = p.out + (size_t)(row0 + r) * p.out_stride + head * VD + col;
