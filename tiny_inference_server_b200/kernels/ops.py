@@ -1743,7 +1743,7 @@ def bitmap_set(bitmap_row: torch.Tensor, tokens: torch.Tensor) -> None:
 
 
 #: (row, choice) pairs up to which bfloat16 experts run with every chosen expert's matrices streamed once (csrc/moe_few.cu);
-#: TIS_MOE_FEW_MAX_PAIRS overrides (0: never).  us, 16 experts of 1024, width 1536, 3 a row, against a dot product per element: 1 row
+#: TIS_MOE_FEW_MAX_PAIRS overrides (0: never; the kernel takes MOE_FEW_PAIRS at most).  us, 16 experts of 1024, width 1536, 3 a row, against a dot product per element: 1 row
 #: 22 -> 15, 8 rows 43 -> 42, 16 rows 66 -> 46, 31 rows 103 -> 47; experts of 2048, width 3072: 4 rows 87 -> 87, 16 rows 191 -> 146
 MOE_FEW_MAX_PAIRS = int(os.environ.get("TIS_MOE_FEW_MAX_PAIRS", "96"))
 #: the experts, and the width, up to which they always do; beyond either, one row of 128 experts at most, and three
@@ -1751,18 +1751,39 @@ MOE_FEW_MAX_PAIRS = int(os.environ.get("TIS_MOE_FEW_MAX_PAIRS", "96"))
 #: rows seldom share an expert, and a dot product per pair spreads better (32 experts of 768, width 2048, 4 a row: 1 row 25 -> 18 us,
 #: but 8 rows 50 -> 56; 24 rows 121 -> 78; 8 of 2048, width 4096, 2 a row: 4 rows 70 -> 75, 16 rows 206 -> 91)
 MOE_FEW_MAX_EXPERTS, MOE_FEW_MAX_WIDTH = 16, 3072
+MOE_FEW_PAIRS = 384
 #: (token, choice) pairs from which bfloat16 expert products go to the tiles on the tensor cores (rows sorted by expert on
 #: the device) instead of one dot product per output element; TIS_MOE_GROUPED_MIN_PAIRS overrides (0: never)
 MOE_GROUPED_MIN_PAIRS = int(os.environ.get("TIS_MOE_GROUPED_MIN_PAIRS", "96"))
 #: pairs from which they go to the tcgen05 kernel (tiles of 128 rows, TMA-fed, accumulator in tensor memory) where width and
 #: hidden size are multiples of 64; TIS_MOE_TC_MIN_PAIRS overrides (0: never)
 MOE_TC_MIN_PAIRS = int(os.environ.get("TIS_MOE_TC_MIN_PAIRS", "1024"))
-#: the same for the width MOE_TC_WIDE and more, up to MOE_TC_WIDE_MAX_EXPERTS experts: the mma.sync tiles walk the width with few CTAs in
+#: the same for the width MOE_TC_WIDE and more, up to MOE_TC_WIDE_MAX_EXPERTS experts (TIS_MOE_TC_WIDE_MIN_PAIRS overrides, 0: as any
+#: width; where only TIS_MOE_TC_MIN_PAIRS is given it holds for every width): the mma.sync tiles walk the width with few CTAs in
 #: flight, TMA keeps more of it on its way.  us, 16 experts: 1024 of width 1536, 128 rows 110 -> 57; 2048 of 3072, 64 rows 208 -> 127;
 #: 256 of 512, 40 rows 33 -> 22.5; 128 of 256, 40 rows 19.7 -> 20.1
 #: (hence the width); 128 experts of 512, width 1024, 12 rows of 8: 90 -> 101 (hence the experts)
-MOE_TC_WIDE_MIN_PAIRS = int(os.environ.get("TIS_MOE_TC_WIDE_MIN_PAIRS", "96"))
+MOE_TC_WIDE_MIN_PAIRS = int(os.environ.get("TIS_MOE_TC_WIDE_MIN_PAIRS", "0" if "TIS_MOE_TC_MIN_PAIRS" in os.environ else "96"))
 MOE_TC_WIDE, MOE_TC_WIDE_MAX_EXPERTS = 512, 32
+
+
+def _experts_route(pairs: int, rows: int, d: int, hidden: int, experts: int) -> str:
+    """Which kernels bfloat16 experts of this size are for, if the operands suit them: ``few`` (else as if there were none),
+    ``tc``, ``grouped`` or ``dots``."""
+    streamed = (experts <= MOE_FEW_MAX_EXPERTS and d <= MOE_FEW_MAX_WIDTH) or (rows == 1 and experts <= 128) or pairs >= 3 * experts
+    if pairs <= min(MOE_FEW_MAX_PAIRS, MOE_FEW_PAIRS) and streamed and d % 32 == 0 and hidden % 32 == 0:
+        return "few"
+    return _many_experts_route(pairs, d, hidden, experts)
+
+
+def _many_experts_route(pairs: int, d: int, hidden: int, experts: int) -> str:
+    if MOE_GROUPED_MIN_PAIRS <= 0:
+        return "dots"
+    wide = d >= MOE_TC_WIDE and experts <= MOE_TC_WIDE_MAX_EXPERTS and MOE_TC_WIDE_MIN_PAIRS > 0
+    tc_from = min(MOE_TC_MIN_PAIRS, MOE_TC_WIDE_MIN_PAIRS) if wide else MOE_TC_MIN_PAIRS
+    if MOE_TC_MIN_PAIRS > 0 and pairs >= tc_from and d % 64 == 0 and hidden % 64 == 0:
+        return "tc"
+    return "grouped" if pairs >= MOE_GROUPED_MIN_PAIRS else "dots"
 
 
 def moe_experts(x: torch.Tensor, chosen: torch.Tensor, weights: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor,
@@ -1781,10 +1802,12 @@ def moe_experts(x: torch.Tensor, chosen: torch.Tensor, weights: torch.Tensor, w_
     top = chosen.shape[1]
     experts, hidden = w_gate_up.shape[0], w_gate_up.shape[-2]
     act_code = ACTIVATIONS[act] if act is not None else -1
-    streamed = (experts <= MOE_FEW_MAX_EXPERTS and d <= MOE_FEW_MAX_WIDTH) or (n == 1 and experts <= 128) or n * top >= 3 * experts
-    if (n * top <= MOE_FEW_MAX_PAIRS and x.dtype == torch.bfloat16 and streamed and d % 32 == 0 and hidden % 32 == 0
-            and x.stride(1) == 1 and x.stride(0) % 8 == 0 and (x.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0
-            and (shared is None or shared.stride(1) == 1)):
+    route = _experts_route(n * top, n, d, hidden, experts) if x.dtype == torch.bfloat16 else "dots"
+    if route == "few" and not (x.stride(1) == 1 and x.stride(0) % 8 == 0
+                               and (x.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0
+                               and (shared is None or shared.stride(1) == 1)):
+        route = _many_experts_route(n * top, d, hidden, experts)
+    if route == "few":
         lib = library()
         hid = torch.empty((n * top, hidden), dtype=x.dtype, device=x.device)
         out = torch.empty((n, d), dtype=x.dtype, device=x.device)
@@ -1794,11 +1817,9 @@ def moe_experts(x: torch.Tensor, chosen: torch.Tensor, weights: torch.Tensor, w_
                                shared.stride(0) if shared is not None else 0, _p(shared_gate), _p(out), _p(hid), n, d, top, experts,
                                hidden, act_code, form, int(weigh_input), _stream()), lib)
         return out
-    grouped = (x.dtype == torch.bfloat16 and MOE_GROUPED_MIN_PAIRS > 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
+    grouped = (route in ("tc", "grouped") and x.stride(1) == 1 and x.stride(0) % 8 == 0
                and x.data_ptr() % 16 == 0 and (shared is None or (shared.stride(1) == 1 and shared.stride(0) % 2 == 0)))
-    wide = d >= MOE_TC_WIDE and experts <= MOE_TC_WIDE_MAX_EXPERTS
-    tc_from = min(MOE_TC_MIN_PAIRS, MOE_TC_WIDE_MIN_PAIRS) if wide else MOE_TC_MIN_PAIRS
-    if grouped and MOE_TC_MIN_PAIRS > 0 and n * top >= tc_from and d % 64 == 0 and hidden % 64 == 0:
+    if grouped and route == "tc":
         # many rows: 128-row tiles on the tcgen05 tensor cores, the stacked weights as TMA boxes where they lie
         lib = library()
         tiles = lib.tis_moe_tc_tiles(n * top, experts)
