@@ -316,3 +316,22 @@ def test_a_step_with_single_rows_beside_long_portions(rule, lengths):
     assert _off(got_o, want_o) < 3e-6 and _off(got_s, want_s) < 3e-6
     for r0, m in zip(case.first, case.lengths):                              # every request for itself
         assert _off(got_o[r0:r0 + m], want_o[r0:r0 + m]) < 6e-6
+
+
+@pytest.mark.gpu
+def test_without_memory_for_the_scratch_the_step_is_walked(monkeypatch):
+    from tiny_inference_server_b200.kernels import ops
+    case = Case("gated", 64, 64, (300, 2), torch.float32, seed=15)
+    walked_o, walked_s = case.call(ops, case.segments(False))
+    empty = torch.empty
+
+    def full(*size, **options):
+        if len(size) == 1 and isinstance(size[0], int) and size[0] > 100000:
+            raise torch.cuda.OutOfMemoryError("no memory left")
+        return empty(*size, **options)
+
+    segments, before = case.segments(True), ops.calls["recurrence_chunked"]
+    monkeypatch.setattr(torch, "empty", full)
+    got_o, got_s = case.call(ops, segments)
+    assert ops.calls["recurrence_chunked"] == before
+    assert torch.equal(got_o, walked_o) and torch.equal(got_s, walked_s)

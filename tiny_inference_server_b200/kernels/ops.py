@@ -1213,8 +1213,12 @@ def _chunks(lib, decay: str, qkv: torch.Tensor, a_in, gate, out, state: torch.Te
                                                ctypes.c_size_t(state.stride(0)), rows, requests, n, num_heads, qk_heads, k_dim, v_dim)
     if not floats or 4 * floats > CHUNKED_MAX_BYTES:
         return None
+    try:
+        scratch = torch.empty(floats, dtype=torch.float32, device=qkv.device)
+    except torch.cuda.OutOfMemoryError:
+        return None                                                         # the walk needs none
     calls["recurrence_chunked"] += 1
-    return _Chunks(torch.empty(floats, dtype=torch.float32, device=qkv.device), requests, rows, requests < int(segments[1]))
+    return _Chunks(scratch, requests, rows, requests < int(segments[1]))
 
 
 def _recurrence(lib, decay: str, chunks: Optional[_Chunks], n: int, requests: Optional[int], num_heads: int, k_dim: int, v_dim: int,
