@@ -16,6 +16,7 @@ def steps_of_any_size(monkeypatch):
     """The tcgen05 kernel also where a step's work is too small for it to pay."""
     from tiny_inference_server_b200.kernels import ops
     monkeypatch.setattr(ops, "WINDOW_ATTENTION_TC_MIN_WORK", 0)
+    monkeypatch.setattr(ops, "WINDOW_ATTENTION_TC_MIXED_ROWS", 0)
 
 
 class _Step:
@@ -201,3 +202,12 @@ def test_shares_of_a_row_keep_all_clusters_resident():
     assert ops._decode_shares(two, 0, 16, 1000) == 8 and ops._decode_shares(two, 0, 400, 4096) == 1
     assert ops._decode_shares(one, 0, 8, 4096) == 8 and ops._decode_shares(one, 0, 32, 4096) == 4
     assert ops._decode_shares(two, 0, 1, 63) == 1 and ops._decode_shares(two, 0, 1, 64) == 2       # a tile of keys each
+
+
+def test_when_long_portions_are_worth_a_launch(monkeypatch):
+    from tiny_inference_server_b200.kernels import ops
+    monkeypatch.undo()
+    assert ops._wide_tiles_pay(2048, 0, 1024, 12) and not ops._wide_tiles_pay(1200, 0, 1024, 12)
+    # beside other tiles, in which one launch runs as long as the rows alone, only portions that take as long themselves
+    assert not ops._wide_tiles_pay(1024 + 8, 8, 4000, 12) and not ops._wide_tiles_pay(31 + 512, 31, 4000, 12)
+    assert ops._wide_tiles_pay(3072 + 8, 8, 4000, 12)

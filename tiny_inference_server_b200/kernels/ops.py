@@ -1024,11 +1024,24 @@ WINDOW_ATTENTION_TC = os.environ.get("TIS_WINDOW_ATTENTION_TC", "1") != "0"
 #: prompts, 12 heads, 96 us a layer with the mma.sync kernel, 103 with this one, 154 rows in two 97 and 113; 2048 rows at a window
 #: of 1024 177 and 105 us
 WINDOW_ATTENTION_TC_MIN_WORK = 1 << 24
+#: (rows of the long portions * query heads) from which they do in a step with other tiles as well.  The others' launch comes behind,
+#: where in one launch they run beside the portions, and each of their rows is a chain along its keys: 8 rows at 4000 keys beside a
+#: portion of 1024, 12 heads, window 1024 88 us on the mma.sync kernel alone, 109 on both; without a window 297 and 336, of
+#: which the rows alone take 274 and the portion 84 or 19.  The chain grows with the keys as the portion's time on the mma.sync kernel does
+WINDOW_ATTENTION_TC_MIXED_ROWS = 1 << 15
 
 
 #: decode steps of at most 16 query heads a kv head run on the kernel whose key shares are a cluster, where it takes their
 #: widths and pages; TIS_WINDOW_ATTENTION_DECODE=0 keeps them on the mma.sync kernel
 WINDOW_ATTENTION_DECODE = os.environ.get("TIS_WINDOW_ATTENTION_DECODE", "1") != "0"
+
+
+def _wide_tiles_pay(rows: int, others: int, keys: int, num_heads: int) -> bool:
+    """Whether a step's long portions are worth a launch of the tcgen05 kernel: its rows, the tiles beside the long portions, the keys
+    that a row can see."""
+    if rows * keys * num_heads < WINDOW_ATTENTION_TC_MIN_WORK:
+        return False
+    return others <= 0 or (rows - others) * num_heads >= WINDOW_ATTENTION_TC_MIXED_ROWS
 
 
 def _decode_shares(wlib, form: int, clusters: int, keys: int) -> int:
@@ -1101,7 +1114,7 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
               and out.data_ptr() % 16 == 0
               and (gate is None or gate_per_head or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0)))
         reach = getattr(step, "max_position", 0) + 1
-        tc = tc and n * (min(int(window), reach) if window else reach) * num_heads >= WINDOW_ATTENTION_TC_MIN_WORK
+        tc = tc and _wide_tiles_pay(n, count - tiles.rows_in_wide, min(int(window), reach) if window else reach, num_heads)
         if tc and (wide_count >= TC_ATTENTION_MIN_TILES or getattr(step, "max_position", 0) < TC_ATTENTION_SHORT_CONTEXT):
             calls["window_attention_tc"] += 1
             _check(wlib.tis_window_attention_tc(_p(q), q.stride(0), n, _p(gate), gate_row, int(gate_per_head), _p(out), out.stride(0),
