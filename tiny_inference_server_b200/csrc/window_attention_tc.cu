@@ -6,15 +6,14 @@
 //   * keys and values have widths of their own; their rows lie in the pages as they are, so the TMA engine swizzles the boxes;
 //   * the value rows may be the first TIS_VD elements of the key rows (SHARED): the key tile is then read a second time as the
 //     values, there is no ring of values and a slot is free when the tile's second product is done;
-//   * the bias costs a logarithm an element.  The first pass over a row of scores, which finds the maximum, does without it
-//     where it can: any reference that is not far above the maximum serves the softmax, and the bias of the nearest key bounds
-//     the others (r1, r2 >= 0).  Where the bias varies by more than 2^BIAS_SLACK within the tile, it is taken in both passes;
+//   * the bias costs a logarithm an element.  The first pass over a row of scores, which finds the maximum, leaves them in
+//     tensor memory with their bias and masked, so that the second pass takes only the exponentials;
 //   * rows of the value tile that no row of queries sees (before the window, behind the last row, pages of others) are zeroed:
 //     a probability of 0 must not meet what another request left there.
 // Bound by the chain of a tile through scores, softmax and second product (two tiles side by side), as attention_tc.cu.
 // Against the mma.sync kernel, which reads every operand fragment from shared memory per warp of 16 rows: 2048 rows, 12 query
-// heads of 128 on 3 kv heads, window 1024, with bias and gate 117 -> 43 us; 1024 rows behind 1024 cached, 12 heads on one
-// compressed row of 192 (values 128) 201 -> 45 us.
+// heads of 128 on 3 kv heads, window 1024, with bias 103 -> 33 us; 1024 rows behind 1024 cached, 12 heads on one
+// compressed row of 192 (values 128) 201 -> 41 us (replayed from a graph); outputs against 64 bits 0.97 to 1.0 times as far off.
 #include "tc_common.cuh"
 
 #ifndef TIS_KD
@@ -46,8 +45,6 @@ constexpr int SLOTS = 2;                    // per ring
 constexpr unsigned TMEM_COLS = 512;
 constexpr unsigned COL_S = 0;               // two score buffers of 128 columns
 constexpr unsigned COL_O = 256;             // two output accumulators of up to 128 columns
-constexpr float RESCALE_STEP = 8.f;         // in units of log2
-constexpr float BIAS_SLACK = 60.f;          // the same: how far above a row's maximum its reference may lie
 
 struct WtcParams {
     bf16* out; int out_stride;
@@ -284,9 +281,9 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             // this group hands P over): first the maximum, then the exponentials.
             const bool whole = kt + BN - 1 <= pos0 && kt >= lo_last;      // every row of the tile sees every key
             const bool plain = whole && row_ok;
-            // the scores of half a tile (`bound`: through the tanh; `biased`: scaled to units of log2 and with their bias, else
-            // the scale is left to the caller)
-            auto load64 = [&](int half, float (&s)[64], bool bound, bool biased) {
+            // the scores of half a tile, masked (`bound`: through the tanh).  With a bias: scaled to units of log2, by the first
+            // pass, which writes them back; without: the scale is left to the caller
+            auto load64 = [&](int half, float (&s)[64], bool bound, bool first) {
                 tmem_ld32_issue(tmem_base + lane_bits + col_s + half * 64, s);
                 tmem_ld32_issue(tmem_base + lane_bits + col_s + half * 64 + 32, s + 32);
                 tmem_ld_wait();
@@ -295,35 +292,30 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 #pragma unroll
                     for (int e = 0; e < 64; ++e) s[e] = soft_capped(s[e], p.cap);
                 }
-                if (BIAS && biased) {
+                if (BIAS && first) {
                     const float d0 = (float)(qpos - kt - half * 64);
 #pragma unroll
                     for (int e = 0; e < 64; ++e)
                         s[e] = fmaf(s[e], p.scale_log2, -b1 * fast_log2(fmaf(b2, d0 - (float)e, 1.f)));
                 }
-                if (!plain) {
+                if (!plain && (!BIAS || first)) {
 #pragma unroll
                     for (int e = 0; e < 64; ++e) {
                         const int key = kt + half * 64 + e;
                         s[e] = (row_ok && key <= qpos && key >= lo_r) ? s[e] : -INFINITY;
                     }
                 }
+                if (BIAS && first) {
+                    tmem_st32(tmem_base + lane_bits + col_s + half * 64, reinterpret_cast<const float(&)[32]>(s[0]));
+                    tmem_st32(tmem_base + lane_bits + col_s + half * 64 + 32, reinterpret_cast<const float(&)[32]>(s[32]));
+                }
             };
-            // the row's maximum: of the raw scores (the scale is positive), where the bias allows it with the bias of the
-            // nearest key on top
-            float near_bias = 0.f;
-            bool exact = false;
-            if (BIAS) {
-                const float near = (float)max(0, qpos - (kt + BN - 1)), far = (float)max(0, qpos - max(kt, lo_r));
-                const float near_log = fast_log2(fmaf(b2, near, 1.f));
-                near_bias = -b1 * near_log;
-                exact = !__all_sync(0xffffffffu, b1 >= 0.f && b2 >= 0.f && b1 * (fast_log2(fmaf(b2, far, 1.f)) - near_log) <= BIAS_SLACK);
-            }
+            // the row's maximum, without a bias of the raw scores (the scale is positive)
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll 1
             for (int half = 0; half < 2; ++half) {
                 float s[64];
-                load64(half, s, false, exact);
+                load64(half, s, false, true);
 #pragma unroll
                 for (int e = 0; e < 64; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], s[e]);
             }
@@ -331,9 +323,10 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             const bool capped = !BIAS && p.cap.k != 0.f;
             float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
             if (capped && mx > -INFINITY) mx = soft_capped(mx, p.cap);
-            if (!exact) mx = fmaf(mx, p.scale_log2, near_bias);
-            // raise the reference maximum only when the row's maximum left it far behind
-            const bool raise = mx > m_used + RESCALE_STEP || (m_used == -INFINITY && mx > -INFINITY);
+            if (!BIAS) mx *= p.scale_log2;
+            // the reference is the row's maximum itself, so that the largest probability is 1 and not rounded.  (Raised only
+            // when the maximum had left it far behind: 1 to 2 % more error of the outputs, 2 % less time.)
+            const bool raise = mx > m_used;
             float alpha = 1.f;
             if (raise) {
                 alpha = m_used == -INFINITY ? 0.f : fast_exp2(m_used - mx);
@@ -360,7 +353,7 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 #pragma unroll 1
             for (int half = 0; half < 2; ++half) {
                 float s[64];
-                load64(half, s, capped, true);
+                load64(half, s, capped, false);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {             // eight keys: one 16-byte chunk of the row of P
                     unsigned pk[4];
@@ -372,7 +365,6 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                         __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
                         pk[e >> 1] = *reinterpret_cast<unsigned*>(&h);
                         // the sum of what the product sees: a row that is nearly all one key's comes out as that key's value
-                        // (the reference is not the row's maximum, so its probability is not 1 before the division)
                         ps4[e >> 1] += __uint_as_float(pk[e >> 1] << 16) + __uint_as_float(pk[e >> 1] & 0xffff0000u);
                     }
                     *reinterpret_cast<uint4*>(prow + half * HALF_BYTES + ((c ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
