@@ -1100,7 +1100,7 @@ delta_rule_split_kernel(const T* __restrict__ qkv, int ld, const T* __restrict__
     // of rows that are not the first of their request leave at once)
     const int r0 = seg_row0 != nullptr ? seg_row0[blockIdx.z] : (int)blockIdx.z;
     const int slot = row_slot[r0];
-    if (slot < 0) return;
+    if (slot < 0) { pdl_wait(); return; }               // (a grid that waited for nothing would let the next one run ahead)
     if (r0 > 0 && row_slot[r0 - 1] == slot) return;
     const int rows = row_last[r0] - r0 + 1;
     const int kvh = head / (H / G);
