@@ -285,13 +285,14 @@ def test_who_is_taken_in_chunks():
         assert list(seg.rows) == [m for m in ordered if m >= segment_plan.LISTED_ROWS]
         return ops._chunk_portions(decay, seg, sum(lengths))
 
-    assert portions("channel", [1] * 31 + [159]) == (0, 0)
-    assert portions("channel", [1] * 31 + [160]) == (1, 160)
-    assert portions("bonus", [1] * 31 + [511]) == (0, 0)
+    assert portions("channel", [159]) == (0, 0) and portions("channel", [160]) == (1, 160)
+    assert portions("channel", [1] * 31 + [239]) == (0, 0) and portions("channel", [1] * 31 + [240]) == (1, 240)
+    assert portions("channel", [20] * 20 + [224]) == (0, 0) and portions("channel", [1] * 7 + [224]) == (1, 224)
+    assert portions("bonus", [1] * 31 + [511]) == (0, 0) and portions("bonus", [1] * 31 + [512]) == (1, 512)
     assert portions("gated", [1, 300, 1, 47, 48, 700]) == (3, 1048)
-    assert portions("channel", [112] * 4) == (4, 448)
+    assert portions("channel", [128] * 4) == (4, 512) and portions("channel", [64] * 16 + [224]) == (17, 1248)
     assert portions("channel", [64] * 16) == (0, 0)                          # none of them long
-    assert portions("bonus", [112] * 4) == (0, 0)
+    assert portions("bonus", [128] * 8) == (0, 0) and portions("bonus", [192] * 8) == (8, 1536)
     assert portions("step", [1] * 8) == (0, 0)
     arrays, facts = planner.plan_decode(5)
     assert ops._chunk_portions("step", planner.bind({k: torch.tensor(v) for k, v in arrays.items()}, facts), 5) == (0, 0)
@@ -300,7 +301,7 @@ def test_who_is_taken_in_chunks():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("rule", RULES)
-@pytest.mark.parametrize("lengths", [(1, 1, 200, 5, 530, 1), (530,) + (1,) * 40, (47, 600, 48)])
+@pytest.mark.parametrize("lengths", [(1, 1, 200, 5, 530, 1), (530,) + (1,) * 40, (40, 600, 48)])
 def test_a_step_with_single_rows_beside_long_portions(rule, lengths):
     """Long portions in chunks, the other requests token by token, both against the recurrence in float64."""
     from tiny_inference_server_b200.kernels import ops, segment_plan

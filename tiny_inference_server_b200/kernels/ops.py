@@ -1174,15 +1174,22 @@ def _recurrence_spread(requests: Optional[int], num_heads: int, v_dim: int) -> i
 
 #: rows of a step's longest request from which the matrix-state recurrences run in chunks of 64 tokens
 #: (csrc/chunked_recurrence.cu) instead of token by token, by the kind of decay: the chunks have a time of their own, and the
-#: walks take unlike times a token.  Measured on a B200 at 12 heads of 128 x 128 in bfloat16, us token by token / in chunks,
-#: one request of 128, 200, 512 rows: delta rule 82 / 86, 126 / 106, 309 / 115; gated linear attention 59 / 68, 90 / 86,
-#: 218 / 80; state space 65 / 61, 100 / 76, 248 / 71; with a bonus 27 / 64, 40 / 81, 92 / 87
-CHUNKED_MIN_ROWS = {"channel": 160, "head": 160, "constant": 224, "forget": 208, "gated": 208, "step": 160, "bonus": 512}
+#: walks take unlike times a token.  Measured on a B200 at 12 heads of 128 x 128 in bfloat16, us token by token / in chunks, one
+#: request of 160, 224, 448 rows: delta rule 101 / 99, 139 / 104, 271 / 103, with a decay per head 87 / 97, 120 / 102, 234 / 101;
+#: constant decay 67 / 86, 95 / 85, 202 / 92; gated linear attention (and, like it, the forget gate) 72 / 81, 99 / 80, 192 / 90;
+#: state space 80 / 74, 110 / 73, 217 / 81 (8 heads of 64 x 64: 28 / 31, 38 / 32); with a bonus 33 / 81, 43 / 78, 82 / 87
+CHUNKED_MIN_ROWS = {"channel": 160, "head": 208, "constant": 224, "forget": 208, "gated": 192, "step": 192, "bonus": 512}
 if "TIS_CHUNKED_MIN_ROWS" in os.environ:
     CHUNKED_MIN_ROWS = dict.fromkeys(CHUNKED_MIN_ROWS, int(os.environ["TIS_CHUNKED_MIN_ROWS"]))
-#: several requests: from that many rows of the longest, and that many times the rows above in all that may be long.  Four
-#: requests of 112 rows: delta rule 163 / 119, gated 131 / 81, with a bonus 51 / 77; of 500: 713 / 236, 581 / 138, 212 / 133
-CHUNKED_PORTION_ROWS, CHUNKED_TOTAL = 96, 2
+#: several requests of CHUNKED_PORTION_ROWS and more: the rows of a step's portions from which they do.  4 of 128, 8 of 128, 8 of 192
+#: rows: delta rule 185 / 115, 275 / 136, 410 / 158 (24 heads, 8 of 96: 205 / 217); constant decay 80 / 97, 152 / 109, 225 / 115
+#: (8 heads of 64 x 64, 8 of 128: 42 / 44); gated 149 / 96, 224 / 106, 336 / 110; with a bonus 57 / 93, 108 / 104, 159 / 108
+CHUNKED_PORTION_ROWS = 128
+CHUNKED_TOTAL_ROWS = {"channel": 384, "head": 512, "constant": 1152, "forget": 512, "gated": 384, "step": 512, "bonus": 1152}
+#: with others in the step, which are walked behind the chunks and not beside the long walk: CHUNKED_BESIDE_OTHERS rows at least, and 1.5
+#: rows for each of them and 2 for each row of the longest.  Delta rule, 31 single rows beside 160 rows 111 / 131, beside 512 337 / 160;
+#: 100 beside 224 154 / 212; 20 of 20 rows beside 224 154 / 180; 7 single rows beside 224 161 / 128
+CHUNKED_BESIDE_OTHERS = 192
 #: scratch of the chunked form above which a step is walked token by token all the same (it grows with the rows: 147 KB a
 #: chunk and head of 128 x 128, 213 KB with the delta rule)
 CHUNKED_MAX_BYTES = 1 << 30
@@ -1200,10 +1207,13 @@ def _chunk_portions(decay: str, segments, n: int):
     least = CHUNKED_MIN_ROWS[decay]
     if len(segments) < 4:                                                   # rows not known one by one: all or none
         return (count, n) if longest >= least else (0, 0)
-    total = sum(segments[3])
-    if longest < least and not (longest >= CHUNKED_PORTION_ROWS and total >= CHUNKED_TOTAL * least):
-        return 0, 0
-    return len(segments[3]), total
+    total, others = sum(segments[3]), count - len(segments[3])
+    more = int(1.5 * others + 2 * segments[4]) if others else 0
+    if longest >= max(least, CHUNKED_BESIDE_OTHERS + more if others else 0):
+        return len(segments[3]), total
+    if longest >= CHUNKED_PORTION_ROWS and total >= CHUNKED_TOTAL_ROWS[decay] + 2 * more:
+        return len(segments[3]), total
+    return 0, 0
 
 
 class _Chunks(NamedTuple):
