@@ -203,15 +203,19 @@ def test_tiles_cover_the_rows_once():
 
 
 def test_shares_of_a_row_keep_all_clusters_resident():
-    from types import SimpleNamespace
     from tiny_inference_server_b200.kernels import ops
     # as a device answers whose clusters of 16 do not fill it: two CTAs an SM, and one
-    two = SimpleNamespace(decode_clusters={(0, 1): 296, (0, 2): 148, (0, 4): 72, (0, 8): 34, (0, 16): 14})
-    one = SimpleNamespace(decode_clusters={(0, 1): 148, (0, 2): 74, (0, 4): 36, (0, 8): 16, (0, 16): 7})
-    assert ops._decode_shares(two, 0, 14, 4096) == 16 and ops._decode_shares(two, 0, 15, 4096) == 8
-    assert ops._decode_shares(two, 0, 16, 1000) == 8 and ops._decode_shares(two, 0, 400, 4096) == 1
-    assert ops._decode_shares(one, 0, 8, 4096) == 8 and ops._decode_shares(one, 0, 32, 4096) == 4
-    assert ops._decode_shares(two, 0, 1, 63) == 1 and ops._decode_shares(two, 0, 1, 64) == 2       # a tile of keys each
+    two = {(0, 1): 296, (0, 2): 148, (0, 4): 71, (0, 8): 33, (0, 16): 14}
+    one = {(0, 1): 148, (0, 2): 74, (0, 4): 33, (0, 8): 15, (0, 16): 7}
+    shares = ops._decode_shares
+    assert shares(two, 0, 14, 4096, 128, 8) == 16 and shares(two, 0, 15, 4096, 128, 8) == 8
+    assert shares(two, 0, 16, 1000, 128, 4) == 8 and shares(two, 0, 400, 4096, 128, 4) == 1
+    assert shares(one, 0, 32, 8000, 256, 2) == 4 and shares(one, 0, 8, 1000, 256, 2) == 8
+    assert shares(two, 0, 1, 63, 128, 4) == 1 and shares(two, 0, 1, 64, 128, 4) == 2                # a tile of keys each
+    # few rows, many keys: more shares than a cluster has
+    assert shares(two, 0, 1, 8000, 192, 16) == 16 and shares(two, 0, 1, 16000, 192, 16) == 0
+    assert shares(two, 0, 3, 64000, 128, 8) == 16 and shares(one, 0, 16, 16000, 256, 2) == 0
+    assert shares(one, 0, 256, 100, 256, 2) == 0 and shares(one, 0, 64, 100, 256, 2) == 2
 
 
 def test_when_long_portions_are_worth_a_launch(monkeypatch):

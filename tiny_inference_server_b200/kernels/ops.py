@@ -1044,13 +1044,29 @@ def _wide_tiles_pay(rows: int, others: int, keys: int, num_heads: int) -> bool:
     return others <= 0 or (rows - others) * num_heads >= WINDOW_ATTENTION_TC_MIXED_ROWS
 
 
-def _decode_shares(wlib, form: int, clusters: int, keys: int) -> int:
-    """Shares of the keys of a row, a cluster of CTAs: as many as keep all clusters resident at once, a tile of 64 keys each at least.
-    A second wave of a few clusters would cost as much as the first, and clusters do not fill the device as single CTAs do."""
-    splits = 16
-    while splits > 1 and (splits > keys // 64 + 1 or wlib.decode_clusters[form, splits] < clusters):
+def _merged_shares(tiles: int, keys: int) -> int:
+    """Shares of the keys of a decode step's tiles on the mma.sync kernel: about two CTAs an SM in all."""
+    return max(1, min(keys // 64 + 1, WINDOW_ATTENTION_CTAS // max(1, tiles), 64))
+
+
+def _decode_shares(resident, form: int, clusters: int, keys: int, k_dim: int, group: int) -> int:
+    """Shares of the keys of a row on the decode kernel, a cluster of CTAs; 0: the mma.sync kernel is the faster one.
+
+    As many shares as keep all clusters resident at once, a tile of 64 keys each at least: a second wave of a few clusters would cost
+    as much as the first, and clusters do not fill the device as single CTAs do (the device is asked: 15 clusters of 8 at one CTA an SM, 14 of
+    16 at two; 33 clusters of 8 took 21 us, of 4 29; 16 of 16 26 us, of 8 18).  At most 16 shares a row, where the mma.sync kernel takes up to 64 and a merge: with
+    few rows and many keys that wins.  us: 6 and one tile after the other here, 10 and likewise there, a tile (four times as many
+    warps on it here) 1.0 for keys of less than 128 elements, 1.2, and 1.55 above 192, there 3.65, 5.0, with 16 query heads a kv
+    head 3.0; measured from 100 to 64000 keys and 1 to 128 rows: 1 row, 16 heads on a row of 192, 16000 keys 26 here, 25 there, 8000
+    keys 16.5 and 19; 4 rows, 4 kv heads of 256, 8000 keys 53 and 48, 8 rows 53 and 84."""
+    splits, tiles = 16, keys // 64 + 1
+    while splits > 1 and (splits > tiles or resident[form, splits] < clusters):
         splits //= 2
-    return splits
+    if k_dim > 192 and clusters > resident[form, 1] // 2 and tiles <= 2:
+        return 0                                                            # (64 and 128 rows of 100 keys on 4 kv heads: 15.1 and 14.6, 29.8 and 27.8)
+    here = 6 + (1.0 if k_dim < 128 else 1.2 if k_dim <= 192 else 1.55) * tiles / splits
+    there = 10 + (3.0 if group == 16 else 3.65 if k_dim < 128 else 5.0) * tiles / _merged_shares(clusters, keys)
+    return splits if here <= there else 0
 
 
 def _window_boxes(page_size: int, heads: int, k_dim: int, v_dim: int, k_strides, v_strides, same_start: bool) -> int:
@@ -1100,8 +1116,10 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
         keys = 0
         if decode:
             keys = step.max_position + 1 if not window else min(int(window), step.max_position + 1)
+        splits = 0
         if decode and count == n and boxes & wlib.decode_forms and num_heads // kv_heads <= 16 and WINDOW_ATTENTION_DECODE:
-            splits = _decode_shares(wlib, boxes - 1, count * kv_heads, keys)
+            splits = _decode_shares(wlib.decode_clusters, boxes - 1, count * kv_heads, keys, k_dim, num_heads // kv_heads)
+        if splits:
             calls["window_attention_decode"] += 1
             _check(wlib.tis_window_attention_decode(_p(q), q.stride(0), _p(gate), gate_row, int(gate_per_head), _p(out), out.stride(0),
                                                     _p(k_pages), kps, _p(v_pages), vps, int(boxes == 2), _p(block_table),
@@ -1130,8 +1148,7 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
         # (about two CTAs per SM in all), whose partial results a second launch merges
         splits, partial = 1, None
         if decode:
-            key_tiles = keys // 64 + 1
-            splits = max(1, min(key_tiles, WINDOW_ATTENTION_CTAS // max(1, count * kv_heads), 64))
+            splits = _merged_shares(count * kv_heads, keys)
             if splits > 1:
                 wlib.tis_window_attention_partial_floats.restype = ctypes.c_size_t
                 partial = torch.empty(wlib.tis_window_attention_partial_floats(count, kv_heads, splits), dtype=torch.float32,
