@@ -699,8 +699,8 @@ template <int K, int NT> struct DeltaSmem {
 
 // The chain of the delta rule: per chunk U = U0 - W S and S <- diag(decay) S + Kd^T U, 8 NT columns of one head's state a
 // CTA.  The state lives in the registers of the warps that sum it and, for the next chunk's first product, in shared
-// memory; the next chunk's operands are copied while this one's run.  Bound by the two products' tensor instructions
-// (768 cycles each at 16 columns) and what stands between them: two barriers, the operands' split.
+// memory; the next chunk's operands are copied while this one's run.  Bound by the chain of the two products (seven tensor
+// instructions a step of 16 along the sum) and what stands between them: two barriers, the operands' split.
 template <int K, int V, int NT>
 __global__ void __launch_bounds__(256, 1) chunk_delta_kernel(const ChunkArgs p) {
     typedef DeltaSmem<K, NT> L;

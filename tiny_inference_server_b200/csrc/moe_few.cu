@@ -5,7 +5,8 @@
 // rows of an mma.sync tile and up to 32 (row, choice) pairs of the expert its columns.  The summed index may run in any order
 // that both operands agree on: a lane's 16 bytes of a matrix row (eight neighbouring elements) are its share of two products,
 // and the same eight elements of its column's input row, so both come from global memory in 16-byte loads, as they lie.
-// 8 rows of 1536, 16 experts of 1024 hidden elements, 3 a row: 25 + 21 us before, 21 + 23 us now (cold, under the profiler).  More rows share an expert's bytes, where before each read them again.
+// 8 rows of 1536, 16 experts of 1024 hidden elements, 3 a row: 21 + 23 us, 25 + 21 with a dot product per element (cold, under the
+// profiler): so few rows seldom share an expert.  With more rows they do: a layer of 31 rows 47 us, 103 with dot products.
 #include "common.cuh"
 
 namespace {

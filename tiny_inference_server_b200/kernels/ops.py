@@ -1110,15 +1110,18 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
         row0, rows, count = tiles.rows
         wlib = window_attention_library(k_dim, v_dim)
         gate_row = gate.stride(0) if gate is not None else 0
-        boxes = _window_boxes(page_size, kv_heads, k_dim, v_dim, (kps.value, khs.value, k_dim), (vps.value, vhs.value, v_row),
-                              k_pages.data_ptr() == v_pages.data_ptr())
+        reach = getattr(step, "max_position", 0) + 1
+        keys = min(int(window), reach) if window else reach                 # that a row can see
         decode = getattr(step, "decode_only", False) and count > 0
-        keys = 0
-        if decode:
-            keys = step.max_position + 1 if not window else min(int(window), step.max_position + 1)
-        splits = 0
-        if decode and count == n and boxes & wlib.decode_forms and num_heads // kv_heads <= 16 and WINDOW_ATTENTION_DECODE:
-            splits = _decode_shares(wlib.decode_clusters, boxes - 1, count * kv_heads, keys, k_dim, num_heads // kv_heads)
+        wide0, wide, wide_count = tiles.wide
+        tc = bool(WINDOW_ATTENTION_TC and wide_count and _wide_tiles_pay(n, count - tiles.rows_in_wide, keys, num_heads)
+                  and (wide_count >= TC_ATTENTION_MIN_TILES or reach <= TC_ATTENTION_SHORT_CONTEXT))
+        boxes = splits = 0                                                  # (the host's time counts: asked for only where it matters)
+        if tc or (decode and count == n and num_heads // kv_heads <= 16 and WINDOW_ATTENTION_DECODE):
+            boxes = _window_boxes(page_size, kv_heads, k_dim, v_dim, (kps.value, khs.value, k_dim), (vps.value, vhs.value, v_row),
+                                  k_pages.data_ptr() == v_pages.data_ptr())
+            if not tc and boxes & wlib.decode_forms:
+                splits = _decode_shares(wlib.decode_clusters, boxes - 1, count * kv_heads, keys, k_dim, num_heads // kv_heads)
         if splits:
             calls["window_attention_decode"] += 1
             _check(wlib.tis_window_attention_decode(_p(q), q.stride(0), _p(gate), gate_row, int(gate_per_head), _p(out), out.stride(0),
@@ -1127,13 +1130,8 @@ def window_attention(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.T
                                                     num_heads, kv_heads, page_size, code, _f(scale), _f(cap), _p(bias_slope),
                                                     _p(bias_rate), _p(sink), splits, _p(fault), _stream()), wlib)
             return out
-        wide0, wide, wide_count = tiles.wide
-        tc = (WINDOW_ATTENTION_TC and wide_count and boxes & wlib.tc_forms and scale > 0 and out.stride(0) % 8 == 0
-              and out.data_ptr() % 16 == 0
-              and (gate is None or gate_per_head or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0)))
-        reach = getattr(step, "max_position", 0) + 1
-        tc = tc and _wide_tiles_pay(n, count - tiles.rows_in_wide, min(int(window), reach) if window else reach, num_heads)
-        if tc and (wide_count >= TC_ATTENTION_MIN_TILES or getattr(step, "max_position", 0) < TC_ATTENTION_SHORT_CONTEXT):
+        if (tc and boxes & wlib.tc_forms and scale > 0 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0
+                and (gate is None or gate_per_head or (gate.stride(0) % 8 == 0 and gate.data_ptr() % 16 == 0))):
             calls["window_attention_tc"] += 1
             _check(wlib.tis_window_attention_tc(_p(q), q.stride(0), n, _p(gate), gate_row, int(gate_per_head), _p(out), out.stride(0),
                                                 _p(k_pages), kps, _p(v_pages), vps, int(boxes == 2), _p(block_table),
@@ -1203,6 +1201,7 @@ if "TIS_CHUNKED_MIN_ROWS" in os.environ:
 #: (8 heads of 64 x 64, 8 of 128: 42 / 44); gated 149 / 96, 224 / 106, 336 / 110; with a bonus 57 / 93, 108 / 104, 159 / 108
 CHUNKED_PORTION_ROWS = 128
 CHUNKED_TOTAL_ROWS = {"channel": 384, "head": 512, "constant": 1152, "forget": 512, "gated": 384, "step": 512, "bonus": 1152}
+CHUNKED_LEAST_ROWS = min(CHUNKED_PORTION_ROWS, *CHUNKED_MIN_ROWS.values())          # of the longest in any case
 #: with others in the step, which are walked behind the chunks and not beside the long walk: CHUNKED_BESIDE_OTHERS rows at least, and 1.5
 #: rows for each of them and 2 for each row of the longest.  Delta rule, 31 single rows beside 160 rows 111 / 131, beside 512 337 / 160;
 #: 100 beside 224 154 / 212; 20 of 20 rows beside 224 154 / 180; 7 single rows beside 224 161 / 128
@@ -1244,6 +1243,8 @@ class _Chunks(NamedTuple):
 def _chunks(lib, decay: str, qkv: torch.Tensor, a_in, gate, out, state: torch.Tensor, segments, num_heads: int, qk_heads: int,
             k_dim: int, v_dim: int) -> Optional[_Chunks]:
     """The chunked part of a recurrence, or None: token by token.  ``gate``: a tensor, or its (address, row stride)."""
+    if segments is None or (len(segments) > 2 and segments[2] < CHUNKED_LEAST_ROWS):
+        return None
     n = qkv.shape[0]
     requests, rows = _chunk_portions(decay, segments, n)
     if not requests:
@@ -1261,19 +1262,27 @@ def _chunks(lib, decay: str, qkv: torch.Tensor, a_in, gate, out, state: torch.Te
     return _Chunks(scratch, requests, rows, requests < int(segments[1]))
 
 
+_NO_CHUNKS = (ctypes.c_void_p(0), ctypes.c_size_t(0), 0, 0)
+
+
 def _recurrence(lib, decay: str, chunks: Optional[_Chunks], n: int, requests: Optional[int], num_heads: int, k_dim: int, v_dim: int,
                 device):
     """(how the walk shares out a head's columns, 32-bit scratch for outputs that a launch of its own normalises, the launchers'
     arguments for the chunked part); counts what is launched beyond the one kernel that every call counts."""
     global launches
-    walked = chunks is None or chunks.others
+    if chunks is None:
+        apart = bool(lib.tis_delta_rule_splits(k_dim, v_dim))
+        launches += int(decay == "constant" or (apart and decay != "step"))
+        raw = None
+        if apart or decay in ("constant", "step"):
+            raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=device)
+        return _recurrence_spread(requests, num_heads, v_dim), raw, _NO_CHUNKS
+    walked = chunks.others
     apart = walked and bool(lib.tis_delta_rule_splits(k_dim, v_dim))       # the walk leaves its outputs to the norm
     raw = None
     if apart or decay in ("constant", "step"):
         raw = torch.empty((n, num_heads * v_dim), dtype=torch.float32, device=device)
-    launches += (3 if chunks is not None else -1) + int(walked) + int(decay == "constant" or (apart and decay != "step"))
-    if chunks is None:
-        return _recurrence_spread(requests, num_heads, v_dim), raw, (_p(None), ctypes.c_size_t(0), 0, 0)
+    launches += 3 + int(walked) + int(decay == "constant" or (apart and decay != "step"))
     requests = None if requests is None else max(1, requests - chunks.requests)
     return (_recurrence_spread(requests, num_heads, v_dim), raw,
             (_p(chunks.scratch), ctypes.c_size_t(chunks.scratch.numel()), chunks.requests, chunks.rows))
@@ -1538,7 +1547,7 @@ def time_mix(rkvg: torch.Tensor, w_in: torch.Tensor, u: torch.Tensor, w_bias: to
     n = rkvg.shape[0]
     if rkvg.dtype != w_in.dtype or rkvg.stride(1) != 1 or w_in.stride(1) != 1:
         raise KernelError("time_mix: the rows and the decays' projection are dense and of one type")
-    chunks = _chunks(lib, "bonus", rkvg, w_in, (_p(rkvg[:, 3 * num_heads * dim:]), rkvg.stride(0)), out, state, segments,
+    chunks = _chunks(lib, "bonus", rkvg, w_in, (ctypes.c_void_p(rkvg.data_ptr() + 3 * num_heads * dim * rkvg.element_size()), rkvg.stride(0)), out, state, segments,
                      num_heads, num_heads, dim, dim)
     narrow, raw, chunk_args = _recurrence(lib, "bonus", chunks, n, requests, num_heads, dim, dim, rkvg.device)
     _check(lib.tis_time_mix(_dt(rkvg), _p(rkvg), rkvg.stride(0), _p(w_in), w_in.stride(0), _p(u), _p(w_bias), _p(norm_weight),
