@@ -19,7 +19,7 @@ import torch
 from . import build as _build
 
 _lib = None
-ABI_VERSION = 16
+ABI_VERSION = 17
 #: launches of this library's kernels so far (library matrix products are not counted)
 launches = 0
 #: calls by kind, for tests that must know which kernel a product or an attention went to
@@ -442,6 +442,43 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None
     return out
 
 
+#: float32 products of at least SPLIT_MIN_ROWS rows and enough work go to the tcgen05 kernel of split operands
+#: (csrc/gemm_split.cu) instead of the library's product on the CUDA cores.  A tile's time is K / 32 steps of 1.2 us (half of
+#: them where two CTAs share one) whatever its rows and columns are, so a small result does not pay: measured on a B200, us
+#: library / split, at M x N of 1.0e5 (128 x 1536 x K) 43 / 46 at K 1536, 82 / 97 at 4096; 3.1e5 (200 x 1536) 47 / 44, 111 / 95;
+#: 4.0e5 (65 x 6144) 49 / 46; 1.2e6 (777 x 1536) 111 / 46, 277 / 95; 4.8e6 (777 x 6144) 301 / 137; 1.3e7 (2048 x 6144) 660 / 261.
+#: With a short K the launch counts: 333 x 512 x 1344 (2.3e8) 21 / 26, 512 x 512 x 1344 (3.5e8) 29 / 26, 1024 x 128 x 1536
+#: (2.0e8) 19 / 21, 2048 x 128 x 1536 (4.0e8) 31 / 21.  Up to 64 rows the library streams the weights faster (16 x 1536 x
+#: 49152: 121 / 150).  TIS_SPLIT_MIN_ROWS overrides (0: never).
+SPLIT_MIN_ROWS = int(os.environ.get("TIS_SPLIT_MIN_ROWS", "65"))
+SPLIT_MIN_RESULT = 300_000
+SPLIT_MIN_WORK = 350_000_000
+
+
+def _split_ok(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor]) -> bool:
+    return (a.dtype == torch.float32 and w.dtype == torch.float32 and 0 < SPLIT_MIN_ROWS <= a.shape[0]
+            and a.shape[0] * w.shape[1] >= SPLIT_MIN_RESULT and a.shape[0] * w.shape[1] * a.shape[1] >= SPLIT_MIN_WORK
+            and a.stride(1) == 1 and w.stride(1) == 1 and a.shape[1] % 4 == 0 and w.shape[1] % 4 == 0
+            and a.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and a.stride(0) >= a.shape[1] > 0 and w.stride(0) >= w.shape[1]
+            and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and (out is None or (out.dtype == torch.float32 and out.stride(1) == 1 and out.stride(0) % 4 == 0
+                                 and out.stride(0) >= w.shape[1] and out.data_ptr() % 16 == 0)))
+
+
+def gemm_split(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``a (n, K) @ w (K, N)`` in float32 on the tcgen05 tensor cores, operands split in three bfloat16 numbers (all of
+    their 24 bits), sums of 32 terms added in 32 bits."""
+    lib = library()
+    n, k = a.shape
+    cols = w.shape[1]
+    if out is None:
+        out = torch.empty((n, cols), dtype=torch.float32, device=a.device)
+    calls["gemm_split"] += 1
+    _check(lib.tis_gemm_split(_p(a), a.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), n, cols, k, _p(tc_fault()),
+                              _stream()), lib)
+    return out
+
+
 #: bfloat16 library products go to cuBLAS directly (the same kernels as torch.mm, a third of the host
 #: time per call); TIS_LIBRARY_GEMM=torch sends them through torch.mm instead
 LIBRARY_GEMM_DIRECT = os.environ.get("TIS_LIBRARY_GEMM", "direct") != "torch"
@@ -527,6 +564,8 @@ def gemm(a, w: torch.Tensor, out: Optional[torch.Tensor] = None, sink: Optional[
         a = scaled.dense()
     if _tc_ok(a, w, TC_PLAIN_MIN_ROWS) and (out is None or (out.stride(1) == 1 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0)):
         return gemm_tc(a, w, out)
+    if _split_ok(a, w, out):
+        return gemm_split(a, w, out)
     direct = _library_gemm(a, w, out, False)
     if direct is not None:
         return direct
