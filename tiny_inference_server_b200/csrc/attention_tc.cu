@@ -3,26 +3,34 @@
 //
 // A CTA owns up to 128 consecutive rows (positions pos0..pos0+rows-1) of one request and one
 // query head, and walks the keys 128 at a time.  Three roles, specialised by warp:
-//   warps 0 and 10   the TMA engine's clients: warp 0 brings the Q tile once (128-byte swizzle)
-//            and then the keys of every key tile, warp 10 the values, each into a ring of
+//   warps 0, 12 and 2, 13   the TMA engine's clients: warp 0 brings the Q tile once (128-byte
+//            swizzle), warps 0 and 12 the keys of every key tile, 2 and 13 the values, each pair into a ring of
 //            shared-memory slots of its own (keys are needed early, values late: with rings of
 //            their own the key loads run ahead), one box of 64 elements x page_size rows per page
-//            and half of the head (lanes order the pages of a tile side by side).  The cache
+//            and half of the head, a lane a box (a warp orders one in about 75 cycles).  The cache
 //            keeps rows XOR-swizzled by the position, so the boxes, copied as the bytes lie, are
 //            at once the swizzled operand tiles;
-//   warps 1 and 11   issue the products (one lane each; warp 1 also owns the tensor memory):
+//   warps 1 and 3   issue the products (one lane each; warp 1 also owns the tensor memory):
 //            warp 1 S = Q K^T into one of two score buffers in tensor memory (keys as the K-major
-//            operand), warp 11 O += P V (values as the MN-major operand, P from shared memory);
+//            operand), warp 3 O += P V (values as the MN-major operand, P from shared memory);
 //            two issuing threads, so that one's wait for a barrier does not idle the tensor cores;
-//   warps 2-5 and 6-9: two softmax groups, one thread per query row each.  Even key tiles go
+//   warps 4-7 and 8-11: two softmax groups, one thread per query row each.  Even key tiles go
 //            to the first group, odd ones to the second, each with a score buffer, a P buffer,
 //            an output accumulator in tensor memory and running maximum and sum of its own, so
 //            the softmax of one tile runs under the products and the softmax of the next; the
-//            two halves are merged at the end.  A thread reads its row of S (tcgen05.ld),
-//            scales, masks, does the online softmax in float32 and writes P in bfloat16 into
-//            shared memory in the operand layout.  The running maximum is only raised when the
-//            row's new maximum exceeds it by more than 2^8 (the exponentials stay small enough);
-//            O in tensor memory is then rescaled (tcgen05.ld, tcgen05.st).
+//            two halves are merged at the end.  A thread reads its row of S (tcgen05.ld) into
+//            registers and gives the buffer back at once, so that the scores of the group's next
+//            tile are there when it comes to them; it scales, masks, does the online softmax in
+//            float32 and writes P in bfloat16 into shared memory in the operand layout.  The
+//            running maximum is only raised when the row's new maximum exceeds it by more than
+//            2^8 (the exponentials stay small enough); O in tensor memory is then rescaled
+//            (tcgen05.ld, tcgen05.st).
+//            The two groups take turns with their exponentials; the merged rows leave through shared memory, whole rows a warp.
+// A key tile takes about 1800 cycles: a group's scores, maximum, exponentials (1500, the special function unit needs 1024) and
+// hand-overs, half of that with two groups.  Measured before (scores read twice from tensor memory, which held up the next
+// tile's; one warp that read a page's number when it ordered its boxes, 2300 cycles a tile) and after, 12 heads on 3 kv heads of
+// 128, pages of 16: 2048 rows 28.9 -> 23.3 us, two prompts of 2048 rows together 35.7 -> 22.4, 1024 rows behind 1024
+// 28.3 -> 22.5, 300 rows 13.0 -> 9.9; 24 heads on 8, 2048 rows 55.5 -> 44.0.
 // All hand-offs are mbarriers with bounded waits; a wait that runs out sets the fault word and
 // every role leaves; tensor memory is freed on every path.
 #include "tc_common.cuh"
@@ -41,12 +49,13 @@ constexpr int HD = TIS_HD;
 constexpr int HALVES = HD / 64;             // 128-byte column blocks of a row
 constexpr int BM = 128;                     // query rows of a CTA
 constexpr int BN = 128;                     // keys of a tile
-constexpr int NTH = 384;
+constexpr int NTH = 512;
 constexpr int HALF_BYTES = 128 * 128;       // 128 rows x 128 bytes: one swizzled column block
 constexpr int Q_BYTES = HALVES * HALF_BYTES;
 constexpr int P_BYTES = 2 * HALF_BYTES;     // 128 rows x 128 keys, bfloat16 (one per softmax group)
 constexpr int SLOT_BYTES = HALVES * HALF_BYTES;   // keys or values of one tile
 constexpr int SLOTS = HD == 128 ? 2 : 4;     // per ring (keys, values)
+constexpr int PAGES_AHEAD = 3;
 constexpr unsigned TMEM_COLS = 512;
 constexpr unsigned COL_S = 0;               // two score buffers of 128 columns
 constexpr unsigned COL_O = 256;             // two output accumulators of up to 128 columns
@@ -79,7 +88,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     unsigned char* p_smem = base + Q_BYTES;
     unsigned char* k_slots = p_smem + 2 * P_BYTES;
     unsigned char* v_slots = k_slots + SLOTS * SLOT_BYTES;
-    __shared__ unsigned long long q_full, full_k[SLOTS], empty_k[SLOTS], full_v[SLOTS], empty_v[SLOTS], s_full[2], p_full[2], o_done[2];
+    __shared__ unsigned long long q_full, full_k[SLOTS], empty_k[SLOTS], full_v[SLOTS], empty_v[SLOTS], s_full[2], s_free[2], p_full[2], o_done[2], turn[2];
     __shared__ unsigned tmem_base_slot;
     __shared__ int abort_flag;
 
@@ -106,11 +115,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     if (threadIdx.x == 0) {
         mbar_init(&q_full, 1);
         for (int s = 0; s < SLOTS; ++s) {
-            mbar_init(&full_k[s], 1); mbar_init(&empty_k[s], 1);
-            mbar_init(&full_v[s], 1); mbar_init(&empty_v[s], 1);
+            mbar_init(&full_k[s], 2); mbar_init(&empty_k[s], 1);
+            mbar_init(&full_v[s], 2); mbar_init(&empty_v[s], 1);
         }
         mbar_init(&s_full[0], 1); mbar_init(&s_full[1], 1);
+        mbar_init(&s_free[0], 4); mbar_init(&s_free[1], 4);
         mbar_init(&p_full[0], 4); mbar_init(&p_full[1], 4);
+        mbar_init(&turn[0], 4); mbar_init(&turn[1], 4);
         mbar_init(&o_done[0], 1); mbar_init(&o_done[1], 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -125,98 +136,104 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
     volatile int* abort = &abort_flag;
     pdl_wait();                                           // q and the cache rows of this step come from the kernel before
 
-    if (warp == 0 || warp == 10) {
-        // ---- loads: warp 0 keys (and Q), warp 10 values -----------------------------------------
-        const int kv = warp == 0 ? 0 : 1;
-        unsigned long long* full = kv ? full_v : full_k;
-        unsigned long long* empty = kv ? empty_v : empty_k;
-        unsigned char* ring = kv ? v_slots : k_slots;
-        const int ppt = BN / p.page_size;                 // pages of a key tile (1..8)
-        const int* bt = p.block_table + (size_t)slot * p.bt_stride;
-        auto page_of = [&](int j) -> int {
-            if (lane >= ppt) return 0;
-            const int key0 = tile_begin + j * BN + lane * p.page_size;
-            if (key0 >= hi || key0 + p.page_size <= lo_first) return 0;   // no row sees it: any page will do
-            const int pg = bt[key0 / p.page_size];
-            if (pg < 0 || pg >= p.num_pages) { atomicExch(p.fault, 3); return 0; }
-            return pg;
-        };
-        if (kv == 0 && lane == 0) {
-            mbar_arrive_expect_tx(&q_full, Q_BYTES);
+    // 512 threads are launched with 128 registers each, 65536 in all: 256 x 40 + 256 x 216
+    if (warp < 4 || warp >= 12) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;\n" ::);
+        if (warp == 0 || warp == 2 || warp == 12 || warp == 13) {
+            // ---- loads: warps 0 and 12 keys (and Q), warps 2 and 13 values ----------------------------
+            const int kv = warp == 0 || warp == 12 ? 0 : 1, part = warp >= 12 ? 1 : 0;
+            unsigned long long* full = kv ? full_v : full_k;
+            unsigned long long* empty = kv ? empty_v : empty_k;
+            unsigned char* ring = kv ? v_slots : k_slots;
+            const int ppt = BN / p.page_size, boxes = ppt * HALVES;           // pages of a key tile (1..8), its boxes
+            const bool mine = lane < boxes && (lane & 1) == part;             // a lane a box, the two warps taking turns
+            const int part_bytes = (boxes + 1 - part) / 2 * p.page_size * 128, in_tile = lane / HALVES * p.page_size;
+            const int* bt = p.block_table + (size_t)slot * p.bt_stride;
+            // the page of a lane's keys in tile j, looked at when its copies are ordered: the table's entries are on their way
+            // PAGES_AHEAD tiles earlier (read when they are needed they cost a tile 800 of 2300 cycles)
+            auto page_of = [&](int j) -> int {
+                const int key0 = tile_begin + j * BN + in_tile;
+                if (j >= T || !mine || key0 >= hi || key0 + p.page_size <= lo_first) return 0;  // no row sees it: any page will do
+                return bt[key0 / p.page_size];
+            };
+            if (warp == 0 && lane == 0) {
+                mbar_arrive_expect_tx(&q_full, Q_BYTES);
 #pragma unroll
-            for (int hh = 0; hh < HALVES; ++hh)
-                tma_load_2d(q_smem + hh * HALF_BYTES, &map_q, head * HD + hh * 64, row0, &q_full);
-        }
-        int page_next = page_of(0);
-        for (int j = 0; j < T; ++j) {
-            const int page = page_next;
-            page_next = j + 1 < T ? page_of(j + 1) : 0;
-            const int s = j % SLOTS;
-            int got = 1;
-            if (lane == 0) got = mbar_wait(&empty[s], ((j / SLOTS) & 1) ^ 1, abort, p.fault, 6) ? 1 : 0;
-            got = __shfl_sync(0xffffffffu, got, 0);
-            if (!got) break;
-            if (lane == 0) mbar_arrive_expect_tx(&full[s], SLOT_BYTES);
-            __syncwarp();
-            if (lane < ppt) {
-                unsigned char* dst = ring + (size_t)s * SLOT_BYTES + lane * p.page_size * 128;
-                const int y = ((page * 2 + kv) * p.KVH + kvh) * p.page_size;
-#pragma unroll
-                for (int hh = 0; hh < HALVES; ++hh) tma_load_2d(dst + hh * HALF_BYTES, &map_kv, hh * 64, y, &full[s]);
+                for (int hh = 0; hh < HALVES; ++hh)
+                    tma_load_2d(q_smem + hh * HALF_BYTES, &map_q, head * HD + hh * 64, row0, &q_full);
             }
-        }
-    } else if (warp == 1) {
-        // ---- products, first kind: S_j = Q K_j^T into score buffer j & 1 ----------------------------
-        if (lane == 0) {
-            constexpr unsigned IDESC_S = instr_desc(BM, BN, false);
-            const unsigned long long q_desc0 = smem_desc(smem_u32(q_smem), 16, 1024);
-            const unsigned long long k_desc0 = smem_desc(smem_u32(k_slots), 16, 1024);
-            bool ok = mbar_wait(&q_full, 0, abort, p.fault, 6);
-            for (int j = 0; j < T && ok; ++j) {
-                const int g = j & 1, i = j >> 1, s = j % SLOTS;
-                // the group has read the scores of its tile before (it hands P over after that)
-                if (i > 0 && !mbar_wait(&p_full[g], (i - 1) & 1, abort, p.fault, 6)) break;
-                if (!mbar_wait(&full_k[s], (j / SLOTS) & 1, abort, p.fault, 6)) break;
-                fence_after();
-                // descriptors differ from the ring's first one only in the start address (units of 16 bytes)
-                const unsigned long long kd = k_desc0 + (unsigned long long)((s * SLOT_BYTES) >> 4);
-                const unsigned d = tmem_base + COL_S + g * BN;
+            int pages[PAGES_AHEAD];
 #pragma unroll
-                for (int kk = 0; kk < HD / 16; ++kk) {
-                    const unsigned long long off = (unsigned long long)(((kk >> 2) * HALF_BYTES + (kk & 3) * 32) >> 4);
-                    umma(d, q_desc0 + off, kd + off, IDESC_S, kk != 0);
-                }
-                umma_commit(&empty_k[s]);
-                umma_commit(&s_full[g]);
-            }
-        }
-    } else if (warp == 11) {
-        // ---- products, second kind: O_g += P_j V_j.  An issuing thread of its own: while one thread
-        // waits for a barrier the other keeps the tensor cores fed. ------------------------------------
-        if (lane == 0) {
-            constexpr unsigned IDESC_O = instr_desc(BM, HD, true);
-            const unsigned long long p_desc0 = smem_desc(smem_u32(p_smem), 16, 1024);
-            const unsigned long long v_desc0 = smem_desc(smem_u32(v_slots), HALF_BYTES, 1024);
+            for (int a = 0; a < PAGES_AHEAD; ++a) pages[a] = page_of(a);
             for (int j = 0; j < T; ++j) {
-                const int g = j & 1, i = j >> 1, s = j % SLOTS;
-                if (!mbar_wait(&p_full[g], i & 1, abort, p.fault, 6)) break;
-                if (!mbar_wait(&full_v[s], (j / SLOTS) & 1, abort, p.fault, 6)) break;
-                fence_after();
-                const unsigned long long vd = v_desc0 + (unsigned long long)((s * SLOT_BYTES) >> 4);
-                const unsigned long long pd = p_desc0 + (unsigned long long)((g * P_BYTES) >> 4);
-                const unsigned d = tmem_base + COL_O + g * 128;
+                int page = pages[0];
 #pragma unroll
-                for (int kk = 0; kk < BN / 16; ++kk) {    // 16 keys: 32 bytes along a row of P, 16 rows of V
-                    umma(d, pd + (unsigned long long)(((kk >> 2) * HALF_BYTES + (kk & 3) * 32) >> 4),
-                         vd + (unsigned long long)((kk * 2048) >> 4), IDESC_O, (i | kk) != 0);
+                for (int a = 1; a < PAGES_AHEAD; ++a) pages[a - 1] = pages[a];
+                pages[PAGES_AHEAD - 1] = page_of(j + PAGES_AHEAD);
+                const int s = j % SLOTS;
+                if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ((j / SLOTS) & 1) ^ 1, abort, p.fault, 6))) break;
+                if (page < 0 || page >= p.num_pages) { atomicExch(p.fault, 3); page = 0; }
+                if (lane == 0) mbar_arrive_expect_tx(&full[s], part_bytes);
+                __syncwarp();
+                if (mine) {
+                    const int half = lane % HALVES;
+                    tma_load_2d(ring + (size_t)s * SLOT_BYTES + half * HALF_BYTES + in_tile * 128, &map_kv, half * 64,
+                                ((page * 2 + kv) * p.KVH + kvh) * p.page_size, &full[s]);
                 }
-                umma_commit(&empty_v[s]);
-                umma_commit(&o_done[g]);
+            }
+        } else if (warp == 1) {
+            // ---- products, first kind: S_j = Q K_j^T into score buffer j & 1 ----------------------------
+            if (lane == 0) {
+                constexpr unsigned IDESC_S = instr_desc(BM, BN, false);
+                const unsigned long long q_desc0 = smem_desc(smem_u32(q_smem), 16, 1024);
+                const unsigned long long k_desc0 = smem_desc(smem_u32(k_slots), 16, 1024);
+                bool ok = mbar_wait(&q_full, 0, abort, p.fault, 6);
+                for (int j = 0; j < T && ok; ++j) {
+                    const int g = j & 1, i = j >> 1, s = j % SLOTS;
+                    // the group has the scores of its tile before in registers
+                    if (!(i > 0 ? mbar_wait_both(&s_free[g], (i - 1) & 1, &full_k[s], (j / SLOTS) & 1, abort, p.fault, 6)
+                                : mbar_wait(&full_k[s], (j / SLOTS) & 1, abort, p.fault, 6))) break;
+                    fence_after();
+                    // descriptors differ from the ring's first one only in the start address (units of 16 bytes)
+                    const unsigned long long kd = k_desc0 + (unsigned long long)((s * SLOT_BYTES) >> 4);
+                    const unsigned d = tmem_base + COL_S + g * BN;
+#pragma unroll
+                    for (int kk = 0; kk < HD / 16; ++kk) {
+                        const unsigned long long off = (unsigned long long)(((kk >> 2) * HALF_BYTES + (kk & 3) * 32) >> 4);
+                        umma(d, q_desc0 + off, kd + off, IDESC_S, kk != 0);
+                    }
+                    umma_commit(&empty_k[s]);
+                    umma_commit(&s_full[g]);
+                }
+            }
+        } else if (warp == 3) {
+            // ---- products, second kind: O_g += P_j V_j.  An issuing thread of its own: while one thread
+            // waits for a barrier the other keeps the tensor cores fed. ------------------------------------
+            if (lane == 0) {
+                constexpr unsigned IDESC_O = instr_desc(BM, HD, true);
+                const unsigned long long p_desc0 = smem_desc(smem_u32(p_smem), 16, 1024);
+                const unsigned long long v_desc0 = smem_desc(smem_u32(v_slots), HALF_BYTES, 1024);
+                for (int j = 0; j < T; ++j) {
+                    const int g = j & 1, i = j >> 1, s = j % SLOTS;
+                    if (!mbar_wait_both(&p_full[g], i & 1, &full_v[s], (j / SLOTS) & 1, abort, p.fault, 6)) break;
+                    fence_after();
+                    const unsigned long long vd = v_desc0 + (unsigned long long)((s * SLOT_BYTES) >> 4);
+                    const unsigned long long pd = p_desc0 + (unsigned long long)((g * P_BYTES) >> 4);
+                    const unsigned d = tmem_base + COL_O + g * 128;
+#pragma unroll
+                    for (int kk = 0; kk < BN / 16; ++kk) {    // 16 keys: 32 bytes along a row of P, 16 rows of V
+                        umma(d, pd + (unsigned long long)(((kk >> 2) * HALF_BYTES + (kk & 3) * 32) >> 4),
+                             vd + (unsigned long long)((kk * 2048) >> 4), IDESC_O, (i | kk) != 0);
+                    }
+                    umma_commit(&empty_v[s]);
+                    umma_commit(&o_done[g]);
+                }
             }
         }
     } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;\n" ::);
         // ---- softmax: one thread per query row in each of the two groups ----------------------
-        const int g = warp >= 6 ? 1 : 0;                  // warps 2-5 and 6-9
+        const int g = warp >= 8 ? 1 : 0;                  // warps 4-7 and 8-11
         const int quarter = warp & 3;                     // the lanes of tensor memory this warp may touch
         const int r = quarter * 32 + lane;
         const bool row_ok = r < nrows && p.row_slot[row0 + r] >= 0;
@@ -229,6 +246,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
         const bool warp_has_rows = __any_sync(0xffffffffu, row_ok);
         float m_used = -INFINITY, l_sum = 0.f;
         bool ok = true;
+        // before the exponentials of the group's tile i: the products of its tile before are done, and the other group's
+        // exponentials of the tile before in the row's order.  (Left to themselves the groups come to their exponentials
+        // together and share the units: each 2000 cycles for what takes one alone 1100.)
+        auto wait_turn = [&](int i) {
+            if (g == 0) return i == 0 || mbar_wait_both(&o_done[0], (i - 1) & 1, &turn[0], (i - 1) & 1, abort, p.fault, 6);
+            return i == 0 ? mbar_wait(&turn[1], 0, abort, p.fault, 6)
+                          : mbar_wait_both(&o_done[1], (i - 1) & 1, &turn[1], i & 1, abort, p.fault, 6);
+        };
         int i = 0;                                        // tiles of this group so far
         for (int j = g; j < T; j += 2, ++i) {
             if (!__all_sync(0xffffffffu, mbar_wait(&s_full[g], i & 1, abort, p.fault, 6))) { ok = false; break; }
@@ -241,50 +266,40 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                         *reinterpret_cast<uint4*>(pg_smem + r * 128 + (c >> 3) * HALF_BYTES + ((c & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
                     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 }
-                // it follows every phase of o_done all the same: a wait for the last one alone could return a phase early (the
-                // parity of the phase before the one before), and the merge below writes where P lies
-                if (i > 0 && !__all_sync(0xffffffffu, mbar_wait(&o_done[g], (i - 1) & 1, abort, p.fault, 6))) { ok = false; break; }
+                // it follows every phase of o_done and turn all the same: a wait for the last one alone could return a phase
+                // early (the parity of the phase before the one before), and the merge below writes where P lies
+                if (!__all_sync(0xffffffffu, wait_turn(i))) { ok = false; break; }
+                if (lane == 0) mbar_arrive(&turn[1 - g]);
                 fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&p_full[g]);
+                if (lane == 0) { mbar_arrive(&s_free[g]); mbar_arrive(&p_full[g]); }
                 continue;
             }
             const int kt = tile_begin + j * BN;
-            // Two passes over the row of S, 64 columns at a time (the row stays in tensor memory until
-            // this group hands P over): first the maximum, then the exponentials.
             const bool whole = kt + BN - 1 <= pos0 && kt >= lo_last;      // every row of the tile sees every key
-            const bool plain = whole && row_ok;
-            auto load64 = [&](int half, float (&s)[64], bool bound) {
-                tmem_ld32_issue(tmem_base + lane_bits + col_s + half * 64, s);
-                tmem_ld32_issue(tmem_base + lane_bits + col_s + half * 64 + 32, s + 32);
-                tmem_ld_wait();
-                tmem_ld_arrived(s);
-                if (bound) {
+            float s[BN];
 #pragma unroll
-                    for (int e = 0; e < 64; ++e) s[e] = soft_capped(s[e], p.cap);
-                }
-                if (!plain) {
+            for (int c = 0; c < BN / 32; ++c) tmem_ld32_issue(tmem_base + lane_bits + col_s + c * 32, s + c * 32);
+            tmem_ld_wait();
+            tmem_ld_arrived(s);
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[g]);
+            if (p.cap.k != 0.f) {
 #pragma unroll
-                    for (int e = 0; e < 64; ++e) {
-                        const int key = kt + half * 64 + e;
-                        s[e] = (row_ok && key <= qpos && key >= lo_r) ? s[e] : -INFINITY;
-                    }
-                }
-            };
-            // the row's maximum of the raw scores (the scale is positive), four chains side by side
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                float s[64];
-                load64(half, s, false);
-#pragma unroll
-                for (int e = 0; e < 64; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], s[e]);
+                for (int e = 0; e < BN; ++e) s[e] = soft_capped(s[e], p.cap);
             }
-            // (the bound never falls: the maximum of the bounded scores is the bounded maximum)
-            const bool capped = p.cap.k != 0.f;
-            float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            if (capped && mx > -INFINITY) mx = soft_capped(mx, p.cap);
-            mx *= p.scale_log2;
+            if (!(whole && row_ok)) {
+                // keys lo_r .. qpos, counted from the tile's first; a padding row sees none
+                const int from = row_ok ? lo_r - kt : 1 << 20, span = row_ok ? qpos - lo_r : 0;
+#pragma unroll
+                for (int e = 0; e < BN; ++e) s[e] = (unsigned)(e - from) <= (unsigned)span ? s[e] : -INFINITY;
+            }
+            // the row's maximum (the scale is positive), four chains side by side
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int e = 0; e < BN; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], s[e]);
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
             // raise the reference maximum only when the row's maximum left it far behind
             const bool raise = mx > m_used + RESCALE_STEP || (m_used == -INFINITY && mx > -INFINITY);
             float alpha = 1.f;
@@ -294,7 +309,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 l_sum *= alpha;
             }
             // the products of the group's tile before are done: O may be rescaled, P overwritten
-            if (i > 0 && !__all_sync(0xffffffffu, mbar_wait(&o_done[g], (i - 1) & 1, abort, p.fault, 6))) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, wait_turn(i))) { ok = false; break; }
             if (i > 0 && __any_sync(0xffffffffu, raise)) {
                 fence_after();
 #pragma unroll 1
@@ -310,23 +325,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             const float neg_m = m_used == -INFINITY ? 0.f : -m_used;
             float ps4[4] = {0.f, 0.f, 0.f, 0.f};
             unsigned char* prow = pg_smem + r * 128;
-#pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                float s[64];
-                load64(half, s, capped);
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {             // eight keys: one 16-byte chunk of the row of P
-                    unsigned pk[4];
+            for (int c = 0; c < BN / 8; ++c) {            // eight keys: one 16-byte chunk of the row of P
+                unsigned pk[4];
 #pragma unroll
-                    for (int e = 0; e < 8; e += 2) {
-                        const float a = fast_exp2(fmaf(s[c * 8 + e], p.scale_log2, neg_m));   // 2^-inf = 0 for masked keys
-                        const float b = fast_exp2(fmaf(s[c * 8 + e + 1], p.scale_log2, neg_m));
-                        ps4[e >> 1] += a + b;
-                        __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-                        pk[e >> 1] = *reinterpret_cast<unsigned*>(&h);
-                    }
-                    *reinterpret_cast<uint4*>(prow + half * HALF_BYTES + ((c ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                for (int e = 0; e < 8; e += 2) {
+                    const float a = fast_exp2(fmaf(s[c * 8 + e], p.scale_log2, neg_m));       // 2^-inf = 0 for masked keys
+                    const float b = fast_exp2(fmaf(s[c * 8 + e + 1], p.scale_log2, neg_m));
+                    ps4[e >> 1] += a + b;
+                    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+                    pk[e >> 1] = *reinterpret_cast<unsigned*>(&h);
                 }
+                *reinterpret_cast<uint4*>(prow + (c >> 3) * HALF_BYTES + (((c & 7) ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                if (c == BN / 16 - 1 && lane == 0) mbar_arrive(&turn[1 - g]);
             }
             l_sum += (ps4[0] + ps4[1]) + (ps4[2] + ps4[3]);
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -334,7 +345,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_full[g]);
         }
-        // ---- merge the two groups' halves; each group stores half of the columns -------------
+        // ---- merge the two groups' halves, each group half of the columns, and store them through the ring of keys, which
+        // has no more copies or products to come once both groups' last products are done --------------------------
+        typedef StagedRows<HD> Rows;
+        float* stage = reinterpret_cast<float*>(k_slots);
         if (i > 0 && ok) ok = __all_sync(0xffffffffu, mbar_wait(&o_done[g], (i - 1) & 1, abort, p.fault, 6));
         // the group's P buffer is free now: it carries the row's maximum and sum to the other group
         reinterpret_cast<float*>(pg_smem)[r] = m_used;
@@ -354,7 +368,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             float inv = l > 0.f ? 1.f / l : 0.f;
             if (p.gate != nullptr && r < nrows) inv /= 1.f + __expf(-__bfloat162float(p.gate[(size_t)(row0 + r) * p.ldg + head]));
             constexpr int COLS = HD / 2;                  // this group's share of the columns
-#pragma unroll 1
+#pragma unroll
             for (int c = 0; c < COLS / 32; ++c) {
                 const int col = g * COLS + c * 32;
                 float o0[32], o1[32];
@@ -363,15 +377,22 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                 tmem_ld_wait();
                 tmem_ld_arrived(o0);
                 if (T >= 2) tmem_ld_arrived(o1);
-                if (r < nrows) {                          // padding rows inside the tile get zeros
+                // padding rows inside the tile get zeros
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) o0[e] = row_ok ? (o0[e] * w0 + (T >= 2 ? o1[e] * w1 : 0.f)) * inv : 0.f;
-                    bf16* dst = p.out + (size_t)(row0 + r) * p.out_stride + head * HD + col;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) store8(dst + q * 8, o0 + q * 8);
-                }
+                for (int e = 0; e < 32; ++e) o0[e] = row_ok ? (o0[e] * w0 + (T >= 2 ? o1[e] * w1 : 0.f)) * inv : 0.f;
+                stage_put<HD>(stage, r, col, o0);
             }
             fence_before();
+        }
+        asm volatile("bar.sync 1, 256;\n" ::: "memory");
+        if (!*abort) {
+            const int first = Rows::row(warp - 4, lane, 0), col = Rows::col(lane);
+            bf16* dst = p.out + (size_t)(row0 + first) * p.out_stride + head * HD + col;
+#pragma unroll 4
+            for (int i = 0; i < Rows::STEPS; ++i, dst += (size_t)Rows::ROWS * p.out_stride) {
+                const float4 v = Rows::get(stage, first + i * Rows::ROWS, col);
+                if (first + i * Rows::ROWS < nrows) store4(dst, v);
+            }
         }
     }
 

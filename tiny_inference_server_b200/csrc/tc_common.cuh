@@ -40,6 +40,23 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
     return false;
 }
 
+// The same for two phases at once: the looks at the two barriers overlap (one that is complete already still takes some
+// hundred cycles).
+__device__ __forceinline__ bool mbar_wait_both(unsigned long long* a, unsigned parity_a, unsigned long long* b, unsigned parity_b,
+                                               volatile int* abort, int* fault, int code) {
+    unsigned done_a = 0, done_b = 0;
+    for (int spin = 0; spin < MBAR_SPINS; ++spin) {
+        asm volatile("{\n.reg .pred p, q;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%2], %3;\n"
+                     "mbarrier.try_wait.parity.shared::cta.b64 q, [%4], %5;\nselp.u32 %0, 1, 0, p;\nselp.u32 %1, 1, 0, q;\n}\n"
+                     : "=r"(done_a), "=r"(done_b) : "r"(smem_u32(a)), "r"(parity_a), "r"(smem_u32(b)), "r"(parity_b) : "memory");
+        if (done_a & done_b) return true;
+        if ((spin & 1023) == 1023 && *abort) return false;
+    }
+    *abort = 1;
+    atomicExch(fault, code);
+    return false;
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
                  ::"r"(smem_u32(dst)), "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
@@ -149,6 +166,35 @@ __device__ __forceinline__ void store8(bf16* p, const float* v) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
     *reinterpret_cast<uint4*>(p) = raw;
+}
+
+// A tile of up to 128 rows of W float32 columns (64, 128) that threads hold row by row goes to memory through shared memory, so that
+// a warp writes whole rows and reads a gate's whole rows.  16-byte pieces lie at their place XOR (row mod 8).
+template <int W> __device__ __forceinline__ void stage_put(float* stage, int row, int col, const float (&v)[32]) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(stage + row * W + (((col >> 2) + q) ^ (row & 7)) * 4) =
+            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+}
+// The rows of one of eight warps, sixteen: lane's place in the i-th step.
+template <int W> struct StagedRows {
+    static constexpr int LANES = W / 4, ROWS = 32 / LANES, STEPS = 16 / ROWS;       // lanes a row, rows a step, steps
+    static __device__ __forceinline__ int row(int warp8, int lane, int i) { return warp8 * 16 + i * ROWS + lane / LANES; }
+    static __device__ __forceinline__ int col(int lane) { return lane % LANES * 4; }
+    static __device__ __forceinline__ float4 get(const float* stage, int r, int col) {
+        return *reinterpret_cast<const float4*>(stage + r * W + ((col >> 2) ^ (r & 7)) * 4);
+    }
+};
+// a / b to two last places over the whole range (results below 2^-126 included), without the branch of the rounded division,
+// which keeps neighbouring divisions from running side by side: a row's gates took 700 cycles, with this 100
+__device__ __forceinline__ float divided(float a, float b) {
+    float q;
+    asm("div.full.f32 %0, %1, %2;\n" : "=f"(q) : "f"(a), "f"(b));
+    return q;
+}
+__device__ __forceinline__ void store4(bf16* p, const float4& v) {
+    __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+    *reinterpret_cast<uint2*>(p) = *reinterpret_cast<uint2*>(h);
 }
 
 // ---- host side: tensor maps ---------------------------------------------------------------

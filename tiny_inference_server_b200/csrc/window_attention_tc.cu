@@ -6,14 +6,15 @@
 //   * keys and values have widths of their own; their rows lie in the pages as they are, so the TMA engine swizzles the boxes;
 //   * the value rows may be the first TIS_VD elements of the key rows (SHARED): the key tile is then read a second time as the
 //     values, there is no ring of values and a slot is free when the tile's second product is done;
-//   * the bias costs a logarithm an element.  The first pass over a row of scores, which finds the maximum, leaves them in
-//     tensor memory with their bias and masked, so that the second pass takes only the exponentials;
+//   * the bias costs a logarithm an element;
 //   * rows of the value tile that no row of queries sees (before the window, behind the last row, pages of others) are zeroed:
 //     a probability of 0 must not meet what another request left there.
 // Bound by the chain of a tile through scores, softmax and second product (two tiles side by side), as attention_tc.cu.
 // Against the mma.sync kernel, which reads every operand fragment from shared memory per warp of 16 rows: 2048 rows, 12 query
 // heads of 128 on 3 kv heads, window 1024, with bias 103 -> 33 us; 1024 rows behind 1024 cached, 12 heads on one
-// compressed row of 192 (values 128) 201 -> 41 us (replayed from a graph); outputs against 64 bits 0.97 to 1.0 times as far off.
+// compressed row of 192 (values 128) 201 -> 39 us (replayed from a graph); outputs against 64 bits 0.97 to 1.0 times as far off.
+// With a gate the division a/(1 + e^-g) was 13000 of a tile's last cycles, an element after the other; now 4000 (same rows with
+// bias and gate 44 -> 35 us).
 #include "tc_common.cuh"
 
 #ifndef TIS_KD
@@ -36,12 +37,13 @@ constexpr int KD = TIS_KD, VD = TIS_VD;
 constexpr int K_BLOCKS = KD / 64, V_BLOCKS = VD / 64;       // 128-byte column blocks of a row
 constexpr int BM = 128;                     // query rows of a CTA
 constexpr int BN = 128;                     // keys of a tile
-constexpr int NTH = 384;
+constexpr int NTH = 512;
 constexpr int HALF_BYTES = 128 * 128;       // 128 rows x 128 bytes: one swizzled column block
 constexpr int Q_BYTES = K_BLOCKS * HALF_BYTES;
 constexpr int P_BYTES = 2 * HALF_BYTES;     // 128 rows x 128 keys, bfloat16 (one per softmax group)
 constexpr int K_BYTES = K_BLOCKS * HALF_BYTES, V_BYTES = V_BLOCKS * HALF_BYTES;      // keys, values of one tile
 constexpr int SLOTS = 2;                    // per ring
+constexpr int PAGES_AHEAD = 3;
 constexpr unsigned TMEM_COLS = 512;
 constexpr unsigned COL_S = 0;               // two score buffers of 128 columns
 constexpr unsigned COL_O = 256;             // two output accumulators of up to 128 columns
@@ -94,7 +96,7 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     unsigned char* p_smem = base + Q_BYTES;
     unsigned char* k_slots = p_smem + 2 * P_BYTES;
     unsigned char* v_slots = SHARED ? k_slots : k_slots + SLOTS * K_BYTES;
-    __shared__ unsigned long long q_full, full_k[SLOTS], empty_k[SLOTS], full_v[SLOTS], empty_v[SLOTS], s_full[2], p_full[2], o_done[2];
+    __shared__ unsigned long long q_full, full_k[SLOTS], empty_k[SLOTS], full_v[SLOTS], empty_v[SLOTS], s_full[2], s_free[2], p_full[2], o_done[2], turn[2];
     __shared__ unsigned tmem_base_slot;
     __shared__ int abort_flag;
 
@@ -121,11 +123,13 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     if (threadIdx.x == 0) {
         mbar_init(&q_full, 1);
         for (int s = 0; s < SLOTS; ++s) {
-            mbar_init(&full_k[s], 1); mbar_init(&empty_k[s], 1);
-            mbar_init(&full_v[s], 1); mbar_init(&empty_v[s], 1);
+            mbar_init(&full_k[s], SHARED ? 4 : 2); mbar_init(&empty_k[s], 1);
+            mbar_init(&full_v[s], 2); mbar_init(&empty_v[s], 1);
         }
         mbar_init(&s_full[0], 1); mbar_init(&s_full[1], 1);
+        mbar_init(&s_free[0], 4); mbar_init(&s_free[1], 4);
         mbar_init(&p_full[0], 4); mbar_init(&p_full[1], 4);
+        mbar_init(&turn[0], 4); mbar_init(&turn[1], 4);
         mbar_init(&o_done[0], 1); mbar_init(&o_done[1], 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -141,108 +145,115 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     volatile int* abort = &abort_flag;
     pdl_wait();                                           // q and the cache rows of this step come from the kernel before
 
-    if (warp == 0 || (warp == 10 && !SHARED)) {
-        // ---- loads: warp 0 keys (and Q), warp 10 values -----------------------------------------
-        const int kv = warp == 0 ? 0 : 1;
-        unsigned long long* full = kv ? full_v : full_k;
-        unsigned long long* empty = kv ? empty_v : empty_k;
-        unsigned char* ring = kv ? v_slots : k_slots;
-        const int ppt = BN / p.page_size;                 // pages of a key tile (1..8)
-        const int* bt = p.block_table + (size_t)slot * p.bt_stride;
-        auto page_of = [&](int j) -> int {
-            if (lane >= ppt) return 0;
-            const int key0 = tile_begin + j * BN + lane * p.page_size;
-            if (key0 >= hi || key0 + p.page_size <= lo_first) return 0;   // no row sees it: any page will do
-            const int pg = bt[key0 / p.page_size];
-            if (pg < 0 || pg >= p.num_pages) { atomicExch(p.fault, 5); return 0; }
-            return pg;
-        };
-        if (kv == 0 && lane == 0) {
-            mbar_arrive_expect_tx(&q_full, Q_BYTES);
+    // 512 threads are launched with 128 registers each, 65536 in all: 256 x 40 + 256 x 216
+    if (warp < 4 || warp >= 12) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;\n" ::);
+        if (warp == 0 || warp == 2 || warp == 12 || warp == 13) {
+            // ---- loads: warps 0 and 12 keys (and Q), warps 2 and 13 values, or keys as well --------------
+            const int kv = SHARED || warp == 0 || warp == 12 ? 0 : 1, parts = SHARED ? 4 : 2;
+            const int part = (warp >= 12 ? 1 : 0) + (SHARED && (warp == 2 || warp == 13) ? 2 : 0);
+            unsigned long long* full = kv ? full_v : full_k;
+            unsigned long long* empty = kv ? empty_v : empty_k;
+            unsigned char* ring = kv ? v_slots : k_slots;
+            const int blocks = kv ? V_BLOCKS : K_BLOCKS, boxes = BN / p.page_size * blocks;    // boxes of a key tile (1..32)
+            const bool mine = lane < boxes && lane % parts == part;           // a lane a box, the warps taking turns
+            const int part_bytes = (boxes + parts - 1 - part) / parts * p.page_size * 128, in_tile = lane / blocks * p.page_size;
+            const int* bt = p.block_table + (size_t)slot * p.bt_stride;
+            // (as in attention_tc.cu: read PAGES_AHEAD tiles before they are looked at)
+            auto page_of = [&](int j) -> int {
+                const int key0 = tile_begin + j * BN + in_tile;
+                if (j >= T || !mine || key0 >= hi || key0 + p.page_size <= lo_first) return 0;  // no row sees it: any page will do
+                return bt[key0 / p.page_size];
+            };
+            if (warp == 0 && lane == 0) {
+                mbar_arrive_expect_tx(&q_full, Q_BYTES);
 #pragma unroll
-            for (int hh = 0; hh < K_BLOCKS; ++hh)
-                tma_load_2d(q_smem + hh * HALF_BYTES, &map_q, head * KD + hh * 64, row0, &q_full);
-        }
-        int page_next = page_of(0);
-        for (int j = 0; j < T; ++j) {
-            const int page = page_next;
-            page_next = j + 1 < T ? page_of(j + 1) : 0;
-            const int s = j % SLOTS;
-            int got = 1;
-            if (lane == 0) got = mbar_wait(&empty[s], ((j / SLOTS) & 1) ^ 1, abort, p.fault, 6) ? 1 : 0;
-            got = __shfl_sync(0xffffffffu, got, 0);
-            if (!got) break;
-            if (lane == 0) mbar_arrive_expect_tx(&full[s], kv ? V_BYTES : K_BYTES);
-            __syncwarp();
-            if (lane < ppt) {
-                unsigned char* dst = ring + (size_t)s * (kv ? V_BYTES : K_BYTES) + lane * p.page_size * 128;
-                const CUtensorMap* map = kv ? &map_v : &map_k;
-                for (int hh = 0; hh < (kv ? V_BLOCKS : K_BLOCKS); ++hh)
-                    tma_load_3d(dst + hh * HALF_BYTES, map, hh * 64, kvh * p.page_size, page, &full[s]);
+                for (int hh = 0; hh < K_BLOCKS; ++hh)
+                    tma_load_2d(q_smem + hh * HALF_BYTES, &map_q, head * KD + hh * 64, row0, &q_full);
             }
-        }
-    } else if (warp == 1) {
-        // ---- products, first kind: S_j = Q K_j^T into score buffer j & 1 ----------------------------
-        constexpr unsigned IDESC_S = instr_desc(BM, BN, false);
-        const unsigned long long q_desc0 = smem_desc(smem_u32(q_smem), 16, 1024);
-        const unsigned long long k_desc0 = smem_desc(smem_u32(k_slots), 16, 1024);
-        bool ok = mbar_wait(&q_full, 0, abort, p.fault, 6);
-        for (int j = 0; j < T; ++j) {
-            const int g = j & 1, i = j >> 1, s = j % SLOTS;
-            // the group has read the scores of its tile before (it hands P over after that)
-            ok = ok && (i == 0 || mbar_wait(&p_full[g], (i - 1) & 1, abort, p.fault, 6));
-            ok = ok && mbar_wait(&full_k[s], (j / SLOTS) & 1, abort, p.fault, 6);
-            if (!__all_sync(0xffffffffu, ok)) break;
-            if (SHARED && (j == 0 || j == T - 1))
-                zero_rows(k_slots + s * K_BYTES, V_BLOCKS, lo_first - (tile_begin + j * BN), hi - (tile_begin + j * BN), lane);
-            if (lane == 0) {
-                fence_after();
-                // descriptors differ from the ring's first one only in the start address (units of 16 bytes)
-                const unsigned long long kd = k_desc0 + (unsigned long long)((s * K_BYTES) >> 4);
-                const unsigned d = tmem_base + COL_S + g * BN;
+            int pages[PAGES_AHEAD];
 #pragma unroll
-                for (int kk = 0; kk < KD / 16; ++kk) {
-                    const unsigned long long off = (unsigned long long)(((kk >> 2) * HALF_BYTES + (kk & 3) * 32) >> 4);
-                    umma(d, q_desc0 + off, kd + off, IDESC_S, kk != 0);
+            for (int a = 0; a < PAGES_AHEAD; ++a) pages[a] = page_of(a);
+            for (int j = 0; j < T; ++j) {
+                int page = pages[0];
+#pragma unroll
+                for (int a = 1; a < PAGES_AHEAD; ++a) pages[a - 1] = pages[a];
+                pages[PAGES_AHEAD - 1] = page_of(j + PAGES_AHEAD);
+                const int s = j % SLOTS;
+                if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ((j / SLOTS) & 1) ^ 1, abort, p.fault, 6))) break;
+                if (page < 0 || page >= p.num_pages) { atomicExch(p.fault, 5); page = 0; }
+                if (lane == 0) mbar_arrive_expect_tx(&full[s], part_bytes);
+                __syncwarp();
+                if (mine) {
+                    const int block = lane % blocks;
+                    tma_load_3d(ring + (size_t)s * (kv ? V_BYTES : K_BYTES) + block * HALF_BYTES + in_tile * 128, kv ? &map_v : &map_k,
+                                block * 64, kvh * p.page_size, page, &full[s]);
                 }
-                if (!SHARED) umma_commit(&empty_k[s]);
-                umma_commit(&s_full[g]);
             }
-            __syncwarp();
-        }
-    } else if (warp == 11) {
-        // ---- products, second kind: O_g += P_j V_j.  An issuing warp of its own: while one waits for a barrier the
-        // other keeps the tensor cores fed. --------------------------------------------------------------
-        constexpr unsigned IDESC_O = instr_desc(BM, VD, true);
-        constexpr int SLOT = SHARED ? K_BYTES : V_BYTES;
-        const unsigned long long p_desc0 = smem_desc(smem_u32(p_smem), 16, 1024);
-        const unsigned long long v_desc0 = smem_desc(smem_u32(v_slots), HALF_BYTES, 1024);
-        for (int j = 0; j < T; ++j) {
-            const int g = j & 1, i = j >> 1, s = j % SLOTS;
-            bool ok = SHARED || mbar_wait(&full_v[s], (j / SLOTS) & 1, abort, p.fault, 6);
-            if (!__all_sync(0xffffffffu, ok)) break;
-            if (!SHARED && (j == 0 || j == T - 1))
-                zero_rows(v_slots + s * V_BYTES, V_BLOCKS, lo_first - (tile_begin + j * BN), hi - (tile_begin + j * BN), lane);
-            ok = mbar_wait(&p_full[g], i & 1, abort, p.fault, 6);
-            if (!__all_sync(0xffffffffu, ok)) break;
-            if (lane == 0) {
-                fence_after();
-                const unsigned long long vd = v_desc0 + (unsigned long long)((s * SLOT) >> 4);
-                const unsigned long long pd = p_desc0 + (unsigned long long)((g * P_BYTES) >> 4);
-                const unsigned d = tmem_base + COL_O + g * 128;
+        } else if (warp == 1) {
+            // ---- products, first kind: S_j = Q K_j^T into score buffer j & 1 ----------------------------
+            constexpr unsigned IDESC_S = instr_desc(BM, BN, false);
+            const unsigned long long q_desc0 = smem_desc(smem_u32(q_smem), 16, 1024);
+            const unsigned long long k_desc0 = smem_desc(smem_u32(k_slots), 16, 1024);
+            bool ok = mbar_wait(&q_full, 0, abort, p.fault, 6);
+            for (int j = 0; j < T; ++j) {
+                const int g = j & 1, i = j >> 1, s = j % SLOTS;
+                // the group has the scores of its tile before in registers
+                ok = ok && (i == 0 ? mbar_wait(&full_k[s], (j / SLOTS) & 1, abort, p.fault, 6)
+                                   : mbar_wait_both(&s_free[g], (i - 1) & 1, &full_k[s], (j / SLOTS) & 1, abort, p.fault, 6));
+                if (!__all_sync(0xffffffffu, ok)) break;
+                if (SHARED && (j == 0 || j == T - 1))
+                    zero_rows(k_slots + s * K_BYTES, V_BLOCKS, lo_first - (tile_begin + j * BN), hi - (tile_begin + j * BN), lane);
+                if (lane == 0) {
+                    fence_after();
+                    // descriptors differ from the ring's first one only in the start address (units of 16 bytes)
+                    const unsigned long long kd = k_desc0 + (unsigned long long)((s * K_BYTES) >> 4);
+                    const unsigned d = tmem_base + COL_S + g * BN;
 #pragma unroll
-                for (int kk = 0; kk < BN / 16; ++kk) {    // 16 keys: 32 bytes along a row of P, 16 rows of V
-                    umma(d, pd + (unsigned long long)(((kk >> 2) * HALF_BYTES + (kk & 3) * 32) >> 4),
-                         vd + (unsigned long long)((kk * 2048) >> 4), IDESC_O, (i | kk) != 0);
+                    for (int kk = 0; kk < KD / 16; ++kk) {
+                        const unsigned long long off = (unsigned long long)(((kk >> 2) * HALF_BYTES + (kk & 3) * 32) >> 4);
+                        umma(d, q_desc0 + off, kd + off, IDESC_S, kk != 0);
+                    }
+                    if (!SHARED) umma_commit(&empty_k[s]);
+                    umma_commit(&s_full[g]);
                 }
-                umma_commit(SHARED ? &empty_k[s] : &empty_v[s]);
-                umma_commit(&o_done[g]);
+                __syncwarp();
             }
-            __syncwarp();
+        } else if (warp == 3) {
+            // ---- products, second kind: O_g += P_j V_j.  An issuing warp of its own: while one waits for a barrier the
+            // other keeps the tensor cores fed. --------------------------------------------------------------
+            constexpr unsigned IDESC_O = instr_desc(BM, VD, true);
+            constexpr int SLOT = SHARED ? K_BYTES : V_BYTES;
+            const unsigned long long p_desc0 = smem_desc(smem_u32(p_smem), 16, 1024);
+            const unsigned long long v_desc0 = smem_desc(smem_u32(v_slots), HALF_BYTES, 1024);
+            for (int j = 0; j < T; ++j) {
+                const int g = j & 1, i = j >> 1, s = j % SLOTS;
+                bool ok = SHARED || mbar_wait(&full_v[s], (j / SLOTS) & 1, abort, p.fault, 6);
+                if (!__all_sync(0xffffffffu, ok)) break;
+                if (!SHARED && (j == 0 || j == T - 1))
+                    zero_rows(v_slots + s * V_BYTES, V_BLOCKS, lo_first - (tile_begin + j * BN), hi - (tile_begin + j * BN), lane);
+                ok = mbar_wait(&p_full[g], i & 1, abort, p.fault, 6);
+                if (!__all_sync(0xffffffffu, ok)) break;
+                if (lane == 0) {
+                    fence_after();
+                    const unsigned long long vd = v_desc0 + (unsigned long long)((s * SLOT) >> 4);
+                    const unsigned long long pd = p_desc0 + (unsigned long long)((g * P_BYTES) >> 4);
+                    const unsigned d = tmem_base + COL_O + g * 128;
+#pragma unroll
+                    for (int kk = 0; kk < BN / 16; ++kk) {    // 16 keys: 32 bytes along a row of P, 16 rows of V
+                        umma(d, pd + (unsigned long long)(((kk >> 2) * HALF_BYTES + (kk & 3) * 32) >> 4),
+                             vd + (unsigned long long)((kk * 2048) >> 4), IDESC_O, (i | kk) != 0);
+                    }
+                    umma_commit(SHARED ? &empty_k[s] : &empty_v[s]);
+                    umma_commit(&o_done[g]);
+                }
+                __syncwarp();
+            }
         }
-    } else if (warp >= 2 && warp < 10) {
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;\n" ::);
         // ---- softmax: one thread per query row in each of the two groups ----------------------
-        const int g = warp >= 6 ? 1 : 0;                  // warps 2-5 and 6-9
+        const int g = warp >= 8 ? 1 : 0;                  // warps 4-7 and 8-11
         const int quarter = warp & 3;                     // the lanes of tensor memory this warp may touch
         const int r = quarter * 32 + lane;
         const bool row_ok = r < nrows && p.row_slot[row0 + r] >= 0;
@@ -256,6 +267,14 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         const bool warp_has_rows = __any_sync(0xffffffffu, row_ok);
         float m_used = -INFINITY, l_sum = 0.f;
         bool ok = true;
+        // before the exponentials of the group's tile i: the products of its tile before are done, and the other group's
+        // exponentials of the tile before in the row's order.  (Left to themselves the groups come to their exponentials
+        // together and share the units: each 2000 cycles for what takes one alone 1100.)
+        auto wait_turn = [&](int i) {
+            if (g == 0) return i == 0 || mbar_wait_both(&o_done[0], (i - 1) & 1, &turn[0], (i - 1) & 1, abort, p.fault, 6);
+            return i == 0 ? mbar_wait(&turn[1], 0, abort, p.fault, 6)
+                          : mbar_wait_both(&o_done[1], (i - 1) & 1, &turn[1], i & 1, abort, p.fault, 6);
+        };
         int i = 0;                                        // tiles of this group so far
         for (int j = g; j < T; j += 2, ++i) {
             if (!__all_sync(0xffffffffu, mbar_wait(&s_full[g], i & 1, abort, p.fault, 6))) { ok = false; break; }
@@ -268,61 +287,45 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                         *reinterpret_cast<uint4*>(pg_smem + r * 128 + (c >> 3) * HALF_BYTES + ((c & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
                     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 }
-                // it follows every phase of o_done all the same: a wait for the last one alone could return a phase early (the
-                // parity of the phase before the one before), and the merge below writes where P lies
-                if (i > 0 && !__all_sync(0xffffffffu, mbar_wait(&o_done[g], (i - 1) & 1, abort, p.fault, 6))) { ok = false; break; }
+                // it follows every phase of o_done and turn all the same: a wait for the last one alone could return a phase
+                // early (the parity of the phase before the one before), and the merge below writes where P lies
+                if (!__all_sync(0xffffffffu, wait_turn(i))) { ok = false; break; }
+                if (lane == 0) mbar_arrive(&turn[1 - g]);
                 fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&p_full[g]);
+                if (lane == 0) { mbar_arrive(&s_free[g]); mbar_arrive(&p_full[g]); }
                 continue;
             }
             const int kt = tile_begin + j * BN;
-            // Two passes over the row of S, 64 columns at a time (the row stays in tensor memory until
-            // this group hands P over): first the maximum, then the exponentials.
             const bool whole = kt + BN - 1 <= pos0 && kt >= lo_last;      // every row of the tile sees every key
-            const bool plain = whole && row_ok;
-            // the scores of half a tile, masked (`bound`: through the tanh).  With a bias: scaled to units of log2, by the first
-            // pass, which writes them back; without: the scale is left to the caller
-            auto load64 = [&](int half, float (&s)[64], bool bound, bool first) {
-                tmem_ld32_issue(tmem_base + lane_bits + col_s + half * 64, s);
-                tmem_ld32_issue(tmem_base + lane_bits + col_s + half * 64 + 32, s + 32);
-                tmem_ld_wait();
-                tmem_ld_arrived(s);
-                if (!BIAS && bound) {
+            float s[BN];
 #pragma unroll
-                    for (int e = 0; e < 64; ++e) s[e] = soft_capped(s[e], p.cap);
-                }
-                if (BIAS && first) {
-                    const float d0 = (float)(qpos - kt - half * 64);
+            for (int c = 0; c < BN / 32; ++c) tmem_ld32_issue(tmem_base + lane_bits + col_s + c * 32, s + c * 32);
+            tmem_ld_wait();
+            tmem_ld_arrived(s);
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[g]);
+            // with a bias: in units of log2 from here on; without, the scale is left to the exponentials
+            if (BIAS) {
+                const float d0 = (float)(qpos - kt);
 #pragma unroll
-                    for (int e = 0; e < 64; ++e)
-                        s[e] = fmaf(s[e], p.scale_log2, -b1 * fast_log2(fmaf(b2, d0 - (float)e, 1.f)));
-                }
-                if (!plain && (!BIAS || first)) {
+                for (int e = 0; e < BN; ++e) s[e] = fmaf(s[e], p.scale_log2, -b1 * fast_log2(fmaf(b2, d0 - (float)e, 1.f)));
+            } else if (p.cap.k != 0.f) {
 #pragma unroll
-                    for (int e = 0; e < 64; ++e) {
-                        const int key = kt + half * 64 + e;
-                        s[e] = (row_ok && key <= qpos && key >= lo_r) ? s[e] : -INFINITY;
-                    }
-                }
-                if (BIAS && first) {
-                    tmem_st32(tmem_base + lane_bits + col_s + half * 64, reinterpret_cast<const float(&)[32]>(s[0]));
-                    tmem_st32(tmem_base + lane_bits + col_s + half * 64 + 32, reinterpret_cast<const float(&)[32]>(s[32]));
-                }
-            };
-            // the row's maximum, without a bias of the raw scores (the scale is positive)
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                float s[64];
-                load64(half, s, false, true);
-#pragma unroll
-                for (int e = 0; e < 64; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], s[e]);
+                for (int e = 0; e < BN; ++e) s[e] = soft_capped(s[e], p.cap);
             }
-            // (the bound never falls: the maximum of the bounded scores is the bounded maximum)
-            const bool capped = !BIAS && p.cap.k != 0.f;
+            if (!(whole && row_ok)) {
+                // keys lo_r .. qpos, counted from the tile's first; a padding row sees none
+                const int from = row_ok ? lo_r - kt : 1 << 20, span = row_ok ? qpos - lo_r : 0;
+#pragma unroll
+                for (int e = 0; e < BN; ++e) s[e] = (unsigned)(e - from) <= (unsigned)span ? s[e] : -INFINITY;
+            }
+            // the row's maximum (the scale is positive)
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int e = 0; e < BN; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], s[e]);
             float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            if (capped && mx > -INFINITY) mx = soft_capped(mx, p.cap);
             if (!BIAS) mx *= p.scale_log2;
             // the reference is the row's maximum itself, so that the largest probability is 1 and not rounded.  (Raised only
             // when the maximum had left it far behind: 1 to 2 % more error of the outputs, 2 % less time.)
@@ -334,41 +337,43 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 l_sum *= alpha;
             }
             // the products of the group's tile before are done: O may be rescaled, P overwritten
-            if (i > 0 && !__all_sync(0xffffffffu, mbar_wait(&o_done[g], (i - 1) & 1, abort, p.fault, 6))) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, wait_turn(i))) { ok = false; break; }
             if (i > 0 && __any_sync(0xffffffffu, raise)) {
                 fence_after();
 #pragma unroll 1
-                for (int c = 0; c < VD / 32; ++c) {
-                    float o[32];
-                    tmem_ld32(tmem_base + lane_bits + col_o + c * 32, o);
+                for (int c = 0; c < VD / 64; ++c) {
+                    float o[2][32];
+                    const unsigned at = tmem_base + lane_bits + col_o + c * 64;
+                    tmem_ld32_issue(at, o[0]);
+                    tmem_ld32_issue(at + 32, o[1]);
+                    tmem_ld_wait();
+                    tmem_ld_arrived(o[0]);
+                    tmem_ld_arrived(o[1]);
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) o[e] *= alpha;
-                    tmem_st32(tmem_base + lane_bits + col_o + c * 32, o);
+                    for (int e = 0; e < 64; ++e) o[e >> 5][e & 31] *= alpha;
+                    tmem_st32(at, o[0]);
+                    tmem_st32(at + 32, o[1]);
                 }
                 fence_before();
             }
             const float neg_m = m_used == -INFINITY ? 0.f : -m_used;
             float ps4[4] = {0.f, 0.f, 0.f, 0.f};
             unsigned char* prow = pg_smem + r * 128;
-#pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                float s[64];
-                load64(half, s, capped, false);
+            const float sc = BIAS ? 1.f : p.scale_log2;
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {             // eight keys: one 16-byte chunk of the row of P
-                    unsigned pk[4];
+            for (int c = 0; c < BN / 8; ++c) {            // eight keys: one 16-byte chunk of the row of P
+                unsigned pk[4];
 #pragma unroll
-                    for (int e = 0; e < 8; e += 2) {
-                        const float sc = BIAS ? 1.f : p.scale_log2;
-                        const float a = fast_exp2(fmaf(s[c * 8 + e], sc, neg_m));             // 2^-inf = 0 for masked keys
-                        const float b = fast_exp2(fmaf(s[c * 8 + e + 1], sc, neg_m));
-                        __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-                        pk[e >> 1] = *reinterpret_cast<unsigned*>(&h);
-                        // the sum of what the product sees: a row that is nearly all one key's comes out as that key's value
-                        ps4[e >> 1] += __uint_as_float(pk[e >> 1] << 16) + __uint_as_float(pk[e >> 1] & 0xffff0000u);
-                    }
-                    *reinterpret_cast<uint4*>(prow + half * HALF_BYTES + ((c ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                for (int e = 0; e < 8; e += 2) {
+                    const float a = fast_exp2(fmaf(s[c * 8 + e], sc, neg_m));                 // 2^-inf = 0 for masked keys
+                    const float b = fast_exp2(fmaf(s[c * 8 + e + 1], sc, neg_m));
+                    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+                    pk[e >> 1] = *reinterpret_cast<unsigned*>(&h);
+                    // the sum of what the product sees: a row that is nearly all one key's comes out as that key's value
+                    ps4[e >> 1] += __uint_as_float(pk[e >> 1] << 16) + __uint_as_float(pk[e >> 1] & 0xffff0000u);
                 }
+                *reinterpret_cast<uint4*>(prow + (c >> 3) * HALF_BYTES + (((c & 7) ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                if (c == BN / 16 - 1 && lane == 0) mbar_arrive(&turn[1 - g]);
             }
             l_sum += (ps4[0] + ps4[1]) + (ps4[2] + ps4[3]);
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -376,7 +381,23 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_full[g]);
         }
-        // ---- merge the two groups' halves; each group stores half of the columns -------------
+        // ---- merge the two groups' halves, each group half of the columns, and store them through the ring of keys, which
+        // has no more copies or products to come once both groups' last products are done --------------------------
+        typedef StagedRows<VD> Rows;
+        float* stage = reinterpret_cast<float*>(k_slots);
+        const int first = Rows::row(warp - 4, lane, 0), col = Rows::col(lane);
+        bf16* dst = p.out + (size_t)(row0 + first) * p.out_stride + head * VD + col;
+        const bool gated = p.gate != nullptr && !p.gate_per_head;
+        uint2 gates[4];                                   // of the next four steps, on their way
+        auto fetch_gates = [&](int i0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int at = first + (i0 + i) * Rows::ROWS;
+                gates[i] = make_uint2(0u, 0u);
+                if (gated && at < nrows) gates[i] = *reinterpret_cast<const uint2*>(p.gate + (size_t)(row0 + at) * p.ldg + (size_t)head * VD + col);
+            }
+        };
+        fetch_gates(0);
         if (i > 0 && ok) ok = __all_sync(0xffffffffu, mbar_wait(&o_done[g], (i - 1) & 1, abort, p.fault, 6));
         // the group's P buffer is free now: it carries the row's maximum and sum to the other group
         reinterpret_cast<float*>(pg_smem)[r] = m_used;
@@ -396,7 +417,7 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             float inv = l > 0.f ? 1.f / l : 0.f;
             if (p.gate != nullptr && p.gate_per_head && r < nrows) inv /= 1.f + __expf(-__bfloat162float(p.gate[(size_t)(row0 + r) * p.ldg + head]));
             constexpr int COLS = VD / 2;                  // this group's share of the columns
-#pragma unroll 1
+#pragma unroll
             for (int c = 0; c < COLS / 32; ++c) {
                 const int col = g * COLS + c * 32;
                 float o0[32], o1[32];
@@ -405,25 +426,34 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 tmem_ld_wait();
                 tmem_ld_arrived(o0);
                 if (T >= 2) tmem_ld_arrived(o1);
-                if (r < nrows) {                          // padding rows inside the tile get zeros
+                // padding rows inside the tile get zeros
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) o0[e] = row_ok ? (o0[e] * w0 + (T >= 2 ? o1[e] * w1 : 0.f)) * inv : 0.f;
-                    if (p.gate != nullptr && !p.gate_per_head) {
-                        const bf16* gr = p.gate + (size_t)(row0 + r) * p.ldg + (size_t)head * VD + col;
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            float gv[8];
-                            Vec16<bf16>::load(gr + q * 8, gv);
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) o0[q * 8 + e] /= 1.f + __expf(-gv[e]);
-                        }
-                    }
-                    bf16* dst = p.out + (size_t)(row0 + r) * p.out_stride + head * VD + col;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) store8(dst + q * 8, o0 + q * 8);
-                }
+                for (int e = 0; e < 32; ++e) o0[e] = row_ok ? (o0[e] * w0 + (T >= 2 ? o1[e] * w1 : 0.f)) * inv : 0.f;
+                stage_put<VD>(stage, r, col, o0);
             }
             fence_before();
+        }
+        asm volatile("bar.sync 1, 256;\n" ::: "memory");
+        if (!*abort) {
+#pragma unroll 1                                          // (code that runs once takes longer to fetch than to run)
+            for (int i0 = 0; i0 < Rows::STEPS; i0 += 4, dst += (size_t)4 * Rows::ROWS * p.out_stride) {
+                uint2 now[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) now[i] = gates[i];
+                if (i0 + 4 < Rows::STEPS) fetch_gates(i0 + 4);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int at = first + (i0 + i) * Rows::ROWS;
+                    float4 v = Rows::get(stage, at, col);
+                    if (gated) {
+                        v.x = divided(v.x, 1.f + __expf(-__uint_as_float(now[i].x << 16)));
+                        v.y = divided(v.y, 1.f + __expf(-__uint_as_float(now[i].x & 0xffff0000u)));
+                        v.z = divided(v.z, 1.f + __expf(-__uint_as_float(now[i].y << 16)));
+                        v.w = divided(v.w, 1.f + __expf(-__uint_as_float(now[i].y & 0xffff0000u)));
+                    }
+                    if (at < nrows) store4(dst + (size_t)i * Rows::ROWS * p.out_stride, v);
+                }
+            }
         }
     }
 
