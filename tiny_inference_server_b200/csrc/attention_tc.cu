@@ -7,7 +7,7 @@
 //            swizzle), warps 0 and 12 the keys of every key tile, 2 and 13 the values, each pair into a ring of
 //            shared-memory slots of its own (keys are needed early, values late: with rings of
 //            their own the key loads run ahead), one box of 64 elements x page_size rows per page
-//            and half of the head, a lane a box (a warp orders one in about 75 cycles).  The cache
+//            and half of the head, a lane a box (a lane knows its page).  The cache
 //            keeps rows XOR-swizzled by the position, so the boxes, copied as the bytes lie, are
 //            at once the swizzled operand tiles;
 //   warps 1 and 3   issue the products (one lane each; warp 1 also owns the tensor memory):
@@ -183,17 +183,18 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
             }
         } else if (warp == 1) {
             // ---- products, first kind: S_j = Q K_j^T into score buffer j & 1 ----------------------------
-            if (lane == 0) {
-                constexpr unsigned IDESC_S = instr_desc(BM, BN, false);
-                const unsigned long long q_desc0 = smem_desc(smem_u32(q_smem), 16, 1024);
-                const unsigned long long k_desc0 = smem_desc(smem_u32(k_slots), 16, 1024);
-                bool ok = mbar_wait(&q_full, 0, abort, p.fault, 6);
-                for (int j = 0; j < T && ok; ++j) {
-                    const int g = j & 1, i = j >> 1, s = j % SLOTS;
-                    // the group has the scores of its tile before in registers
-                    if (!(i > 0 ? mbar_wait_both(&s_free[g], (i - 1) & 1, &full_k[s], (j / SLOTS) & 1, abort, p.fault, 6)
-                                : mbar_wait(&full_k[s], (j / SLOTS) & 1, abort, p.fault, 6))) break;
-                    fence_after();
+            constexpr unsigned IDESC_S = instr_desc(BM, BN, false);
+            const unsigned long long q_desc0 = smem_desc(smem_u32(q_smem), 16, 1024);
+            const unsigned long long k_desc0 = smem_desc(smem_u32(k_slots), 16, 1024);
+            bool ok = mbar_wait(&q_full, 0, abort, p.fault, 6);
+            for (int j = 0; j < T; ++j) {
+                const int g = j & 1, i = j >> 1, s = j % SLOTS;
+                // the group has the scores of its tile before in registers
+                ok = ok && (i > 0 ? mbar_wait_both(&s_free[g], (i - 1) & 1, &full_k[s], (j / SLOTS) & 1, abort, p.fault, 6)
+                                  : mbar_wait(&full_k[s], (j / SLOTS) & 1, abort, p.fault, 6));
+                if (!__all_sync(0xffffffffu, ok)) break;
+                fence_after();
+                if (elect_one()) {
                     // descriptors differ from the ring's first one only in the start address (units of 16 bytes)
                     const unsigned long long kd = k_desc0 + (unsigned long long)((s * SLOT_BYTES) >> 4);
                     const unsigned d = tmem_base + COL_S + g * BN;
@@ -205,18 +206,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     umma_commit(&empty_k[s]);
                     umma_commit(&s_full[g]);
                 }
+                __syncwarp();
             }
         } else if (warp == 3) {
             // ---- products, second kind: O_g += P_j V_j.  An issuing thread of its own: while one thread
             // waits for a barrier the other keeps the tensor cores fed. ------------------------------------
-            if (lane == 0) {
-                constexpr unsigned IDESC_O = instr_desc(BM, HD, true);
-                const unsigned long long p_desc0 = smem_desc(smem_u32(p_smem), 16, 1024);
-                const unsigned long long v_desc0 = smem_desc(smem_u32(v_slots), HALF_BYTES, 1024);
-                for (int j = 0; j < T; ++j) {
-                    const int g = j & 1, i = j >> 1, s = j % SLOTS;
-                    if (!mbar_wait_both(&p_full[g], i & 1, &full_v[s], (j / SLOTS) & 1, abort, p.fault, 6)) break;
-                    fence_after();
+            constexpr unsigned IDESC_O = instr_desc(BM, HD, true);
+            const unsigned long long p_desc0 = smem_desc(smem_u32(p_smem), 16, 1024);
+            const unsigned long long v_desc0 = smem_desc(smem_u32(v_slots), HALF_BYTES, 1024);
+            for (int j = 0; j < T; ++j) {
+                const int g = j & 1, i = j >> 1, s = j % SLOTS;
+                if (!__all_sync(0xffffffffu, mbar_wait_both(&p_full[g], i & 1, &full_v[s], (j / SLOTS) & 1, abort, p.fault, 6))) break;
+                fence_after();
+                if (elect_one()) {
                     const unsigned long long vd = v_desc0 + (unsigned long long)((s * SLOT_BYTES) >> 4);
                     const unsigned long long pd = p_desc0 + (unsigned long long)((g * P_BYTES) >> 4);
                     const unsigned d = tmem_base + COL_O + g * 128;
@@ -228,6 +230,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant_
                     umma_commit(&empty_v[s]);
                     umma_commit(&o_done[g]);
                 }
+                __syncwarp();
             }
         }
     } else {

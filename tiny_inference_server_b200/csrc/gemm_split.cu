@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_split_kernel(const SplitParams p)
         }
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 48;\n" ::);
-        if (warp == (CONV + SUMS) / 32 && lane == 0) {
+        if (warp == (CONV + SUMS) / 32) {
             constexpr unsigned IDESC = instr_desc(BM, BN, true);
             const unsigned long long x0 = smem_desc64(smem_u32(stages)), w0 = smem_desc(smem_u32(stages) + 3 * A_PLANE, W_BOX, 1024);
             int it = 0;
@@ -237,21 +237,24 @@ __global__ void __launch_bounds__(NTH, 1) gemm_split_kernel(const SplitParams p)
                 place(unit, m0, n0, first, last);
                 for (int step = first; step < last; ++step, ++it) {
                     const int s = it % STAGES, b = it & 1;
-                    if (!mbar_wait(&acc_empty[b], ((it >> 1) & 1) ^ 1, abort, p.fault, 5) ||
-                        !mbar_wait(&full[s], (it / STAGES) & 1, abort, p.fault, 5)) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait_both(&acc_empty[b], ((it >> 1) & 1) ^ 1, &full[s], (it / STAGES) & 1, abort,
+                                                                p.fault, 5))) { ok = false; break; }
                     fence_after();
-                    // descriptors differ from the first stage's in the start address only (units of 16 bytes)
-                    const unsigned long long xs = x0 + (unsigned)(s * STAGE_BYTES >> 4), ws = w0 + (unsigned)(s * STAGE_BYTES >> 4);
-                    const unsigned d = tmem_base + b * ACC_COLS;
-                    auto product = [&](int i, int j, bool begun) {      // planes i of x, j of W
+                    if (elect_one()) {
+                        // descriptors differ from the first stage's in the start address only (units of 16 bytes)
+                        const unsigned long long xs = x0 + (unsigned)(s * STAGE_BYTES >> 4), ws = w0 + (unsigned)(s * STAGE_BYTES >> 4);
+                        const unsigned d = tmem_base + b * ACC_COLS;
+                        auto product = [&](int i, int j, bool begun) {      // planes i of x, j of W
 #pragma unroll
-                        for (int kk = 0; kk < BK / 16; ++kk)
-                            umma(d, xs + ((i * A_PLANE + kk * 32) >> 4), ws + ((j * W_PLANE + kk * 2048) >> 4), IDESC, begun || kk > 0);
-                    };
-                    product(0, 2, false); product(2, 0, true); product(1, 1, true);
-                    product(0, 1, true); product(1, 0, true); product(0, 0, true);
-                    umma_commit(&empty[s]);
-                    umma_commit(&acc_full[b]);
+                            for (int kk = 0; kk < BK / 16; ++kk)
+                                umma(d, xs + ((i * A_PLANE + kk * 32) >> 4), ws + ((j * W_PLANE + kk * 2048) >> 4), IDESC, begun || kk > 0);
+                        };
+                        product(0, 2, false); product(2, 0, true); product(1, 1, true);
+                        product(0, 1, true); product(1, 0, true); product(0, 0, true);
+                        umma_commit(&empty[s]);
+                        umma_commit(&acc_full[b]);
+                    }
+                    __syncwarp();
                 }
             }
         }

@@ -13,6 +13,15 @@ namespace tc {
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
+// One lane of a whole warp.  Behind this (and not behind a lane's number) the compiler knows that a single thread orders copies
+// and products, and takes their operands from uniform registers; behind `lane == 0` each copy or product cost about 70 cycles
+// and a look at a barrier 200.
+__device__ __forceinline__ bool elect_one() {
+    unsigned one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
+
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count));
 }
@@ -23,38 +32,34 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar, i
     asm volatile("{\n.reg .b64 st;\nmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}\n"
                  ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ bool mbar_done(unsigned long long* bar, unsigned parity) {
+    unsigned done;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return done != 0;
+}
 // Bounded wait for the phase with this parity.  Returns false when it ran out (the fault word
 // is set to `code`) or when another role gave up before (`abort`); the caller then leaves its loop.
+// The first look is apart from the loop: a look takes 40 cycles, as a turn of the loop
+// 150 to 220, for a phase that was complete already, in every hand-over of every role.
 constexpr int MBAR_SPINS = 1 << 20;
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, volatile int* abort, int* fault,
-                                          int code) {
-    unsigned done = 0;
+__device__ __forceinline__ bool mbar_wait_on(unsigned long long* bar, unsigned parity, volatile int* abort, int* fault, int code) {
     for (int spin = 0; spin < MBAR_SPINS; ++spin) {
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-        if (done) return true;
+        if (mbar_done(bar, parity)) return true;
         if ((spin & 1023) == 1023 && *abort) return false;
     }
     *abort = 1;
     atomicExch(fault, code);
     return false;
 }
-
-// The same for two phases at once: the looks at the two barriers overlap (one that is complete already still takes some
-// hundred cycles).
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, volatile int* abort, int* fault, int code) {
+    return mbar_done(bar, parity) || mbar_wait_on(bar, parity, abort, fault, code);
+}
+// The same for two phases, the first looks at the two barriers side by side.
 __device__ __forceinline__ bool mbar_wait_both(unsigned long long* a, unsigned parity_a, unsigned long long* b, unsigned parity_b,
                                                volatile int* abort, int* fault, int code) {
-    unsigned done_a = 0, done_b = 0;
-    for (int spin = 0; spin < MBAR_SPINS; ++spin) {
-        asm volatile("{\n.reg .pred p, q;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%2], %3;\n"
-                     "mbarrier.try_wait.parity.shared::cta.b64 q, [%4], %5;\nselp.u32 %0, 1, 0, p;\nselp.u32 %1, 1, 0, q;\n}\n"
-                     : "=r"(done_a), "=r"(done_b) : "r"(smem_u32(a)), "r"(parity_a), "r"(smem_u32(b)), "r"(parity_b) : "memory");
-        if (done_a & done_b) return true;
-        if ((spin & 1023) == 1023 && *abort) return false;
-    }
-    *abort = 1;
-    atomicExch(fault, code);
-    return false;
+    const bool done_a = mbar_done(a, parity_a), done_b = mbar_done(b, parity_b);
+    return (done_a || mbar_wait_on(a, parity_a, abort, fault, code)) && (done_b || mbar_wait_on(b, parity_b, abort, fault, code));
 }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
@@ -185,13 +190,6 @@ template <int W> struct StagedRows {
         return *reinterpret_cast<const float4*>(stage + r * W + ((col >> 2) ^ (r & 7)) * 4);
     }
 };
-// a / b to two last places over the whole range (results below 2^-126 included), without the branch of the rounded division,
-// which keeps neighbouring divisions from running side by side: a row's gates took 700 cycles, with this 100
-__device__ __forceinline__ float divided(float a, float b) {
-    float q;
-    asm("div.full.f32 %0, %1, %2;\n" : "=f"(q) : "f"(a), "f"(b));
-    return q;
-}
 __device__ __forceinline__ void store4(bf16* p, const float4& v) {
     __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
     *reinterpret_cast<uint2*>(p) = *reinterpret_cast<uint2*>(h);

@@ -204,8 +204,8 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 if (!__all_sync(0xffffffffu, ok)) break;
                 if (SHARED && (j == 0 || j == T - 1))
                     zero_rows(k_slots + s * K_BYTES, V_BLOCKS, lo_first - (tile_begin + j * BN), hi - (tile_begin + j * BN), lane);
-                if (lane == 0) {
-                    fence_after();
+                fence_after();
+                if (elect_one()) {
                     // descriptors differ from the ring's first one only in the start address (units of 16 bytes)
                     const unsigned long long kd = k_desc0 + (unsigned long long)((s * K_BYTES) >> 4);
                     const unsigned d = tmem_base + COL_S + g * BN;
@@ -234,8 +234,8 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     zero_rows(v_slots + s * V_BYTES, V_BLOCKS, lo_first - (tile_begin + j * BN), hi - (tile_begin + j * BN), lane);
                 ok = mbar_wait(&p_full[g], i & 1, abort, p.fault, 6);
                 if (!__all_sync(0xffffffffu, ok)) break;
-                if (lane == 0) {
-                    fence_after();
+                fence_after();
+                if (elect_one()) {
                     const unsigned long long vd = v_desc0 + (unsigned long long)((s * SLOT) >> 4);
                     const unsigned long long pd = p_desc0 + (unsigned long long)((g * P_BYTES) >> 4);
                     const unsigned d = tmem_base + COL_O + g * 128;
