@@ -398,15 +398,16 @@ def gemm_skinny(a, w: torch.Tensor, out: Optional[torch.Tensor] = None, swiglu: 
     return result if sink is not None else out
 
 
-#: The tcgen05 kernel of this library (csrc/gemm_tc.cu) against the library product, measured on a
-#: B200 at the 0.9B model's shapes (replayed from CUDA graphs, weights rotated through more than L2):
-#: gate/up with the SwiGLU gating in its epilogue it wins from about 3000 rows (4096 rows: 78 against
-#: 94 us for the library product plus the gating kernel; 2048 rows: 52 against 49 us); plain products
-#: it loses (2048 x 1536 x 4096: 28 against 19.5 us — one CTA per tile moves more bytes from L2 per
-#: multiply-add than the library's two-CTA tiles).  So by default it takes gate/up products of at
-#: least TC_MIN_ROWS rows and no plain ones; TIS_TC_MIN_ROWS / TIS_TC_PLAIN_MIN_ROWS in the
-#: environment override the two limits (0 = never).
-TC_MIN_ROWS = int(os.environ.get("TIS_TC_MIN_ROWS", "3072"))
+#: The tcgen05 kernel of this library (csrc/gemm_tc.cu) against the library product, measured on a B200 (replayed from CUDA
+#: graphs, weights rotated through more than L2).  Gate/up with the gating in its epilogue, us library product and gating kernel /
+#: own, at 65, 128, 200, 300, 400, 512, 640, 1024, 2048 rows: K 1536, hidden 4096 11.2 / 9.4, 10.6 / 8.8, 12.1 / 10.3, 13.4 / 14.3,
+#: 14.9 / 14.4, 16.3 / 14.5, 21.8 / 20.3, 27.5 / 22.2, 48.5 / 37.8; K 3072, hidden 8192 21.2 / 19.4, 24.1 / 19.9, 25.7 / 24.3,
+#: 30.5 / 38.1, 36.5 / 39.1, 42.7 / 40.3, 60.7 / 55.7, 84 / 75, 180 / 129; K 4096, hidden 14336 40.9 / 38.9, 49.5 / 39.2, 55 / 53,
+#: 65 / 91, 85 / 94, 102 / 95, 150 / 122, 206 / 167, 345 / 308; K 1536, hidden 1024 7.3 / 7.4 .. 16.1 / 13.9.  It loses where the
+#: last tile of 256 rows is mostly empty: up to 256 rows (one tile) and from four fifths of the tiles' rows on it takes them.
+#: Plain products it loses (2048 x 1536 x 2304: 12.1 / 16.2, 2048 x 3072 x 12352 102 / 109): by default it takes none.
+#: TIS_TC_MIN_ROWS / TIS_TC_PLAIN_MIN_ROWS in the environment override the two limits (0 = never).
+TC_MIN_ROWS = int(os.environ.get("TIS_TC_MIN_ROWS", "65"))
 TC_PLAIN_MIN_ROWS = int(os.environ.get("TIS_TC_PLAIN_MIN_ROWS", "0"))
 _tc_fault = None
 
@@ -426,11 +427,16 @@ def _tc_ok(a: torch.Tensor, w: torch.Tensor, min_rows: int) -> bool:
             and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def _tc_tiles_full(n: int) -> bool:
+    """Whether ``n`` rows fill four fifths of the tiles of 256 rows they take, or one tile has them all."""
+    return n <= 256 or 5 * n >= 4 * 256 * -(-n // 256)
+
+
 def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, swiglu: bool = False,
-            form: GateForm = SILU) -> torch.Tensor:
+            form: GateForm = SILU, shape: int = -1) -> torch.Tensor:
     """``a (n, K) @ w (K, N)`` in bfloat16 on the tcgen05 tensor cores (TMA-fed, accumulator in
     tensor memory); with ``swiglu`` the columns of ``w`` are [32 gate | 32 up] blocks and the
-    result is (n, N/2)."""
+    result is (n, N/2).  ``shape``: the tile (0 .. 5; -1: the kernel's choice)."""
     lib = library()
     n, k = a.shape
     cols = w.shape[1]
@@ -438,7 +444,7 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None
         out = torch.empty((n, cols // 2 if swiglu else cols), dtype=a.dtype, device=a.device)
     calls["gemm_tc"] += 1
     _check(lib.tis_gemm_tc(_p(a), a.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), n, cols, k,
-                           EPI_SWIGLU if swiglu else EPI_STORE, form, _p(tc_fault()), _stream()), lib)
+                           EPI_SWIGLU if swiglu else EPI_STORE, form, shape, _p(tc_fault()), _stream()), lib)
     return out
 
 
@@ -589,7 +595,7 @@ def gemm_swiglu(a, w_gu: torch.Tensor, hidden: int, block: int, form: GateForm =
         return gemm_swap(scaled if scaled is not None else a, w_gu, swiglu=True, form=form)
     if scaled is not None:
         a = scaled.dense()
-    if block == 32 and _tc_ok(a, w_gu, TC_MIN_ROWS) and w_gu.shape[1] % 64 == 0:
+    if block == 32 and _tc_ok(a, w_gu, TC_MIN_ROWS) and _tc_tiles_full(a.shape[0]) and w_gu.shape[1] % 64 == 0:
         return gemm_tc(a, w_gu, swiglu=True, form=form)
     gu = gemm(a, w_gu)
     out = torch.empty((a.shape[0], hidden), dtype=a.dtype, device=a.device)
