@@ -93,9 +93,12 @@ causal_conv_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ w
         if (k < hist) st[(size_t)k * C + c] = h[k];
 }
 
-// The same for channel counts and row strides that are multiples of a 16-byte vector: a thread owns a (row, vector
-// of channels) and the taps are a template parameter, so that weights and history stay in registers.
-template <typename T, int TAPS>
+// The same for channel counts and row strides that are multiples of a 16-byte vector: a thread owns a vector of channels and
+// ROWS neighbouring rows, and the taps are a template parameter, so that weights and inputs stay in registers: the weights of
+// eight channels are as many bytes as eight rows of inputs.  Rows whose inputs all lie in this step and in one request are
+// taken together, their loads on their way at once; the others one by one.  Measured at 2048 rows of 2304 channels, four taps,
+// us with a row a thread / so: 12.4 / 6.0, with silu (and its rounded division) 16.2 / 8.2.
+template <typename T, int TAPS, int ROWS>
 __global__ void __launch_bounds__(128)
 causal_conv_vec_kernel(const T* __restrict__ x, int ldx, const float* __restrict__ w, float* __restrict__ state,
                        size_t state_stride, T* __restrict__ out, int ldo, const int* __restrict__ row_slot,
@@ -104,13 +107,16 @@ causal_conv_vec_kernel(const T* __restrict__ x, int ldx, const float* __restrict
     constexpr int N = Vec16<T>::N, HIST = TAPS - 1;
     pdl_launch_dependents();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * N;
-    const int r = blockIdx.y;
+    const int r0 = blockIdx.y * ROWS;
     if (c >= C) return;
-    const int slot = row_slot[r];
-    if (slot < 0) return;
-    int back = 0;
-    while (back < HIST && r - back - 1 >= 0 && row_slot[r - back - 1] == slot) ++back;
-    if (back > 0 && back < HIST) return;              // computed by the thread of the request's first row
+    // whether rows r0 - HIST .. r0 + ROWS - 1 are one request's
+    bool together = ROWS > 1 && r0 >= HIST && r0 + ROWS <= n;
+    if (together) {
+        const int slot = row_slot[r0];
+        together = slot >= 0;
+#pragma unroll
+        for (int k = -HIST; k < ROWS; ++k) together = together && row_slot[r0 + k] == slot;
+    }
     float wt[N][TAPS];
 #pragma unroll
     for (int j = 0; j < TAPS; ++j)
@@ -128,61 +134,88 @@ causal_conv_vec_kernel(const T* __restrict__ x, int ldx, const float* __restrict
         for (int e = 0; e < N; ++e) {
             acc[e] += b0[e];
             if (residual) acc[e] += cur[e];
-            if (act_silu) acc[e] = acc[e] / (1.f + expf(-acc[e]));
+            if (act_silu) acc[e] = sizeof(T) == 2 ? divided(acc[e], 1.f + expf(-acc[e])) : acc[e] / (1.f + expf(-acc[e]));
         }
         Vec16<T>::store(out + row * ldo + c, acc);
     };
-    if (back == HIST) {
-        float acc[N], cur[N];
+    if (together) {
+        float in[ROWS + HIST][N];
 #pragma unroll
-        for (int e = 0; e < N; ++e) acc[e] = 0.f;
+        for (int k = 0; k < ROWS + HIST; ++k) Vec16<T>::load(x + (size_t)(r0 - HIST + k) * ldx + c, in[k]);
+        // (the request's state is seen to by whoever has its first row)
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) {
-            Vec16<T>::load(x + (size_t)(r - HIST + j) * ldx + c, cur);
+        for (int i = 0; i < ROWS; ++i) {
+            float acc[N];
 #pragma unroll
-            for (int e = 0; e < N; ++e) acc[e] = fmaf(wt[e][j], cur[e], acc[e]);
+            for (int e = 0; e < N; ++e) acc[e] = 0.f;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j)
+#pragma unroll
+                for (int e = 0; e < N; ++e) acc[e] = fmaf(wt[e][j], in[i + j][e], acc[e]);
+            finish(acc, in[i + HIST], (size_t)(r0 + i));
         }
-        finish(acc, cur, (size_t)r);
         return;
     }
-    const int rows = row_last[r] - r + 1;
-    float* st = state + (size_t)slot * state_stride;
-    float h[HIST > 0 ? HIST : 1][N];
+#pragma unroll 1
+    for (int r = r0; r < min(r0 + ROWS, n); ++r) {
+        const int slot = row_slot[r];
+        if (slot < 0) continue;
+        int back = 0;
+        while (back < HIST && r - back - 1 >= 0 && row_slot[r - back - 1] == slot) ++back;
+        if (back > 0 && back < HIST) continue;              // computed by the thread of the request's first row
+        if (back == HIST) {
+            float acc[N], cur[N];
 #pragma unroll
-    for (int k = 0; k < HIST; ++k)
+            for (int e = 0; e < N; ++e) acc[e] = 0.f;
 #pragma unroll
-        for (int e = 0; e < N; ++e) h[k][e] = st[(size_t)k * C + c + e];
-    const int mine = rows < HIST ? rows : HIST;
-    for (int i = 0; i < mine; ++i) {
-        float acc[N], cur[N];
-        Vec16<T>::load(x + (size_t)(r + i) * ldx + c, cur);
+            for (int j = 0; j < TAPS; ++j) {
+                Vec16<T>::load(x + (size_t)(r - HIST + j) * ldx + c, cur);
 #pragma unroll
-        for (int e = 0; e < N; ++e) {
-            float a = 0.f;                              // the taps in the order of the other path: bit-equal results
+                for (int e = 0; e < N; ++e) acc[e] = fmaf(wt[e][j], cur[e], acc[e]);
+            }
+            finish(acc, cur, (size_t)r);
+            continue;
+        }
+        const int rows = row_last[r] - r + 1;
+        float* st = state + (size_t)slot * state_stride;
+        float h[HIST > 0 ? HIST : 1][N];
 #pragma unroll
-            for (int k = 0; k < HIST; ++k) a = fmaf(wt[e][k], h[k][e], a);
-            acc[e] = fmaf(wt[e][HIST], cur[e], a);
+        for (int k = 0; k < HIST; ++k)
+#pragma unroll
+            for (int e = 0; e < N; ++e) h[k][e] = st[(size_t)k * C + c + e];
+        const int mine = rows < HIST ? rows : HIST;
+        for (int i = 0; i < mine; ++i) {
+            float acc[N], cur[N];
+            Vec16<T>::load(x + (size_t)(r + i) * ldx + c, cur);
+#pragma unroll
+            for (int e = 0; e < N; ++e) {
+                float a = 0.f;                              // the taps in the order of the other paths: bit-equal results
+#pragma unroll
+                for (int k = 0; k < HIST; ++k) a = fmaf(wt[e][k], h[k][e], a);
+                acc[e] = fmaf(wt[e][HIST], cur[e], a);
+            }
+#pragma unroll
+            for (int k = 0; k + 1 < HIST; ++k)
+#pragma unroll
+                for (int e = 0; e < N; ++e) h[k][e] = h[k + 1][e];
+            if (HIST > 0) {
+#pragma unroll
+                for (int e = 0; e < N; ++e) h[HIST - 1][e] = cur[e];
+            }
+            finish(acc, cur, (size_t)(r + i));
+        }
+        if (rows > HIST) {
+#pragma unroll
+            for (int k = 0; k < HIST; ++k) Vec16<T>::load(x + (size_t)(r + rows - HIST + k) * ldx + c, h[k]);
         }
 #pragma unroll
-        for (int k = 0; k + 1 < HIST; ++k)
+        for (int k = 0; k < HIST; ++k)
 #pragma unroll
-            for (int e = 0; e < N; ++e) h[k][e] = h[k + 1][e];
-        if (HIST > 0) {
-#pragma unroll
-            for (int e = 0; e < N; ++e) h[HIST - 1][e] = cur[e];
-        }
-        finish(acc, cur, (size_t)(r + i));
+            for (int e = 0; e < N; ++e) st[(size_t)k * C + c + e] = h[k][e];
     }
-    if (rows > HIST) {
-#pragma unroll
-        for (int k = 0; k < HIST; ++k) Vec16<T>::load(x + (size_t)(r + rows - HIST + k) * ldx + c, h[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < HIST; ++k)
-#pragma unroll
-        for (int e = 0; e < N; ++e) st[(size_t)k * C + c + e] = h[k][e];
 }
 
+constexpr int CONV_MIN_ROWS = 640;      // from which a thread takes neighbouring rows (us a row a thread / four: 300 rows 4.1 / 4.9, 512 4.6 / 4.6, 768 5.7 / 4.8)
 template <typename T, int TAPS>
 static void launch_causal_conv_vec(const T* x, int ldx, const float* w, float* state, size_t state_stride, T* out, int ldo,
                                    const int* row_slot, const int* row_last, int n, int C, int residual, int act_silu,
@@ -190,8 +223,13 @@ static void launch_causal_conv_vec(const T* x, int ldx, const float* w, float* s
     constexpr int N = Vec16<T>::N;
     const int vecs = C / N;
     const int threads = vecs >= 128 ? 128 : (vecs + 31) / 32 * 32;
-    tis_launch(causal_conv_vec_kernel<T, TAPS>, dim3((vecs + threads - 1) / threads, n), dim3(threads), 0, stream, x, ldx, w,
-               state, state_stride, out, ldo, row_slot, row_last, n, C, residual, act_silu, bias);
+    constexpr int ROWS = 4;
+    if (n >= CONV_MIN_ROWS)
+        tis_launch(causal_conv_vec_kernel<T, TAPS, ROWS>, dim3((vecs + threads - 1) / threads, (n + ROWS - 1) / ROWS), dim3(threads), 0,
+                   stream, x, ldx, w, state, state_stride, out, ldo, row_slot, row_last, n, C, residual, act_silu, bias);
+    else
+        tis_launch(causal_conv_vec_kernel<T, TAPS, 1>, dim3((vecs + threads - 1) / threads, n), dim3(threads), 0, stream, x, ldx, w,
+                   state, state_stride, out, ldo, row_slot, row_last, n, C, residual, act_silu, bias);
 }
 
 TIS_API int tis_causal_conv(int dtype, const void* x, int ldx, const float* w, float* state, size_t state_stride,
@@ -364,6 +402,67 @@ norm_mix_store_vec_kernel(T* __restrict__ qkv, int ld, int nq, int nk, int nv, c
     }
 }
 
+// The same in one pass, a vector of queries, keys or values a thread: rows of at most 1024 vectors in all.  The two sums of squares
+// are added up together, with one barrier.  Bound by the chain from the row's slot to its page and the loads' latency; with more
+// rows than a wave of CTAs holds (288 threads each here) the kernel above is the faster one.  Rows of 1536 + 384 + 384, us above /
+// here: 300 rows 4.9 / 3.7, 512 6.8 / 4.0, 768 7.2 / 6.0, 1024 7.1 / 8.3, 2048 11.6 / 11.9.
+constexpr int NORM_MIX_ONCE_ROWS = 900;
+template <typename T>
+__global__ void __launch_bounds__(1024)
+norm_mix_store_once_kernel(T* __restrict__ qkv, int ld, int nq, int nk, int nv, const float* __restrict__ wq,
+                           const float* __restrict__ wk, float eps, const T* __restrict__ v_other, int ld_other,
+                           const float* __restrict__ lambda, T* __restrict__ k_pages, size_t k_page_stride,
+                           size_t k_head_stride, T* __restrict__ v_pages, size_t v_page_stride, size_t v_head_stride,
+                           int kv_heads, int page_size, int num_pages, const int* __restrict__ block_table, int bt_stride,
+                           const int* __restrict__ positions, const int* __restrict__ row_slot, int* __restrict__ fault) {
+    constexpr int N = Vec16<T>::N;
+    __shared__ float red[2][32];
+    pdl_launch_dependents();
+    const int r = blockIdx.x;
+    const int slot = row_slot[r], pos = positions[r];
+    if (slot < 0) return;
+    const int page = block_table[(size_t)slot * bt_stride + pos / page_size];
+    const int i = threadIdx.x * N, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const bool is_q = i < nq, is_k = !is_q && i < nq + nk, is_v = i >= nq + nk && i < nq + nk + nv;
+    const float* w = is_q ? wq : is_k ? wk : nullptr;       // (of this thread's elements)
+    float x[N], y[N], f[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) { x[e] = 0.f; f[e] = w != nullptr ? w[(is_q ? i : i - nq) + e] : 1.f; }
+    const float lam = is_v && v_other != nullptr && lambda != nullptr ? lambda[0] : 0.f;
+    pdl_wait();
+    T* row = qkv + (size_t)r * ld;
+    if (is_q || is_k || is_v) Vec16<T>::load(row + i, x);
+    if (is_v && v_other != nullptr) Vec16<T>::load(v_other + (size_t)r * ld_other + i - nq - nk, y);
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < N; ++e) ss = fmaf(x[e], x[e], ss);
+    const float sq = warp_sum(is_q ? ss : 0.f), sk = warp_sum(is_k ? ss : 0.f);
+    if (lane == 0) { red[0][warp] = sq; red[1][warp] = sk; }
+    __syncthreads();
+    const float q_sum = warp_sum(lane < warps ? red[0][lane] : 0.f), k_sum = warp_sum(lane < warps ? red[1][lane] : 0.f);
+    const float factor = w == nullptr ? 1.f : is_q ? rsqrtf(q_sum / (float)nq + eps) : rsqrtf(k_sum / (float)nk + eps);
+    const bool bad = page < 0 || page >= num_pages;
+    if (bad && threadIdx.x == 0) atomicExch(fault, 3);
+    const int in_page = pos % page_size;
+    if (is_q && wq != nullptr) {
+#pragma unroll
+        for (int e = 0; e < N; ++e) x[e] = x[e] * factor * f[e];
+        Vec16<T>::store(row + i, x);
+    } else if (is_k && !bad) {
+        const int k_dim = nk / kv_heads, head = (i - nq) / k_dim, e0 = i - nq - head * k_dim;
+#pragma unroll
+        for (int e = 0; e < N; ++e) x[e] = x[e] * factor * f[e];
+        Vec16<T>::store(k_pages + (size_t)page * k_page_stride + (size_t)head * k_head_stride + (size_t)in_page * k_dim + e0, x);
+    } else if (is_v && !bad) {
+        const int v_dim = nv / kv_heads, head = (i - nq - nk) / v_dim, e0 = i - nq - nk - head * v_dim;
+        if (v_other != nullptr) {
+#pragma unroll
+            for (int e = 0; e < N; ++e) x[e] = (1.f - lam) * x[e] + lam * y[e];
+        }
+        Vec16<T>::store(v_pages + (size_t)page * v_page_stride + (size_t)head * v_head_stride + (size_t)in_page * v_dim + e0, x);
+    }
+}
+
 TIS_API int tis_norm_mix_store(int dtype, void* qkv, int ld, int nq, int nk, int nv, const float* wq, const float* wk,
                                float eps, const void* v_other, int ld_other, const float* lambda, void* k_pages,
                                size_t k_page_stride, size_t k_head_stride, void* v_pages, size_t v_page_stride,
@@ -381,6 +480,15 @@ TIS_API int tis_norm_mix_store(int dtype, void* qkv, int ld, int nq, int nk, int
     if (nq % per == 0 && kd % per == 0 && vd % per == 0 && ld % per == 0 && (v_other == nullptr || ld_other % per == 0) &&
         k_page_stride % per == 0 && k_head_stride % per == 0 && v_page_stride % per == 0 && v_head_stride % per == 0 &&
         ((uintptr_t)qkv | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)v_other) % 16 == 0) {
+        const int vecs = (nq + nk + nv) / per;
+        if (vecs <= 1024 && n < NORM_MIX_ONCE_ROWS) {
+            TIS_DISPATCH_DTYPE(dtype, T,
+                tis_launch(norm_mix_store_once_kernel<T>, dim3(n), dim3((vecs + 31) / 32 * 32), 0, stream, (T*)qkv, ld, nq, nk, nv, wq, wk,
+                           eps, (const T*)v_other, ld_other, lambda, (T*)k_pages, k_page_stride, k_head_stride, (T*)v_pages,
+                           v_page_stride, v_head_stride, kv_heads, page_size, num_pages, block_table, bt_stride, positions, row_slot,
+                           fault));
+            return tis_check_launch("norm_mix_store");
+        }
         TIS_DISPATCH_DTYPE(dtype, T,
             tis_launch(norm_mix_store_vec_kernel<T>, dim3(n), dim3(256), 0, stream, (T*)qkv, ld, nq, nk, nv, wq, wk, eps,
                        (const T*)v_other, ld_other, lambda, (T*)k_pages, k_page_stride, k_head_stride, (T*)v_pages,
