@@ -77,13 +77,15 @@ def _p(t: Optional[torch.Tensor]):
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+#: (torch.cuda.current_device() without its check that CUDA is initialised: ``library()`` has seen to that)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
 
 
 def _stream():
     """torch's current CUDA stream as a raw handle (the direct getter is 40 times cheaper than going
     through a Stream object, and this runs once per launch)."""
     if _raw_stream is not None:
-        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
+        return ctypes.c_void_p(_raw_stream(_current_device()))
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
@@ -507,22 +509,24 @@ def _library_gemm(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor],
     global _blas_state, launches
     if not LIBRARY_GEMM_DIRECT or _blas_state is False:
         return None
-    if (a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or a.stride(1) != 1 or w.stride(1) != 1
-            or a.stride(0) < a.shape[1] or w.stride(0) < w.shape[1]):
+    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
+        return None
+    (n, k), cols = a.shape, w.shape[1]
+    (lda, step_a), (ldw, step_w) = a.stride(), w.stride()
+    if step_a != 1 or step_w != 1 or lda < k or ldw < cols:
         return None
     lib = library()
     if not _blas_workspace(lib, a.device):
         return None
-    n, k = a.shape
-    cols = w.shape[1]
     want = torch.float32 if f32_out else torch.bfloat16
     if out is None:
-        out = torch.empty((n, cols), dtype=want, device=a.device)
+        out, ldo = a.new_empty((n, cols), dtype=want), cols
     elif out.dtype != want or out.stride(1) != 1 or out.stride(0) < cols:
         return None
+    else:
+        ldo = out.stride(0)
     calls["gemm_library"] += 1
-    status = lib.tis_gemm_library(_p(a), a.stride(0), _p(w), w.stride(0), _p(out), out.stride(0), n, cols, k,
-                                  int(f32_out), _stream())
+    status = lib.tis_gemm_library(_p(a), lda, _p(w), ldw, _p(out), ldo, n, cols, k, int(f32_out), _stream())
     if status != 0:
         raise KernelError(lib.tis_last_error().decode())
     return out
@@ -554,18 +558,19 @@ def gemm(a, w: torch.Tensor, out: Optional[torch.Tensor] = None, sink: Optional[
         a = scaled.rows
     if a.dtype == torch.float32 and torch.backends.cuda.matmul.allow_tf32:
         raise KernelError("float32 products must not run in TF32: torch.backends.cuda.matmul.allow_tf32 is set")
-    streams = _stream_pays(a.shape[0], a.shape[1], w.shape[1]) and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-    if (_skinny_ok(a, w) and (streams or _ring_tiles(w.shape[1], a.shape[1]) <= RING_MAX_TILES)) or \
-            (_skinny_ok(a, w, STREAM_MAX_ROWS) and streams):
-        if sink is not None and not _sink_fits(sink, a.shape[0], w.shape[1], out):
-            sink = None
-        return gemm_skinny(scaled if scaled is not None else a, w, out, sink=sink)
-    if _skinny_ok(a, w) and a.shape[1] >= 2 * w.shape[1] and _swap_ok(a, w, out):
-        # a long share of K per CTA and a tall matrix: the tcgen05 kernel with swapped operands
-        if sink is not None and not (_sink_fits(sink, a.shape[0], w.shape[1], out) and sink.values.stride(0) % 4 == 0
-                                     and sink.values.data_ptr() % 16 == 0 and sink.weight.data_ptr() % 16 == 0):
-            sink = None
-        return gemm_swap(scaled if scaled is not None else a, w, out, sink=sink)
+    if a.shape[0] <= max(SKINNY_MAX_ROWS, STREAM_MAX_ROWS):                 # (many rows are not asked about: the host's time counts)
+        streams = _stream_pays(a.shape[0], a.shape[1], w.shape[1]) and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+        if (_skinny_ok(a, w) and (streams or _ring_tiles(w.shape[1], a.shape[1]) <= RING_MAX_TILES)) or \
+                (_skinny_ok(a, w, STREAM_MAX_ROWS) and streams):
+            if sink is not None and not _sink_fits(sink, a.shape[0], w.shape[1], out):
+                sink = None
+            return gemm_skinny(scaled if scaled is not None else a, w, out, sink=sink)
+        if _skinny_ok(a, w) and a.shape[1] >= 2 * w.shape[1] and _swap_ok(a, w, out):
+            # a long share of K per CTA and a tall matrix: the tcgen05 kernel with swapped operands
+            if sink is not None and not (_sink_fits(sink, a.shape[0], w.shape[1], out) and sink.values.stride(0) % 4 == 0
+                                         and sink.values.data_ptr() % 16 == 0 and sink.weight.data_ptr() % 16 == 0):
+                sink = None
+            return gemm_swap(scaled if scaled is not None else a, w, out, sink=sink)
     if scaled is not None:
         a = scaled.dense()
     if _tc_ok(a, w, TC_PLAIN_MIN_ROWS) and (out is None or (out.stride(1) == 1 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0)):
@@ -993,11 +998,12 @@ def causal_conv(x: torch.Tensor, weight: torch.Tensor, state: torch.Tensor, out:
 def _page_strides(pages: torch.Tensor, width: int, free_rows: bool = False):
     """(page stride, head stride) of a view [pages, kv_heads, page_size, width] whose rows are dense; with
     ``free_rows`` also the stride from row to row, which may then exceed the width (a slice of wider rows)."""
-    if pages.stride(3) != 1 or (pages.stride(2) != width if not free_rows else pages.stride(2) < width):
+    page, head, row, step = pages.stride()                  # (one call: the host's time counts)
+    if step != 1 or (row != width if not free_rows else row < width):
         raise KernelError("cache pages: the rows of a kv head must lie one after the other")
     if free_rows:
-        return ctypes.c_size_t(pages.stride(0)), ctypes.c_size_t(pages.stride(1)), int(pages.stride(2))
-    return ctypes.c_size_t(pages.stride(0)), ctypes.c_size_t(pages.stride(1))
+        return ctypes.c_size_t(page), ctypes.c_size_t(head), int(row)
+    return ctypes.c_size_t(page), ctypes.c_size_t(head)
 
 
 def norm_mix_store(qkv: torch.Tensor, nq: int, nk: int, nv: int, q_weight: Optional[torch.Tensor],
@@ -1053,12 +1059,13 @@ WINDOW_ATTENTION_CTAS = 2 * 148
 def window_attention_mma_usable(q: torch.Tensor, gate, out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
                                 gate_per_head: bool = False) -> bool:
     k_dim, v_dim = k_pages.shape[3], v_pages.shape[3]
-    return (WINDOW_ATTENTION_MMA and v_pages.stride(2) % 8 == 0 and q.dtype == torch.bfloat16 and k_dim % 16 == 0 and v_dim % 16 == 0
-            and 16 <= k_dim <= 256 and 16 <= v_dim <= 256 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0
-            and out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0
+    k_page, k_head, _, _ = k_pages.stride()
+    v_page, v_head, v_row, _ = v_pages.stride()
+    return (WINDOW_ATTENTION_MMA and (v_row | k_page | k_head | v_page | v_head) % 8 == 0 and q.dtype == torch.bfloat16
+            and k_dim % 16 == 0 and v_dim % 16 == 0 and 16 <= k_dim <= 256 and 16 <= v_dim <= 256
+            and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0
             and (gate is None or gate_per_head or (gate.stride(0) % 2 == 0 and gate.data_ptr() % 4 == 0))
-            and all(s % 8 == 0 for s in (k_pages.stride(0), k_pages.stride(1), v_pages.stride(0), v_pages.stride(1)))
-            and k_pages.data_ptr() % 16 == 0 and v_pages.data_ptr() % 16 == 0)
+            and (k_pages.data_ptr() | v_pages.data_ptr()) % 16 == 0)
 
 
 #: long portions of prompts run on the tcgen05 kernel where it takes their widths and pages;
