@@ -141,18 +141,36 @@ __device__ __forceinline__ float gated_unit(float g, float u, const GateForm& f)
     u = fminf(fmaxf(u, -f.limit), f.limit);
     return g / (1.f + expf(-g * fmaf(f.c3 * g, g, f.c1))) * (u + f.shift);
 }
-// a / b to two last places over the whole range (results below 2^-126 included), without the branch of the rounded division,
-// which keeps neighbouring divisions from running side by side: sixteen rows of an attention tile's gates took 11000 cycles, now 4000
-__device__ __forceinline__ float divided(float a, float b) {
-    float q;
-    asm("div.full.f32 %0, %1, %2;\n" : "=f"(q) : "f"(a), "f"(b));
-    return q;
+// a / b for b >= 1 (or NaN), rounded to nearest as `/` rounds it, without the operator's branch, which keeps neighbouring divisions from
+// running side by side (and takes zeros, as rows beyond the last one give them, the long way): gate/up of 200 rows, 1536 x
+// 8192, with the gating in its epilogue 19.4 us by the operator, 11.1 so; of 2048 rows 42.6 and 40.8; a convolution of 2048 x 2304
+// with silu 11.0 and 9.7.  (div.full.f32, two last places off, 10.4, 39.3 and 8.0.)
+// The method is Markstein's (IBM Journal of Research and Development 34, 1990): y is the reciprocal to half a last place, v = a y
+// is off by a last place at most, the remainder a - b v comes out of a multiply-add exactly, and v + (a - b v) y rounds as a / b
+// does, because y's error moves that sum by less than a quotient of two 24-bit numbers stays away from where rounding turns.
+// Large b and small a are scaled by powers of two first, so that nothing on the way is subnormal; results below
+// 2^-126 are rounded once more when the scale is taken back.  Infinities, NaN and zeros come out as from the operator.
+__device__ __forceinline__ float quotient(float a, float b) {
+    const bool large = b >= 0x1p64f, small = fabsf(a) < 0x1p-30f;
+    const float d = b * (large ? 0x1p-64f : 1.f), n = a * (small ? 0x1p64f : 1.f);
+    float y0;
+    asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(y0) : "f"(d));
+    const float y = fmaf(fmaf(-d, y0, 1.f), y0, y0), v = n * y;
+    const float q = copysignf(fmaf(fmaf(-d, v, n), y, v), n);               // (a zero's sign)
+    return (fabsf(v) < INFINITY ? q : n * y0) * ((large ? 0x1p-64f : 1.f) * (small ? 0x1p-64f : 1.f));
 }
-// the same with the faster exponential and division, for results that are rounded to bfloat16
+// the same with the faster exponential, for results that are rounded to bfloat16
 __device__ __forceinline__ float gated_unit_fast(float g, float u, const GateForm& f) {
     g = fminf(g, f.limit);
     u = fminf(fmaxf(u, -f.limit), f.limit);
-    return divided(g, 1.f + __expf(-g * fmaf(f.c3 * g, g, f.c1))) * (u + f.shift);
+    return g / (1.f + __expf(-g * fmaf(f.c3 * g, g, f.c1))) * (u + f.shift);
+}
+// and the same numbers in an epilogue, where a few warps have many units each and wait for every one of them.  (With many warps an SM the
+// operator's fewer instructions count: the gating kernel at 300 rows of 4096 takes 4.3 us with it and 5.9 with the other.)
+__device__ __forceinline__ float gated_unit_epilogue(float g, float u, const GateForm& f) {
+    g = fminf(g, f.limit);
+    u = fminf(fmaxf(u, -f.limit), f.limit);
+    return quotient(g, 1.f + __expf(-g * fmaf(f.c3 * g, g, f.c1))) * (u + f.shift);
 }
 
 // Block-wide sum / max for blockDim.x a multiple of 32 (<= 1024); `red` holds 33 floats.

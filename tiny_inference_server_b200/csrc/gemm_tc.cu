@@ -228,7 +228,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& map_a, const CUt
                     tmem_ld_arrived(g);
                     tmem_ld_arrived(u);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) g[i] = gated_unit_fast(g[i], u[i], p.gate);
+                    for (int i = 0; i < 32; ++i) g[i] = gated_unit_epilogue(g[i], u[i], p.gate);
                     if (row < p.M && n0 + c * 64 < p.N) {
                         bf16* o = p.out + (size_t)row * p.ldo + (n0 >> 1) + c * 32;
 #pragma unroll

@@ -152,7 +152,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                 if (GATED) {
                     tmem_ld_arrived(u);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) g[i] = gated_unit_fast(g[i] * iw, u[i] * iw, p.gate);
+                    for (int i = 0; i < 32; ++i) g[i] = gated_unit_epilogue(g[i] * iw, u[i] * iw, p.gate);
                 } else if (p.act >= 0) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) g[i] = tile_act(g[i] * iw, p.act);

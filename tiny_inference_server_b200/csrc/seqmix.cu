@@ -134,7 +134,11 @@ causal_conv_vec_kernel(const T* __restrict__ x, int ldx, const float* __restrict
         for (int e = 0; e < N; ++e) {
             acc[e] += b0[e];
             if (residual) acc[e] += cur[e];
-            if (act_silu) acc[e] = sizeof(T) == 2 ? divided(acc[e], 1.f + expf(-acc[e])) : acc[e] / (1.f + expf(-acc[e]));
+            if (act_silu) {
+                // (a row a thread: many warps, which the operator's fewer instructions suit; 300 rows 4.8 us, by quotient 5.4)
+                const float den = 1.f + expf(-acc[e]);
+                acc[e] = ROWS > 1 ? quotient(acc[e], den) : acc[e] / den;
+            }
         }
         Vec16<T>::store(out + row * ldo + c, acc);
     };

@@ -446,10 +446,10 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     const int at = first + (i0 + i) * Rows::ROWS;
                     float4 v = Rows::get(stage, at, col);
                     if (gated) {
-                        v.x = divided(v.x, 1.f + __expf(-__uint_as_float(now[i].x << 16)));
-                        v.y = divided(v.y, 1.f + __expf(-__uint_as_float(now[i].x & 0xffff0000u)));
-                        v.z = divided(v.z, 1.f + __expf(-__uint_as_float(now[i].y << 16)));
-                        v.w = divided(v.w, 1.f + __expf(-__uint_as_float(now[i].y & 0xffff0000u)));
+                        v.x = quotient(v.x, 1.f + __expf(-__uint_as_float(now[i].x << 16)));
+                        v.y = quotient(v.y, 1.f + __expf(-__uint_as_float(now[i].x & 0xffff0000u)));
+                        v.z = quotient(v.z, 1.f + __expf(-__uint_as_float(now[i].y << 16)));
+                        v.w = quotient(v.w, 1.f + __expf(-__uint_as_float(now[i].y & 0xffff0000u)));
                     }
                     if (at < nrows) store4(dst + (size_t)i * Rows::ROWS * p.out_stride, v);
                 }
