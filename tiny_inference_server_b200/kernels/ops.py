@@ -464,7 +464,16 @@ SPLIT_MIN_WORK = 350_000_000
 
 
 def _split_ok(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor]) -> bool:
-    return (a.dtype == torch.float32 and w.dtype == torch.float32 and 0 < SPLIT_MIN_ROWS <= a.shape[0]
+    """What the kernel takes.  Everything else stays with torch.mm: operands that do not fit together, of which it says so, a
+    result on top of an operand, and operands that want a gradient."""
+    if a.dtype != torch.float32 or w.dtype != torch.float32 or a.dim() != 2 or w.dim() != 2 or not a.is_cuda or a.device != w.device:
+        return False
+    if a.shape[1] != w.shape[0] or (torch.is_grad_enabled() and (a.requires_grad or w.requires_grad)):
+        return False
+    if out is not None and (out.device != a.device or out.shape != (a.shape[0], w.shape[1])
+                            or out.untyped_storage().data_ptr() in (a.untyped_storage().data_ptr(), w.untyped_storage().data_ptr())):
+        return False
+    return (0 < SPLIT_MIN_ROWS <= a.shape[0]
             and a.shape[0] * w.shape[1] >= SPLIT_MIN_RESULT and a.shape[0] * w.shape[1] * a.shape[1] >= SPLIT_MIN_WORK
             and a.stride(1) == 1 and w.stride(1) == 1 and a.shape[1] % 4 == 0 and w.shape[1] % 4 == 0
             and a.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and a.stride(0) >= a.shape[1] > 0 and w.stride(0) >= w.shape[1]
