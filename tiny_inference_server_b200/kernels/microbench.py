@@ -5,6 +5,8 @@
     python -m tiny_inference_server_b200.kernels.microbench rowwise --tokens 2048
     python -m tiny_inference_server_b200.kernels.microbench gemm --rows 8        (weight-streaming kernel)
     python -m tiny_inference_server_b200.kernels.microbench gemm --rows 4096     (tcgen05 kernel, above 64 rows)
+    python -m tiny_inference_server_b200.kernels.microbench gemm-float32         (32-bit products on the tensor cores
+        beside the library's, and with numbers that have to be computed again)
     python -m tiny_inference_server_b200.kernels.microbench prefill --tokens 2048 --layers 4
     python -m tiny_inference_server_b200.kernels.microbench sampling --rows 8 --vocab 49152
     python -m tiny_inference_server_b200.kernels.microbench seqmix --window 1024   (windowed attention, short
@@ -1122,6 +1124,34 @@ def gemm(args):
               f"{2 * n * K * N / a / 1e6:6.1f} TFLOP/s)   library {b:7.2f} us{extra}")
 
 
+def gemm_float32(args):
+    """The library's product and the one of split operands (csrc/gemm_split.cu) at both sides of the limits between them
+    (``SPLIT_MIN_ROWS`` and what follows it in ops.py), then the latter with marked elements."""
+    def inputs(M, K, N):
+        weights = [torch.randn(K, N, device="cuda") * 0.02 for _ in range(max(2, (150 << 20) // (K * N * 4) + 1))]
+        return torch.randn(M, K, device="cuda"), weights
+
+    def times(M, K, N, *fns):
+        a, ws = inputs(M, K, N)
+        return [_graph_time(lambda i: fn(a, ws[i % len(ws)]), 16) for fn in fns]
+
+    for M, K, N in ((16, 1536, 49152), (64, 1536, 6144), (65, 1536, 6144), (65, 4096, 6144), (128, 1536, 1536), (128, 4096, 1536), (200, 1536, 1536),
+                    (200, 4096, 1536), (100, 1536, 6144), (128, 1536, 4608), (256, 1536, 1536), (300, 1536, 1536), (777, 1536, 1536), (777, 4096, 1536), (777, 1536, 6144),
+                    (2048, 1536, 6144), (2048, 3072, 12352), (333, 512, 1344), (400, 512, 1344), (512, 512, 1344), (1024, 128, 1536), (1536, 128, 1536), (2048, 128, 1536)):
+        library, split = times(M, K, N, torch.mm, ops.gemm_split)
+        print(f"float32 {M:5d} x {K:5d} x {N:6d} (result {M * N:9d}, work {M * N * K:.1e}): library {library:8.2f} us   split {split:8.2f} us "
+              f"({2 * M * K * N / split / 1e6:6.1f} TFLOP/s)")
+    for M, K, N in ((777, 1536, 1536), (777, 1536, 6144)):
+        a, ws = inputs(M, K, N)
+        one, row = a.clone(), [w.clone() for w in ws]
+        one[5, 3] = float("nan")
+        for w in row:
+            w[2] = float("inf")
+        t = [_graph_time(fn, 16) for fn in (lambda i: torch.mm(a, ws[i % len(ws)]), lambda i: ops.gemm_split(a, ws[i % len(ws)]),
+                                            lambda i: ops.gemm_split(one, ws[i % len(ws)]), lambda i: ops.gemm_split(a, row[i % len(ws)]))]
+        print(f"float32 {M:5d} x {K:5d} x {N:6d}: library {t[0]:8.2f} us   split {t[1]:8.2f}   a NaN in x {t[2]:8.2f}   a row of infinities in W {t[3]:8.2f}")
+
+
 def prefill(args):
     """One step of ``--tokens`` prompt tokens through ``--layers`` layers of the model."""
     from ..config import EngineConfig
@@ -1241,7 +1271,7 @@ def timeline(args):
 
 def main(argv=None):
     ap = argparse.ArgumentParser(prog="microbench", description=__doc__.split("\n\n")[0])
-    ap.add_argument("what", choices=["attention", "attention-prefill", "rowwise", "gemm", "prefill", "sampling", "timeline",
+    ap.add_argument("what", choices=["attention", "attention-prefill", "rowwise", "gemm", "gemm-float32", "prefill", "sampling", "timeline",
                                      "seqmix", "latent-linear-routed", "differential-latent-forget", "gated-space-tied", "normed-shared-clamped", "scan-mix-chunked", "all"])
     ap.add_argument("--rank", type=int, default=128, help="latent-linear-routed: compressed elements a token")
     ap.add_argument("--rot", type=int, default=64, help="latent-linear-routed: rotated elements a token")
@@ -1283,6 +1313,8 @@ def main(argv=None):
         for n in ([args.rows] if args.what == "gemm" else [1, 8, 16]):
             args.rows = n
             gemm(args)
+    if args.what in ("gemm-float32", "all"):
+        gemm_float32(args)
     if args.what in ("prefill", "all"):
         prefill(args)
     if args.what in ("sampling", "all"):

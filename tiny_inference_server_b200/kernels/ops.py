@@ -452,12 +452,13 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None
 
 #: float32 products of at least SPLIT_MIN_ROWS rows and enough work go to the tcgen05 kernel of split operands
 #: (csrc/gemm_split.cu) instead of the library's product on the CUDA cores.  A tile's time is K / 32 steps of 1.2 us (half of
-#: them where two CTAs share one) whatever its rows and columns are, so a small result does not pay: measured on a B200, us
-#: library / split, at M x N of 1.0e5 (128 x 1536 x K) 43 / 46 at K 1536, 82 / 97 at 4096; 3.1e5 (200 x 1536) 47 / 44, 111 / 95;
-#: 4.0e5 (65 x 6144) 49 / 46; 1.2e6 (777 x 1536) 111 / 46, 277 / 95; 4.8e6 (777 x 6144) 301 / 137; 1.3e7 (2048 x 6144) 660 / 261.
-#: With a short K the launch counts: 333 x 512 x 1344 (2.3e8) 21 / 26, 512 x 512 x 1344 (3.5e8) 29 / 26, 1024 x 128 x 1536
-#: (2.0e8) 19 / 21, 2048 x 128 x 1536 (4.0e8) 31 / 21.  Up to 64 rows the library streams the weights faster (16 x 1536 x
-#: 49152: 121 / 150).  TIS_SPLIT_MIN_ROWS overrides (0: never).
+#: them where two CTAs share one) whatever its rows and columns are, so a small result does not pay: measured on a B200
+#: (microbench gemm-float32), us library / split, at M x N of 2.0e5 (128 x 1536) 38 / 43 at K 1536, 75 / 93 at 4096; 3.1e5 (200 x
+#: 1536) 40.5 / 41.7, 101 / 91; 4.0e5 (65 x 6144) 43.4 / 41.7, 109 / 95; 4.6e5 (300 x 1536) 41.2 / 42.0; 6.1e5 (100 x 6144) 64 / 42;
+#: 1.2e6 (777 x 1536) 105 / 42, 271 / 89; 4.8e6 (777 x 6144) 295 / 131; 1.3e7 (2048 x 6144) 652 / 247.  With a short K the
+#: launch counts: 400 x 512 x 1344 (2.8e8) 17.8 / 20.0, 512 x 512 x 1344 (3.5e8) 27 / 20.5, 1536 x 128 x 1536 (3.0e8) 15.8 / 15.3,
+#: 2048 x 128 x 1536 (4.0e8) 25 / 15.  Up to 64 rows the library streams the weights faster (16 x 1536 x 49152: 109 / 137).
+#: TIS_SPLIT_MIN_ROWS overrides (0: never).
 SPLIT_MIN_ROWS = int(os.environ.get("TIS_SPLIT_MIN_ROWS", "65"))
 SPLIT_MIN_RESULT = 300_000
 SPLIT_MIN_WORK = 350_000_000
