@@ -92,3 +92,19 @@ def test_norms_in_one_pass(dtype, nq, G, kd, vd, norms, mix):
     live = slot >= 0
     torch.testing.assert_close(q[live][:, :nq].double(), want[live], rtol=1e-5 if dtype == torch.float32 else 2.0 ** -7, atol=1e-5)
     assert torch.equal(q[~live], qkv[~live])
+
+
+# the first row on a 16-byte boundary, and four, eight and twelve bytes behind one; rows of whole vectors and others
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+@pytest.mark.parametrize("d", [8, 72, 1536, 12, 7])
+def test_embeddings_into_a_view(dtype, shift, d):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(d)
+    table = torch.randn(50, d, generator=g, device="cuda").to(dtype)
+    tokens = torch.randint(0, 50, (13,), generator=g, device="cuda").to(torch.int32)
+    flat = torch.full((13 * d + 8,), 7.0, device="cuda")
+    out = flat[shift:shift + 13 * d].view(13, d)
+    ops.embed_rows(table, tokens, out, 0.75)
+    assert torch.equal(out, table[tokens.long()].float() * 0.75)
+    assert bool((flat[:shift] == 7.0).all()) and bool((flat[shift + 13 * d:] == 7.0).all())

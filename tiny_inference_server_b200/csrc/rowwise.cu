@@ -19,11 +19,11 @@ __global__ void embed_rows_kernel(const T* __restrict__ table, const int* __rest
     const T* src = table + (size_t)tokens[r] * d;
     float* dst = out + (size_t)r * d;
     constexpr int N = Vec16<T>::N;
-    if (d % N == 0) {
+    if (d % N == 0 && (uintptr_t)out % 16 == 0) {
         for (int i = threadIdx.x * N; i < d; i += blockDim.x * N) {
             float v[N];
             Vec16<T>::load(src + i, v);
-            // (d is a multiple of four here: the rows of the stream lie on 16-byte boundaries.  Stored number by number, a
+            // (d is a multiple of four: all rows lie on 16-byte boundaries if the first one does.  Stored number by number, a
             // lane's eight beside the next lane's: 15.5 us for 2048 rows of 1536, 5.2 so)
 #pragma unroll
             for (int j = 0; j < N; j += 4)
