@@ -108,3 +108,31 @@ def test_embeddings_into_a_view(dtype, shift, d):
     ops.embed_rows(table, tokens, out, 0.75)
     assert torch.equal(out, table[tokens.long()].float() * 0.75)
     assert bool((flat[:shift] == 7.0).all()) and bool((flat[shift + 13 * d:] == 7.0).all())
+
+
+# both sides of the limits: by rows (narrow rows), by threads (wide ones); 1024 vectors a row, and more than one pass takes
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq,G,kd,vd,counts", [(40, 1, 8, 8, (899, 900)), (3072, 8, 128, 128, (272, 274, 546, 547)), (3072, 8, 64, 64, (341, 342, 683, 684)),
+                                               (6144, 8, 128, 128, (341, 342))])
+def test_norms_at_the_limits_of_one_pass(dtype, nq, G, kd, vd, counts):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(nq)
+    nk, nv, page = G * kd, G * vd, 16
+    for n in counts:
+        pages = -(-n // page)
+        slot, pos = torch.zeros(n, dtype=torch.int32, device="cuda"), torch.arange(n, dtype=torch.int32, device="cuda")
+        table = torch.randperm(pages, generator=torch.Generator().manual_seed(1)).to(torch.int32).cuda()[None]
+        qkv = torch.randn(n, nq + nk + nv, generator=g, device="cuda").to(dtype)
+        wq, wk = torch.randn(nq, generator=g, device="cuda"), torch.randn(nk, generator=g, device="cuda")
+        k_pages, v_pages = (torch.zeros(pages, G, page, m, dtype=dtype, device="cuda") for m in (kd, vd))
+        fault, got = torch.zeros(4, dtype=torch.int32, device="cuda"), qkv.clone()
+        ops.norm_mix_store(got, nq, nk, nv, wq, wk, 1e-6, None, None, k_pages, v_pages, table, pos, slot, page, fault)
+        assert int(fault[0]) == 0
+        q, k, v = qkv.double().split([nq, nk, nv], 1)
+        # a sum of squares in 32 bits, three products, then the result's own rounding
+        tol = dict(rtol=1e-5, atol=1e-6) if dtype == torch.float32 else dict(rtol=2.0 ** -7, atol=1e-6)
+        torch.testing.assert_close(got[:, :nq].double(), q / torch.sqrt((q * q).mean(-1, keepdim=True) + 1e-6) * wq.double(), **tol)
+        keys = k_pages[table[0].long()].transpose(1, 2).reshape(pages * page, nk)[:n]
+        values = v_pages[table[0].long()].transpose(1, 2).reshape(pages * page, nv)[:n]
+        torch.testing.assert_close(keys.double(), k / torch.sqrt((k * k).mean(-1, keepdim=True) + 1e-6) * wk.double(), **tol)
+        assert torch.equal(values, v.to(dtype))

@@ -407,10 +407,13 @@ norm_mix_store_vec_kernel(T* __restrict__ qkv, int ld, int nq, int nk, int nv, c
 }
 
 // The same in one pass, a vector of queries, keys or values a thread: rows of at most 1024 vectors in all.  The two sums of squares
-// are added up together, with one barrier.  Bound by the chain from the row's slot to its page and the loads' latency; with more
-// rows than a wave of CTAs holds (288 threads each here) the kernel above is the faster one.  Rows of 1536 + 384 + 384, us above /
-// here: 300 rows 4.9 / 3.7, 512 6.8 / 4.0, 768 7.2 / 6.0, 1024 7.1 / 8.3, 2048 11.6 / 11.9.
-constexpr int NORM_MIX_ONCE_ROWS = 900;
+// are added up together, with one barrier.  Bound by the chain from the row's slot to its page and the loads' latency; with much more
+// than a wave of CTAs (148 x 2048 threads) the kernel above is the faster one, and a row's threads are as many as its vectors.
+// us above / here, bfloat16, rows of 1536 + 384 + 384 (288 threads): 300 rows 5.1 / 3.5, 700 7.1 / 6.0, 900 7.2 / 6.1, 1100 7.0 / 6.8;
+// 2048 + 512 + 512 (384): 700 7.9 / 5.8, 900 7.9 / 7.4, 1100 7.8 / 8.3; 3072 + 1024 + 1024 (640): 500 9.7 / 9.1, 600 10.0 / 11.1, 900
+// 10.1 / 15.4; 4096 + 1024 + 1024 (768): 400 8.4 / 7.8, 600 11.2 / 12.2; 6144 + 1024 + 1024 (1024): 300 9.4 / 9.0, 600 13.8 / 14.7.
+// float32, 1536 + 384 + 384 (576): 600 6.7 / 5.3, 900 6.8 / 7.2; 2048 + 512 + 512 (768): 400 5.7 / 4.9, 900 7.5 / 9.6.
+constexpr int NORM_MIX_ONCE_ROWS = 900, NORM_MIX_ONCE_THREADS = 350000;
 template <typename T>
 __global__ void __launch_bounds__(1024)
 norm_mix_store_once_kernel(T* __restrict__ qkv, int ld, int nq, int nk, int nv, const float* __restrict__ wq,
@@ -484,10 +487,10 @@ TIS_API int tis_norm_mix_store(int dtype, void* qkv, int ld, int nq, int nk, int
     if (nq % per == 0 && kd % per == 0 && vd % per == 0 && ld % per == 0 && (v_other == nullptr || ld_other % per == 0) &&
         k_page_stride % per == 0 && k_head_stride % per == 0 && v_page_stride % per == 0 && v_head_stride % per == 0 &&
         ((uintptr_t)qkv | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)v_other) % 16 == 0) {
-        const int vecs = (nq + nk + nv) / per;
-        if (vecs <= 1024 && n < NORM_MIX_ONCE_ROWS) {
+        const int vecs = (nq + nk + nv) / per, threads = (vecs + 31) / 32 * 32;
+        if (threads <= 1024 && n < NORM_MIX_ONCE_ROWS && n * threads < NORM_MIX_ONCE_THREADS) {
             TIS_DISPATCH_DTYPE(dtype, T,
-                tis_launch(norm_mix_store_once_kernel<T>, dim3(n), dim3((vecs + 31) / 32 * 32), 0, stream, (T*)qkv, ld, nq, nk, nv, wq, wk,
+                tis_launch(norm_mix_store_once_kernel<T>, dim3(n), dim3(threads), 0, stream, (T*)qkv, ld, nq, nk, nv, wq, wk,
                            eps, (const T*)v_other, ld_other, lambda, (T*)k_pages, k_page_stride, k_head_stride, (T*)v_pages,
                            v_page_stride, v_head_stride, kv_heads, page_size, num_pages, block_table, bt_stride, positions, row_slot,
                            fault));
