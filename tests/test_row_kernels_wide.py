@@ -23,15 +23,16 @@ def _rows(lengths, device="cuda"):
 
 
 # one request; portions that begin and end inside a thread's four rows, shorter than the taps, single rows and padding between; a
-# number of rows that is no multiple of four
+# number of rows that is no multiple of four; few channels (a row a thread) and so many that a thread takes four
+@pytest.mark.parametrize("C", [72, 1808])
 @pytest.mark.parametrize("lengths", [[777], [1, 2, 3, 700, 1, 1, 5, 64], [640, -3, 9, 1, -1, 2, 130], [1] * 660])
 @pytest.mark.parametrize("taps", [2, 3, 4, 5])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("silu", [False, True])
-def test_convolution_of_many_rows(lengths, taps, dtype, silu):
+def test_convolution_of_many_rows(lengths, taps, dtype, silu, C):
     ops = _ops()
     g = torch.Generator(device="cuda").manual_seed(taps)
-    n, C = sum(abs(x) for x in lengths), 72
+    n = sum(abs(x) for x in lengths)
     slot, last = _rows(lengths)
     x = torch.randn(n, C + 8, generator=g, device="cuda").to(dtype)[:, :C]
     w = torch.randn(taps, C, generator=g, device="cuda")

@@ -219,7 +219,11 @@ causal_conv_vec_kernel(const T* __restrict__ x, int ldx, const float* __restrict
     }
 }
 
-constexpr int CONV_MIN_ROWS = 640;      // from which a thread takes neighbouring rows (us a row a thread / four: 300 rows 4.1 / 4.9, 512 4.6 / 4.6, 768 5.7 / 4.8)
+// Rows times channels from which a thread takes neighbouring rows: below, a row a thread keeps more loads on their way.  us a row
+// a thread / four, bfloat16: 256 channels 2048 rows 3.0 / 3.7; 768 1400 rows 4.0 / 4.2, 2048 5.0 / 4.2; 1536 600 4.0 / 4.3, 800 4.6 / 4.5;
+// 2304 450 4.2 / 4.5, 600 5.2 / 4.7; 4096 300 4.5 / 4.9, 450 5.6 / 5.1; 5120 150 4.4 / 5.3, 300 5.5 / 5.1, 600 7.9 / 5.3; float32: 256
+// 2048 3.2 / 3.4; 768 1400 4.3 / 3.8; 1536 600 3.5 / 4.0, 800 4.3 / 4.0; 2304 450 4.0 / 3.9; 5120 150 3.3 / 3.9, 300 5.0 / 4.2.
+constexpr size_t CONV_MIN_ELEMENTS = 1150000;
 template <typename T, int TAPS>
 static void launch_causal_conv_vec(const T* x, int ldx, const float* w, float* state, size_t state_stride, T* out, int ldo,
                                    const int* row_slot, const int* row_last, int n, int C, int residual, int act_silu,
@@ -228,7 +232,7 @@ static void launch_causal_conv_vec(const T* x, int ldx, const float* w, float* s
     const int vecs = C / N;
     const int threads = vecs >= 128 ? 128 : (vecs + 31) / 32 * 32;
     constexpr int ROWS = 4;
-    if (n >= CONV_MIN_ROWS)
+    if ((size_t)n * C >= CONV_MIN_ELEMENTS)
         tis_launch(causal_conv_vec_kernel<T, TAPS, ROWS>, dim3((vecs + threads - 1) / threads, (n + ROWS - 1) / ROWS), dim3(threads), 0,
                    stream, x, ldx, w, state, state_stride, out, ldo, row_slot, row_last, n, C, residual, act_silu, bias);
     else
