@@ -59,3 +59,43 @@ def test_errors_stay_errors():
     # the same operands without any of this
     ops.gemm(a, w, out=torch.empty(OUT, device="cuda"))
     assert ops.calls["gemm_split"] == before + 1
+
+
+def _bf16(rows, cols, ld=None, at=1 << 20):
+    t = _like(rows, cols, at=at, dtype=torch.bfloat16)
+    t.stride = lambda i=None: (cols if ld is None else ld, 1) if i is None else (cols if ld is None else ld, 1)[i]
+    return t
+
+
+@pytest.mark.parametrize("a,w,taken", [
+    (_bf16(128, 256), _bf16(256, 512), True),
+    (_bf16(128, 256, ld=512), _bf16(256, 512, ld=1024), True),
+    (_bf16(128, 256, ld=0), _bf16(256, 512), False),                        # one row, seen 128 times
+    (_bf16(128, 256, ld=8), _bf16(256, 512), False),                        # rows that overlap
+    (_bf16(128, 256), _bf16(256, 512, ld=0), False),
+    (_bf16(128, 0, ld=8), _bf16(0, 512), False),                            # empty sums
+    (_bf16(128, 256), _bf16(248, 512), False),
+])
+def test_what_the_bfloat16_kernel_of_many_rows_is_given(a, w, taken):
+    assert ops._tc_ok(a, w, 65) is taken
+
+
+def test_the_library_is_given_operands_that_fit(monkeypatch):
+    def reached():
+        raise AssertionError("the library's product was asked for")
+    monkeypatch.setattr(ops, "LIBRARY_GEMM_DIRECT", True)
+    monkeypatch.setattr(ops, "_blas_state", None)
+    monkeypatch.setattr(ops, "library", reached)
+    assert ops._library_gemm(_bf16(128, 256), _bf16(248, 512), None, False) is None
+    with pytest.raises(AssertionError):
+        ops._library_gemm(_bf16(128, 256), _bf16(256, 512), None, False)
+
+
+@pytest.mark.gpu
+def test_rows_that_are_one_row():
+    """Gate/up of a row that is expanded to many, as before the kernel took steps from 65 rows on."""
+    row, w = torch.randn(1, 256, device="cuda").to(torch.bfloat16), torch.randn(256, 256, device="cuda").to(torch.bfloat16) * 0.1
+    got = ops.gemm_swiglu(row.expand(200, 256), w, 128, 32)
+    torch.testing.assert_close(got, ops.gemm_swiglu(row.expand(200, 256).contiguous(), w, 128, 32), rtol=2e-2, atol=2e-3)
+    with pytest.raises(RuntimeError):
+        ops.gemm(row.expand(200, 256).contiguous(), w[:248])

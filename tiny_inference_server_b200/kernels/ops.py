@@ -423,7 +423,10 @@ def tc_fault() -> torch.Tensor:
 
 
 def _tc_ok(a: torch.Tensor, w: torch.Tensor, min_rows: int) -> bool:
-    return (min_rows > 0 and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+    """What the tcgen05 kernel takes: also no rows that lie on one another (its maps have no stride of zero), no empty sums."""
+    if min_rows <= 0 or a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or a.shape[1] != w.shape[0]:
+        return False
+    return (a.stride(0) >= a.shape[1] > 0 and w.stride(0) >= w.shape[1]
             and a.shape[0] >= min_rows and w.stride(1) == 1 and a.stride(1) == 1
             and a.shape[1] % 8 == 0 and w.shape[1] % 8 == 0 and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
             and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
@@ -521,9 +524,9 @@ def _library_gemm(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor],
         return None
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         return None
-    (n, k), cols = a.shape, w.shape[1]
+    (n, k), (rows, cols) = a.shape, w.shape
     (lda, step_a), (ldw, step_w) = a.stride(), w.stride()
-    if step_a != 1 or step_w != 1 or lda < k or ldw < cols:
+    if step_a != 1 or step_w != 1 or lda < k or ldw < cols or rows != k:
         return None
     lib = library()
     if not _blas_workspace(lib, a.device):
