@@ -437,10 +437,10 @@ norm_mix_store_once_kernel(T* __restrict__ qkv, int ld, int nq, int nk, int nv, 
     const bool is_q = i < nq, is_k = !is_q && i < nq + nk, is_v = i >= nq + nk && i < nq + nk + nv;
     const float* w = is_q ? wq : is_k ? wk : nullptr;       // (of this thread's elements)
     float x[N], y[N], f[N];
+    pdl_wait();                                             // (weights and lambda may be a kernel's output, too)
 #pragma unroll
     for (int e = 0; e < N; ++e) { x[e] = 0.f; f[e] = w != nullptr ? w[(is_q ? i : i - nq) + e] : 1.f; }
     const float lam = is_v && v_other != nullptr && lambda != nullptr ? lambda[0] : 0.f;
-    pdl_wait();
     T* row = qkv + (size_t)r * ld;
     if (is_q || is_k || is_v) Vec16<T>::load(row + i, x);
     if (is_v && v_other != nullptr) Vec16<T>::load(v_other + (size_t)r * ld_other + i - nq - nk, y);
