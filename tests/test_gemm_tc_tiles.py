@@ -31,3 +31,25 @@ def test_tiles(M, K, N, shape):
         torch.testing.assert_close(gated[:, :N // 2].double(), unit, rtol=1e-2, atol=1e-3)
         assert bool((gated[:, N // 2:] == 7.0).all())
     assert int(ops.tc_fault()[0]) == 0
+
+
+def _gated(a, w, block):
+    """silu(gate) * up in 64 bits, gate and up columns in alternating blocks."""
+    gate, up = (a.double() @ w.double()).view(a.shape[0], -1, 2, block).unbind(2)
+    return (torch.nn.functional.silu(gate) * up).reshape(a.shape[0], -1)
+
+
+# the first rows that go there; one full tile of 256 and one row more; nine tenths of two, three and four tiles; full tiles
+@pytest.mark.parametrize("rows,fused", [(64, False), (65, True), (256, True), (257, False), (460, False), (461, True), (512, True), (513, False),
+                                        (691, False), (692, True), (768, True), (921, False), (922, True)])
+def test_which_way_gate_and_up_go(rows, fused):
+    from tiny_inference_server_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    K, H = 256, 128
+    wide = torch.randn(rows, K + 8, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(K, 2 * H, generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+    for a, block, taken in ((wide[:, 8:], 32, fused), (wide[:, 8:], 64, False), (wide[:, 4:K + 4], 32, False)):   # (the last: 8 bytes behind a boundary)
+        before = ops.calls["gemm_tc"]
+        got = ops.gemm_swiglu(a, w, H, block)
+        assert ops.calls["gemm_tc"] == before + taken
+        torch.testing.assert_close(got.double(), _gated(a, w, block), rtol=2e-2, atol=2e-3)

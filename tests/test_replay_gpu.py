@@ -261,7 +261,7 @@ def test_replay_at_the_sizes_of_the_0_9b_model(mode, dtype, tmp_path, tmp_path_f
 
 def test_replay_with_the_tcgen05_products(tmp_path, tmp_path_factory, monkeypatch):
     """The same replay with every product of 128 rows or more on the tcgen05 kernel (by default
-    only very long portions go there): whole prompts of 150 and 200 tokens in one step."""
+    only gate/up products go there): whole prompts of 150 and 200 tokens in one step."""
     from tiny_inference_server_b200.kernels import ops
     monkeypatch.setattr(ops, "TC_MIN_ROWS", 128)
     monkeypatch.setattr(ops, "TC_PLAIN_MIN_ROWS", 128)

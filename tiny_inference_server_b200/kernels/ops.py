@@ -401,12 +401,15 @@ def gemm_skinny(a, w: torch.Tensor, out: Optional[torch.Tensor] = None, swiglu: 
 
 
 #: The tcgen05 kernel of this library (csrc/gemm_tc.cu) against the library product, measured on a B200 (replayed from CUDA
-#: graphs, weights rotated through more than L2).  Gate/up with the gating in its epilogue, us library product and gating kernel /
-#: own, at 65, 128, 200, 300, 400, 512, 640, 1024, 2048 rows: K 1536, hidden 4096 11.2 / 9.4, 10.6 / 8.8, 12.1 / 10.3, 13.4 / 14.3,
-#: 14.9 / 14.4, 16.3 / 14.5, 21.8 / 20.3, 27.5 / 22.2, 48.5 / 37.8; K 3072, hidden 8192 21.2 / 19.4, 24.1 / 19.9, 25.7 / 24.3,
-#: 30.5 / 38.1, 36.5 / 39.1, 42.7 / 40.3, 60.7 / 55.7, 84 / 75, 180 / 129; K 4096, hidden 14336 40.9 / 38.9, 49.5 / 39.2, 55 / 53,
-#: 65 / 91, 85 / 94, 102 / 95, 150 / 122, 206 / 167, 345 / 308; K 1536, hidden 1024 7.3 / 7.4 .. 16.1 / 13.9.  It loses where the
-#: last tile of 256 rows is mostly empty: up to 256 rows (one tile) and from four fifths of the tiles' rows on it takes them.
+#: graphs, weights rotated through more than L2; microbench gemm).  Gate/up with the gating in its epilogue, us library product and
+#: gating kernel / own, at 65, 128, 200, 256, 300, 440, 480, 640, 768, 870, 950, 1024, 2048 rows: K 1536, hidden 4096 9.7 / 9.1,
+#: 9.9 / 9.3, 11.6 / 11.3, 11.4 / 11.3, 13.0 / 15.7, 15.0 / 16.1, 16.0 / 16.0, 22 / 21.6, 22.7 / 21.9, 24.9 / 23.6, 26.6 / 23.7, 27.7 / 23.7,
+#: 49.7 / 40.2; K 3072, hidden 8192 20.3 / 20.2, 23.4 / 20.5, 25.0 / 25.7, 27.0 / 25.9, 30 / 40, 38 / 42, 42.6 / 42.2, 60.5 / 58.5,
+#: 63.9 / 60.3, 72 / 76, 77.1 / 77.0, 81 / 78, 160 / 138; K 4096, hidden 14336 39.9 / 39.7, 49 / 40, 55.5 / 55.2, 58 / 56, 66 / 94,
+#: 89 / 98, 106 / 100, 155 / 128, 163 / 132, 167 / 180, 179 / 178, 210 / 177, 385 / 316; K 1536, hidden 1024 9.2 / 10.4, 9.3 / 10.5, 9.9 / 10.7,
+#: 8.2 / 8.8, 8.2 / 8.7, 8.5 / 9.1, 9.0 / 9.0, 9.4 / 10.1, 10.0 / 10.1, 10.3 / 10.4, 11.2 / 10.5, 10.8 / 10.5, 16.6 / 15.8 (and one call of the
+#: host's less, some 6 us).  It loses where the last tile of 256 rows is partly empty: up to 256 rows (one tile) and from nine
+#: tenths of the tiles' rows on it takes them.
 #: Plain products it loses (2048 x 1536 x 2304: 12.1 / 16.2, 2048 x 3072 x 12352 102 / 109): by default it takes none.
 #: TIS_TC_MIN_ROWS / TIS_TC_PLAIN_MIN_ROWS in the environment override the two limits (0 = never).
 TC_MIN_ROWS = int(os.environ.get("TIS_TC_MIN_ROWS", "65"))
@@ -433,8 +436,8 @@ def _tc_ok(a: torch.Tensor, w: torch.Tensor, min_rows: int) -> bool:
 
 
 def _tc_tiles_full(n: int) -> bool:
-    """Whether ``n`` rows fill four fifths of the tiles of 256 rows they take, or one tile has them all."""
-    return n <= 256 or 5 * n >= 4 * 256 * -(-n // 256)
+    """Whether ``n`` rows fill nine tenths of the tiles of 256 rows they take, or one tile has them all."""
+    return n <= 256 or 10 * n >= 9 * 256 * -(-n // 256)
 
 
 def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, swiglu: bool = False,
