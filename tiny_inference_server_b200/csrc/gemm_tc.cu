@@ -24,9 +24,9 @@
 // word, lets every role leave its loop, and the tensor memory is freed before the CTA ends;
 // the two CTAs of a cluster end together.
 // A stage of 128 along K takes its products 1024 cycles (BN = 256) and some 300 to hand over; with wide tiles the operands from L2
-// bound it.  Measured on a B200, us, the library's product and the gating kernel / this: 2048 x 1536 x 8192 48.5 / 37.8 (one CTA a tile,
-// a look at a barrier 200 cycles and rounded divisions in the gating before: 52), 2048 x 3072 x 16384 159 / 129, 1024 x 1536 x
-// 8192 27.5 / 22.2, 128 x 1536 x 8192 10.6 / 8.8.  Plain products it loses (2048 x 1536 x 2304 12.1 / 16.2, 2048 x 4096 x 1536
+// bound it.  Measured on a B200, us, the library's product and the gating kernel / this: 2048 x 1536 x 8192 49.7 / 40.2 (one CTA a tile,
+// a look at a barrier 200 cycles and the division operator in the gating before: 52), 2048 x 3072 x 16384 160 / 138, 1024 x 1536 x
+// 8192 27.7 / 23.7, 128 x 1536 x 8192 9.9 / 9.3.  Plain products it loses (2048 x 1536 x 2304 12.1 / 16.2, 2048 x 4096 x 1536
 // 20.1 / 24.8, 2048 x 3072 x 12352 102 / 109): the library splits their sums, and its clusters fetch a tile once for several CTAs.
 #include "tc_common.cuh"
 

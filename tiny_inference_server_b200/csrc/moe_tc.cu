@@ -11,8 +11,9 @@
 // Roles, hand-offs, bounded waits and the double-buffered accumulator are those of gemm_tc.cu; tiles whose table entry
 // is negative (beyond the last expert's rows) are skipped by every role alike.
 // Bound by the operands from L2 (48 KB a step of 64 along K and CTA).  Measured on a B200, both products of 2048 rows, 3 of 16 experts of
-// 1024, width 1536, with sort, gather and sum: 160 -> 108 us since copies and products are ordered behind elect.sync and a barrier
-// that is complete costs one look.
+// 1024, width 1536, with sort, gather and sum, replayed from a graph: 159 us, and 107 since copies and products are ordered behind
+// elect.sync, a complete barrier costs one look and gates are divided by quotient() (the whole layer 198 and 144; called from Python,
+// whose calls it waits for, 175 and 150).
 #include "tc_common.cuh"
 
 namespace {
@@ -181,8 +182,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
 }
 
 // xs[place] = x[pair / top] for every place of the sorted order that a (token, choice) pair takes; a warp a place, 16-byte vectors,
-// four of a lane on their way at a time (both products of 2048 rows with sort, gather and sum, 6144 places of 1536 taken: 108 us with a
-// CTA a place and a vector a thread, 105 so).
+// four of a lane on their way at a time (both products of 2048 rows with sort, gather and sum, 6144 places of 1536 taken: 3 us
+// less than with a CTA a place and a vector a thread).
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const bf16* __restrict__ x, int ldx, const int* __restrict__ sorted_pair, int top, bf16* __restrict__ xs,
                   int d, int places) {

@@ -13,8 +13,8 @@
 // Against the mma.sync kernel, which reads every operand fragment from shared memory per warp of 16 rows: 2048 rows, 12 query
 // heads of 128 on 3 kv heads, window 1024, with bias 103 -> 33 us; 1024 rows behind 1024 cached, 12 heads on one
 // compressed row of 192 (values 128) 201 -> 39 us (replayed from a graph); outputs against 64 bits 0.97 to 1.0 times as far off.
-// With a gate the division a/(1 + e^-g) was 13000 of a tile's last cycles, an element after the other; now 4000 (same rows with
-// bias and gate 44 -> 35 us).
+// With a gate the division a/(1 + e^-g) was 13000 of a tile's last cycles, an element after the other: same rows with bias and gate
+// 44 us, with rows stored from shared memory and quotient() 37.
 #include "tc_common.cuh"
 
 #ifndef TIS_KD
